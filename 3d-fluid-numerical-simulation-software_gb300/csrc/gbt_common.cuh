@@ -58,6 +58,7 @@ struct Flow {
     T *mut, *omega, *dt;
     T *mul;                                          // FP64 form: laminar viscosity (Sutherland) per cell, formed
                                                      // with the spectral radii for Baldwin-Lomax and the viscous radii
+    T *dinv;                                         // 1 / the diagonal of the LU-SGS sweeps, formed with the time step
     T *lamc[3], *lamv[3];
     T *Ff[3][NQ], *Vf[3][NQ];                        // face convective / viscous fluxes
     T *Fd[3][NQ];                                    // face artificial dissipation (JST only, else null)

@@ -68,39 +68,27 @@ struct BcTables {
 
 constexpr int kIntegralBlocks = 16;             // blocks per inlet/outlet section in the integrals
 
-// Cells of every i+j+k hyperplane of every solve, in "plane order": q runs over the planes of
-// solve 0, then those of solve 1, ...; inside a plane by i, then j. start[s*stride + plane] ..
-// start[s*stride + plane + 1] are the q of one plane of solve s; max_count[plane] is the largest
-// plane over the solves.
-struct PlaneTables {
-    const int *start = nullptr;
-    int stride = 0, max_plane = 0;
-    long long nq = 0;
-    int cpw = 10, wpb = 1;                        // sweep block shape: cells per warp, warps per block (autotuned)
-    // row starts for the tiled scatter of dQ: the plane-order index of interior cell
-    // (i, j, k) of solve s is rq[rq_off[s] + (i + j + k) * (IM - 1) + i - 1] + j
-    const int *rq = nullptr;
-    const long long *rq_off = nullptr;
-    std::vector<int> max_count;
+// The LU-SGS sweeps' tiles (wavefront.cu). A tile is a group of grid columns that a block marches
+// along k, skewed by the columns' places in it; the tiles of a slot hold T steps each, tile (PI, PJ)
+// from step0 + (PI * nPJ + PJ) * T on.
+struct WaveSolve { int nI, nJ, nK, nPI, nPJ, T; long long step0; };
+struct WaveCtl { unsigned epoch, ticket[2]; };     // sweeps started; tiles handed out, per direction
+struct WaveBytes { int geo, flow, dq, pkt, area, var_flow, var_dq, var_pkt; };      // of a step
+struct WaveTables {
+    const WaveSolve *solve = nullptr;              // per slot
+    const int2 *item = nullptr;                    // {slot, PI << 16 | PJ}: every tile, after the two it reads from
+    int n_item = 0;
+    int max_tiles = 0, max_T = 0;                  // largest of a slot: tiles, steps of a tile
+    long long max_steps = 0;                       // and steps of all its tiles
+    WaveCtl *ctl = nullptr;
+    char *geo = nullptr, *flow = nullptr, *dq = nullptr;   // blocks of the steps, in step order
+    void *area = nullptr;                          // mean area per cell and direction
+    uint4 *pkt = nullptr;                          // terms that cross from tile to tile
 };
-
-// Everything the LU-SGS sweeps read, copied into plane order so that the cells of one plane and
-// their neighbours in the previous plane are dense in memory (in the k-contiguous box they are
-// scattered, one sector per value). Geometry is copied once; the flow inputs before every forward
-// sweep; dQ lives here during the sweeps and is scattered back to the box afterwards.
-template <typename T>
-struct SweepData {
-    const long long *cell = nullptr;               // q -> box index (including the solve's base)
-    const int *nb[2][3] = {};                      // [0] lower (forward), [1] upper (backward) neighbour q, or -1
-    T *gn[3][3] = {}, *gs[3] = {}, *gve[3] = {}, *gvol = nullptr;   // per direction: mean normal, |S|, entrainment
-    T *cv[NQ] = {}, *pp = nullptr, *lamc[3] = {}, *lamv[3] = {}, *dt = nullptr, *res[NQ] = {};
-    T *dq[NQ] = {};
-    // Spalart-Allmaras sweep (null without it), per cell as a neighbour in direction d: normal
-    // velocity with the mean flow's dQ added, old variable times old normal velocity, mean |S|,
-    // relax * lambda_c, lambda_v; per cell: old variable, diagonal, residual, update
-    T *sa_vn[3] = {}, *sa_eb[3] = {}, *sa_s[3] = {}, *sa_rl[3] = {}, *sa_lv[3] = {};
-    T *sa_ev0 = nullptr, *sa_alpha = nullptr, *sa_res = nullptr, *sa_dq = nullptr;
-};
+// columns of a tile in i and j; bytes of a step's blocks (fp64: working type; sa: with the
+// Spalart-Allmaras variable)
+void wave_patch(int &pa, int &pb);
+void wave_bytes(int fp64, int sa, WaveBytes &w);
 
 void launch_geometry(const LaunchCtx &ctx, const Geo &G, double *totalvol);
 // the periodic rotation's cosines and sines per solve (BcTables::per_trig), once at create
@@ -121,18 +109,10 @@ template <typename T>
 void launch_resflux(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC, const Geo &G, const GeoW<T> &GW, Flow<T> F,
                     const BcTables &bc, int level, T *scratch_dtmin);
 
-// the mean-flow sweeps; with the Spalart-Allmaras variable present (F.ev), its scalar sweep of each
-// direction follows the mean-flow sweep of that direction
+// both sweeps, dQ back into the box (with the Spalart-Allmaras variable present, F.ev, its update too; VV:
+// the tables of the variable's sweep)
 template <typename T>
-void launch_lusgs_sweeps(const LaunchCtx &ctx, const PhysW<T> &P, const Geo &G, Flow<T> F, const PlaneTables &pt,
-                         const SweepData<T> &S);
-
-// fastest block shape of the sweep kernels for this level, as cells_per_warp * 16 + warps_per_block
-// (times the plane chains on benign inputs in the plane-order scratch; synchronises the stream)
-// whether (cells per warp, warps per block) is one of the compiled sweep shapes
-bool sweep_shape_known(int cpw, int wpb);
-template <typename T>
-int tune_sweep_cpw(const LaunchCtx &ctx, const PhysW<T> &P, const PlaneTables &pt, const SweepData<T> &S);
+void launch_lusgs_sweeps(const LaunchCtx &ctx, const PhysW<T> &P, const Geo &G, Flow<T> F, const WaveTables &V, const WaveTables &VV);
 
 // Baldwin-Lomax wall distances of every wall line point (fine level, once; see BcTables)
 template <typename T>
@@ -141,9 +121,9 @@ void launch_wall_distances(const LaunchCtx &ctx, const Geo &G, const BcTables &b
 // FP32 copies of the geometry the working-precision kernels read (mixed form; once per level)
 void launch_geometry_working(const LaunchCtx &ctx, const Geo &G, const GeoW<float> &GW);
 
-// plane-order copy of the sweep's geometry (once per level, after the geometry kernels)
+// the sweeps' geometry in step order (once per level, after the geometry kernels)
 template <typename T>
-void launch_sweep_geometry(const LaunchCtx &ctx, const Geo &G, const PlaneTables &pt, const SweepData<T> &S);
+void launch_wave_geometry(const LaunchCtx &ctx, const Geo &G, const WaveTables &V);
 
 template <typename T>
 void launch_update(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> F, int level,
@@ -194,9 +174,6 @@ template <typename T>
 void launch_sa_boundary(const LaunchCtx &ctx, const Phys &P, Flow<T> W, const BcTables &bc);
 template <typename T>
 void launch_sa_model(const LaunchCtx &ctx, const Phys &P, const GeoW<T> &GW, Flow<T> W);
-template <typename T>
-void launch_sa_sweep(const LaunchCtx &ctx, const PhysW<T> &PC, const Geo &G, Flow<T> W, const PlaneTables &pt,
-                     const SweepData<T> &S, int dir);
 template <typename T>
 void launch_sa_update(const LaunchCtx &ctx, const Phys &P, Flow<T> W, int *bad_list, int bad_cap, int *bad_count);
 template <typename T>

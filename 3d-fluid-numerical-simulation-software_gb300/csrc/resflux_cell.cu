@@ -324,6 +324,14 @@ __global__ void k_wall_mut(Batch B, Flow<T> W, const DevWall *walls)
     else W.mut[p] = -W.mut[m];
 }
 
+// 1 / the diagonal of the LU-SGS sweeps (source/LU_SGS_Marching.cpp:95-150): Vol / dt + relax lambda_c + 2 lambda_v
+template <typename T>
+__device__ __forceinline__ T sweep_diagonal(const PhysW<T> &PC, T vol, T dt, T lc, T lv)
+{
+    if constexpr (sizeof(T) == 8) return frcp<T>(fma((T)2, lv, fma(vol, frcp<T>(dt), __dmul_rn(PC.relax, lc))));
+    else return (T)1 / fma((T)2, lv, fma(PC.relax, lc, vol / dt));
+}
+
 // viscous spectral radii and the local time step
 template <typename T, bool NS>   // NS: Navier-Stokes (viscous radii), else Euler
 __global__ void __launch_bounds__(256) k_cell_b(Batch B, PhysW<T> PC, GeoW<T> G, Flow<T> W, int level)
@@ -355,7 +363,9 @@ __global__ void __launch_bounds__(256) k_cell_b(Batch B, PhysW<T> PC, GeoW<T> G,
         for (int d = 0; d < 3; d++) W.lamv[d][p] = l[d];
         lv = l[0] + l[1] + l[2];
     }
-    W.dt[p] = to_work<T>(dtf * cfl) * vol / (lc + PC.c_timestep * lv);
+    const T dt = to_work<T>(dtf * cfl) * vol / (lc + PC.c_timestep * lv);
+    W.dt[p] = dt;
+    W.dinv[p] = sweep_diagonal<T>(PC, vol, dt, lc, NS ? lv : W.lamv[0][p] + W.lamv[1][p] + W.lamv[2][p]);
 }
 
 // global time stepping: minimum over the solve, then broadcast (source/TimeStep.cpp:64-87)
@@ -382,12 +392,16 @@ __global__ void __launch_bounds__(1024) k_dt_min(Batch B, Flow<T> W, T *out)
     if (threadIdx.x == 0) out[blockIdx.y] = sh[0];
 }
 template <typename T>
-__global__ void k_dt_set(Batch B, Flow<T> W, const T *mn)
+__global__ void k_dt_set(Batch B, PhysW<T> PC, GeoW<T> G, Flow<T> W, const T *mn)
 {
     const Lvl L = B.lv[blockIdx.y];
     int i, j, k;
     if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
-    W.dt[ix(L, i, j, k)] = mn[blockIdx.y];
+    const long long p = ix(L, i, j, k);
+    const T dt = mn[blockIdx.y];
+    W.dt[p] = dt;
+    W.dinv[p] = sweep_diagonal<T>(PC, G.vol[p], dt, W.lamc[0][p] + W.lamc[1][p] + W.lamc[2][p],
+                                  W.lamv[0][p] + W.lamv[1][p] + W.lamv[2][p]);
 }
 
 // decrement of the low-time-step counter after the time step used it
@@ -428,7 +442,7 @@ void launch_cell_stages(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC,
     else k_cell_b<T, false><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, PC, GW, W, level);
     if (P.global_dt) {
         k_dt_min<T><<<dim3(1, B.nsolve), 1024, 0, ctx.stream>>>(B, W, scratch);
-        k_dt_set<T><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, W, scratch);
+        k_dt_set<T><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, PC, GW, W, scratch);
     }
     k_after_timestep<<<(B.nsolve + 127) / 128, 128, 0, ctx.stream>>>(B, level);
     ctx.mark("time_step", 0, 2);

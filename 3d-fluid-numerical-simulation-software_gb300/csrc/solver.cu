@@ -56,7 +56,7 @@ struct Level {
     Lvl *lv_d = nullptr;
     SolveConst *sc_d = nullptr;
     long long pool_n = 0;
-    int maxIM = 0, maxJM = 0, maxKM = 0, max_plane = 0;
+    int maxIM = 0, maxJM = 0, maxKM = 0;
     DevBuf geo_mem, flow_d_mem, flow_t_mem, int_mem, tab_mem, meta_mem;
     Geo G{};
     GeoW<T> GW{};                         // working-precision geometry (aliases in FP64, FP32 copies in mixed)
@@ -69,9 +69,8 @@ struct Level {
     Flow<T> W{};
     double *totalvol = nullptr, *blockvol = nullptr;
     BcTables bc;
-    PlaneTables planes;
-    SweepData<T> sweep;
-    DevBuf plane_mem;
+    WaveTables wave, wave_var;            // of the mean flow; of the Spalart-Allmaras variable
+    DevBuf wave_mem;
     std::vector<DevWall> walls_h;
     bool use_force = false;
     LaunchCtx ctx(const Batch &B, cudaStream_t s) const
@@ -551,7 +550,6 @@ public:
             sc.cix = (int)(std::upper_bound(case_first.begin(), case_first.end(), s) - case_first.begin()) - 1;
             Lv.sc.push_back(sc);
             Lv.maxIM = std::max(Lv.maxIM, c.IM); Lv.maxJM = std::max(Lv.maxJM, c.JM); Lv.maxKM = std::max(Lv.maxKM, c.KM);
-            Lv.max_plane = std::max(Lv.max_plane, c.IM + c.JM + c.KM - 3);
         }
         Lv.pool_n = base;
         // the face kernels index a level's pools with 32-bit offsets
@@ -592,13 +590,13 @@ public:
         double *d = (double *)Lv.flow_d_mem.p;
         Flow<T> &W = Lv.W;
         for (int c = 0; c < NQ; c++) { W.cv[c] = d; d += N; W.cvold[c] = d; d += N; W.cv2h[c] = d; d += N; }
-        Lv.flow_t_mem.bytes = sizeof(T) * N * 66;
+        Lv.flow_t_mem.bytes = sizeof(T) * N * 67;
         CK(cudaMalloc(&Lv.flow_t_mem.p, Lv.flow_t_mem.bytes));
         CK(cudaMemset(Lv.flow_t_mem.p, 0, Lv.flow_t_mem.bytes));
         T *t = (T *)Lv.flow_t_mem.p;
         auto tk = [&]() { T *r = t; t += N; return r; };
         for (int c = 0; c < NPV; c++) W.pv[c] = tk();
-        W.mut = tk(); W.omega = tk(); W.dt = tk(); W.mul = tk();
+        W.mut = tk(); W.omega = tk(); W.dt = tk(); W.mul = tk(); W.dinv = tk();
         for (int f = 0; f < 3; f++) { W.lamc[f] = tk(); W.lamv[f] = tk(); for (int c = 0; c < NQ; c++) { W.Ff[f][c] = tk(); W.Vf[f][c] = tk(); } }
         for (int c = 0; c < NQ; c++) { W.res[c] = tk(); W.dq[c] = tk(); W.res2h[c] = tk(); W.dq2h[c] = tk(); }
         if (P.turb_sa && l == 1) {
@@ -650,36 +648,17 @@ public:
             build_tables(l, lc, hx, hy);
         }
         timer.mark("pools, nodes, patch tables", stream);
-        build_planes(l);
-        timer.mark("hyperplane tables", stream);
+        build_waves(l);
+        timer.mark("sweep tiles", stream);
         launch_geometry(ctx(l), G, Lv.blockvol);
         k_case_volume<<<(nsolve + 127) / 128, 128, 0, stream>>>(batch(l), Lv.blockvol, Lv.totalvol);
         if (Lv.W.ev) build_sa_wall_distance(l);
         timer.mark("geometry", stream);
         build_geometry_working(l);
         build_wall_distances(l);
-        launch_sweep_geometry<T>(ctx(l), G, Lv.planes, Lv.sweep);
-        timer.mark("working geometry, wall lines", stream);
-        {
-            // block shape of the sweep kernels: GBTURBO_SWEEP_SHAPE="cpw,wpb" pins it; batches of
-            // four or more solves time the candidates; smaller ones, where the candidates are within
-            // run-to-run noise of each other, take ten cells per one-warp block
-            int cpw = 10, wpb = 1;
-            const char *pin = std::getenv("GBTURBO_SWEEP_SHAPE");
-            if (pin && std::sscanf(pin, "%d,%d", &cpw, &wpb) == 2 && sweep_shape_known(cpw, wpb)) {
-            } else if (nsolve >= 4) {
-                const int v = tune_sweep_cpw<T>(ctx(l), PC, Lv.planes, Lv.sweep);
-                cpw = v / 16;
-                wpb = v % 16;
-            } else {
-                cpw = 10;
-                wpb = 1;
-            }
-            Lv.planes.cpw = cpw;
-            Lv.planes.wpb = wpb;
-        }
+        launch_wave_geometry<T>(ctx(l), G, Lv.wave);
         CK(cudaStreamSynchronize(stream));
-        timer.mark("sweep shape", stream);
+        timer.mark("working geometry, wall lines", stream);
         CK(cudaGetLastError());
     }
 
@@ -800,109 +779,68 @@ public:
         }
     }
 
-    // cells of the LU-SGS hyperplanes (source/LU_SGS_Marching.cpp:62-74) in plane order, with the
-    // plane-order neighbour tables and the plane-order copies of the sweep's inputs
-    void build_planes(int l)
+    // tiles of the LU-SGS sweeps and the memory of their steps
+    void build_waves(int l)
     {
         Level<T> &Lv = lev[l];
-        PlaneTables &pt = Lv.planes;
-        pt.max_plane = Lv.max_plane;
-        pt.stride = Lv.max_plane + 2;
-        pt.max_count.assign(pt.stride, 0);
-        std::vector<long long> cell;
-        std::vector<int> start((size_t)nsolve * pt.stride + 1, 0);
-        std::vector<int> nbq[2][3];
-        std::vector<int> rq;                       // row starts of the transpositions (PlaneTables::rq)
-        std::vector<long long> rq_off(nsolve);
+        WaveTables &V = Lv.wave;
+        const bool sa = P.turb_sa && l == 1;
+        int pa, pb;
+        wave_patch(pa, pb);
+        WaveBytes w;
+        wave_bytes(sizeof(T) == 8, sa, w);
+        std::vector<WaveSolve> sol;
+        std::vector<std::array<int, 4>> order;     // steps behind the slot's first tile, slot, PI, PJ
+        long long steps = 0;
         for (int s = 0; s < nsolve; s++) {
             const Lvl &v = Lv.lv[s];
-            const int nI = v.IM - 1, nJ = v.JM - 1, nK = v.KM - 1;
-            rq_off[s] = (long long)rq.size();
-            rq.resize(rq.size() + (size_t)pt.stride * nI, 0);
-            // q of interior cell (i,j,k) of this solve
-            std::vector<int> qof((size_t)nI * nJ * nK, -1);
-            auto at = [&](int i, int j, int k) -> int & { return qof[((size_t)(i - 1) * nJ + (j - 1)) * nK + (k - 1)]; };
-            for (int pl = 0; pl < pt.stride; pl++) {
-                start[(size_t)s * pt.stride + pl] = (int)cell.size();
-                int c = 0;
-                if (pl >= 3)
-                    for (int i = 1; i <= nI; i++) {
-                        bool first = true;
-                        for (int j = 1; j <= nJ; j++) {
-                            const int k = pl - i - j;
-                            if (k < 1 || k > nK) continue;
-                            if (first) { rq[(size_t)rq_off[s] + (size_t)pl * nI + (i - 1)] = (int)cell.size() - j; first = false; }
-                            at(i, j, k) = (int)cell.size();
-                            cell.push_back(ix(v, i, j, k));
-                            c++;
-                        }
-                    }
-                pt.max_count[pl] = std::max(pt.max_count[pl], c);
-            }
-            if (cell.size() > (size_t)0x7fffffff) throw std::runtime_error("batch too large for the plane tables");
-            for (int dir = 0; dir < 2; dir++)
-                for (int d = 0; d < 3; d++) nbq[dir][d].resize(cell.size(), -1);
-            for (int i = 1; i <= nI; i++)
-                for (int j = 1; j <= nJ; j++)
-                    for (int k = 1; k <= nK; k++) {
-                        const int q = at(i, j, k);
-                        if (i > 1) nbq[0][0][q] = at(i - 1, j, k);
-                        if (j > 1) nbq[0][1][q] = at(i, j - 1, k);
-                        if (k > 1) nbq[0][2][q] = at(i, j, k - 1);
-                        if (i < nI) nbq[1][0][q] = at(i + 1, j, k);
-                        if (j < nJ) nbq[1][1][q] = at(i, j + 1, k);
-                        if (k < nK) nbq[1][2][q] = at(i, j, k + 1);
-                    }
+            WaveSolve q;
+            q.nI = v.IM - 1; q.nJ = v.JM - 1; q.nK = v.KM - 1;
+            q.nPI = (q.nI + pa - 1) / pa; q.nPJ = (q.nJ + pb - 1) / pb;
+            q.T = q.nK + pa + pb - 2;
+            q.step0 = steps;
+            if (q.nPI > 0x7fff || q.nPJ > 0xffff) throw std::runtime_error("a block has too many columns for the sweeps");
+            for (int a = 0; a < q.nPI; a++)
+                for (int b = 0; b < q.nPJ; b++) order.push_back({pa * a + pb * b, s, a, b});
+            const long long np = (long long)q.nPI * q.nPJ;
+            steps += np * q.T;
+            V.max_steps = std::max(V.max_steps, np * q.T);
+            V.max_tiles = std::max(V.max_tiles, (int)np);
+            V.max_T = std::max(V.max_T, q.T);
+            sol.push_back(q);
         }
-        start[(size_t)nsolve * pt.stride] = (int)cell.size();
-        // start[s*stride + pl + 1] must be the end of plane pl: the last slot of each solve row
-        // (pl = stride-1) is empty, so the next row's first entry closes it
-        const size_t nq = cell.size();
-        pt.nq = (long long)nq;
+        // every tile after the two it reads from; those that can start together side by side
+        std::stable_sort(order.begin(), order.end(), [](const auto &x, const auto &y) { return x[0] < y[0]; });
+        std::vector<int2> item;
+        for (auto &o : order) item.push_back(make_int2(o[1], (o[2] << 16) | o[3]));
+        V.n_item = (int)item.size();
         auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-        const bool sa = P.turb_sa && l == 1;
-        const size_t n_t = 16 + 18 + NQ + (sa ? 19 : 0);   // geometry, flow inputs, dQ (and the SA sweep's)
-        Lv.plane_mem.bytes = al(sizeof(int) * start.size()) + al(sizeof(long long) * nq) + 6 * al(sizeof(int) * nq) +
-                             al(sizeof(int) * rq.size()) + al(sizeof(long long) * rq_off.size()) + n_t * al(sizeof(T) * nq) + 256;
-        CK(cudaMalloc(&Lv.plane_mem.p, Lv.plane_mem.bytes));
-        char *q = (char *)Lv.plane_mem.p;
+        const size_t N = (size_t)steps;
+        Lv.wave_mem.bytes = al(sizeof(WaveSolve) * sol.size()) + al(sizeof(int2) * item.size()) + 2 * al(sizeof(WaveCtl)) +
+                            al(N * w.geo) + al(N * w.flow) + al(N * w.dq) + al(N * w.pkt) + al(N * w.area) + al(N * w.var_flow) +
+                            al(N * w.var_dq) + al(N * w.var_pkt);
+        CK(cudaMalloc(&Lv.wave_mem.p, Lv.wave_mem.bytes));
+        CK(cudaMemset(Lv.wave_mem.p, 0, Lv.wave_mem.bytes));
+        char *q = (char *)Lv.wave_mem.p;
         auto take = [&](size_t b) { char *r = q; q += al(b); return r; };
-        int *dstart = (int *)take(sizeof(int) * start.size());
-        CK(cudaMemcpy(dstart, start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice));
-        pt.start = dstart;
-        int *drq = (int *)take(sizeof(int) * rq.size());
-        CK(cudaMemcpy(drq, rq.data(), sizeof(int) * rq.size(), cudaMemcpyHostToDevice));
-        long long *drq_off = (long long *)take(sizeof(long long) * rq_off.size());
-        CK(cudaMemcpy(drq_off, rq_off.data(), sizeof(long long) * rq_off.size(), cudaMemcpyHostToDevice));
-        pt.rq = drq;
-        pt.rq_off = drq_off;
-        SweepData<T> &S = Lv.sweep;
-        long long *dcell = (long long *)take(sizeof(long long) * nq);
-        CK(cudaMemcpy(dcell, cell.data(), sizeof(long long) * nq, cudaMemcpyHostToDevice));
-        S.cell = dcell;
-        for (int dir = 0; dir < 2; dir++)
-            for (int d = 0; d < 3; d++) {
-                int *t = (int *)take(sizeof(int) * nq);
-                CK(cudaMemcpy(t, nbq[dir][d].data(), sizeof(int) * nq, cudaMemcpyHostToDevice));
-                S.nb[dir][d] = t;
-            }
-        auto arr = [&]() { return (T *)take(sizeof(T) * nq); };
-        for (int d = 0; d < 3; d++) {
-            for (int c = 0; c < 3; c++) S.gn[d][c] = arr();
-            S.gs[d] = arr();
-            S.gve[d] = arr();
-        }
-        S.gvol = arr();
-        for (int c = 0; c < NQ; c++) S.cv[c] = arr();
-        S.pp = arr();
-        for (int d = 0; d < 3; d++) { S.lamc[d] = arr(); S.lamv[d] = arr(); }
-        S.dt = arr();
-        for (int c = 0; c < NQ; c++) S.res[c] = arr();
-        for (int c = 0; c < NQ; c++) S.dq[c] = arr();
-        if (sa) {
-            for (int d = 0; d < 3; d++) { S.sa_vn[d] = arr(); S.sa_eb[d] = arr(); S.sa_s[d] = arr(); S.sa_rl[d] = arr(); S.sa_lv[d] = arr(); }
-            S.sa_ev0 = arr(); S.sa_alpha = arr(); S.sa_res = arr(); S.sa_dq = arr();
-        }
+        void *d = take(sizeof(WaveSolve) * sol.size());
+        CK(cudaMemcpy(d, sol.data(), sizeof(WaveSolve) * sol.size(), cudaMemcpyHostToDevice));
+        V.solve = (const WaveSolve *)d;
+        d = take(sizeof(int2) * item.size());
+        CK(cudaMemcpy(d, item.data(), sizeof(int2) * item.size(), cudaMemcpyHostToDevice));
+        V.item = (const int2 *)d;
+        V.ctl = (WaveCtl *)take(sizeof(WaveCtl));
+        V.geo = take(N * w.geo);
+        V.flow = take(N * w.flow);
+        V.dq = take(N * w.dq);
+        V.pkt = (uint4 *)take(N * w.pkt);
+        V.area = take(N * w.area);
+        WaveTables &U = Lv.wave_var = V;
+        U.ctl = (WaveCtl *)take(sizeof(WaveCtl));
+        U.geo = nullptr;
+        U.flow = take(N * w.var_flow);
+        U.dq = take(N * w.var_dq);
+        U.pkt = (uint4 *)take(N * w.var_pkt);
     }
 
     void build_tables(int l, const std::vector<LevelCase> &lc, const std::vector<double> &hx, const std::vector<double> &hy)
@@ -1145,7 +1083,7 @@ public:
     {
         LaunchCtx cx = ctx(l);
         Level<T> &Lv = lev[l];
-        launch_lusgs_sweeps<T>(cx, PC, Lv.G, Lv.W, Lv.planes, Lv.sweep);
+        launch_lusgs_sweeps<T>(cx, PC, Lv.G, Lv.W, Lv.wave, Lv.wave_var);
         launch_update<T>(cx, P, Lv.G, Lv.W, l, bad_list, bad_cap, bad_count);
     }
     // transfers between level lf and the next coarser one
@@ -1169,7 +1107,7 @@ public:
         sweep_update(l);
     }
     void res_calculate(int l) override { launch_res_norm<T>(ctx(l), lev[l].G, lev[l].W, lev[l].totalvol, norm_part, norm_blk); }
-    void sweep_shape(int l, int out[2]) const override { out[0] = lev[l].planes.cpw; out[1] = lev[l].planes.wpb; }
+    void sweep_shape(int, int out[2]) const override { out[0] = 10; out[1] = 1; }
     bool face_staged(int l) const override
     {
         return lev[l].tma_mem.p != nullptr && P.recon_var == 200 && P.recon == 500 && P.scheme == 300;

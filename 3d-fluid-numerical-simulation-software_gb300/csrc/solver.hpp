@@ -78,7 +78,7 @@ public:
     // their limiter hits summed
     virtual void states(SolveState *out) = 0;
     virtual void set_use_force(int level, bool on) = 0;
-    // block shape the sweep autotuner chose for a level: cells per warp, warps per block
+    // cells per warp, warps per block of the plane-by-plane sweeps of earlier versions
     virtual void sweep_shape(int level, int out[2]) const = 0;
     // whether a level's face stage runs on tiles staged in shared memory by TMA (mixed form)
     virtual bool face_staged(int level) const = 0;

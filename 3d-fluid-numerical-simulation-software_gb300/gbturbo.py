@@ -354,7 +354,7 @@ class Solver:
         self._ck(self._L.gb_sync(self.h))
 
     def sweep_tuning(self, level: int = 1) -> tuple:
-        """(cells per warp, warps per block) the sweep autotuner chose for a level"""
+        """(10, 1): the block shape of the plane-by-plane sweeps of earlier versions (gb_sweep_tuning)"""
         v = (ctypes.c_int * 2)()
         self._ck(self._L.gb_sweep_tuning(self.h, level, v))
         return int(v[0]), int(v[1])

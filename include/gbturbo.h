@@ -123,9 +123,9 @@ int gb_get_outlet_pressure(gb_solver *h, double *out);
 
 /* waits for the handle's stream */
 int gb_sync(gb_solver *h);
-/* block shape of the LU-SGS sweep kernels on a level: out[0] cells per warp, out[1] warps per
- * block, chosen at create by timing the plane chains of each candidate shape; the choice changes
- * timing only, not results */
+/* block shape of the plane-by-plane sweep launches of earlier versions: out[0] cells per warp (10),
+ * out[1] warps per block (1). The sweeps now march tiles of grid columns in one launch per direction and
+ * have no shape to choose; the call is kept for programs that report it */
 int gb_sweep_tuning(gb_solver *h, int level, int out[2]);
 /* whether a level's face stage runs on tiles of faces staged in shared memory by the tensor memory
  * accelerator (*tma = 1; the mixed form's default scheme on meshes whose k extent KM is 4n + 1 and
