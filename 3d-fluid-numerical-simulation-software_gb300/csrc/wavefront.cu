@@ -57,7 +57,7 @@ constexpr int kSlots = kGroup * kStages;        // steps whose terms are kept: t
                                                 // are never overwritten before they are sent
 constexpr int kAhead = 4;                       // steps that the incoming warp asks ahead
 constexpr unsigned kWaitLimit = 1u << 21;       // polls of a wait before it gives up (seconds)
-constexpr int kSteps32 = 32;                    // steps of a block of the gather and scatter kernels
+constexpr int kSteps32 = 16;                    // steps of a block of the FP32 gather kernel
 
 // bytes of a step's blocks, packets of an edge cell and of a step
 //   FP32: geo {n_d, V_entrainment,d} at 3 cell + d; flow {h_d, c_d} at 3 cell + d of the forward sweep, {rho, m},
@@ -534,9 +534,12 @@ __device__ __forceinline__ void next_sweep(const WaveTables &V)
     }
 }
 
-// FP32: a block takes 32 steps of a tile; a warp reads 32 consecutive k of a column (each column its own
-// 32, shifted by a + b), and the block writes its steps as contiguous pieces through shared memory
-__global__ void __launch_bounds__(256) k_wave_gather32(Batch B, PhysW<float> P, Flow<float> W, WaveTables V)
+// FP32: a block takes 16 steps of a tile, one thread per cell: a half-warp reads 16 consecutive k of a column
+// (each column its own 16, shifted by a + b), and the block writes its steps as contiguous pieces through
+// shared memory. Bound by the latency of its loads, some 30 per cell: with 32 steps and four cells per
+// thread one after another it took 43 us on the 129x49x49 passage and 168 us per cycle on 32 solves of
+// 25x25x65 nodes, one cell per thread 15 and 64 (40 for the bytes of the latter).
+__global__ void __launch_bounds__(NC * kSteps32) k_wave_gather32(Batch B, PhysW<float> P, Flow<float> W, WaveTables V)
 {
     using L = Lay<float, MEAN>;
     constexpr int NF = L::flow / 16, ND = L::dq / 16, stride = NF + ND + 1;      // quads per step, and in shared memory
@@ -546,49 +549,53 @@ __global__ void __launch_bounds__(256) k_wave_gather32(Batch B, PhysW<float> P, 
     const Chunk c = chunk_of(V, kSteps32);
     if (!c.live) return;
     const Lvl Lv = B.lv[blockIdx.y];
-    const int b = threadIdx.x >> 5, st = threadIdx.x & 31;
-    const int j = c.PJ * PB + b + 1;
-    const long long sn[3] = {(long long)Lv.NJ * Lv.NK, Lv.NK, 1};
-#pragma unroll
-    for (int a = 0; a < PA; a++) {
-        const int i = c.PI * PA + a + 1, k = c.t0 + st - a - b + 1, cell = a * PB + b;
-        float4 o = {1.0f, 0, 0, 0}, x = {0, 0, 1.0f, 0}, r = {0, 0, 0, 0};
-        float2 hc[2][3] = {};
-        float r4 = 0.0f;
-        if (i <= c.S.nI && j <= c.S.nJ && k >= 1 && k <= c.S.nK) {
-            const long long p = ix(Lv, i, j, k);
-            o = make_float4(f64_to_f32_rn(W.cv[0][p]), f64_to_f32_rn(W.cv[1][p]), f64_to_f32_rn(W.cv[2][p]), f64_to_f32_rn(W.cv[3][p]));
-            x = make_float4(f64_to_f32_rn(W.cv[4][p]), W.pv[PP][p], 1.0f / o.x, 0.0f);
-            const float inva = W.dinv[p];
-            r = make_float4(__fmul_rn(-W.res[0][p], inva), __fmul_rn(-W.res[1][p], inva), __fmul_rn(-W.res[2][p], inva),
-                            __fmul_rn(-W.res[3][p], inva));
-            r4 = __fmul_rn(-W.res[4][p], inva);
-            const float *area = (const float *)V.area + (c.step + st) * (3 * NC) + 3 * cell;
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                // what the cell's term is scaled with is the diagonal of the cell that receives it (one that
-                // lies outside the box has none and receives nothing)
-                const float h = 0.5f * area[d], q = __fmaf_rn(0.5f, __fmul_rn(P.relax, W.lamc[d][p]), W.lamv[d][p]);
-                const float up = W.dinv[p + sn[d]], dn = W.dinv[p - sn[d]];
-                hc[0][d] = make_float2(__fmul_rn(h, up), __fmul_rn(q, up));
-                hc[1][d] = make_float2(__fmul_rn(h, dn), __fmul_rn(q, dn));
-            }
-        }
-        char *t = smem + st * stride * 16;
+    const int cell = threadIdx.x / kSteps32, st = threadIdx.x % kSteps32, a = cell / PB, b = cell % PB;
+    const int i = c.PI * PA + a + 1, j = c.PJ * PB + b + 1, k = c.t0 + st - a - b + 1;
+    float4 o = {1.0f, 0, 0, 0}, x = {0, 0, 1.0f, 0}, r = {0, 0, 0, 0};
+    float2 hc[2][3] = {};
+    float r4 = 0.0f;
+    if (i <= c.S.nI && j <= c.S.nJ && k >= 1 && k <= c.S.nK) {
+        const long long p = ix(Lv, i, j, k);
+        const long long sn[3] = {(long long)Lv.NJ * Lv.NK, Lv.NK, 1};
+        const double q0 = W.cv[0][p], q1 = W.cv[1][p], q2 = W.cv[2][p], q3 = W.cv[3][p], q4 = W.cv[4][p];
+        const float *area = (const float *)V.area + (c.step + st) * (3 * NC) + 3 * cell;
+        const float inva = W.dinv[p];
+        float lc[3], lv[3], ar[3], up[3], dn[3];
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            ((float2 *)t)[3 * cell + d] = hc[0][d];
-            ((float2 *)(t + L::flow - L::ends))[3 * cell + d] = hc[1][d];
+            lc[d] = W.lamc[d][p]; lv[d] = W.lamv[d][p]; ar[d] = area[d];
+            // what the cell's term is scaled with is the diagonal of the cell that receives it (one that
+            // lies outside the box has none and receives nothing)
+            up[d] = W.dinv[p + sn[d]]; dn[d] = W.dinv[p - sn[d]];
         }
-        ((float4 *)(t + L::ends))[cell] = o;
-        ((float4 *)(t + L::ends))[NC + cell] = x;
-        ((float4 *)(t + L::flow))[cell] = r;
-        ((float *)(t + L::flow))[4 * NC + cell] = r4;
+        const float s0 = W.res[0][p], s1 = W.res[1][p], s2 = W.res[2][p], s3 = W.res[3][p], s4 = W.res[4][p];
+        x.y = W.pv[PP][p];
+        o = make_float4(f64_to_f32_rn(q0), f64_to_f32_rn(q1), f64_to_f32_rn(q2), f64_to_f32_rn(q3));
+        x.x = f64_to_f32_rn(q4);
+        x.z = 1.0f / o.x;
+        r = make_float4(__fmul_rn(-s0, inva), __fmul_rn(-s1, inva), __fmul_rn(-s2, inva), __fmul_rn(-s3, inva));
+        r4 = __fmul_rn(-s4, inva);
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const float h = 0.5f * ar[d], q = __fmaf_rn(0.5f, __fmul_rn(P.relax, lc[d]), lv[d]);
+            hc[0][d] = make_float2(__fmul_rn(h, up[d]), __fmul_rn(q, up[d]));
+            hc[1][d] = make_float2(__fmul_rn(h, dn[d]), __fmul_rn(q, dn[d]));
+        }
     }
+    char *t = smem + st * stride * 16;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        ((float2 *)t)[3 * cell + d] = hc[0][d];
+        ((float2 *)(t + L::flow - L::ends))[3 * cell + d] = hc[1][d];
+    }
+    ((float4 *)(t + L::ends))[cell] = o;
+    ((float4 *)(t + L::ends))[NC + cell] = x;
+    ((float4 *)(t + L::flow))[cell] = r;
+    ((float *)(t + L::flow))[4 * NC + cell] = r4;
     __syncthreads();
     float4 *df = (float4 *)(V.flow + c.step * L::flow), *dd = (float4 *)(V.dq + c.step * L::dq);
-    for (int e = threadIdx.x; e < c.nt * NF; e += 256) df[e] = tile[(e / NF) * stride + e % NF];
-    for (int e = threadIdx.x; e < c.nt * ND; e += 256) dd[e] = tile[(e / ND) * stride + NF + e % ND];
+    for (int e = threadIdx.x; e < c.nt * NF; e += NC * kSteps32) df[e] = tile[(e / NF) * stride + e % NF];
+    for (int e = threadIdx.x; e < c.nt * ND; e += NC * kSteps32) dd[e] = tile[(e / ND) * stride + NF + e % ND];
 }
 
 // FP64: one thread per cell and step, eight steps per block (a 32-byte sector of a column's row serves four
@@ -750,7 +757,7 @@ __global__ void __launch_bounds__(256) k_wave_scatter_var(Batch B, Flow<T> W, Wa
     W.dq_ev[ix(B.lv[blockIdx.y], i, j, k)] = ((const T *)(VV.dq + (c.step + st) * Lay<T, VAR>::dq))[cell];
 }
 
-constexpr unsigned kGatherBytes = 32 * (Lay<float, MEAN>::flow + Lay<float, MEAN>::dq + 16);
+constexpr unsigned kGatherBytes = kSteps32 * (Lay<float, MEAN>::flow + Lay<float, MEAN>::dq + 16);
 
 // (shared memory beyond the default limit has to be asked for, once per kernel and device)
 template <typename T, Kind K>
@@ -800,7 +807,7 @@ void launch_lusgs_sweeps(const LaunchCtx &ctx, const PhysW<T> &P, const Geo &G, 
 {
     auto chunks = [&](int steps) { return dim3((unsigned)(V.max_tiles * ((V.max_T + steps - 1) / steps)), ctx.batch.nsolve); };
     ctx.mark("sweep_forward", 1, 2);
-    if constexpr (sizeof(T) == 4) k_wave_gather32<<<chunks(kSteps32), 256, kGatherBytes, ctx.stream>>>(ctx.batch, P, W, V);
+    if constexpr (sizeof(T) == 4) k_wave_gather32<<<chunks(kSteps32), NC * kSteps32, kGatherBytes, ctx.stream>>>(ctx.batch, P, W, V);
     else k_wave_gather64<<<chunks(8), 256, 0, ctx.stream>>>(ctx.batch, P, W, V);
     march<T, 1, MEAN>(ctx, V, P.gm1);
     ctx.mark("sweep_forward", 0, 2);
