@@ -51,6 +51,7 @@ struct BcTables {
     int max_outlet_im = 0, max_outlet_jm = 0;
     double *outlet_cu = nullptr;                  // per outlet patch: mass-weighted swirl of each radial row
     double *integ_part = nullptr;                 // per solve and section: kIntegralBlocks partial sums of 3
+    unsigned *integ_count = nullptr;              // per solve: blocks of a launch that are done
     // Baldwin-Lomax wall distances (fine level): record w holds, for point n0 = 1..N-1 of each of
     // its wall-normal lines t, the distance of cell n0 from the line's wall-face centre at
     // wall_dist[wall_dist_off[w] + (n0 - 1) * lines(w) + t], in the working precision
@@ -66,7 +67,7 @@ struct BcTables {
     long long n_sa_gather = 0;
 };
 
-constexpr int kIntegralBlocks = 16;             // blocks per inlet/outlet section in the integrals
+constexpr int kIntegralBlocks = 32;             // blocks per inlet/outlet section in the integrals
 
 // The LU-SGS sweeps' tiles (wavefront.cu). A tile is a group of grid columns that a block marches
 // along k, skewed by the columns' places in it; the tiles of a slot hold T steps each, tile (PI, PJ)
@@ -131,7 +132,7 @@ void launch_update(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> F,
 
 template <typename T>
 void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> F, const double *totalvol, double *partials,
-                     int nblk);
+                     int nblk, unsigned *count);
 
 // residual norm with scratch in a static device array; copies the norms to host_out if given
 template <typename T>

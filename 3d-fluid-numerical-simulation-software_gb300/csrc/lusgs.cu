@@ -203,72 +203,111 @@ void launch_limiter(const LaunchCtx &ctx, const Phys &P, Flow<T> W, int level, i
     k_limiter<T><<<(B.nsolve + 31) / 32, 32, 0, ctx.stream>>>(B, P, W, level, bad_list, bad_cap, bad_count);
 }
 
-// ---- residual norm: sum |(Q_old - Q)/Q_old| * Vol / V_total, FP64, fixed-order two-stage sum ----
+// whether this block is the last of its group to get here (all threads call it; what the group's blocks
+// wrote before is then visible). The counter is put back to zero for the next launch.
+__device__ __forceinline__ bool last_block(unsigned *count, unsigned blocks)
+{
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(count, 1u) == blocks - 1;
+        if (last) *count = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// ---- residual norm: sum |(Q_old - Q)/Q_old| * Vol / V_total, FP64, in a fixed order: each thread four or
+// more cells, the threads of a block, the blocks of a case (its last block to arrive sums them for every
+// slot). Bound by its FP64 instructions: 45 per cell in the FP64 form (25 us for the 129x49x49 passage),
+// 5 in the mixed form, whose reductions counted more. With 304 blocks for every slot, each reduced by 25
+// shuffled additions per warp, and the blocks' sums added up by five threads of a second kernel it took 62
+// and 46 us, and 195 us for 32 solves of 25x25x65 nodes; now 33, 20 and 48.
+constexpr int kNormThreads = 256, kNormCells = 4 * kNormThreads;
+__host__ __device__ inline int norm_blocks(const Lvl &L, int most)
+{
+    const int n = ((L.IM - 1) * (L.JM - 1) * (L.KM - 1) + kNormCells - 1) / kNormCells;
+    return n < most ? n : most;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_norm_partial(Batch B, Geo G, Flow<T> W, double *partials, int nblk)
+__global__ void __launch_bounds__(kNormThreads) k_norm(Batch B, Geo G, Flow<T> W, double *partials, int nblk, const double *totalvol,
+                                                       unsigned *count)
 {
     const int s = blockIdx.y;
     const Lvl L = B.lv[s];
+    const int nb = norm_blocks(L, nblk);
+    if ((int)blockIdx.x >= nb) return;
     const int nI = L.IM - 1, nJ = L.JM - 1, nK = L.KM - 1;
     const unsigned n = (unsigned)nI * (unsigned)nJ * (unsigned)nK;
     double acc[5] = {0, 0, 0, 0, 0};
-    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (unsigned)nblk * blockDim.x) {
+    for (unsigned t = blockIdx.x * kNormThreads + threadIdx.x; t < n; t += (unsigned)nb * kNormThreads) {
         const unsigned q = t / (unsigned)nK, r = q / (unsigned)nJ;
         const int k = (int)(t - q * (unsigned)nK) + 1, j = (int)(q - r * (unsigned)nJ) + 1, i = (int)r + 1;
         const long long p = ix(L, i, j, k);
         const double vol = G.vol[p];
+        double o[5], c[5];
 #pragma unroll
-        for (int c = 0; c < 5; c++) {
-            const double o = W.cvold[c][p];
-            acc[c] += rel_change_t<T>(o, W.cv[c][p]) * vol;
-        }
-    }
-    __shared__ double sh[8][5];
+        for (int m = 0; m < 5; m++) { o[m] = W.cvold[m][p]; c[m] = W.cv[m][p]; }
 #pragma unroll
-    for (int c = 0; c < 5; c++) {
-        double v = acc[c];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][c] = v;
+        for (int m = 0; m < 5; m++) acc[m] += rel_change_t<T>(o[m], c[m]) * vol;
     }
+    __shared__ double sh[5][kNormThreads];
+#pragma unroll
+    for (int m = 0; m < 5; m++) sh[m][threadIdx.x] = acc[m];
     __syncthreads();
-    if (threadIdx.x < 5) {
+    const int m = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto warp_sum = [](double v) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        return v;
+    };
+    if (m < 5) {                                  // one warp per component
         double v = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) v += sh[w][threadIdx.x];
-        partials[((long long)s * nblk + blockIdx.x) * 5 + threadIdx.x] = v;
+        for (int e = lane; e < kNormThreads; e += 32) v += sh[m][e];
+        v = warp_sum(v);
+        if (lane == 0) partials[((long long)s * nblk + blockIdx.x) * 5 + m] = v;
     }
-}
-
-// the norm of a case: the partials of its blocks in block order, over the case's volume (every
-// slot of the case computes the same sum and keeps it)
-__global__ void k_norm_final(Batch B, const double *partials, int nblk, const double *totalvol)
-{
-    const int s = blockIdx.x;
-    if (threadIdx.x >= 5) return;
     const SolveConst &sc = B.sc[s];
+    unsigned blocks = 0;
+    for (int q = sc.lead; q < sc.lead + sc.nblk; q++) blocks += (unsigned)norm_blocks(B.lv[q], nblk);
+    if (!last_block(count + sc.lead, blocks) || m >= 5) return;
+    // the norm of the case: the sums of its slots over the case's volume (every slot keeps it)
     double v = 0;
-    for (int q = sc.lead; q < sc.lead + sc.nblk; q++)
-        for (int b = 0; b < nblk; b++) v += partials[((long long)q * nblk + b) * 5 + threadIdx.x];
-    v = v / totalvol[s];
-    B.st[s].res[threadIdx.x] = v;
-    if (threadIdx.x == 0 && !isfinite(v)) B.st[s].status |= GBT_STATUS_NAN;
+    for (int q = sc.lead; q < sc.lead + sc.nblk; q++) {
+        const int nq = norm_blocks(B.lv[q], nblk);
+        for (int e = lane; e < nq; e += 32) v += __ldcg(&partials[((long long)q * nblk + e) * 5 + m]);
+    }
+    v = warp_sum(v);
+    if (lane != 0) return;
+    for (int q = sc.lead; q < sc.lead + sc.nblk; q++) {
+        const double w = v / totalvol[q];
+        B.st[q].res[m] = w;
+        if (m == 0 && !isfinite(w)) B.st[q].status |= GBT_STATUS_NAN;
+    }
 }
 
 template <typename T>
-void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> W, const double *totalvol, double *partials, int nblk)
+void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> W, const double *totalvol, double *partials, int nblk, unsigned *count)
 {
     const Batch &B = ctx.batch;
-    ctx.mark("res_norm", 1, 2);
-    k_norm_partial<T><<<dim3(nblk, B.nsolve), 256, 0, ctx.stream>>>(B, G, W, partials, nblk);
-    k_norm_final<<<B.nsolve, 32, 0, ctx.stream>>>(B, partials, nblk, totalvol);
-    ctx.mark("res_norm", 0, 2);
+    ctx.mark("res_norm", 1, 1);
+    const Lvl most = {ctx.maxIM, ctx.maxJM, ctx.maxKM, 0, 0, 0};
+    k_norm<T><<<dim3(norm_blocks(most, nblk), B.nsolve), kNormThreads, 0, ctx.stream>>>(B, G, W, partials, nblk, totalvol, count);
+    ctx.mark("res_norm", 0, 1);
 }
 
-// ---- inlet/outlet integrals (source/Ouput.cpp:9-107,282-300) ----
-// partial sums over one section (inlet or outlet k face): mass flow, sum Pt^((g-1)/g) * m and
-// sum Tt * m; grid (kIntegralBlocks, solves, 2 sections), so the FP64 powers spread over the SMs
+// ---- inlet/outlet integrals (source/Ouput.cpp:9-107,282-300)
+// Partial sums over one section (inlet or outlet k face): mass flow, sum Pt^((g-1)/g) * m and sum Tt * m;
+// grid (kIntegralBlocks, solves, 2 sections). With Pt = p fac^(g/(g-1)) the power is p^((g-1)/g) fac, one
+// FP64 power per point instead of two, and Ma^2 needs no roots. The last block of a solve adds its
+// blocks' sums up in their order and forms the reported values, a lane per section where they are powers.
+// Bound by the latency of the FP64 chains: 48 us per evaluation of the 129x49x49 passage as two kernels
+// with two powers per point, sums and powers of a solve on one thread, now 26.
 template <typename T>
-__global__ void __launch_bounds__(128) k_section_partial(Batch B, Phys P, Geo G, Flow<T> W, const DevInOut *inl,
-                                                         const DevInOut *outl, double *part)
+__global__ void __launch_bounds__(128) k_integrals(Batch B, Phys P, Geo G, Flow<T> W, const DevInOut *inl, const DevInOut *outl,
+                                                   double *part, unsigned *count)
 {
     const int s = blockIdx.y, sec = blockIdx.z;
     // the section's block: the case's Inlet[1] / Outlet[1] may lie in any of its blocks
@@ -287,11 +326,9 @@ __global__ void __launch_bounds__(128) k_section_partial(Batch B, Phys P, Geo G,
         const double w = 0.5 * ((double)W.pv[PW][p] + (double)W.pv[PW][q]);
         const double mc = d * (u * G.S[2][0][p] + v * G.S[2][1][p] + w * G.S[2][2][p]);
         const double tf = 0.5 * ((double)W.pv[PT][p] + (double)W.pv[PT][q]);
-        const double Ma = sqrt(u * u + v * v + w * w) / sqrt(g * R * tf);
-        const double fac = 1.0 + g1 / 2.0 * Ma * Ma;
-        const double Pt = (double)W.pv[PP][p] * pow(fac, g / g1);
+        const double fac = 1.0 + g1 / 2.0 * ((u * u + v * v + w * w) / (g * R * tf));
         m += mc;
-        pm += pow(Pt, g1 / g) * mc;
+        pm += pow((double)W.pv[PP][p], g1 / g) * fac * mc;
         tm += (double)W.pv[PT][p] * fac * mc;
     }
     __shared__ double sh[3][4];
@@ -307,29 +344,27 @@ __global__ void __launch_bounds__(128) k_section_partial(Batch B, Phys P, Geo G,
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) v += sh[threadIdx.x][w];
         part[(((long long)s * 2 + sec) * kIntegralBlocks + blockIdx.x) * 3 + threadIdx.x] = v;
     }
-}
-
-// inlet/outlet integrals (source/Ouput.cpp:9-107,282-300): partials summed in block order
-__global__ void k_integrals(Batch B, Phys P, const DevInOut *inl, const DevInOut *outl, const double *part)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= B.nsolve) return;
-    double a[3] = {0, 0, 0}, b[3] = {0, 0, 0};
-    for (int blk = 0; blk < kIntegralBlocks; blk++)
-        for (int c = 0; c < 3; c++) {
-            a[c] += part[(((long long)s * 2 + 0) * kIntegralBlocks + blk) * 3 + c];
-            b[c] += part[(((long long)s * 2 + 1) * kIntegralBlocks + blk) * 3 + c];
-        }
-    const double g = P.gamma, g1 = g - 1.0, R = P.rgas;
+    if (!last_block(count + s, 2 * kIntegralBlocks) || threadIdx.x >= 32) return;
+    // lanes 0..2: the inlet's sums, 3..5: the outlet's
+    const int lane = threadIdx.x;
+    double sum = 0;
+    if (lane < 6)
+        for (int b = 0; b < kIntegralBlocks; b++) sum += __ldcg(&part[(((long long)s * 2 + lane / 3) * kIntegralBlocks + b) * 3 + lane % 3]);
+    double a[3], b[3];
+    for (int c = 0; c < 3; c++) {
+        a[c] = __shfl_sync(0xffffffffu, sum, c);
+        b[c] = __shfl_sync(0xffffffffu, sum, 3 + c);
+    }
     // blade count of the inlet's and of the outlet's block (source/Ouput.cpp:288,294)
     const double mi = a[0] * P.dens_ref * P.vel_ref * B.sc[inl[s].solve].nblade;
     const double mo = b[0] * P.dens_ref * P.vel_ref * B.sc[outl[s].solve].nblade;
-    const double pti = pow(a[1] / a[0], g / g1) * P.dens_ref * P.vel_ref * P.vel_ref;
-    const double pto = pow(b[1] / b[0], g / g1) * P.dens_ref * P.vel_ref * P.vel_ref;
+    const double pt = pow(lane == 0 ? a[1] / a[0] : b[1] / b[0], g / g1) * P.dens_ref * P.vel_ref * P.vel_ref;
+    const double pti = __shfl_sync(0xffffffffu, pt, 0), pto = __shfl_sync(0xffffffffu, pt, 1);
     const double tti = a[2] / a[0] * P.temp_ref, tto = b[2] / b[0] * P.temp_ref;
     const double PR = pto / pti;
     const double Ladk = g / g1 * R * tti * (pow(PR, g1 / g) - 1.0);
     const double Lk = g / g1 * R * tti * (tto / tti - 1.0);
+    if (lane != 0) return;
     SolveState &st = B.st[s];
     st.m_in = mi; st.m_out = mo; st.pr = PR; st.eff = Ladk / Lk;
     st.m_ratio = fabs((mi - mo) / mi);
@@ -341,9 +376,8 @@ void launch_integrals(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T>
 {
     // first inlet and first outlet patch of every solve (the reference reports Inlet[1], Outlet[1])
     const Batch &B = ctx.batch;
-    k_section_partial<T><<<dim3(kIntegralBlocks, B.nsolve, 2), 128, 0, ctx.stream>>>(B, P, G, W, bc.inlet_first,
-                                                                                      bc.outlet_first, bc.integ_part);
-    k_integrals<<<(B.nsolve + 31) / 32, 32, 0, ctx.stream>>>(B, P, bc.inlet_first, bc.outlet_first, bc.integ_part);
+    k_integrals<T><<<dim3(kIntegralBlocks, B.nsolve, 2), 128, 0, ctx.stream>>>(B, P, G, W, bc.inlet_first, bc.outlet_first,
+                                                                               bc.integ_part, bc.integ_count);
 }
 
 // CFL ramp of the driver (source/Solver.cpp:49-60): x1.2 whenever the density residual falls
@@ -368,7 +402,7 @@ void launch_cfl_ramp(const LaunchCtx &ctx, int iter)
     template void launch_update<T>(const LaunchCtx &, const Phys &, const Geo &, Flow<T>, int, int *, int, int *);     \
     template void launch_primitive<T>(const LaunchCtx &, const Phys &, Flow<T>);                                       \
     template void launch_limiter<T>(const LaunchCtx &, const Phys &, Flow<T>, int, int *, int, int *);                 \
-    template void launch_res_norm<T>(const LaunchCtx &, const Geo &, Flow<T>, const double *, double *, int);          \
+    template void launch_res_norm<T>(const LaunchCtx &, const Geo &, Flow<T>, const double *, double *, int, unsigned *);          \
     template void launch_integrals<T>(const LaunchCtx &, const Phys &, const Geo &, Flow<T>, const BcTables &);
 GBT_INST(double)
 GBT_INST(float)

@@ -322,7 +322,8 @@ public:
     const int bad_cap = 4096;
     double *norm_part = nullptr;
     double *init_q = nullptr;             // uniform start: five conserved values per slot
-    const int norm_blk = 304;            // two blocks per SM: the FP64 divisions spread over all SMs
+    const int norm_blk = 304;            // most blocks of a slot in the residual norm: two per SM
+    unsigned *norm_count = nullptr;       // per case (its first slot): blocks of a launch that are done
     T *dtmin = nullptr;
     cudaGraphExec_t graphs[3] = {nullptr, nullptr, nullptr};
     int phase_runs[3] = {0, 0, 0};        // iterations run in each driver phase (graphs: see iterate)
@@ -505,7 +506,7 @@ public:
         CK(cudaMemcpy(st_d, st.data(), st_mem.bytes, cudaMemcpyHostToDevice));
         // scratch: limiter lists, norm partials, global-dt minima
         size_t sb = sizeof(int) * (size_t)nsolve * (bad_cap + 1) + sizeof(double) * (size_t)nsolve * (norm_blk + 1) * 5 +
-                    sizeof(T) * nsolve + 256;
+                    sizeof(unsigned) * nsolve + sizeof(T) * nsolve + 256;
         scratch_mem.bytes = sb;
         CK(cudaMalloc(&scratch_mem.p, sb));
         char *q = (char *)scratch_mem.p;
@@ -513,6 +514,8 @@ public:
         init_q = (double *)q; q += sizeof(double) * (size_t)nsolve * 5;
         bad_list = (int *)q; q += sizeof(int) * (size_t)nsolve * bad_cap;
         bad_count = (int *)q; q += sizeof(int) * nsolve;
+        norm_count = (unsigned *)q; q += sizeof(unsigned) * nsolve;
+        CK(cudaMemset(norm_count, 0, sizeof(unsigned) * nsolve));
         dtmin = (T *)(((uintptr_t)q + 15) & ~(uintptr_t)15);
         timer.mark("solve state and scratch", stream);
         for (int l = 1; l <= ng; l++) build_level(l);
@@ -999,7 +1002,7 @@ public:
         size_t tot = bytes(inl.size(), sizeof(DevInOut)) + bytes(outl.size(), sizeof(DevInOut)) + bytes(inl1.size(), sizeof(DevInOut)) +
                      bytes(outl1.size(), sizeof(DevInOut)) + bytes(walls.size(), sizeof(DevWall)) + bytes(pdst.size(), 8) * 2 +
                      bytes(pmeta.size(), 4) + bytes(outl.size() * (size_t)(bc.max_outlet_im + 1), 8) +
-                     bytes((size_t)nsolve * 2 * kIntegralBlocks * 3, 8) + bytes(sa_dst_h.size(), 8) * 2 +
+                     bytes((size_t)nsolve * 2 * kIntegralBlocks * 3, 8) + bytes((size_t)nsolve, 4) + bytes(sa_dst_h.size(), 8) * 2 +
                      bytes(mixes.size(), sizeof(DevMix)) + bytes(mixes.size() * (size_t)bc.max_mix_rows * kMixVals, 8) +
                      bytes((size_t)nsolve * 4, 8) + 256;
         CK(cudaMalloc(&Lv.tab_mem.p, tot));
@@ -1027,6 +1030,8 @@ public:
         bc.mix_avg = (double *)up(nullptr, 0, 8); q += bytes(mixes.size() * (size_t)bc.max_mix_rows * kMixVals, 8);
         bc.outlet_cu = (double *)up(nullptr, 0, 8); q += bytes(outl.size() * (size_t)(bc.max_outlet_im + 1), 8);
         bc.integ_part = (double *)up(nullptr, 0, 8); q += bytes((size_t)nsolve * 2 * kIntegralBlocks * 3, 8);
+        const std::vector<unsigned> zeros(nsolve, 0);
+        bc.integ_count = (unsigned *)up(zeros.data(), zeros.size(), 4);
         double *trig = (double *)up(nullptr, 0, 8); q += bytes((size_t)nsolve * 4, 8);
         bc.per_trig = trig;
         launch_periodic_trig(ctx(l), trig);
@@ -1106,7 +1111,7 @@ public:
         { Mark m(this, "mg_forcing"); launch_forcing_keep<T>(ctx(l), lev[l].W); }
         sweep_update(l);
     }
-    void res_calculate(int l) override { launch_res_norm<T>(ctx(l), lev[l].G, lev[l].W, lev[l].totalvol, norm_part, norm_blk); }
+    void res_calculate(int l) override { launch_res_norm<T>(ctx(l), lev[l].G, lev[l].W, lev[l].totalvol, norm_part, norm_blk, norm_count); }
     void sweep_shape(int, int out[2]) const override { out[0] = 10; out[1] = 1; }
     bool face_staged(int l) const override
     {
@@ -1132,7 +1137,7 @@ public:
         launch_interpolate<T>(ctx(1), ctx(2), lev[1].W, lev[2].W, init);
     }
     void delta_cons() override { need_mg(); Mark m(this, "mg_delta"); launch_delta<T>(ctx(2), lev[2].W); }
-    void integrals(int l) override { Mark m(this, "integrals", 2); launch_integrals<T>(ctx(l), P, lev[l].G, lev[l].W, lev[l].bc); }
+    void integrals(int l) override { Mark m(this, "integrals", 1); launch_integrals<T>(ctx(l), P, lev[l].G, lev[l].W, lev[l].bc); }
     void set_use_force(int l, bool on) override { lev[l].use_force = on; }
     void need_mg() const { if (ng < 2) throw std::runtime_error("the case runs on a single grid level"); }
 
