@@ -21,12 +21,10 @@ __device__ __forceinline__ void st_state(Flow<T> &W, long long g, const double c
 
 // inlet: Riemann invariant from the interior, total pressure/temperature and flow direction
 template <typename T>
-__global__ void __launch_bounds__(32) k_bc_inlet(Batch B, Phys P, Geo G, Flow<T> W, const DevInOut *pat)
+__device__ __forceinline__ void bc_inlet(const Batch &B, const Phys &P, const Geo &G, Flow<T> &W, const DevInOut &pt, int t)
 {
-    const DevInOut pt = pat[blockIdx.y];
     const Lvl L = B.lv[pt.solve];
     const int ni = pt.ie - pt.is + 1, nj = pt.je - pt.js + 1;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ni * nj) return;
     const int i = pt.is + t / nj, j = pt.js + t % nj;
     const bool low = (pt.ks == 1);
@@ -61,27 +59,22 @@ __global__ void __launch_bounds__(32) k_bc_inlet(Batch B, Phys P, Geo G, Flow<T>
     for (int nd = 1; nd <= P.ndummy; nd++) st_state(W, ix(L, i, j, low ? -nd : L.KM + nd), c, q);
 }
 
-// axial outlet in three launches spread over the SMs: mass-weighted swirl per radial row (one
-// warp per row, lanes over the pitch), radial equilibrium marched from p_out at i = IM/2 using
-// the previous ghost density (one warp per pitch line), then ghosts extrapolated from the last
-// interior layer (one thread per face)
+// axial outlet in two parts: mass-weighted swirl per radial row (one warp per row, lanes over the pitch),
+// then, one warp per pitch line, radial equilibrium marched from p_out at i = IM/2 using the previous ghost
+// density, and the ghosts extrapolated from the last interior layer. The sine and cosine of the faces'
+// polar angles are formed once per level (k_outlet_trig, the same function).
 template <typename T>
-__global__ void __launch_bounds__(256) k_outlet_swirl(Batch B, Geo G, Flow<T> W, const DevInOut *pat, double *cu_all,
-                                                      int cu_stride)
+__device__ __forceinline__ void bc_swirl(const Batch &B, const Geo &G, Flow<T> &W, const DevInOut &pt, const double2 *trig, double *cu, int i)
 {
-    const DevInOut pt = pat[blockIdx.y];
     const Lvl L = B.lv[pt.solve];
     const int JM = L.JM, KM = L.KM;
     const int lane = threadIdx.x & 31;
-    const int i = 1 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (i > L.IM - 1) return;
     double acc = 0.0, sa = 0.0;
     for (int j = 1 + lane; j <= JM - 1; j += 32) {
         const long long p = ix(L, i, j, KM - 1), f = ix(L, i, j, KM);
-        const double th = G.th[2][f];
-        double sn, cs;
-        sincos(th, &sn, &cs);
-        const double ct = -1.0 * (double)W.pv[PU][p] * sn + (double)W.pv[PV][p] * cs;
+        const double2 sc = trig[(i - 1) * (JM - 1) + j - 1];
+        const double ct = -1.0 * (double)W.pv[PU][p] * sc.x + (double)W.pv[PV][p] * sc.y;
         acc = acc + ct * G.s[2][f];
         sa = sa + G.s[2][f];
     }
@@ -89,7 +82,18 @@ __global__ void __launch_bounds__(256) k_outlet_swirl(Batch B, Geo G, Flow<T> W,
         acc += __shfl_down_sync(0xffffffffu, acc, o);
         sa += __shfl_down_sync(0xffffffffu, sa, o);
     }
-    if (lane == 0) cu_all[(long long)blockIdx.y * cu_stride + i] = acc / sa;
+    if (lane == 0) cu[i] = acc / sa;
+}
+
+__global__ void k_outlet_trig(Batch B, Geo G, const DevInOut *pat, double2 *trig, long long stride)
+{
+    const DevInOut pt = pat[blockIdx.y];
+    const Lvl L = B.lv[pt.solve];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (L.IM - 1) * (L.JM - 1)) return;
+    double sn, cs;
+    sincos(G.th[2][ix(L, 1 + t / (L.JM - 1), 1 + t % (L.JM - 1), L.KM)], &sn, &cs);
+    trig[blockIdx.y * stride + t] = make_double2(sn, cs);
 }
 
 // The march p_i = p_(i+1) - t_i (towards the hub) and p_i = p_(i-1) + u_i (towards the casing)
@@ -97,18 +101,26 @@ __global__ void __launch_bounds__(256) k_outlet_swirl(Batch B, Geo G, Flow<T> W,
 // rows at a time and adds them up with a warp scan (a different association of the same sums
 // than the reference's running total).
 template <typename T>
-__global__ void __launch_bounds__(32) k_outlet_march(Batch B, Geo G, Flow<T> W, const DevInOut *pat, const double *cu_all,
-                                                     int cu_stride)
+__device__ __forceinline__ void bc_outlet_line(const Batch &B, const Phys &P, const Geo &G, Flow<T> &W, const DevInOut &pt,
+                                               const double *cu, int j)
 {
-    const DevInOut pt = pat[blockIdx.y];
     const Lvl L = B.lv[pt.solve];
     const int IM = L.IM, KM = L.KM;
-    const int j = 1 + blockIdx.x, lane = threadIdx.x;
+    const int lane = threadIdx.x & 31;
     if (j > L.JM - 1) return;
-    const double *cu = cu_all + (long long)blockIdx.y * cu_stride;
     const int iref = (int)(0.5 * IM);
-    const double pout = B.st[pt.solve].pout;
-    if (lane == 0) W.pv[PP][ix(L, iref, j, KM)] = (T)pout;
+    const double pout = B.st[pt.solve].pout, g1 = P.gamma - 1.0;
+    auto fill = [&](int i, double press) {
+        const long long g = ix(L, i, j, KM), p = ix(L, i, j, KM - 1);
+        const double d = W.cv[0][p];
+        const double pr = (double)(T)press;
+        const double u = W.pv[PU][p], v = W.pv[PV][p], w = W.pv[PW][p];
+        const double c[5] = {d, W.cv[1][p], W.cv[2][p], W.cv[3][p], pr / g1 + d * (u * u + v * v + w * w) / 2.0};
+        const T q[6] = {(T)d, (T)u, (T)v, (T)w, (T)pr, (T)(pr / P.rgas / d)};
+        st_state(W, g, c, q);
+        for (int nd = 1; nd <= P.ndummy; nd++) st_state(W, ix(L, i, j, KM + nd), c, q);
+    };
+    if (lane == 0) fill(iref, pout);
     // towards the hub: i = iref-1, iref-2, ..., 1
     double carry = 0.0;
     for (int base = 0; base < iref - 1; base += 32) {
@@ -123,7 +135,7 @@ __global__ void __launch_bounds__(32) k_outlet_march(Batch B, Geo G, Flow<T> W, 
             const double v = __shfl_up_sync(0xffffffffu, t, o);
             if (lane >= o) t += v;
         }
-        if (i >= 1) W.pv[PP][ix(L, i, j, KM)] = (T)(pout - (carry + t));
+        if (i >= 1) fill(i, pout - (carry + t));
         carry += __shfl_sync(0xffffffffu, t, 31);
     }
     // towards the casing: i = iref+1, ..., IM-1, radii of the k = KM-1 face row as the reference takes them
@@ -140,42 +152,20 @@ __global__ void __launch_bounds__(32) k_outlet_march(Batch B, Geo G, Flow<T> W, 
             const double v = __shfl_up_sync(0xffffffffu, u, o);
             if (lane >= o) u += v;
         }
-        if (i <= IM - 1) W.pv[PP][ix(L, i, j, KM)] = (T)(pout + (carry + u));
+        if (i <= IM - 1) fill(i, pout + (carry + u));
         carry += __shfl_sync(0xffffffffu, u, 31);
     }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_outlet_fill(Batch B, Phys P, Flow<T> W, const DevInOut *pat)
-{
-    const DevInOut pt = pat[blockIdx.y];
-    const Lvl L = B.lv[pt.solve];
-    const int IM = L.IM, JM = L.JM, KM = L.KM;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (IM - 1) * (JM - 1)) return;
-    const double g1 = P.gamma - 1.0;
-    const int i = 1 + t / (JM - 1), j = 1 + t % (JM - 1);
-    const long long g = ix(L, i, j, KM), p = ix(L, i, j, KM - 1);
-    const double d = W.cv[0][p];
-    const double pr = (double)W.pv[PP][g];
-    const double u = W.pv[PU][p], v = W.pv[PV][p], w = W.pv[PW][p];
-    const double c[5] = {d, W.cv[1][p], W.cv[2][p], W.cv[3][p], pr / g1 + d * (u * u + v * v + w * w) / 2.0};
-    const T q[6] = {(T)d, (T)u, (T)v, (T)w, (T)pr, (T)(pr / P.rgas / d)};
-    st_state(W, g, c, q);
-    for (int nd = 1; nd <= P.ndummy; nd++) st_state(W, ix(L, i, j, KM + nd), c, q);
 }
 
 // no-slip wall: ghost keeps p, T, rho, rho*E of the first cell, relative velocity reflected;
 // reconstruction layers = mean of ghost and first cell
 template <typename T>
-__global__ void k_bc_wall(Batch B, Phys P, Geo G, Flow<T> W, const DevWall *walls)
+__device__ __forceinline__ void bc_wall(const Batch &B, const Phys &P, const Geo &G, Flow<T> &W, const DevWall &wl, unsigned t)
 {
-    const DevWall wl = walls[blockIdx.y];
     const Lvl L = B.lv[wl.solve];
-    const int ni = wl.ie - wl.is + 1, nj = wl.je - wl.js + 1, nk = wl.ke - wl.ks + 1;
-    int i, j, k;
-    if (!box_index(ni, nj, nk, i, j, k)) return;
-    i += wl.is - 1; j += wl.js - 1; k += wl.ks - 1;
+    const unsigned ni = (unsigned)(wl.ie - wl.is + 1), nj = (unsigned)(wl.je - wl.js + 1), nk = (unsigned)(wl.ke - wl.ks + 1);
+    if (t >= ni * nj * nk) return;
+    const int i = wl.is + (int)(t / nk / nj), j = wl.js + (int)(t / nk % nj), k = wl.ks + (int)(t % nk);
     const int f = (wl.face - 1) / 2;
     const bool lo = wl.face % 2 == 1;
     const long long sn = f == 0 ? (long long)L.NJ * L.NK : (f == 1 ? (long long)L.NK : 1LL);
@@ -204,11 +194,9 @@ __global__ void k_bc_wall(Batch B, Phys P, Geo G, Flow<T> W, const DevWall *wall
 // periodic exchange: ghost/dummy <- interior cell of the partner face, velocity and momentum
 // rotated about z by +-delta_th
 template <typename T>
-__global__ void k_bc_periodic(Batch B, Flow<T> W, const long long *dst, const long long *src, const int *meta,
-                              const double *trig, long long n)
+__device__ __forceinline__ void bc_periodic(const Batch &B, Flow<T> &W, const long long *dst, const long long *src, const int *meta,
+                                            const double *trig, long long t)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
     const int mt = meta[t];
     const int s = mt >> 2, sg = (mt & 3) - 1;
     const long long a = src[t], b = dst[t];
@@ -356,22 +344,80 @@ __global__ void k_mix_fill(Batch B, Phys P, Flow<T> W, const DevMix *mix, int ma
     for (int nd = 1; nd <= P.ndummy; nd++) st_state(W, gp + step * nd, c, q);
 }
 
+// The fills in two launches, each block with one part of the work: first the outlets' swirl, the walls and the
+// periodic and interface copies, then the inlets and the outlets' lines. None of them reads what another
+// one writes (they read interior cells, and an outlet's line its own ghost's density), so they can run
+// side by side as long as no cell belongs to two of them (BcTables::apart; the parts come one after
+// another, as in the reference, where one does). Bound by the latency of the FP64 chains of the inlet's
+// state: as six launches in a row 69 us per evaluation of the 129x49x49 passage, as two 35.
+constexpr int kBcThreads = 128;
+struct BcParts { unsigned first[3]; };              // blocks of the first parts of a launch, summed up
+template <typename T>
+__global__ void __launch_bounds__(kBcThreads) k_bc_first(Batch B, Phys P, Geo G, Flow<T> W, BcTables bc, BcParts n, unsigned per_outlet,
+                                                         unsigned per_wall)
+{
+    unsigned b = blockIdx.x;
+    if (b < n.first[0]) {
+        const unsigned o = b / per_outlet;
+        bc_swirl<T>(B, G, W, bc.outlet[o], bc.outlet_trig + o * bc.outlet_trig_stride, bc.outlet_cu + (long long)o * (bc.max_outlet_im + 1),
+                    1 + (int)((b - o * per_outlet) * (kBcThreads / 32) + (threadIdx.x >> 5)));
+    } else if (b < n.first[1]) {
+        b -= n.first[0];
+        const unsigned o = b / per_wall;
+        bc_wall<T>(B, P, G, W, bc.wall[o], (b - o * per_wall) * kBcThreads + threadIdx.x);
+    } else {
+        const long long t = (long long)(b - n.first[1]) * kBcThreads + threadIdx.x;
+        if (t < bc.n_per) bc_periodic<T>(B, W, bc.per_dst, bc.per_src, bc.per_meta, bc.per_trig, t);
+    }
+}
+template <typename T>
+__global__ void __launch_bounds__(kBcThreads) k_bc_second(Batch B, Phys P, Geo G, Flow<T> W, BcTables bc, BcParts n, unsigned per_inlet,
+                                                          unsigned per_outlet)
+{
+    unsigned b = blockIdx.x;
+    if (b < n.first[0]) {
+        const unsigned o = b / per_inlet;
+        bc_inlet<T>(B, P, G, W, bc.inlet[o], (int)((b - o * per_inlet) * kBcThreads + threadIdx.x));
+    } else {
+        b -= n.first[0];
+        const unsigned o = b / per_outlet;
+        bc_outlet_line<T>(B, P, G, W, bc.outlet[o], bc.outlet_cu + (long long)o * (bc.max_outlet_im + 1),
+                          1 + (int)((b - o * per_outlet) * (kBcThreads / 32) + (threadIdx.x >> 5)));
+    }
+}
+
+void launch_outlet_trig(const LaunchCtx &ctx, const Geo &G, const BcTables &bc)
+{
+    if (bc.n_outlet)
+        k_outlet_trig<<<dim3((bc.max_outlet_im * bc.max_outlet_jm + 255) / 256, bc.n_outlet), 256, 0, ctx.stream>>>(
+            ctx.batch, G, bc.outlet, bc.outlet_trig, bc.outlet_trig_stride);
+}
+
 template <typename T>
 void launch_boundary(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> W, const BcTables &bc)
 {
     const Batch &B = ctx.batch;
-    // 32-thread blocks: the FP64 powers and roots of the inlet state spread over many SMs
-    if (bc.n_inlet) k_bc_inlet<T><<<dim3((bc.max_inlet + 31) / 32, bc.n_inlet), 32, 0, ctx.stream>>>(B, P, G, W, bc.inlet);
-    if (bc.n_outlet) {
-        const int cs = bc.max_outlet_im + 1;
-        k_outlet_swirl<T><<<dim3((bc.max_outlet_im + 7) / 8, bc.n_outlet), 256, 0, ctx.stream>>>(B, G, W, bc.outlet, bc.outlet_cu, cs);
-        k_outlet_march<T><<<dim3(bc.max_outlet_jm, bc.n_outlet), 32, 0, ctx.stream>>>(B, G, W, bc.outlet, bc.outlet_cu, cs);
-        k_outlet_fill<T><<<dim3((bc.max_outlet_im * bc.max_outlet_jm + 255) / 256, bc.n_outlet), 256, 0, ctx.stream>>>(B, P, W, bc.outlet);
+    const unsigned w = kBcThreads / 32;
+    const unsigned pin = (unsigned)(bc.max_inlet + kBcThreads - 1) / kBcThreads, prow = (unsigned)(bc.max_outlet_im + w - 1) / w,
+                   pline = (unsigned)(bc.max_outlet_jm + w - 1) / w, pwall = (unsigned)(bc.max_wall + kBcThreads - 1) / kBcThreads;
+    const unsigned nin = pin * bc.n_inlet, nrow = prow * bc.n_outlet, nline = pline * bc.n_outlet, nwall = pwall * bc.n_wall,
+                   nper = (unsigned)((bc.n_per + kBcThreads - 1) / kBcThreads);
+    auto first = [&](unsigned a, unsigned b, unsigned c) {
+        if (a + b + c) k_bc_first<T><<<a + b + c, kBcThreads, 0, ctx.stream>>>(B, P, G, W, bc, BcParts{{a, a + b, a + b + c}}, prow, pwall);
+    };
+    auto second = [&](unsigned a, unsigned b) {
+        if (a + b) k_bc_second<T><<<a + b, kBcThreads, 0, ctx.stream>>>(B, P, G, W, bc, BcParts{{a, a + b, a + b}}, pin, pline);
+    };
+    if (bc.apart) {
+        first(nrow, nwall, nper);
+        second(nin, nline);
+    } else {
+        second(nin, 0);
+        first(nrow, 0, 0);
+        second(0, nline);
+        first(0, nwall, 0);
+        first(0, 0, nper);
     }
-    if (bc.n_wall) k_bc_wall<T><<<dim3((bc.max_wall + 127) / 128, bc.n_wall), 128, 0, ctx.stream>>>(B, P, G, W, bc.wall);
-    if (bc.n_per)
-        k_bc_periodic<T><<<(unsigned)((bc.n_per + 255) / 256), 256, 0, ctx.stream>>>(B, W, bc.per_dst, bc.per_src, bc.per_meta,
-                                                                                   bc.per_trig, bc.n_per);
     if (W.ev) launch_sa_boundary<T>(ctx, P, W, bc);
     if (bc.n_mix) {
         k_mix_average<T><<<dim3(bc.max_mix_rows, bc.n_mix, 2), 32, 0, ctx.stream>>>(B, P, G, W, bc.mix, bc.max_mix_rows, bc.mix_avg);

@@ -50,6 +50,9 @@ struct BcTables {
     long long n_per = 0;
     int max_outlet_im = 0, max_outlet_jm = 0;
     double *outlet_cu = nullptr;                  // per outlet patch: mass-weighted swirl of each radial row
+    double2 *outlet_trig = nullptr;               // per outlet patch and face: sine and cosine of its polar angle
+    long long outlet_trig_stride = 0;
+    bool apart = false;                           // no ghost cell belongs to two of inlet, outlet, wall and periodic fills
     double *integ_part = nullptr;                 // per solve and section: kIntegralBlocks partial sums of 3
     unsigned *integ_count = nullptr;              // per solve: blocks of a launch that are done
     // Baldwin-Lomax wall distances (fine level): record w holds, for point n0 = 1..N-1 of each of
@@ -94,6 +97,8 @@ void wave_bytes(int fp64, int sa, WaveBytes &w);
 void launch_geometry(const LaunchCtx &ctx, const Geo &G, double *totalvol);
 // the periodic rotation's cosines and sines per solve (BcTables::per_trig), once at create
 void launch_periodic_trig(const LaunchCtx &ctx, double *trig);
+// the sines and cosines of the outlets' faces (BcTables::outlet_trig), once per level after the geometry
+void launch_outlet_trig(const LaunchCtx &ctx, const Geo &G, const BcTables &bc);
 
 template <typename T>
 void launch_boundary(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> F, const BcTables &bc);

@@ -174,7 +174,7 @@ template <typename T>
 void launch_resflux(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC, const Geo &G, const GeoW<T> &GW, Flow<T> W,
                     const BcTables &bc, int level, T *scratch)
 {
-    const int nbc = (bc.n_inlet > 0) + 3 * (bc.n_outlet > 0) + (bc.n_wall > 0) + (bc.n_per > 0);
+    const int nbc = bc.apart ? 2 : 5;
     ctx.mark("boundary", 1, nbc);
     launch_boundary<T>(ctx, P, G, W, bc);
     ctx.mark("boundary", 0, nbc);

@@ -655,6 +655,7 @@ public:
         timer.mark("sweep tiles", stream);
         launch_geometry(ctx(l), G, Lv.blockvol);
         k_case_volume<<<(nsolve + 127) / 128, 128, 0, stream>>>(batch(l), Lv.blockvol, Lv.totalvol);
+        launch_outlet_trig(ctx(l), G, Lv.bc);
         if (Lv.W.ev) build_sa_wall_distance(l);
         timer.mark("geometry", stream);
         build_geometry_working(l);
@@ -982,6 +983,50 @@ public:
                 }
             }
         }
+        // whether the ghost cells of inlets, outlets, walls and the gather list are all different ones (then
+        // the fills need no order among each other)
+        {
+            std::vector<unsigned char> owner((size_t)Lv.pool_n, 0);
+            bc.apart = true;
+            auto claim = [&](long long p, unsigned char who) {
+                if (owner[p] && owner[p] != who) bc.apart = false;
+                owner[p] = who;
+            };
+            // (every inlet, outlet and wall patch its own: two patches of a kind may not share a cell either)
+            unsigned char who = 1;
+            auto next = [&] { who = who == 250 ? 1 : who + 1; };
+            for (int s = 0; s < nsolve; s++) {
+                const Lvl &v = Lv.lv[s];
+                const LevelCase &c = lc[s];
+                for (auto &p : c.in) {
+                    next();
+                    for (int i = p.is; i <= p.ie; i++)
+                        for (int j = p.js; j <= p.je; j++)
+                            for (int nd = 0; nd <= P.ndummy; nd++) claim(ix(v, i, j, p.ks == 1 ? -nd : v.KM + nd), who);
+                }
+                for (size_t o = 0; o < c.out.size(); o++) {
+                    next();
+                    for (int i = 1; i <= v.IM - 1; i++)
+                        for (int j = 1; j <= v.JM - 1; j++)
+                            for (int nd = 0; nd <= P.ndummy; nd++) claim(ix(v, i, j, v.KM + nd), who);
+                }
+                for (auto &w : c.walls) {
+                    next();
+                    const int f = (w.face - 1) / 2;
+                    const bool lo = w.face % 2 == 1;
+                    const long long sn = f == 0 ? (long long)v.NJ * v.NK : (f == 1 ? (long long)v.NK : 1LL);
+                    for (int i = w.is; i <= w.ie; i++)
+                        for (int j = w.js; j <= w.je; j++)
+                            for (int k = w.ks; k <= w.ke; k++) {
+                                const long long p = ix(v, i, j, k), g = lo ? p - sn : p;
+                                for (int nd = 0; nd <= P.ndummy; nd++) claim(g + nd * (lo ? -sn : sn), who);
+                            }
+                }
+            }
+            for (long long d : pdst) claim(d, 251);
+            // (nor may the gather list read a cell that one of the fills writes)
+            for (long long p : psrc) if (owner[p]) bc.apart = false;
+        }
         // mixing planes of every case (applied last, source/BoundaryCondition.cpp:59-62)
         std::vector<DevMix> mixes;
         for (int cix = 0; cix < ncase; cix++) {
@@ -1003,6 +1048,7 @@ public:
                      bytes(outl1.size(), sizeof(DevInOut)) + bytes(walls.size(), sizeof(DevWall)) + bytes(pdst.size(), 8) * 2 +
                      bytes(pmeta.size(), 4) + bytes(outl.size() * (size_t)(bc.max_outlet_im + 1), 8) +
                      bytes((size_t)nsolve * 2 * kIntegralBlocks * 3, 8) + bytes((size_t)nsolve, 4) + bytes(sa_dst_h.size(), 8) * 2 +
+                     bytes(outl.size() * (size_t)bc.max_outlet_im * bc.max_outlet_jm, 16) +
                      bytes(mixes.size(), sizeof(DevMix)) + bytes(mixes.size() * (size_t)bc.max_mix_rows * kMixVals, 8) +
                      bytes((size_t)nsolve * 4, 8) + 256;
         CK(cudaMalloc(&Lv.tab_mem.p, tot));
@@ -1032,6 +1078,8 @@ public:
         bc.integ_part = (double *)up(nullptr, 0, 8); q += bytes((size_t)nsolve * 2 * kIntegralBlocks * 3, 8);
         const std::vector<unsigned> zeros(nsolve, 0);
         bc.integ_count = (unsigned *)up(zeros.data(), zeros.size(), 4);
+        bc.outlet_trig_stride = (long long)bc.max_outlet_im * bc.max_outlet_jm;
+        bc.outlet_trig = (double2 *)up(nullptr, 0, 16); q += bytes(outl.size() * (size_t)bc.outlet_trig_stride, 16);
         double *trig = (double *)up(nullptr, 0, 8); q += bytes((size_t)nsolve * 4, 8);
         bc.per_trig = trig;
         launch_periodic_trig(ctx(l), trig);
