@@ -70,6 +70,9 @@ struct BcTables {
     long long n_sa_gather = 0;
 };
 
+// where the integrals put an iteration's row of the history (12 values per case): row iter - *base
+struct HistorySink { double *out; const int *base; int rows, ncase; };
+
 constexpr int kIntegralBlocks = 32;             // blocks per inlet/outlet section in the integrals
 
 // The LU-SGS sweeps' tiles (wavefront.cu). A tile is a group of grid columns that a block marches
@@ -144,7 +147,7 @@ template <typename T>
 void launch_res_norm_static(const LaunchCtx &ctx, const Geo &G, Flow<T> F, const double *totalvol, int ncase, double *host_out);
 
 template <typename T>
-void launch_integrals(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> F, const BcTables &bc);
+void launch_integrals(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> F, const BcTables &bc, const HistorySink &hist);
 
 template <typename T>
 void launch_primitive(const LaunchCtx &ctx, const Phys &P, Flow<T> F);

@@ -307,7 +307,7 @@ void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> W, const double
 // with two powers per point, sums and powers of a solve on one thread, now 26.
 template <typename T>
 __global__ void __launch_bounds__(128) k_integrals(Batch B, Phys P, Geo G, Flow<T> W, const DevInOut *inl, const DevInOut *outl,
-                                                   double *part, unsigned *count)
+                                                   double *part, unsigned *count, HistorySink hist)
 {
     const int s = blockIdx.y, sec = blockIdx.z;
     // the section's block: the case's Inlet[1] / Outlet[1] may lie in any of its blocks
@@ -369,15 +369,24 @@ __global__ void __launch_bounds__(128) k_integrals(Batch B, Phys P, Geo G, Flow<
     st.m_in = mi; st.m_out = mo; st.pr = PR; st.eff = Ladk / Lk;
     st.m_ratio = fabs((mi - mo) / mi);
     if (!isfinite(mi) || !isfinite(mo)) st.status |= GBT_STATUS_NAN;
+    // the iteration's row of the history, by the case's first slot
+    const SolveConst &sc = B.sc[s];
+    const int row = st.iter - *hist.base;
+    if (sc.lead != s || row < 0 || row >= hist.rows) return;
+    double *r = hist.out + ((long long)row * hist.ncase + sc.cix) * 12;
+    r[0] = st.iter;
+    for (int c = 0; c < 5; c++) r[1 + c] = st.res[c];
+    r[6] = mi; r[7] = mo; r[8] = PR; r[9] = st.eff; r[10] = st.m_ratio;
+    r[11] = st.cfl;
 }
 
 template <typename T>
-void launch_integrals(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> W, const BcTables &bc)
+void launch_integrals(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> W, const BcTables &bc, const HistorySink &hist)
 {
     // first inlet and first outlet patch of every solve (the reference reports Inlet[1], Outlet[1])
     const Batch &B = ctx.batch;
     k_integrals<T><<<dim3(kIntegralBlocks, B.nsolve, 2), 128, 0, ctx.stream>>>(B, P, G, W, bc.inlet_first, bc.outlet_first,
-                                                                               bc.integ_part, bc.integ_count);
+                                                                               bc.integ_part, bc.integ_count, hist);
 }
 
 // CFL ramp of the driver (source/Solver.cpp:49-60): x1.2 whenever the density residual falls
@@ -403,7 +412,7 @@ void launch_cfl_ramp(const LaunchCtx &ctx, int iter)
     template void launch_primitive<T>(const LaunchCtx &, const Phys &, Flow<T>);                                       \
     template void launch_limiter<T>(const LaunchCtx &, const Phys &, Flow<T>, int, int *, int, int *);                 \
     template void launch_res_norm<T>(const LaunchCtx &, const Geo &, Flow<T>, const double *, double *, int, unsigned *);          \
-    template void launch_integrals<T>(const LaunchCtx &, const Phys &, const Geo &, Flow<T>, const BcTables &);
+    template void launch_integrals<T>(const LaunchCtx &, const Phys &, const Geo &, Flow<T>, const BcTables &, const HistorySink &);
 GBT_INST(double)
 GBT_INST(float)
 

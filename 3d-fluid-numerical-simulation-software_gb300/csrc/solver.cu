@@ -252,6 +252,23 @@ __global__ void __launch_bounds__(256) k_abs_res_partial(Batch B, const T *res0,
     if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = sh[0];
 }
 
+// Elements e0 .. e0 + n of a field as the caller gets it: the cells [i0, ...] x [j0, ...] x [k0, ...] of a box with
+// the components fastest, in FP64. src: the components' boxes, a set bit of fp32 for the working-precision
+// ones of the mixed form.
+constexpr int kPackComps = 18;
+struct PackList { const void *src[kPackComps]; unsigned fp32; int nc, i0, j0, k0, nj, nk, NJ, NK; };
+__global__ void __launch_bounds__(256) k_pack(PackList a, long long e0, long long n, double *out)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const unsigned long long e = (unsigned long long)(e0 + t);
+    const unsigned cell = (unsigned)(e / (unsigned)a.nc), c = (unsigned)(e - (unsigned long long)cell * (unsigned)a.nc);
+    const unsigned r = cell / (unsigned)a.nk;
+    const int k = a.k0 + (int)(cell - r * (unsigned)a.nk), j = a.j0 + (int)(r % (unsigned)a.nj), i = a.i0 + (int)(r / (unsigned)a.nj);
+    const long long p = ((long long)(i + PAD) * a.NJ + (j + PAD)) * a.NK + (k + PAD);
+    out[t] = (a.fp32 >> c & 1) ? (double)((const float *)a.src[c])[p] : ((const double *)a.src[c])[p];
+}
+
 // volume of a case: its blocks' volumes summed in block order (source/ComputeAllBlockVars.cpp:32)
 __global__ void k_case_volume(Batch B, const double *blockvol, double *casevol)
 {
@@ -325,6 +342,8 @@ public:
     const int norm_blk = 304;            // most blocks of a slot in the residual norm: two per SM
     unsigned *norm_count = nullptr;       // per case (its first slot): blocks of a launch that are done
     T *dtmin = nullptr;
+    DevBuf hist_mem;                      // rows of the history since *hist.base, brought back when they are full
+    HistorySink hist{};
     cudaGraphExec_t graphs[3] = {nullptr, nullptr, nullptr};
     int phase_runs[3] = {0, 0, 0};        // iterations run in each driver phase (graphs: see iterate)
 
@@ -517,6 +536,14 @@ public:
         norm_count = (unsigned *)q; q += sizeof(unsigned) * nsolve;
         CK(cudaMemset(norm_count, 0, sizeof(unsigned) * nsolve));
         dtmin = (T *)(((uintptr_t)q + 15) & ~(uintptr_t)15);
+        // 256 rows of history, fewer for very large batches (about 4 MB)
+        hist.ncase = ncase;
+        hist.rows = (int)std::max<long long>(1, std::min<long long>(256, (4LL << 20) / (96LL * ncase)));
+        hist_mem.bytes = sizeof(double) * 12 * (size_t)hist.rows * ncase + 256;
+        CK(cudaMalloc(&hist_mem.p, hist_mem.bytes));
+        CK(cudaMemset(hist_mem.p, 0, hist_mem.bytes));
+        hist.base = (const int *)hist_mem.p;
+        hist.out = (double *)((char *)hist_mem.p + 256);
         timer.mark("solve state and scratch", stream);
         for (int l = 1; l <= ng; l++) build_level(l);
     }
@@ -525,6 +552,8 @@ public:
     {
         for (auto &g : graphs) if (g) cudaGraphExecDestroy(g);
         for (auto &e : ev_pool) cudaEventDestroy(e);
+        for (auto &e : pin_done) if (e) cudaEventDestroy(e);
+        if (pin) cudaFreeHost(pin);
         if (stream) { cudaStreamSynchronize(stream); cudaStreamDestroy(stream); }
     }
 
@@ -1185,7 +1214,7 @@ public:
         launch_interpolate<T>(ctx(1), ctx(2), lev[1].W, lev[2].W, init);
     }
     void delta_cons() override { need_mg(); Mark m(this, "mg_delta"); launch_delta<T>(ctx(2), lev[2].W); }
-    void integrals(int l) override { Mark m(this, "integrals", 1); launch_integrals<T>(ctx(l), P, lev[l].G, lev[l].W, lev[l].bc); }
+    void integrals(int l) override { Mark m(this, "integrals", 1); launch_integrals<T>(ctx(l), P, lev[l].G, lev[l].W, lev[l].bc, hist); }
     void set_use_force(int l, bool on) override { lev[l].use_force = on; }
     void need_mg() const { if (ng < 2) throw std::runtime_error("the case runs on a single grid level"); }
 
@@ -1264,11 +1293,24 @@ public:
     }
 
     // the driver loop (source/Structured_FV3D.cpp:142-219): step + integrals, one graph per phase
-    void iterate(int n, double *hist) override
+    void iterate(int n, double *hist_out) override
     {
-        std::vector<SolveState> st(nsolve);
+        // the rows stay on the device while the iterations run (a copy and a wait after each left the GPU
+        // idle for 15 to 25 us) and come back together
+        int base = 0, kept = 0;
+        auto bring = [&](int q) {
+            if (!hist_out || kept == 0) return;
+            CK(cudaMemcpyAsync(hist_out + (size_t)(q - kept) * ncase * 12, hist.out, sizeof(double) * 12 * (size_t)kept * ncase,
+                               cudaMemcpyDeviceToHost, stream));
+            CK(cudaStreamSynchronize(stream));
+            kept = 0;
+        };
         for (int q = 0; q < n; q++) {
             iter++;
+            if (hist_out && kept == 0) {
+                base = iter;
+                CK(cudaMemcpyAsync((void *)hist.base, &base, sizeof(int), cudaMemcpyHostToDevice, stream));
+            }
             int ph = phase();
             // a phase graph fixes the reporting level it was captured with: a restarted multigrid
             // case reports the coarse level for its first iterations, which therefore run eagerly
@@ -1296,19 +1338,9 @@ public:
                 integrals(report_level());
                 mass_flow_imposed();
             }
-            if (hist) {
-                CK(cudaMemcpyAsync(st.data(), st_d, sizeof(SolveState) * nsolve, cudaMemcpyDeviceToHost, stream));
-                CK(cudaStreamSynchronize(stream));
-                for (int cix = 0; cix < ncase; cix++) {
-                    const SolveState &a = st[case_first[cix]];
-                    double *r = hist + ((size_t)q * ncase + cix) * 12;
-                    r[0] = a.iter;
-                    for (int c = 0; c < 5; c++) r[1 + c] = a.res[c];
-                    r[6] = a.m_in; r[7] = a.m_out; r[8] = a.pr; r[9] = a.eff; r[10] = a.m_ratio;
-                    r[11] = a.cfl;
-                }
-            }
+            if (hist_out && ++kept == hist.rows) bring(q + 1);
         }
+        bring(n);
         CK(cudaGetLastError());
     }
 
@@ -1345,25 +1377,66 @@ public:
 
     // a box [i0,i1]x[j0,j1]x[k0,k1] of several component arrays, components fastest
     struct Comp { const double *d; const T *t; };
-    long box(const Lvl &v, const std::vector<Comp> &cs, int i0, int i1, int j0, int j1, int k0, int k1, double *out, long cap)
+    long box(int l, const Lvl &v, const std::vector<Comp> &cs, int i0, int i1, int j0, int j1, int k0, int k1, double *out, long cap)
     {
-        long n = (long)(i1 - i0 + 1) * (j1 - j0 + 1) * (k1 - k0 + 1) * (long)cs.size();
+        const long n = (long)(i1 - i0 + 1) * (j1 - j0 + 1) * (k1 - k0 + 1) * (long)cs.size();
         if (n > cap) return -1;
-        std::vector<std::vector<double>> h(cs.size());
-        for (size_t c = 0; c < cs.size(); c++) {
-            if (cs[c].d) fetch(cs[c].d, v, h[c]);
-            else fetch(cs[c].t, v, h[c]);
+        if (cs.size() > (size_t)kPackComps) throw std::runtime_error("too many components");
+        // packed on the device straight into pinned host memory, piece by piece, a piece copied to the caller's
+        // (often untouched) pages by several threads while the next one is packed. One thread that fetched the
+        // boxes one by one and interleaved them took 2.3 ms for the primitive variables of the 129x49x49
+        // passage and 16 ms for those of 32 solves of 25x25x65 nodes, a plain copy into pageable memory 4.2
+        // and 5.3 ms; now 0.9 and 5.9 (from Python, the array it makes included).
+        PackList a{};
+        a.nc = (int)cs.size();
+        for (int c = 0; c < a.nc; c++) {
+            a.src[c] = cs[c].d ? (const void *)(cs[c].d + v.base) : (const void *)(cs[c].t + v.base);
+            if (!cs[c].d && sizeof(T) == 4) a.fp32 |= 1u << c;
         }
-        long q = 0;
-        Lvl z = v;
-        z.base = 0;
-        for (int i = i0; i <= i1; i++)
-            for (int j = j0; j <= j1; j++)
-                for (int k = k0; k <= k1; k++) {
-                    long long p = ix(z, i, j, k);
-                    for (size_t c = 0; c < cs.size(); c++) out[q++] = h[c][(size_t)p];
-                }
+        a.i0 = i0; a.j0 = j0; a.k0 = k0; a.nj = j1 - j0 + 1; a.nk = k1 - k0 + 1; a.NJ = v.NJ; a.NK = v.NK;
+        pinned();
+        const long most = kPinned / 2;
+        long got = 0, had = 0;                       // elements packed, copied
+        for (int q = 0; had < n; q++) {
+            long m = 0;
+            if (got < n) {
+                m = std::min(most, n - got);
+                k_pack<<<(unsigned)((m + 255) / 256), 256, 0, stream>>>(a, got, m, pin_dev + (q & 1) * most);
+                CK(cudaGetLastError());
+                CK(cudaEventRecord(pin_done[q & 1], stream));
+            }
+            if (q > 0) {
+                const long last = std::min(most, n - had);
+                CK(cudaEventSynchronize(pin_done[(q - 1) & 1]));
+                copy_out(out + had, pin + ((q - 1) & 1) * most, last);
+                had += last;
+            }
+            got += m;
+        }
         return n;
+    }
+    // pinned memory of the downloads (elements), allocated by the first one
+    static constexpr long kPinned = 2 << 20;
+    double *pin = nullptr, *pin_dev = nullptr;
+    cudaEvent_t pin_done[2] = {nullptr, nullptr};
+    void pinned()
+    {
+        if (pin) return;
+        for (auto &e : pin_done) if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        CK(cudaHostAlloc(&pin, sizeof(double) * kPinned, cudaHostAllocMapped));
+        CK(cudaHostGetDevicePointer(&pin_dev, pin, 0));
+    }
+    static void copy_out(double *dst, const double *src, long n)
+    {
+        const long per = 1 << 17;                    // a megabyte per thread
+        const long nt = std::min<long>({(n + per - 1) / per, 8, (long)std::max(1u, std::thread::hardware_concurrency())});
+        if (nt <= 1) { std::memcpy(dst, src, sizeof(double) * n); return; }
+        std::vector<std::thread> pool;
+        const long step = (n + nt - 1) / nt;
+        for (long t = 1; t < nt; t++)
+            pool.emplace_back([=] { std::memcpy(dst + t * step, src + t * step, sizeof(double) * std::max(0L, std::min(step, n - t * step))); });
+        std::memcpy(dst, src, sizeof(double) * std::min(step, n));
+        for (auto &t : pool) t.join();
     }
 
     long get_field(int solve, int l, const std::string &name, double *out, long cap) override
@@ -1377,41 +1450,41 @@ public:
         auto D = [](const double *p) { return Comp{p, nullptr}; };
         auto Tt = [](const T *p) { return Comp{nullptr, p}; };
         std::vector<Comp> cs;
-        if (name == "cv") { for (int c = 0; c < 5; c++) cs.push_back(D(W.cv[c])); return box(v, cs, 0, IM, 0, JM, 0, KM, out, cap); }
-        if (name == "pv") { for (int c = 0; c < 6; c++) cs.push_back(Tt(W.pv[c])); return box(v, cs, 0, IM, 0, JM, 0, KM, out, cap); }
-        if (name == "mut") return box(v, {Tt(W.mut)}, 0, IM, 0, JM, 0, KM, out, cap);
+        if (name == "cv") { for (int c = 0; c < 5; c++) cs.push_back(D(W.cv[c])); return box(l, v, cs, 0, IM, 0, JM, 0, KM, out, cap); }
+        if (name == "pv") { for (int c = 0; c < 6; c++) cs.push_back(Tt(W.pv[c])); return box(l, v, cs, 0, IM, 0, JM, 0, KM, out, cap); }
+        if (name == "mut") return box(l, v, {Tt(W.mut)}, 0, IM, 0, JM, 0, KM, out, cap);
         if (name == "ev" || name == "res_ev" || name == "dwall") {
             if (!W.ev) return -1;                  // Spalart-Allmaras cases, fine level
-            if (name == "ev") return box(v, {D(W.ev)}, 0, IM, 0, JM, 0, KM, out, cap);
-            if (name == "res_ev") return box(v, {Tt(W.res_ev)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
-            return box(v, {D(W.dwall)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+            if (name == "ev") return box(l, v, {D(W.ev)}, 0, IM, 0, JM, 0, KM, out, cap);
+            if (name == "res_ev") return box(l, v, {Tt(W.res_ev)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+            return box(l, v, {D(W.dwall)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
         }
-        if (name == "res") { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.res[c])); return box(v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap); }
-        if (name == "dq") { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.dq[c])); return box(v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap); }
-        if (name == "dt") return box(v, {Tt(W.dt)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
-        if (name == "omega") return box(v, {Tt(W.omega)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+        if (name == "res") { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.res[c])); return box(l, v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap); }
+        if (name == "dq") { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.dq[c])); return box(l, v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap); }
+        if (name == "dt") return box(l, v, {Tt(W.dt)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+        if (name == "omega") return box(l, v, {Tt(W.omega)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
         const char *lam[6] = {"lamcI", "lamcJ", "lamcK", "lamvI", "lamvJ", "lamvK"};
         for (int q = 0; q < 6; q++)
-            if (name == lam[q]) return box(v, {Tt(q < 3 ? W.lamc[q] : W.lamv[q - 3])}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+            if (name == lam[q]) return box(l, v, {Tt(q < 3 ? W.lamc[q] : W.lamv[q - 3])}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
         const char *fcn[3] = {"FcI", "FcJ", "FcK"}, *fvn[3] = {"FvI", "FvJ", "FvK"}, *gn[3] = {"faceI", "faceJ", "faceK"};
         for (int f = 0; f < 3; f++) {
             int i1 = f == 0 ? IM : IM - 1, j1 = f == 1 ? JM : JM - 1, k1 = f == 2 ? KM : KM - 1;
-            if (name == fcn[f]) { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.Ff[f][c])); return box(v, cs, 1, i1, 1, j1, 1, k1, out, cap); }
-            if (name == fvn[f]) { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.Vf[f][c])); return box(v, cs, 1, i1, 1, j1, 1, k1, out, cap); }
+            if (name == fcn[f]) { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.Ff[f][c])); return box(l, v, cs, 1, i1, 1, j1, 1, k1, out, cap); }
+            if (name == fvn[f]) { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.Vf[f][c])); return box(l, v, cs, 1, i1, 1, j1, 1, k1, out, cap); }
             if (name == gn[f]) {
                 for (int c = 0; c < 3; c++) cs.push_back(D(G.S[f][c]));
                 cs.push_back(D(G.s[f]));
                 for (int c = 0; c < 3; c++) cs.push_back(D(G.c[f][c]));
                 cs.push_back(D(G.r[f])); cs.push_back(D(G.th[f]));
                 for (int c = 0; c < 9; c++) cs.push_back(D(G.m[f][c]));
-                return box(v, cs, 1, i1, 1, j1, 1, k1, out, cap);
+                return box(l, v, cs, 1, i1, 1, j1, 1, k1, out, cap);
             }
         }
         if (name == "cell") {
             cs.push_back(D(G.vol));
             for (int c = 0; c < 3; c++) cs.push_back(D(G.cc[c]));
             for (int c = 0; c < 9; c++) cs.push_back(D(G.cm[c]));
-            return box(v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+            return box(l, v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
         }
         if (name == "totalvol") {
             if (cap < 1) return -1;

@@ -316,7 +316,7 @@ class Solver:
     def get(self, name: str, solve: int = 0, level: int = 1) -> np.ndarray:
         I, J, K, _ = self.dims(solve, level)
         shape = FIELD_SHAPES[name](I, J, K)
-        out = np.zeros(int(np.prod(shape)))
+        out = np.empty(int(np.prod(shape)))       # (every element is written, or the call fails)
         n = self._L.gb_get_field(self.h, solve, level, name.encode(), _dp(out), out.size)
         if n < 0:
             raise GBError(self._L.gb_last_error().decode())
