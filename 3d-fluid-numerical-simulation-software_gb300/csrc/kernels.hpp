@@ -94,7 +94,7 @@ struct WaveTables {
 };
 // columns of a tile in i and j; bytes of a step's blocks (fp64: working type; sa: with the
 // Spalart-Allmaras variable)
-void wave_patch(int &pa, int &pb);
+void wave_patch(int fp64, int &pa, int &pb);
 void wave_bytes(int fp64, int sa, WaveBytes &w);
 
 void launch_geometry(const LaunchCtx &ctx, const Geo &G, double *totalvol);

@@ -819,7 +819,7 @@ public:
         WaveTables &V = Lv.wave;
         const bool sa = P.turb_sa && l == 1;
         int pa, pb;
-        wave_patch(pa, pb);
+        wave_patch(sizeof(T) == 8, pa, pb);
         WaveBytes w;
         wave_bytes(sizeof(T) == 8, sa, w);
         std::vector<WaveSolve> sol;

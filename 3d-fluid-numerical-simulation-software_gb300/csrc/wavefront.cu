@@ -4,18 +4,19 @@
 //
 // What bounds it: the chain of i + j + k planes, not the arithmetic or the bytes. One kernel launch per
 // plane (programmatic dependent launches, neighbours re-read through L2) cost 1.8 us per plane in FP32 and
-// 3.4 us in FP64. Here a block owns a tile of 4 x 8 grid columns (i, j) and marches it along k skewed: at
+// 3.4 us in FP64. Here a block owns a tile of 4 x 8 grid columns (i, j; 2 x 8 in FP64) and marches it along k skewed: at
 // step t the column (a, b) of the tile is at k = t - a - b, so that the terms it needs from inside the
 // tile are the ones its neighbours formed one step earlier, and a step costs the block one barrier. Tiles
 // run side by side on as many SMs as there are, each a few steps behind the two it reads from.
 //
 // What a step costs is the number of instructions one warp issues (a lone warp of a sub-partition issues
 // one every three to four cycles, and an FP64 instruction holds its sub-partition for some 70): with a
-// lane per cell a step took 337 instructions and 1.3k cycles in FP32. So four lanes share a cell, four
-// warps a step, and everything that is not the cell's arithmetic is done by two further warps of the
-// block:
-//   lane q of a cell   receives component q (and the fifth); lanes 0..2 form the term of direction q, and
-//                      lane 3 the pressure, with the instructions with which the others form their V_n
+// lane per cell a step took 337 instructions and 1.3k cycles in FP32. So four lanes share a cell (eight in
+// FP64, 26 FP64 instructions a step where four lanes took 38), four warps a step, and everything that is
+// not the cell's arithmetic is done by two further warps of the block:
+//   a cell's lanes     receive a component each (FP32: and the fifth); lanes 0..2 form the terms of a direction
+//                      each (FP64: with lanes 4..6, which take its last two components), and lane 3 the
+//                      pressure, with the instructions with which the others form their V_n
 //   the incoming warp  reads the terms that cross into the tile and puts them beside the tile's own
 //   the outgoing warp  sends the terms that leave it and fetches the inputs of later steps
 //
@@ -50,7 +51,11 @@ namespace gbt {
 
 namespace {
 
-constexpr int PA = 4, PB = 8, NC = PA * PB;     // columns of a tile in i and j
+// columns of a tile in i and j, lanes of a cell: 128 lanes a step in both precisions
+constexpr int PB = 8;
+template <typename T> constexpr int kPA = sizeof(T) == 4 ? 4 : 2;
+template <typename T> constexpr int kCells = kPA<T> * PB;
+template <typename T> constexpr int kLanes = 128 / kCells<T>;
 constexpr int kGroup = 2, kStages = 3;          // steps of a stage of the input ring, stages
 constexpr int kSlots = kGroup * kStages;        // steps whose terms are kept: the outgoing warp fetches a stage
                                                 // after it has sent the steps that used it, so a step's terms
@@ -58,18 +63,20 @@ constexpr int kSlots = kGroup * kStages;        // steps whose terms are kept: t
 constexpr int kAhead = 4;                       // steps that the incoming warp asks ahead
 constexpr unsigned kWaitLimit = 1u << 21;       // polls of a wait before it gives up (seconds)
 constexpr int kSteps32 = 16;                    // steps of a block of the FP32 gather kernel
+template <typename T> constexpr int kSteps = 256 / kCells<T>;                   // of the kernels with a thread per cell
 
 // bytes of a step's blocks, packets of an edge cell and of a step
 //   FP32: geo {n_d, V_entrainment,d} at 3 cell + d; flow {h_d, c_d} at 3 cell + d of the forward sweep, {rho, m},
 //         {rho E, p, 1/rho, 0} per cell, {h_d, c_d} of the backward sweep (a sweep copies its own end and the
 //         middle); packets {w_1, w_2, w_3, tag}, {w_4, w_5, 0, tag}
-//   FP64: geo {n_1, n_2}, {n_3, V_entrainment} at 3 cell + d; flow {h_d, c_d} of the forward sweep, {f_1, f_2},
-//         {f_3, f_4}, f_5 at 3 cell + d, Q_1..Q_4, Q_5 per cell, {h_d, c_d} of the backward sweep; packets {w_c, tag}
+//   FP64: geo {n_1, n_2}, {n_3, V_entrainment} at 3 cell + d; flow {h_d, c_d} of the forward sweep, f_1, .., f_5
+//         at 3 cell + d, Q_1..Q_4, Q_5 per cell, {h_d, c_d} of the backward sweep; packets {w_c, tag}
 //   dq:   component q at 4 cell + q, the fifth per cell: the right-hand side, then dQ
 //   the variable's sweep: flow V_d, ev V_old,d, |S_d|, relax lambda_c,d, lambda_v,d at 3 cell + d, ev, alpha per cell;
 //         dq one value per cell; packets {A term, V term, 0, tag} in FP32, one {value, tag} each in FP64
 enum Kind { MEAN, VAR };
 template <typename T, Kind K> struct Lay {
+    static constexpr int PA = kPA<T>, NC = kCells<T>;
     static constexpr int B = sizeof(T), CA = K == VAR ? 2 : 4, CB = K == VAR ? 0 : 1, NV = CA + CB;   // values of a term
     static constexpr int geo = K == VAR ? 0 : 12 * NC * B;
     static constexpr int ends = K == MEAN ? 6 * NC * B : 0;                  // of the flow block, one sweep's own
@@ -179,6 +186,7 @@ template <int DIR> struct CellStep<float, DIR, MEAN> {
     {
         return __fmaf_rn(a2, b2, __fmaf_rn(a0, b0, __fmul_rn(a1, b1)));
     }
+    static constexpr int NC = L::NC;
     static __device__ __forceinline__ void run(const char *in, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
                                                int w_off4, bool active, float gm1, char *dq_out)
     {
@@ -227,57 +235,50 @@ template <int DIR> struct CellStep<float, DIR, MEAN> {
 
 template <int DIR> struct CellStep<double, DIR, MEAN> {
     using L = Lay<double, MEAN>;
+    static constexpr int NC = L::NC;
     static __device__ __forceinline__ void run(const char *in, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
                                                int w_off4, bool active, double gm1, char *dq_out)
     {
-        const int e = 3 * cell + (q < 3 ? q : 0);
+        const int d = q & 3, c = q < 4 ? q : 4, e = 3 * cell + (d < 3 ? d : 0);     // direction, component received
+        const bool low = q < 4;                      // components 1..3 of the direction's term, or 4 and 5
         const double2 *g = (const double2 *)in + e;
         const char *own = in + L::geo + (DIR > 0 ? 0 : L::flow_in - L::ends), *mid = in + L::geo + (DIR > 0 ? L::ends : 0);
-        const double2 *f = (const double2 *)mid + e;
-        const double *c = (const double *)mid + 15 * NC, *fq = (const double *)(in + L::geo + L::flow_in);
-        const double2 g0 = g[0], g1 = g[3 * NC], hc = ((const double2 *)own)[e], f0 = f[0], f1 = f[3 * NC];
-        const double f4 = ((const double *)mid)[12 * NC + e], oq = c[4 * cell + q], o4 = c[4 * NC + cell];
-        const double rq = fq[4 * cell + q], r4 = fq[4 * NC + cell];
+        const double *f = (const double *)mid + (low ? 0 : 9 * NC) + e, *oc = (const double *)mid + 15 * NC + (low ? 4 * cell + c : 4 * NC + cell),
+                     *rc = (const double *)(in + L::geo + L::flow_in) + (low ? 4 * cell + c : 4 * NC + cell);
+        const double2 g0 = g[0], g1 = g[3 * NC], hc = ((const double2 *)own)[e];
+        const double fa = f[0], fb = f[3 * NC], fc = low ? f[6 * NC] : 0.0, o = *oc, r = *rc;
         // received
-        const double sq = __dadd_rn(__dadd_rn(((const double *)(rd + r_off[0]))[q], ((const double *)(rd + r_off[2]))[q]),
-                                    ((const double *)(rd + L::KA))[4 * cell + q]);
-        const double s4 = __dadd_rn(__dadd_rn(((const double *)(rd + r_off[1]))[0], ((const double *)(rd + r_off[3]))[0]),
-                                    ((const double *)(rd + L::KB))[cell]);
-        double dqq = DIR > 0 ? __dadd_rn(rq, sq) : __dadd_rn(rq, -sq), dq4 = DIR > 0 ? __dadd_rn(r4, s4) : __dadd_rn(r4, -s4);
-        if (!active) dqq = dq4 = 0.0;
-        const double nq = __dadd_rn(oq, dqq), ne = __dadd_rn(o4, dq4);
-        const unsigned quad = (threadIdx.x & 31) & ~3u;
-        double d[4], n[4];
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            d[m] = __shfl_sync(0xffffffffu, dqq, quad + m);
-            n[m] = __shfl_sync(0xffffffffu, nq, quad + m);
+        const double s = __dadd_rn(__dadd_rn(*(const double *)(rd + r_off[0]), *(const double *)(rd + r_off[1])), *(const double *)(rd + r_off[2]));
+        const double x = __dadd_rn(r, DIR > 0 ? s : -s), dq = active ? x : 0.0, nq = __dadd_rn(o, dq);
+        const unsigned oct = (threadIdx.x & 31) & ~7u;
+        auto from = [&](double v, int lane) { return __shfl_sync(0xffffffffu, v, oct + lane); };
+        const double n0 = from(nq, 0), n1 = from(nq, 1), n2 = from(nq, 2), n3 = from(nq, 3), n4 = from(nq, 4);
+        const double da = from(dq, low ? 0 : 3), db = from(dq, low ? 1 : 4), dc = from(dq, 2);
+        const double inv = rcp_nr(n0);
+        // lanes 0..2 of a half: V_n - ve; lane 3: p = (gamma - 1)(rho E - |m|^2 / (2 rho))
+        const double mm = fma(n3, d < 3 ? g1.x : n3, fma(n1, d < 3 ? g0.x : n1, __dmul_rn(n2, d < 3 ? g0.y : n2)));
+        const double dn = fma(mm, inv, d < 3 ? -g1.y : -0.0);
+        const double pn = from(__dmul_rn(gm1, fma(-0.5, dn, n4)), 3), ep = __dadd_rn(n4, pn);
+        auto term = [&](double n, double y, double v) {
+            const double w = __dmul_rn(hc.y, v);
+            return fma(hc.x, fma(n, dn, y), DIR > 0 ? w : -w);
+        };
+        const double y = fma(pn, g1.x, -fa);
+        const double ta = term(low ? n0 : n3, low ? -fa : y, da), tb = term(low ? n1 : ep, fma(pn, low ? g0.x : g1.y, -fb), db),
+                     tc = term(n2, fma(pn, g0.y, -fc), dc);
+        if (d < 3) {
+            double *w = (double *)(wr + w_off);
+            if (low) { *(double2 *)w = make_double2(ta, tb); w[2] = tc; }
+            else { w[3] = ta; *(double *)(wr + w_off4) = tb; }
         }
-        const double inv = rcp_nr(n[0]);
-        // lanes 0..2: V_n - ve; lane 3: p = (gamma - 1)(rho E - |m|^2 / (2 rho))
-        const double mm = fma(n[3], q < 3 ? g1.x : n[3], fma(n[1], q < 3 ? g0.x : n[1], __dmul_rn(n[2], q < 3 ? g0.y : n[2])));
-        const double t = fma(mm, inv, q < 3 ? -g1.y : -0.0);
-        const double pr = __dmul_rn(gm1, fma(-0.5, t, ne));
-        const double dn = t, pn = __shfl_sync(0xffffffffu, pr, quad + 3);
-        auto term = [&](double dF, double dd) { return fma(hc.x, dF, DIR > 0 ? __dmul_rn(hc.y, dd) : -__dmul_rn(hc.y, dd)); };
-        const double s0 = term(fma(n[0], dn, -f0.x), d[0]), s1 = term(fma(n[1], dn, fma(pn, g0.x, -f0.y)), d[1]),
-                     s2 = term(fma(n[2], dn, fma(pn, g0.y, -f1.x)), d[2]), s3 = term(fma(n[3], dn, fma(pn, g1.x, -f1.y)), d[3]),
-                     t4 = term(fma(__dadd_rn(ne, pn), dn, fma(pn, g1.y, -f4)), dq4);
-        if (q < 3) {
-            double2 *o = (double2 *)(wr + w_off);
-            o[0] = make_double2(s0, s1);
-            o[1] = make_double2(s2, s3);
-            *(double *)(wr + w_off4) = t4;
-        }
-        double *out = (double *)dq_out;
-        out[4 * cell + q] = dqq;
-        if (q == 0) out[4 * NC + cell] = dq4;
+        if (q < 5) ((double *)dq_out)[low ? 4 * cell + c : 4 * NC + cell] = dq;
     }
 };
 
 // the variable's sweep: A terms of the three directions, then V terms, then the division
 template <typename T, int DIR> struct CellStep<T, DIR, VAR> {
     using L = Lay<T, VAR>;
+    static constexpr int NC = L::NC;
     static __device__ __forceinline__ T add(T a, T b) { if constexpr (sizeof(T) == 4) return __fadd_rn(a, b); else return __dadd_rn(a, b); }
     static __device__ __forceinline__ T mul(T a, T b) { if constexpr (sizeof(T) == 4) return __fmul_rn(a, b); else return __dmul_rn(a, b); }
     static __device__ __forceinline__ void run(const char *in, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
@@ -304,6 +305,7 @@ template <typename T, int DIR, Kind K>
 __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, WaveTables V, T gm1)
 {
     using L = Lay<T, K>;
+    constexpr int PA = L::PA, NC = L::NC;
     extern __shared__ __align__(128) char smem[];
     __shared__ unsigned s_take[2];
     const unsigned base = (unsigned)__cvta_generic_to_shared(smem);
@@ -324,23 +326,29 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
     const bool edges = w.has_i || w.has_j;
     bool ok = true;
     if (warp < 4) {
-        const int a = warp, b = lane >> 2, q = lane & 3, cell = a * PB + b;
+        const int cell = threadIdx.x / kLanes<T>, q = threadIdx.x % kLanes<T>, a = cell / PB, b = cell % PB;
         const bool column = w.PI * PA + a < w.S.nI && w.PJ * PB + b < w.S.nJ;
         constexpr int F = DIR > 0 ? 1 : 0;          // forward: halo first
-        const int r_off[4] = {off_ia<L>(a + 1 - F, b), off_ib<L>(a + 1 - F, b), off_ja<L>(a, b + 1 - F),
-                              off_jb<L>(a, b + 1 - F)};
-        const int w_off = q == 0 ? off_ia<L>(a + F, b) : q == 1 ? off_ja<L>(a, b + F) : L::KA + L::CA * cell * L::B;
-        const int w_off4 = q == 0 ? off_ib<L>(a + F, b) : q == 1 ? off_jb<L>(a, b + F)
-                                                                  : L::KB + L::CB * cell * L::B;
+        // terms read: FP64, component q (or the fifth) of the three directions; otherwise both groups of I and J
+        int r_off[4] = {off_ia<L>(a + 1 - F, b), off_ib<L>(a + 1 - F, b), off_ja<L>(a, b + 1 - F), off_jb<L>(a, b + 1 - F)};
+        if (sizeof(T) == 8 && K == MEAN) {
+            const bool low = q < 4;
+            r_off[0] = low ? r_off[0] + 8 * q : r_off[1];
+            r_off[1] = low ? r_off[2] + 8 * q : r_off[3];
+            r_off[2] = low ? L::KA + 8 * (4 * cell + q) : L::KB + 8 * cell;
+        }
+        const int dir = sizeof(T) == 8 ? q & 3 : q;
+        const int w_off = dir == 0 ? off_ia<L>(a + F, b) : dir == 1 ? off_ja<L>(a, b + F) : L::KA + L::CA * cell * L::B;
+        const int w_off4 = dir == 0 ? off_ib<L>(a + F, b) : dir == 1 ? off_jb<L>(a, b + F) : L::KB + L::CB * cell * L::B;
         char *dq = V.dq + (w.step0 + (DIR > 0 ? 0 : T_ - 1)) * L::dq;
         int k = (DIR > 0 ? 0 : T_ - 1) - a - b;
+        unsigned ph = 0;
         int slot = 0, stage = 0;
-        unsigned ph = 0, sph = 0;
         const char *rd = terms + (kSlots - 1) * L::slot;
         for (int n = 0; n < T_; n += kGroup) {
-            bar_wait(full + 8 * stage, sph, ok);
+            bar_wait(full + 8 * stage, ph, ok);
             const char *in = smem + stage * kGroup * L::step;
-            // (a stage holds its steps in order of t)
+            // (a stage holds its steps in order of t; the last one may hold fewer)
             const int cnt = min(kGroup, T_ - n);
 #pragma unroll
             for (int u = 0; u < kGroup; u++) {
@@ -348,15 +356,15 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
                 if (edges) bar_wait(edge + 8 * slot, ph, ok);
                 char *wr = terms + slot * L::slot;
                 CellStep<T, DIR, K>::run(in + (DIR > 0 ? u : cnt - 1 - u) * L::step, rd, wr, cell, q, r_off, w_off, w_off4,
-                                          column && k >= 0 && k < w.S.nK, gm1, dq);
+                                         column && (unsigned)k < (unsigned)w.S.nK, gm1, dq);
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (threadIdx.x == 0) bar_arrive(done + 8 * slot);
                 rd = wr;
                 k += DIR;
                 dq += DIR * L::dq;
-                if (++slot == kSlots) { slot = 0; ph ^= 1; }
+                slot++;
             }
-            if (++stage == kStages) { stage = 0; sph ^= 1; }
+            if (++stage == kStages) { stage = slot = 0; ph ^= 1; }
         }
     } else if (warp == 4) {
         if (!edges) return;
@@ -539,9 +547,10 @@ __device__ __forceinline__ void next_sweep(const WaveTables &V)
 // shared memory. Bound by the latency of its loads, some 30 per cell: with 32 steps and four cells per
 // thread one after another it took 43 us on the 129x49x49 passage and 168 us per cycle on 32 solves of
 // 25x25x65 nodes, one cell per thread 15 and 64 (40 for the bytes of the latter).
-__global__ void __launch_bounds__(NC * kSteps32) k_wave_gather32(Batch B, PhysW<float> P, Flow<float> W, WaveTables V)
+__global__ void __launch_bounds__(kCells<float> * kSteps32) k_wave_gather32(Batch B, PhysW<float> P, Flow<float> W, WaveTables V)
 {
     using L = Lay<float, MEAN>;
+    constexpr int PA = L::PA, NC = L::NC;
     constexpr int NF = L::flow / 16, ND = L::dq / 16, stride = NF + ND + 1;      // quads per step, and in shared memory
     extern __shared__ __align__(128) char smem[];
     float4 *tile = (float4 *)smem;
@@ -598,20 +607,20 @@ __global__ void __launch_bounds__(NC * kSteps32) k_wave_gather32(Batch B, PhysW<
     for (int e = threadIdx.x; e < c.nt * ND; e += NC * kSteps32) dd[e] = tile[(e / ND) * stride + NF + e % ND];
 }
 
-// FP64: one thread per cell and step, eight steps per block (a 32-byte sector of a column's row serves four
-// of them from L1). Bound by its FP64 instructions, some 75 per cell.
+// FP64: one thread per cell and step, 16 steps per block (a line of a column's row serves them from L1). Bound by its FP64 instructions, some 75 per cell.
 __global__ void __launch_bounds__(256) k_wave_gather64(Batch B, PhysW<double> P, Flow<double> W, WaveTables V)
 {
     using L = Lay<double, MEAN>;
+    constexpr int PA = L::PA, NC = L::NC;
     next_sweep(V);
-    const Chunk c = chunk_of(V, 8);
-    const int cell = threadIdx.x & 31, st = threadIdx.x >> 5, a = cell / PB, b = cell % PB;
+    const Chunk c = chunk_of(V, kSteps<double>);
+    const int cell = threadIdx.x % NC, st = threadIdx.x / NC, a = cell / PB, b = cell % PB;
     if (!c.live || st >= c.nt) return;
     const Lvl Lv = B.lv[blockIdx.y];
     const int i = c.PI * PA + a + 1, j = c.PJ * PB + b + 1, k = c.t0 + st - a - b + 1;
     char *blk = V.flow + (c.step + st) * L::flow;
-    double2 *fw = (double2 *)blk + 3 * cell, *bw = (double2 *)(blk + L::flow - L::ends) + 3 * cell, *f = (double2 *)(blk + L::ends) + 3 * cell;
-    double *f4 = (double *)(blk + L::ends) + 12 * NC + 3 * cell, *oq = (double *)(blk + L::ends) + 15 * NC;
+    double2 *fw = (double2 *)blk + 3 * cell, *bw = (double2 *)(blk + L::flow - L::ends) + 3 * cell;
+    double *f = (double *)(blk + L::ends) + 3 * cell, *oq = (double *)(blk + L::ends) + 15 * NC;
     double *rq = (double *)(V.dq + (c.step + st) * L::dq);
     if (i > c.S.nI || j > c.S.nJ || k < 1 || k > c.S.nK) {
         // (the rest of such a cell's block stays zero)
@@ -631,9 +640,11 @@ __global__ void __launch_bounds__(256) k_wave_gather64(Batch B, PhysW<double> P,
     for (int d = 0; d < 3; d++) {
         const double2 g0 = geo[d], g1 = geo[3 * NC + d];
         const double dv = __dadd_rn(fma(w, g1.x, fma(u, g0.x, __dmul_rn(v, g0.y))), -g1.y);
-        f[d] = make_double2(__dmul_rn(o[0], dv), fma(po, g0.x, __dmul_rn(o[1], dv)));
-        f[3 * NC + d] = make_double2(fma(po, g0.y, __dmul_rn(o[2], dv)), fma(po, g1.x, __dmul_rn(o[3], dv)));
-        f4[d] = fma(po, g1.y, __dmul_rn(ep, dv));
+        f[d] = __dmul_rn(o[0], dv);
+        f[3 * NC + d] = fma(po, g0.x, __dmul_rn(o[1], dv));
+        f[6 * NC + d] = fma(po, g0.y, __dmul_rn(o[2], dv));
+        f[9 * NC + d] = fma(po, g1.x, __dmul_rn(o[3], dv));
+        f[12 * NC + d] = fma(po, g1.y, __dmul_rn(ep, dv));
         // what the cell's term is scaled with is the diagonal of the cell that receives it (one that lies
         // outside the box has none and receives nothing)
         const double h = 0.5 * area[d], q = fma(0.5, __dmul_rn(P.relax, W.lamc[d][p]), W.lamv[d][p]);
@@ -656,9 +667,10 @@ template <typename T, int DIR>
 __global__ void __launch_bounds__(256) k_wave_var(Batch B, PhysW<T> P, Geo G, Flow<T> W, WaveTables V, WaveTables VV)
 {
     using L = Lay<T, VAR>;
+    constexpr int PA = L::PA, NC = L::NC;
     next_sweep(VV);
-    const Chunk c = chunk_of(V, 8);
-    const int cell = threadIdx.x & 31, st = threadIdx.x >> 5, a = cell / PB, b = cell % PB;
+    const Chunk c = chunk_of(V, kSteps<T>);
+    const int cell = threadIdx.x % NC, st = threadIdx.x / NC, a = cell / PB, b = cell % PB;
     if (!c.live || st >= c.nt) return;
     const Lvl Lv = B.lv[blockIdx.y];
     const int i = c.PI * PA + a + 1, j = c.PJ * PB + b + 1, k = c.t0 + st - a - b + 1;
@@ -697,6 +709,7 @@ __global__ void __launch_bounds__(256) k_wave_var(Batch B, PhysW<T> P, Geo G, Fl
 template <typename T>
 __global__ void __launch_bounds__(256) k_wave_geometry(Batch B, Geo G, WaveTables V)
 {
+    constexpr int PA = kPA<T>, NC = kCells<T>;
     const WaveSolve S = V.solve[blockIdx.y];
     const Lvl Lv = B.lv[blockIdx.y];
     const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -725,7 +738,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_wave_scatter(Batch B, Flow<T> W, WaveTables V)
 {
     using L = Lay<T, MEAN>;
-    constexpr int CH = sizeof(T) == 4 ? 32 : 16, NW = L::dq / 16, stride = NW + 1;
+    constexpr int PA = L::PA, NC = L::NC, CH = 32, NW = L::dq / 16, stride = NW + 1;
     __shared__ float4 tile[CH * stride];
     const Chunk c = chunk_of(V, CH);
     if (!c.live) return;
@@ -749,8 +762,9 @@ __global__ void __launch_bounds__(256) k_wave_scatter(Batch B, Flow<T> W, WaveTa
 template <typename T>
 __global__ void __launch_bounds__(256) k_wave_scatter_var(Batch B, Flow<T> W, WaveTables VV)
 {
-    const Chunk c = chunk_of(VV, 8);
-    const int cell = threadIdx.x & 31, st = threadIdx.x >> 5, a = cell / PB, b = cell % PB;
+    constexpr int PA = kPA<T>, NC = kCells<T>;
+    const Chunk c = chunk_of(VV, kSteps<T>);
+    const int cell = threadIdx.x % NC, st = threadIdx.x / NC, a = cell / PB, b = cell % PB;
     if (!c.live || st >= c.nt) return;
     const int i = c.PI * PA + a + 1, j = c.PJ * PB + b + 1, k = c.t0 + st - a - b + 1;
     if (i > c.S.nI || j > c.S.nJ || k < 1 || k > c.S.nK) return;
@@ -775,9 +789,9 @@ void march(const LaunchCtx &ctx, const WaveTables &V, T gm1)
 
 }  // namespace
 
-void wave_patch(int &pa, int &pb)
+void wave_patch(int fp64, int &pa, int &pb)
 {
-    pa = PA;
+    pa = fp64 ? kPA<double> : kPA<float>;
     pb = PB;
 }
 
@@ -786,7 +800,7 @@ void wave_bytes(int fp64, int sa, WaveBytes &w)
     auto set = [&](auto mean, auto var) {
         using L = decltype(mean);
         using X = decltype(var);
-        w = {L::geo, L::flow, L::dq, L::pkt * 16, 3 * NC * L::B, 0, 0, 0};
+        w = {L::geo, L::flow, L::dq, L::pkt * 16, 3 * L::NC * L::B, 0, 0, 0};
         if (sa) { w.var_flow = X::flow; w.var_dq = X::dq; w.var_pkt = X::pkt * 16; }
     };
     if (fp64) set(Lay<double, MEAN>{}, Lay<double, VAR>{});
@@ -799,7 +813,7 @@ void launch_wave_geometry(const LaunchCtx &ctx, const Geo &G, const WaveTables &
     allow_shared<T, MEAN>();
     allow_shared<T, VAR>();
     if (sizeof(T) == 4) cudaFuncSetAttribute(k_wave_gather32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGatherBytes);
-    k_wave_geometry<T><<<ctx.grid_n(V.max_steps * NC, 256), 256, 0, ctx.stream>>>(ctx.batch, G, V);
+    k_wave_geometry<T><<<ctx.grid_n(V.max_steps * kCells<T>, 256), 256, 0, ctx.stream>>>(ctx.batch, G, V);
 }
 
 template <typename T>
@@ -807,13 +821,13 @@ void launch_lusgs_sweeps(const LaunchCtx &ctx, const PhysW<T> &P, const Geo &G, 
 {
     auto chunks = [&](int steps) { return dim3((unsigned)(V.max_tiles * ((V.max_T + steps - 1) / steps)), ctx.batch.nsolve); };
     ctx.mark("sweep_forward", 1, 2);
-    if constexpr (sizeof(T) == 4) k_wave_gather32<<<chunks(kSteps32), NC * kSteps32, kGatherBytes, ctx.stream>>>(ctx.batch, P, W, V);
-    else k_wave_gather64<<<chunks(8), 256, 0, ctx.stream>>>(ctx.batch, P, W, V);
+    if constexpr (sizeof(T) == 4) k_wave_gather32<<<chunks(kSteps32), kCells<float> * kSteps32, kGatherBytes, ctx.stream>>>(ctx.batch, P, W, V);
+    else k_wave_gather64<<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, P, W, V);
     march<T, 1, MEAN>(ctx, V, P.gm1);
     ctx.mark("sweep_forward", 0, 2);
     if (W.ev) {
         ctx.mark("sa_sweeps", 1, 2);
-        k_wave_var<T, 1><<<chunks(8), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
+        k_wave_var<T, 1><<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
         march<T, 1, VAR>(ctx, VV, (T)0);
         ctx.mark("sa_sweeps", 0, 2);
     }
@@ -822,13 +836,13 @@ void launch_lusgs_sweeps(const LaunchCtx &ctx, const PhysW<T> &P, const Geo &G, 
     ctx.mark("sweep_backward", 0, 1);
     if (W.ev) {
         ctx.mark("sa_sweeps", 1, 3);
-        k_wave_var<T, -1><<<chunks(8), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
+        k_wave_var<T, -1><<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
         march<T, -1, VAR>(ctx, VV, (T)0);
-        k_wave_scatter_var<T><<<chunks(8), 256, 0, ctx.stream>>>(ctx.batch, W, VV);
+        k_wave_scatter_var<T><<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, W, VV);
         ctx.mark("sa_sweeps", 0, 3);
     }
     ctx.mark("sweep_scatter", 1, 1);
-    k_wave_scatter<T><<<chunks(sizeof(T) == 4 ? 32 : 16), 256, 0, ctx.stream>>>(ctx.batch, W, V);
+    k_wave_scatter<T><<<chunks(32), 256, 0, ctx.stream>>>(ctx.batch, W, V);
     ctx.mark("sweep_scatter", 0, 1);
 }
 
