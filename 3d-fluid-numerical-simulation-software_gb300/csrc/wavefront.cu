@@ -60,7 +60,10 @@ constexpr int kGroup = 2, kStages = 3;          // steps of a stage of the input
 constexpr int kSlots = kGroup * kStages;        // steps whose terms are kept: the outgoing warp fetches a stage
                                                 // after it has sent the steps that used it, so a step's terms
                                                 // are never overwritten before they are sent
-constexpr int kAhead = 4;                       // steps that the incoming warp asks ahead
+constexpr int kAhead = 2;                       // steps that the incoming warp asks ahead: with one, the answer takes
+                                                // longer than a step; asked earlier, it is more often too early and
+                                                // costs a second round (137, 146, 154, 186 us a forward sweep of the
+                                                // 129x49x49 passage in FP32 with 2, 3, 4, 8)
 constexpr unsigned kWaitLimit = 1u << 21;       // polls of a wait before it gives up (seconds)
 constexpr int kSteps32 = 16;                    // steps of a block of the FP32 gather kernel
 template <typename T> constexpr int kSteps = 256 / kCells<T>;                   // of the kernels with a thread per cell
@@ -773,18 +776,23 @@ __global__ void __launch_bounds__(256) k_wave_scatter_var(Batch B, Flow<T> W, Wa
 
 constexpr unsigned kGatherBytes = kSteps32 * (Lay<float, MEAN>::flow + Lay<float, MEAN>::dq + 16);
 
+// Shared memory of a block of the march. FP64: no more than two blocks on an SM, whose FP64 pipes they share:
+// further ones slow the tiles that the others wait for (forward sweep of four 129x49x49 passages 1110 us
+// with four blocks, 903 with two, 1012 with one; of one 161x65x65 passage 751, 751, 709).
+template <typename T, Kind K> constexpr int kMarchShared = sizeof(T) == 8 && Lay<T, K>::smem < 100000 ? 100000 : Lay<T, K>::smem;
+
 // (shared memory beyond the default limit has to be asked for, once per kernel and device)
 template <typename T, Kind K>
 void allow_shared()
 {
-    cudaFuncSetAttribute(k_wave<T, 1, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay<T, K>::smem);
-    cudaFuncSetAttribute(k_wave<T, -1, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay<T, K>::smem);
+    cudaFuncSetAttribute(k_wave<T, 1, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMarchShared<T, K>);
+    cudaFuncSetAttribute(k_wave<T, -1, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMarchShared<T, K>);
 }
 
 template <typename T, int DIR, Kind K>
 void march(const LaunchCtx &ctx, const WaveTables &V, T gm1)
 {
-    k_wave<T, DIR, K><<<V.n_item, 192, Lay<T, K>::smem, ctx.stream>>>(ctx.batch, V, gm1);
+    k_wave<T, DIR, K><<<V.n_item, 192, kMarchShared<T, K>, ctx.stream>>>(ctx.batch, V, gm1);
 }
 
 }  // namespace
