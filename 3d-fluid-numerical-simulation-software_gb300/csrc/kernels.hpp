@@ -73,6 +73,9 @@ struct BcTables {
 // where the integrals put an iteration's row of the history (12 values per case): row iter - *base
 struct HistorySink { double *out; const int *base; int rows, ncase; };
 
+// out-of-range cells of every slot (update.cuh): their list, its length, blocks of a launch that are done
+struct LimitLists { int *list, cap, *count; unsigned *done; };
+
 constexpr int kIntegralBlocks = 32;             // blocks per inlet/outlet section in the integrals
 
 // The LU-SGS sweeps' tiles (wavefront.cu). A tile is a group of grid columns that a block marches
@@ -118,10 +121,11 @@ template <typename T>
 void launch_resflux(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC, const Geo &G, const GeoW<T> &GW, Flow<T> F,
                     const BcTables &bc, int level, T *scratch_dtmin);
 
-// both sweeps, dQ back into the box (with the Spalart-Allmaras variable present, F.ev, its update too; VV:
+// both sweeps, then Q_old = Q, Q += dQ, the primitive variables and the limiter (with the Spalart-Allmaras variable present, F.ev, its update too; VV:
 // the tables of the variable's sweep)
 template <typename T>
-void launch_lusgs_sweeps(const LaunchCtx &ctx, const PhysW<T> &P, const Geo &G, Flow<T> F, const WaveTables &V, const WaveTables &VV);
+void launch_lusgs_sweeps(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC, const Geo &G, Flow<T> F, const WaveTables &V,
+                         const WaveTables &VV, int level, const LimitLists &q);
 
 // Baldwin-Lomax wall distances of every wall line point (fine level, once; see BcTables)
 template <typename T>
@@ -133,10 +137,6 @@ void launch_geometry_working(const LaunchCtx &ctx, const Geo &G, const GeoW<floa
 // the sweeps' geometry in step order (once per level, after the geometry kernels)
 template <typename T>
 void launch_wave_geometry(const LaunchCtx &ctx, const Geo &G, const WaveTables &V);
-
-template <typename T>
-void launch_update(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> F, int level,
-                   int *bad_list, int bad_cap, int *bad_count);
 
 template <typename T>
 void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> F, const double *totalvol, double *partials,
@@ -153,12 +153,18 @@ template <typename T>
 void launch_primitive(const LaunchCtx &ctx, const Phys &P, Flow<T> F);
 
 template <typename T>
-void launch_limiter(const LaunchCtx &ctx, const Phys &P, Flow<T> F, int level, int *bad_list, int bad_cap,
-                    int *bad_count);
+void launch_limiter(const LaunchCtx &ctx, const Phys &P, Flow<T> F, int level, const LimitLists &q);
 
 // multigrid transfer between fine (f) and coarse (c) levels
 template <typename T>
 void launch_restrict(const LaunchCtx &cf, const LaunchCtx &cc, const Geo &Gf, const Geo &Gc, Flow<T> Ff, Flow<T> Fc);
+// restriction or prolongation with the receiving level's primitive variables and limiter
+template <typename T>
+void launch_restrict_primitive(const LaunchCtx &cf, const LaunchCtx &cc, const Phys &P, const Geo &Gf, const Geo &Gc, Flow<T> Ff,
+                               Flow<T> Fc, int level, const LimitLists &q);
+template <typename T>
+void launch_interpolate_primitive(const LaunchCtx &cf, const LaunchCtx &cc, const Phys &P, Flow<T> Ff, Flow<T> Fc, int init_from_coarse,
+                                  int level, const LimitLists &q);
 template <typename T>
 void launch_forcing(const LaunchCtx &cc, Flow<T> Fc);
 template <typename T>

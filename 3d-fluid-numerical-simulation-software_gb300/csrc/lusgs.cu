@@ -1,222 +1,51 @@
-// The update after the LU-SGS sweeps: Q += dQ (FP64 accumulation in both precision forms), the
-// primitive variables (source/PrimitiveVars.cpp:7-28), detection of out-of-range cells for the
-// limiter (source/Limit_FlowVars.cpp:8-118), and the residual norm (source/ComputeAllBlockVars.cpp:318-372).
+// Primitive variables (source/PrimitiveVars.cpp:7-28) and the limiter (source/Limit_FlowVars.cpp:8-118) by
+// themselves, the residual norm (source/ComputeAllBlockVars.cpp:318-372), the inlet and outlet integrals
+// (source/Ouput.cpp:9-107,282-300) and the CFL ramp.
 #include "gbt_common.cuh"
 #include "kernels.hpp"
 #include "flux.cuh"
+#include "update.cuh"
 
 namespace gbt {
 
-// primitive variables from the conserved ones
-template <typename T>
-__device__ __forceinline__ void prim_from_cons(const Phys &P, const double c[5], T q[6])
-{
-    if constexpr (sizeof(T) == 4) {
-        // mixed form: primitives are stored in FP32, so they are formed in FP32 from the FP64 Q
-        // (conversions by integer operations: the same roundings as the conversion instructions)
-        const float d = f64_to_f32_rn(c[0]), rd = 1.0f / d;
-        const float u = f64_to_f32_rn(c[1]) * rd, v = f64_to_f32_rn(c[2]) * rd, w = f64_to_f32_rn(c[3]) * rd;
-        const float V2 = u * u + v * v + w * w;
-        const float pr = ((float)P.gamma - 1.0f) * (f64_to_f32_rn(c[4]) - d * V2 * 0.5f);
-        q[PD] = d; q[PU] = u; q[PV] = v; q[PW] = w; q[PP] = pr; q[PT] = pr * rd / (float)P.rgas;
-    } else {
-        // one FP64 division by the density, products with its reciprocal (within rounding)
-        const double d = c[0], rd = 1.0 / d, u = c[1] * rd, v = c[2] * rd, w = c[3] * rd;
-        const double V2 = u * u + v * v + w * w;
-        const double pr = (P.gamma - 1.0) * (c[4] - d * V2 * 0.5);
-        q[PD] = (T)d; q[PU] = (T)u; q[PV] = (T)v; q[PW] = (T)w; q[PP] = (T)pr; q[PT] = (T)(pr * rd / P.rgas);
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ bool out_of_range(const T q[6])
-{
-    const T dmin = (T)(double)1.0E-6f, dmax = (T)1000, pmin = (T)(double)1.0E-6f, pmax = (T)1000, vmax = (T)1000;
-    return q[PD] < dmin || q[PD] > dmax || q[PP] < pmin || q[PP] > pmax || q[PU] > vmax || q[PV] > vmax || q[PW] > vmax;
-}
-
-// Q_old = Q; Q += dQ; primitive variables; out-of-range cells appended to the solve's list
-template <typename T>
-__global__ void __launch_bounds__(256) k_update(Batch B, Phys P, Flow<T> W, int *bad_list, int bad_cap, int *bad_count)
+// primitive variables of a level (PRIM), out-of-range cells repaired (LIM)
+template <typename T, bool PRIM, bool LIM>
+__global__ void __launch_bounds__(256) k_primitive(Batch B, Phys P, Flow<T> W, int level, LimitLists q)
 {
     const int s = blockIdx.y;
     const Lvl L = B.lv[s];
+    const unsigned blocks = cell_blocks(L);
+    if (blockIdx.x >= blocks) return;
     int i, j, k;
-    if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
-    const long long p = ix(L, i, j, k);
-    double c[5];
-#pragma unroll
-    for (int n = 0; n < 5; n++) {
-        const double o = W.cv[n][p];
-        W.cvold[n][p] = o;
-        c[n] = o + to_f64<T>(W.dq[n][p]);
-        W.cv[n][p] = c[n];
-    }
-    T q[6];
-    prim_from_cons<T>(P, c, q);
-#pragma unroll
-    for (int n = 0; n < 6; n++) W.pv[n][p] = q[n];
-    if (P.limiter && out_of_range(q)) {
-        int slot = atomicAdd(&bad_count[s], 1);
-        if (slot < bad_cap) bad_list[(long long)s * bad_cap + slot] = (int)(((long long)(i - 1) * (L.JM - 1) + (j - 1)) * (L.KM - 1) + (k - 1));
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_primitive(Batch B, Phys P, Flow<T> W)
-{
-    const Lvl L = B.lv[blockIdx.y];
-    int i, j, k;
-    if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
-    const long long p = ix(L, i, j, k);
-    double c[5];
-#pragma unroll
-    for (int n = 0; n < 5; n++) c[n] = W.cv[n][p];
-    T q[6];
-    prim_from_cons<T>(P, c, q);
-#pragma unroll
-    for (int n = 0; n < 6; n++) W.pv[n][p] = q[n];
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_detect(Batch B, Phys P, Flow<T> W, int *bad_list, int bad_cap, int *bad_count)
-{
-    const int s = blockIdx.y;
-    const Lvl L = B.lv[s];
-    int i, j, k;
-    if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
-    const long long p = ix(L, i, j, k);
-    T q[6];
-#pragma unroll
-    for (int n = 0; n < 6; n++) q[n] = W.pv[n][p];
-    if (out_of_range(q)) {
-        int slot = atomicAdd(&bad_count[s], 1);
-        if (slot < bad_cap) bad_list[(long long)s * bad_cap + slot] = (int)(((long long)(i - 1) * (L.JM - 1) + (j - 1)) * (L.KM - 1) + (k - 1));
-    }
-}
-
-// The reference repairs limited cells one after another in i, j, k order, each from the mean of
-// its in-range neighbours as they are at that moment, so a repaired cell can feed a later one.
-// Rare; one thread per solve replays that order over the (sorted) list of flagged cells. When
-// the list overflowed, the thread scans every cell instead.
-template <typename T>
-__global__ void k_limiter(Batch B, Phys P, Flow<T> W, int level, int *bad_list, int bad_cap, int *bad_count)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= B.nsolve) return;
-    const int n = bad_count[s];
-    if (n == 0) { B.st[s].status &= ~GBT_STATUS_LIMITER; return; }
-    const Lvl L = B.lv[s];
-    const int nI = L.IM - 1, nJ = L.JM - 1, nK = L.KM - 1;
-    int *lst = bad_list + (long long)s * bad_cap;
-    const bool full = n > bad_cap;
-    if (!full) {
-        for (int a = 1; a < n; a++) {                 // insertion sort: lists are short
-            int v = lst[a], b = a - 1;
-            while (b >= 0 && lst[b] > v) { lst[b + 1] = lst[b]; b--; }
-            lst[b + 1] = v;
-        }
-    }
-    const long long total = (long long)nI * nJ * nK;
-    const long long m = full ? total : n;
-    for (long long e = 0; e < m; e++) {
-        const long long lin = full ? e : lst[e];
-        const int i = 1 + (int)(lin / ((long long)nJ * nK)), j = 1 + (int)((lin / nK) % nJ), k = 1 + (int)(lin % nK);
+    if (box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) {
         const long long p = ix(L, i, j, k);
-        T q[6];
-        for (int c = 0; c < 6; c++) q[c] = W.pv[c][p];
-        if (!out_of_range(q)) continue;
-        double d = 0, u = 0, v = 0, w = 0, pr = 0;
-        int kn = 0, i1 = 0, j1 = 0, k1 = 0;
-        for (int ia = -1; ia <= 1; ia++)
-            for (int ja = -1; ja <= 1; ja++)
-                for (int ka = -1; ka <= 1; ka++) {
-                    k1 = k + ka; j1 = j + ja; i1 = i + ia;
-                    if (i1 > 0 && i1 < L.IM && j1 > 0 && j1 < L.JM && k1 > 0 && k1 < L.KM) {
-                        const long long r = ix(L, i1, j1, k1);
-                        T qq[6];
-                        for (int c = 0; c < 6; c++) qq[c] = W.pv[c][r];
-                        if (!out_of_range(qq)) {
-                            d += qq[PD]; u += qq[PU]; v += qq[PV]; w += qq[PW]; pr += qq[PP]; kn++;
-                        }
-                    }
-                }
-        if (kn == 0) {
-            // last visited neighbour (i+1, j+1, k+1), clipped to the admissible range
-            const long long r = ix(L, i1, j1, k1);
-            d = W.pv[PD][r]; u = W.pv[PU][r]; v = W.pv[PV][r]; w = W.pv[PW][r]; pr = W.pv[PP][r];
-            const double lo = (double)1.0E-6f;
-            if (d < lo) d = lo;
-            if (d > 1000.0) d = 1000.0;
-            if (pr < lo) pr = lo;
-            if (pr > 1000.0) pr = 1000.0;
-            if (fabs(u) > 1000.0) u = u < 0 ? -1000.0 : 1000.0;
-            if (fabs(v) > 1000.0) v = v < 0 ? -1000.0 : 1000.0;
-            if (fabs(w) > 1000.0) w = w < 0 ? -1000.0 : 1000.0;
+        T v[6];
+        if constexpr (PRIM) {
+            double c[5];
+#pragma unroll
+            for (int n = 0; n < 5; n++) c[n] = W.cv[n][p];
+            prim_from_cons<T>(P, c, v);
+#pragma unroll
+            for (int n = 0; n < 6; n++) W.pv[n][p] = v[n];
         } else {
-            const double sn1 = (double)(1.0f / (float)kn);
-            d *= sn1; u *= sn1; v *= sn1; w *= sn1; pr *= sn1;
+#pragma unroll
+            for (int n = 0; n < 6; n++) v[n] = W.pv[n][p];
         }
-        W.pv[PD][p] = (T)d; W.pv[PU][p] = (T)u; W.pv[PV][p] = (T)v; W.pv[PW][p] = (T)w; W.pv[PP][p] = (T)pr;
-        W.pv[PT][p] = (T)(pr / d / P.rgas);
-        W.cv[0][p] = d; W.cv[1][p] = d * u; W.cv[2][p] = d * v; W.cv[3][p] = d * w;
-        W.cv[4][p] = pr / (P.gamma - 1.0) + d * (u * u + v * v + w * w) / 2.0;
+        if constexpr (LIM) limit_flag<T>(P, q, L, s, i, j, k, v);
     }
-    B.st[s].flag_low_dt[level] = 10;
-    B.st[s].status |= GBT_STATUS_LIMITER | (full ? GBT_STATUS_LIMITER_OVF : 0);
-    B.st[s].limiter_hits += n;
-}
-
-template <typename T>
-void launch_update(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> W, int level, int *bad_list,
-                   int bad_cap, int *bad_count)
-{
-    (void)G;
-    const Batch &B = ctx.batch;
-    ctx.mark("update_limiter", 1, 2);
-    cudaMemsetAsync(bad_count, 0, sizeof(int) * B.nsolve, ctx.stream);
-    k_update<T><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, P, W, bad_list, bad_cap, bad_count);
-    if (P.limiter) k_limiter<T><<<(B.nsolve + 31) / 32, 32, 0, ctx.stream>>>(B, P, W, level, bad_list, bad_cap, bad_count);
-    if (W.ev) {
-        // the variable's update and Limit_SA after the mean flow's (source/LU_SGS_Marching.cpp:275-277,
-        // source/ComputeAllBlockVars.cpp:257-266); the limiter list is reused
-        launch_sa_update<T>(ctx, P, W, bad_list, bad_cap, bad_count);
-        if (P.limiter) launch_sa_limit<T>(ctx, W, bad_list, bad_cap, bad_count);
-    }
-    ctx.mark("update_limiter", 0, 2);
+    if constexpr (LIM) limit_done<T>(B, P, W, level, q, s, blocks);
 }
 
 template <typename T>
 void launch_primitive(const LaunchCtx &ctx, const Phys &P, Flow<T> W)
 {
-    k_primitive<T><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(ctx.batch, P, W);
+    k_primitive<T, true, false><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(ctx.batch, P, W, 0, {});
 }
 
 template <typename T>
-void launch_limiter(const LaunchCtx &ctx, const Phys &P, Flow<T> W, int level, int *bad_list, int bad_cap,
-                    int *bad_count)
+void launch_limiter(const LaunchCtx &ctx, const Phys &P, Flow<T> W, int level, const LimitLists &q)
 {
-    if (!P.limiter) return;
-    const Batch &B = ctx.batch;
-    cudaMemsetAsync(bad_count, 0, sizeof(int) * B.nsolve, ctx.stream);
-    k_detect<T><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, P, W, bad_list, bad_cap, bad_count);
-    k_limiter<T><<<(B.nsolve + 31) / 32, 32, 0, ctx.stream>>>(B, P, W, level, bad_list, bad_cap, bad_count);
-}
-
-// whether this block is the last of its group to get here (all threads call it; what the group's blocks
-// wrote before is then visible). The counter is put back to zero for the next launch.
-__device__ __forceinline__ bool last_block(unsigned *count, unsigned blocks)
-{
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        last = atomicAdd(count, 1u) == blocks - 1;
-        if (last) *count = 0;
-    }
-    __syncthreads();
-    if (last) __threadfence();
-    return last;
+    if (P.limiter) k_primitive<T, false, true><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(ctx.batch, P, W, level, q);
 }
 
 // ---- residual norm: sum |(Q_old - Q)/Q_old| * Vol / V_total, FP64, in a fixed order: each thread four or
@@ -408,9 +237,8 @@ void launch_cfl_ramp(const LaunchCtx &ctx, int iter)
 }
 
 #define GBT_INST(T)                                                                                                   \
-    template void launch_update<T>(const LaunchCtx &, const Phys &, const Geo &, Flow<T>, int, int *, int, int *);     \
     template void launch_primitive<T>(const LaunchCtx &, const Phys &, Flow<T>);                                       \
-    template void launch_limiter<T>(const LaunchCtx &, const Phys &, Flow<T>, int, int *, int, int *);                 \
+    template void launch_limiter<T>(const LaunchCtx &, const Phys &, Flow<T>, int, const LimitLists &);                 \
     template void launch_res_norm<T>(const LaunchCtx &, const Geo &, Flow<T>, const double *, double *, int, unsigned *);          \
     template void launch_integrals<T>(const LaunchCtx &, const Phys &, const Geo &, Flow<T>, const BcTables &, const HistorySink &);
 GBT_INST(double)

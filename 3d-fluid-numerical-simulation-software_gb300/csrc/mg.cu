@@ -4,33 +4,49 @@
 // corner fill of the coarse ghosts, trilinear 27/9/3/1 prolongation.
 #include "gbt_common.cuh"
 #include "kernels.hpp"
+#include "update.cuh"
 #include <algorithm>
 
 namespace gbt {
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_restrict(Batch Bf, Batch Bc, Geo Gf, Geo Gc, Flow<T> Wf, Flow<T> Wc)
+// PRIM: the coarse level's primitive variables and limiter with it (a launch each otherwise)
+template <typename T, bool PRIM>
+__global__ void __launch_bounds__(256) k_restrict(Batch Bf, Batch Bc, Phys P, Geo Gf, Geo Gc, Flow<T> Wf, Flow<T> Wc, int level,
+                                                  LimitLists lists)
 {
     const int s = blockIdx.y;
     const Lvl F = Bf.lv[s], C = Bc.lv[s];
+    const unsigned blocks = cell_blocks(C);
+    if (blockIdx.x >= blocks) return;
     int i, j, k;
-    if (!box_index(C.IM - 1, C.JM - 1, C.KM - 1, i, j, k)) return;
-    const int i1 = 2 * i - 1, j1 = 2 * j - 1, k1 = 2 * k - 1, i2 = 2 * i, j2 = 2 * j, k2 = 2 * k;
-    const long long f[8] = {ix(F, i1, j1, k1), ix(F, i1, j1, k2), ix(F, i1, j2, k1), ix(F, i1, j2, k2),
-                            ix(F, i2, j1, k1), ix(F, i2, j1, k2), ix(F, i2, j2, k1), ix(F, i2, j2, k2)};
-    const long long p = ix(C, i, j, k);
-    const double vc = Gc.vol[p];
+    if (box_index(C.IM - 1, C.JM - 1, C.KM - 1, i, j, k)) {
+        const int i1 = 2 * i - 1, j1 = 2 * j - 1, k1 = 2 * k - 1, i2 = 2 * i, j2 = 2 * j, k2 = 2 * k;
+        const long long f[8] = {ix(F, i1, j1, k1), ix(F, i1, j1, k2), ix(F, i1, j2, k1), ix(F, i1, j2, k2),
+                                ix(F, i2, j1, k1), ix(F, i2, j1, k2), ix(F, i2, j2, k1), ix(F, i2, j2, k2)};
+        const long long p = ix(C, i, j, k);
+        const double vc = Gc.vol[p];
+        double cons[5];
 #pragma unroll
-    for (int c = 0; c < NQ; c++) {
-        double a = Wf.cv[c][f[0]] * Gf.vol[f[0]];
-        T r = Wf.res[c][f[0]];
+        for (int c = 0; c < NQ; c++) {
+            double a = Wf.cv[c][f[0]] * Gf.vol[f[0]];
+            T r = Wf.res[c][f[0]];
 #pragma unroll
-        for (int q = 1; q < 8; q++) { a = a + Wf.cv[c][f[q]] * Gf.vol[f[q]]; r = r + Wf.res[c][f[q]]; }
-        a = a / vc;
-        Wc.cv2h[c][p] = a;
-        Wc.cv[c][p] = a;
-        Wc.res2h[c][p] = r;
+            for (int q = 1; q < 8; q++) { a = a + Wf.cv[c][f[q]] * Gf.vol[f[q]]; r = r + Wf.res[c][f[q]]; }
+            a = a / vc;
+            Wc.cv2h[c][p] = a;
+            Wc.cv[c][p] = a;
+            cons[c] = a;
+            Wc.res2h[c][p] = r;
+        }
+        if constexpr (PRIM) {
+            T v[6];
+            prim_from_cons<T>(P, cons, v);
+#pragma unroll
+            for (int c = 0; c < 6; c++) Wc.pv[c][p] = v[c];
+            limit_flag<T>(P, lists, C, s, i, j, k, v);
+        }
     }
+    if constexpr (PRIM) limit_done<T>(Bc, P, Wc, level, lists, s, blocks);
 }
 
 // coarse residual replaced by the restricted fine residual through the forcing function:
@@ -145,51 +161,71 @@ __global__ void __launch_bounds__(64) k_corners(Batch B, Flow<T> W)
 
 // fine Q (+)= sum of 27/64, 9/64, 3/64, 1/64 weighted coarse values around the fine cell; the
 // first call after the coarse start-up phase interpolates Q itself, later calls the correction
-template <typename T>
-__global__ void __launch_bounds__(256) k_interpolate(Batch Bf, Batch Bc, Flow<T> Wf, Flow<T> Wc, int init)
+template <typename T, bool PRIM>
+__global__ void __launch_bounds__(256) k_interpolate(Batch Bf, Batch Bc, Phys P, Flow<T> Wf, Flow<T> Wc, int init, int level,
+                                                     LimitLists lists)
 {
     const int s = blockIdx.y;
     const Lvl F = Bf.lv[s], C = Bc.lv[s];
+    const unsigned blocks = cell_blocks(F);
+    if (blockIdx.x >= blocks) return;
     int i, j, k;
-    if (!box_index(F.IM - 1, F.JM - 1, F.KM - 1, i, j, k)) return;
-    // nearest coarse cell and the next one (source/Prolong_Interpolate.cpp:90-119): for an odd
-    // fine index n, (n+1)/2 and (n-1)/2; for an even one, n/2 and n/2+1
-    const int ia1 = (i + 1) >> 1, ia2 = (i & 1) ? (i - 1) >> 1 : (i >> 1) + 1;
-    const int ja1 = (j + 1) >> 1, ja2 = (j & 1) ? (j - 1) >> 1 : (j >> 1) + 1;
-    const int ka1 = (k + 1) >> 1, ka2 = (k & 1) ? (k - 1) >> 1 : (k >> 1) + 1;
-    const long long c111 = ix(C, ia1, ja1, ka1), c112 = ix(C, ia1, ja1, ka2), c121 = ix(C, ia1, ja2, ka1),
-                    c211 = ix(C, ia2, ja1, ka1), c221 = ix(C, ia2, ja2, ka1), c122 = ix(C, ia1, ja2, ka2),
-                    c212 = ix(C, ia2, ja1, ka2), c222 = ix(C, ia2, ja2, ka2);
-    const double a1 = 27.0 / 64.0, a2 = 9.0 / 64.0, a3 = 3.0 / 64.0, a4 = 1.0 / 64.0;
-    const long long p = ix(F, i, j, k);
+    if (box_index(F.IM - 1, F.JM - 1, F.KM - 1, i, j, k)) {
+        // nearest coarse cell and the next one (source/Prolong_Interpolate.cpp:90-119): for an odd
+        // fine index n, (n+1)/2 and (n-1)/2; for an even one, n/2 and n/2+1
+        const int ia1 = (i + 1) >> 1, ia2 = (i & 1) ? (i - 1) >> 1 : (i >> 1) + 1;
+        const int ja1 = (j + 1) >> 1, ja2 = (j & 1) ? (j - 1) >> 1 : (j >> 1) + 1;
+        const int ka1 = (k + 1) >> 1, ka2 = (k & 1) ? (k - 1) >> 1 : (k >> 1) + 1;
+        const long long c111 = ix(C, ia1, ja1, ka1), c112 = ix(C, ia1, ja1, ka2), c121 = ix(C, ia1, ja2, ka1),
+                        c211 = ix(C, ia2, ja1, ka1), c221 = ix(C, ia2, ja2, ka1), c122 = ix(C, ia1, ja2, ka2),
+                        c212 = ix(C, ia2, ja1, ka2), c222 = ix(C, ia2, ja2, ka2);
+        const double a1 = 27.0 / 64.0, a2 = 9.0 / 64.0, a3 = 3.0 / 64.0, a4 = 1.0 / 64.0;
+        const long long p = ix(F, i, j, k);
+        double cons[5];
 #pragma unroll
-    for (int c = 0; c < NQ; c++) {
-        double v;
-        if (init) {
-            const double *q = Wc.cv[c];
-            v = a1 * q[c111] + a2 * (q[c112] + q[c121] + q[c211]) + a3 * (q[c221] + q[c122] + q[c212]) + a4 * q[c222];
-            Wf.cv[c][p] = v;
-        } else {
-            const T *q = Wc.dq2h[c];
-            if constexpr (sizeof(T) == 4) {
-                // mixed form: the correction is summed in FP32 (the weights are exact there) and
-                // accumulated into the FP64 Q
-                const T w = (T)a1 * q[c111] + (T)a2 * (q[c112] + q[c121] + q[c211]) +
-                            (T)a3 * (q[c221] + q[c122] + q[c212]) + (T)a4 * q[c222];
-                v = (double)w;
+        for (int c = 0; c < NQ; c++) {
+            double v;
+            if (init) {
+                const double *q = Wc.cv[c];
+                v = a1 * q[c111] + a2 * (q[c112] + q[c121] + q[c211]) + a3 * (q[c221] + q[c122] + q[c212]) + a4 * q[c222];
+                cons[c] = v;
             } else {
-                v = a1 * (double)q[c111] + a2 * ((double)q[c112] + (double)q[c121] + (double)q[c211]) +
-                    a3 * ((double)q[c221] + (double)q[c122] + (double)q[c212]) + a4 * (double)q[c222];
+                const T *q = Wc.dq2h[c];
+                if constexpr (sizeof(T) == 4) {
+                    // mixed form: the correction is summed in FP32 (the weights are exact there) and
+                    // accumulated into the FP64 Q
+                    const T w = (T)a1 * q[c111] + (T)a2 * (q[c112] + q[c121] + q[c211]) +
+                                (T)a3 * (q[c221] + q[c122] + q[c212]) + (T)a4 * q[c222];
+                    v = (double)w;
+                } else {
+                    v = a1 * (double)q[c111] + a2 * ((double)q[c112] + (double)q[c121] + (double)q[c211]) +
+                        a3 * ((double)q[c221] + (double)q[c122] + (double)q[c212]) + a4 * (double)q[c222];
+                }
+                cons[c] = Wf.cv[c][p] + v;
             }
-            Wf.cv[c][p] = Wf.cv[c][p] + v;
+            Wf.cv[c][p] = cons[c];
+        }
+        if constexpr (PRIM) {
+            T v[6];
+            prim_from_cons<T>(P, cons, v);
+#pragma unroll
+            for (int c = 0; c < 6; c++) Wf.pv[c][p] = v[c];
+            limit_flag<T>(P, lists, F, s, i, j, k, v);
         }
     }
+    if constexpr (PRIM) limit_done<T>(Bf, P, Wf, level, lists, s, blocks);
 }
 
 template <typename T>
 void launch_restrict(const LaunchCtx &cf, const LaunchCtx &cc, const Geo &Gf, const Geo &Gc, Flow<T> Ff, Flow<T> Fc)
 {
-    k_restrict<T><<<cc.grid_cells(256), 256, 0, cc.stream>>>(cf.batch, cc.batch, Gf, Gc, Ff, Fc);
+    k_restrict<T, false><<<cc.grid_cells(256), 256, 0, cc.stream>>>(cf.batch, cc.batch, Phys{}, Gf, Gc, Ff, Fc, 0, {});
+}
+template <typename T>
+void launch_restrict_primitive(const LaunchCtx &cf, const LaunchCtx &cc, const Phys &P, const Geo &Gf, const Geo &Gc, Flow<T> Ff,
+                               Flow<T> Fc, int level, const LimitLists &q)
+{
+    k_restrict<T, true><<<cc.grid_cells(256), 256, 0, cc.stream>>>(cf.batch, cc.batch, P, Gf, Gc, Ff, Fc, level, q);
 }
 template <typename T>
 void launch_forcing(const LaunchCtx &cc, Flow<T> Fc)
@@ -221,7 +257,13 @@ void launch_corner(const LaunchCtx &cc, Flow<T> Fc)
 template <typename T>
 void launch_interpolate(const LaunchCtx &cf, const LaunchCtx &cc, Flow<T> Ff, Flow<T> Fc, int init)
 {
-    k_interpolate<T><<<cf.grid_cells(256), 256, 0, cf.stream>>>(cf.batch, cc.batch, Ff, Fc, init);
+    k_interpolate<T, false><<<cf.grid_cells(256), 256, 0, cf.stream>>>(cf.batch, cc.batch, Phys{}, Ff, Fc, init, 0, {});
+}
+template <typename T>
+void launch_interpolate_primitive(const LaunchCtx &cf, const LaunchCtx &cc, const Phys &P, Flow<T> Ff, Flow<T> Fc, int init, int level,
+                                  const LimitLists &q)
+{
+    k_interpolate<T, true><<<cf.grid_cells(256), 256, 0, cf.stream>>>(cf.batch, cc.batch, P, Ff, Fc, init, level, q);
 }
 
 #define GBT_INST(T)                                                                                                       \
@@ -231,7 +273,11 @@ void launch_interpolate(const LaunchCtx &cf, const LaunchCtx &cc, Flow<T> Ff, Fl
     template void launch_add_forcing<T>(const LaunchCtx &, Flow<T>);                                                     \
     template void launch_delta<T>(const LaunchCtx &, Flow<T>);                                                           \
     template void launch_corner<T>(const LaunchCtx &, Flow<T>);                                                          \
-    template void launch_interpolate<T>(const LaunchCtx &, const LaunchCtx &, Flow<T>, Flow<T>, int);
+    template void launch_interpolate<T>(const LaunchCtx &, const LaunchCtx &, Flow<T>, Flow<T>, int);                    \
+    template void launch_restrict_primitive<T>(const LaunchCtx &, const LaunchCtx &, const Phys &, const Geo &, const Geo &, Flow<T>, \
+                                               Flow<T>, int, const LimitLists &);                                        \
+    template void launch_interpolate_primitive<T>(const LaunchCtx &, const LaunchCtx &, const Phys &, Flow<T>, Flow<T>, int, int, \
+                                                  const LimitLists &);
 GBT_INST(double)
 GBT_INST(float)
 

@@ -304,19 +304,19 @@ __global__ void __launch_bounds__(256) k_bl_merge(Flow<T> W, long long n)
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const unsigned long long b = W.blmin[p];
-    if (b != ~0ull) W.mut[p] = bl_value<T>(b);
+    if (b == ~0ull) return;
+    W.mut[p] = bl_value<T>(b);
+    W.blmin[p] = ~0ull;                                        // not reached, for the next evaluation
 }
 
 // ghost mu_t mirrored across every wall face (source/WallFlux.cpp:106-109,137-140,168-171)
 template <typename T>
-__global__ void k_wall_mut(Batch B, Flow<T> W, const DevWall *walls)
+__device__ __forceinline__ void wall_mut(const Batch &B, const Flow<T> &W, const DevWall &wl, unsigned t)
 {
-    const DevWall wl = walls[blockIdx.y];
     const Lvl L = B.lv[wl.solve];
-    const int ni = wl.ie - wl.is + 1, nj = wl.je - wl.js + 1, nk = wl.ke - wl.ks + 1;
-    int i, j, k;
-    if (!box_index(ni, nj, nk, i, j, k)) return;
-    i += wl.is - 1; j += wl.js - 1; k += wl.ks - 1;
+    const unsigned ni = (unsigned)(wl.ie - wl.is + 1), nj = (unsigned)(wl.je - wl.js + 1), nk = (unsigned)(wl.ke - wl.ks + 1);
+    if (t >= ni * nj * nk) return;
+    const int i = wl.is + (int)(t / nk / nj), j = wl.js + (int)(t / nk % nj), k = wl.ks + (int)(t % nk);
     const int f = (wl.face - 1) / 2;
     const long long p = ix(L, i, j, k);
     const long long m = f == 0 ? ix(L, i - 1, j, k) : (f == 1 ? ix(L, i, j - 1, k) : ix(L, i, j, k - 1));
@@ -332,11 +332,18 @@ __device__ __forceinline__ T sweep_diagonal(const PhysW<T> &PC, T vol, T dt, T l
     else return (T)1 / fma((T)2, lv, fma(PC.relax, lc, vol / dt));
 }
 
-// viscous spectral radii and the local time step
+// viscous spectral radii and the local time step; further blocks fill the walls' ghost mu_t (which this
+// stage does not read)
 template <typename T, bool NS>   // NS: Navier-Stokes (viscous radii), else Euler
-__global__ void __launch_bounds__(256) k_cell_b(Batch B, PhysW<T> PC, GeoW<T> G, Flow<T> W, int level)
+__global__ void __launch_bounds__(256) k_cell_b(Batch B, PhysW<T> PC, GeoW<T> G, Flow<T> W, int level, unsigned cell_blocks,
+                                                const DevWall *walls, unsigned wall_blocks, unsigned n_wall)
 {
     const int s = blockIdx.y;
+    if (blockIdx.x >= cell_blocks) {
+        const unsigned w = (blockIdx.x - cell_blocks) * (unsigned)B.nsolve + blockIdx.y;
+        if (w < n_wall * wall_blocks) wall_mut<T>(B, W, walls[w / wall_blocks], w % wall_blocks * 256 + threadIdx.x);
+        return;
+    }
     const Lvl L = B.lv[s];
     int i, j, k;
     if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
@@ -404,14 +411,6 @@ __global__ void k_dt_set(Batch B, PhysW<T> PC, GeoW<T> G, Flow<T> W, const T *mn
                                   W.lamv[0][p] + W.lamv[1][p] + W.lamv[2][p]);
 }
 
-// decrement of the low-time-step counter after the time step used it
-__global__ void k_after_timestep(Batch B, int level)
-{
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= B.nsolve) return;
-    if (B.st[s].flag_low_dt[level] > 0) B.st[s].flag_low_dt[level] -= 1;
-}
-
 template <typename T>
 void launch_cell_stages(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC, const Geo &G, const GeoW<T> &GW,
                         Flow<T> W, const BcTables &bc,
@@ -422,30 +421,27 @@ void launch_cell_stages(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC,
     if (P.equation_ns) k_cell_a<T, true><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, PC, GW, W);
     else k_cell_a<T, false><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, PC, GW, W);
     ctx.mark("spectral_curl", 0);
-    ctx.mark("baldwin_lomax", 1, 4);
+    ctx.mark("baldwin_lomax", 1, 2);
     if (level == 1 && P.turb_bl && bc.n_wall > 0) {
         // every wall of every solve in one launch (32 lines per block, the points of each line split
-        // over BL_WARPS warps), merged through the per-cell minimum, reset every evaluation
-        cudaMemsetAsync(W.blmin, 0xFF, (size_t)ctx.pool_n * sizeof(unsigned long long), ctx.stream);
+        // over BL_WARPS warps), merged through the per-cell minimum, which the merge resets
         dim3 g((unsigned)((bc.max_wall + 31) / 32), bc.n_wall);
         k_bl<T><<<g, 32 * BL_WARPS, 0, ctx.stream>>>(B, PC, W, bc.wall, 0, bc.wall_dist_off, (const T *)bc.wall_dist);
         k_bl_merge<T><<<(unsigned)((ctx.pool_n + 255) / 256), 256, 0, ctx.stream>>>(W, ctx.pool_n);
     }
     if (level == 1 && P.turb_sa && W.ev) launch_sa_model<T>(ctx, P, GW, W);
-    if (bc.n_wall > 0) {
-        dim3 g((unsigned)((bc.max_wall + 127) / 128), bc.n_wall);
-        k_wall_mut<T><<<g, 128, 0, ctx.stream>>>(B, W, bc.wall);
-    }
-    ctx.mark("baldwin_lomax", 0, 4);
-    ctx.mark("time_step", 1, 2);
-    if (P.equation_ns) k_cell_b<T, true><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, PC, GW, W, level);
-    else k_cell_b<T, false><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, PC, GW, W, level);
+    ctx.mark("baldwin_lomax", 0, 2);
+    ctx.mark("time_step", 1, 1);
+    dim3 g = ctx.grid_cells(256);
+    const unsigned nb = g.x, pw = (unsigned)((bc.max_wall + 255) / 256);
+    g.x += (pw * bc.n_wall + B.nsolve - 1) / B.nsolve;
+    if (P.equation_ns) k_cell_b<T, true><<<g, 256, 0, ctx.stream>>>(B, PC, GW, W, level, nb, bc.wall, pw, bc.n_wall);
+    else k_cell_b<T, false><<<g, 256, 0, ctx.stream>>>(B, PC, GW, W, level, nb, bc.wall, pw, bc.n_wall);
     if (P.global_dt) {
         k_dt_min<T><<<dim3(1, B.nsolve), 1024, 0, ctx.stream>>>(B, W, scratch);
         k_dt_set<T><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, PC, GW, W, scratch);
     }
-    k_after_timestep<<<(B.nsolve + 127) / 128, 128, 0, ctx.stream>>>(B, level);
-    ctx.mark("time_step", 0, 2);
+    ctx.mark("time_step", 0, 1);
 }
 
 template void launch_cell_stages<double>(const LaunchCtx &, const Phys &, const PhysW<double> &, const Geo &,

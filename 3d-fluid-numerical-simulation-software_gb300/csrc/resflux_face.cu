@@ -140,9 +140,11 @@ __global__ void __launch_bounds__(128) k_jst_dissip(Batch B, Phys P, Flow<T> W)
 // terms are compile-time switches (NS, JST), so that every load of a cell is issued before the
 // first sum instead of behind a branch.
 template <typename T, bool NS, bool JST>
-__global__ void __launch_bounds__(256) k_cell_sum(Batch B, GeoW<T> G, Flow<T> W)
+__global__ void __launch_bounds__(256) k_cell_sum(Batch B, GeoW<T> G, Flow<T> W, int level)
 {
     const int s = blockIdx.y;
+    // decrement of the low-time-step counter, after the time step used it
+    if (blockIdx.x == 0 && threadIdx.x == 0 && B.st[s].flag_low_dt[level] > 0) B.st[s].flag_low_dt[level] -= 1;
     const Lvl L = B.lv[s];
     int i, j, k;
     if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
@@ -215,10 +217,10 @@ void launch_resflux(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC, con
     }
     ctx.mark("cell_sum", 1);
     const bool jst = W.Fd[0][0] != nullptr;
-    if (P.equation_ns && !jst) k_cell_sum<T, true, false><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, GW, W);
-    else if (P.equation_ns) k_cell_sum<T, true, true><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, GW, W);
-    else if (!jst) k_cell_sum<T, false, false><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, GW, W);
-    else k_cell_sum<T, false, true><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, GW, W);
+    if (P.equation_ns && !jst) k_cell_sum<T, true, false><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, GW, W, level);
+    else if (P.equation_ns) k_cell_sum<T, true, true><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, GW, W, level);
+    else if (!jst) k_cell_sum<T, false, false><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, GW, W, level);
+    else k_cell_sum<T, false, true><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, GW, W, level);
     ctx.mark("cell_sum", 0);
 }
 

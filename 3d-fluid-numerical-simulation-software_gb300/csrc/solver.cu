@@ -335,8 +335,7 @@ public:
     bool reuse = false;                   // the cases start from a restart file (config "use previous solution")
     bool any_mass = false;                // some case imposes its mass flow through the back pressure
     SolveState *st_d = nullptr;
-    int *bad_list = nullptr, *bad_count = nullptr;
-    const int bad_cap = 4096;
+    LimitLists limits{nullptr, 4096, nullptr, nullptr};
     double *norm_part = nullptr;
     double *init_q = nullptr;             // uniform start: five conserved values per slot
     const int norm_blk = 304;            // most blocks of a slot in the residual norm: two per SM
@@ -524,15 +523,17 @@ public:
         }
         CK(cudaMemcpy(st_d, st.data(), st_mem.bytes, cudaMemcpyHostToDevice));
         // scratch: limiter lists, norm partials, global-dt minima
-        size_t sb = sizeof(int) * (size_t)nsolve * (bad_cap + 1) + sizeof(double) * (size_t)nsolve * (norm_blk + 1) * 5 +
+        size_t sb = sizeof(int) * (size_t)nsolve * (limits.cap + 2) + sizeof(double) * (size_t)nsolve * (norm_blk + 1) * 5 +
                     sizeof(unsigned) * nsolve + sizeof(T) * nsolve + 256;
         scratch_mem.bytes = sb;
         CK(cudaMalloc(&scratch_mem.p, sb));
         char *q = (char *)scratch_mem.p;
         norm_part = (double *)q; q += sizeof(double) * (size_t)nsolve * norm_blk * 5;
         init_q = (double *)q; q += sizeof(double) * (size_t)nsolve * 5;
-        bad_list = (int *)q; q += sizeof(int) * (size_t)nsolve * bad_cap;
-        bad_count = (int *)q; q += sizeof(int) * nsolve;
+        limits.list = (int *)q; q += sizeof(int) * (size_t)nsolve * limits.cap;
+        limits.count = (int *)q; q += sizeof(int) * nsolve;
+        limits.done = (unsigned *)q; q += sizeof(unsigned) * nsolve;
+        CK(cudaMemset(limits.count, 0, 2 * sizeof(int) * nsolve));
         norm_count = (unsigned *)q; q += sizeof(unsigned) * nsolve;
         CK(cudaMemset(norm_count, 0, sizeof(unsigned) * nsolve));
         dtmin = (T *)(((uintptr_t)q + 15) & ~(uintptr_t)15);
@@ -657,6 +658,7 @@ public:
         CK(cudaMalloc(&Lv.int_mem.p, Lv.int_mem.bytes));
         CK(cudaMemset(Lv.int_mem.p, 0, Lv.int_mem.bytes));
         W.blmin = (unsigned long long *)Lv.int_mem.p;
+        CK(cudaMemset(W.blmin, 0xFF, sizeof(unsigned long long) * N));       // (k_bl_merge leaves it like this)
         int *ip = (int *)(W.blmin + N);
         int *wallf[3] = {ip, ip + N, ip + 2 * N};
         for (int f = 0; f < 3; f++) W.wallf[f] = wallf[f];
@@ -1165,8 +1167,7 @@ public:
     {
         LaunchCtx cx = ctx(l);
         Level<T> &Lv = lev[l];
-        launch_lusgs_sweeps<T>(cx, PC, Lv.G, Lv.W, Lv.wave, Lv.wave_var);
-        launch_update<T>(cx, P, Lv.G, Lv.W, l, bad_list, bad_cap, bad_count);
+        launch_lusgs_sweeps<T>(cx, P, PC, Lv.G, Lv.W, Lv.wave, Lv.wave_var, l, limits);
     }
     // transfers between level lf and the next coarser one
     void restrict_lv(int lf)
@@ -1174,10 +1175,16 @@ public:
         Mark m(this, "mg_restrict");
         launch_restrict<T>(ctx(lf), ctx(lf + 1), lev[lf].G, lev[lf + 1].G, lev[lf].W, lev[lf + 1].W);
     }
-    void interpolate_lv(int lf, int init)
+    // the same with the receiving level's primitive variables and limiter
+    void restrict_primitive(int lf)
+    {
+        Mark m(this, "mg_restrict");
+        launch_restrict_primitive<T>(ctx(lf), ctx(lf + 1), P, lev[lf].G, lev[lf + 1].G, lev[lf].W, lev[lf + 1].W, lf + 1, limits);
+    }
+    void interpolate_primitive(int lf, int init)
     {
         Mark m(this, "mg_prolong");
-        launch_interpolate<T>(ctx(lf), ctx(lf + 1), lev[lf].W, lev[lf + 1].W, init);
+        launch_interpolate_primitive<T>(ctx(lf), ctx(lf + 1), P, lev[lf].W, lev[lf + 1].W, init, lf, limits);
     }
     void delta_lv(int lc) { Mark m(this, "mg_delta"); launch_delta<T>(ctx(lc), lev[lc].W); }
     // FAS smoothing of coarse level l (three-level extension): residual at the restricted state,
@@ -1199,7 +1206,7 @@ public:
         launch_res_norm_static<T>(ctx(l), lev[l].G, lev[l].W, lev[l].totalvol, ncase, host_out);
     }
     void primitive_vars(int l) override { Mark m(this, "primitive"); launch_primitive<T>(ctx(l), P, lev[l].W); }
-    void limit_vars(int l) override { Mark m(this, "limiter", 2); launch_limiter<T>(ctx(l), P, lev[l].W, l, bad_list, bad_cap, bad_count); }
+    void limit_vars(int l) override { Mark m(this, "limiter", 1); launch_limiter<T>(ctx(l), P, lev[l].W, l, limits); }
     void corner_treatment(int l) override { Mark m(this, "mg_corner", 2); launch_corner<T>(ctx(l), lev[l].W); }
     void restrict_to_coarse() override
     {
@@ -1237,39 +1244,33 @@ public:
         if (!reuse && iter < coarse_iter) { time_marching(2); res_calculate(2); }
         else if (!reuse && iter == coarse_iter) {
             time_marching(2); res_calculate(2); corner_treatment(2);
-            interpolate(1); primitive_vars(1); limit_vars(1);
+            interpolate_primitive(1, 1);
         } else if (ng == 2) {
             lev[2].use_force = true;
             time_marching(1); res_calculate(1);
             resflux(1);
-            restrict_to_coarse();
-            primitive_vars(2); limit_vars(2);
+            restrict_primitive(1);
             time_marching(2);
             delta_cons();
             corner_treatment(2);
-            interpolate(0);
-            primitive_vars(1); limit_vars(1);
+            interpolate_primitive(1, 0);
         } else {
             // three-level V-cycle (extension): the fine step as in the two-level cycle, then FAS
             // on levels 2 and 3 with the coarse residuals evaluated at the restricted states
             time_marching(1); res_calculate(1);
             resflux(1);
-            restrict_lv(1);
-            primitive_vars(2); limit_vars(2);
+            restrict_primitive(1);
             smooth_fas(2);
             resflux(2);
             { Mark m(this, "mg_forcing"); launch_add_forcing<T>(ctx(2), lev[2].W); }
-            restrict_lv(2);
-            primitive_vars(3); limit_vars(3);
+            restrict_primitive(2);
             smooth_fas(3);
             delta_lv(3);
             corner_treatment(3);
-            interpolate_lv(2, 0);
-            primitive_vars(2); limit_vars(2);
+            interpolate_primitive(2, 0);
             delta_lv(2);
             corner_treatment(2);
-            interpolate_lv(1, 0);
-            primitive_vars(1); limit_vars(1);
+            interpolate_primitive(1, 0);
         }
     }
     // the level whose integrals an iteration reports (source/Structured_FV3D.cpp:150-156: the coarse

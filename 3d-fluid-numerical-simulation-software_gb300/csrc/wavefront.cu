@@ -31,7 +31,8 @@
 // Every input of a step lies in one block of memory ([step][values][cells]) and comes through a ring in
 // shared memory by bulk copies. k_wave_gather writes the blocks with everything a cell can form without
 // its neighbours: the right-hand side, its terms' coefficients and, in FP64, its old fluxes (in FP32 they
-// are formed in the sweep: the bytes cost more there). k_wave_scatter turns dQ back into box order.
+// are formed in the sweep: the bytes cost more there). k_wave_update turns dQ back into box order and
+// applies it.
 //
 // A cell sends one term per direction d (the reference's A and V terms of a neighbour, :95-150, 293-419),
 //   w_d = h_d (F_d(Q + dQ) - F_d(Q)) +- c_d dQ      (+ forward, - backward)
@@ -46,6 +47,7 @@
 #include "gbt_common.cuh"
 #include "kernels.hpp"
 #include "flux.cuh"
+#include "update.cuh"
 
 namespace gbt {
 
@@ -736,30 +738,63 @@ __global__ void __launch_bounds__(256) k_wave_geometry(Batch B, Geo G, WaveTable
     }
 }
 
-// ---- dQ of some steps of a tile back into box order: contiguous pieces in, runs along k out
+// ---- dQ back into box order and applied: Q_old = Q, Q += dQ (FP64 in both precision forms), primitive
+// variables, limiter. A block takes the 32 k of every column of a tile that share a line of the box (the
+// rows' padded index a multiple of 32 on), which lie in up to 42 steps. Bound by HBM (184 bytes a cell in
+// the mixed form) on large batches: 12 solves on three meshes 0.255 ms per cycle as two launches, scatter
+// and update, 0.214 as one; with runs of 16 or 32 k that start anywhere, 0.352 and 0.285.
+constexpr int kRun = 32;
+__host__ __device__ inline int runs_of(int nK) { return (nK + PAD) / kRun + 1; }
 template <typename T>
-__global__ void __launch_bounds__(256) k_wave_scatter(Batch B, Flow<T> W, WaveTables V)
+__global__ void __launch_bounds__(256) k_wave_update(Batch B, Phys P, Flow<T> W, WaveTables V, int level, LimitLists q)
 {
     using L = Lay<T, MEAN>;
-    constexpr int PA = L::PA, NC = L::NC, CH = 32, NW = L::dq / 16, stride = NW + 1;
-    __shared__ float4 tile[CH * stride];
-    const Chunk c = chunk_of(V, CH);
-    if (!c.live) return;
-    const Lvl Lv = B.lv[blockIdx.y];
-    const float4 *src = (const float4 *)(V.dq + c.step * L::dq);
-    for (int e = threadIdx.x; e < c.nt * NW; e += 256) tile[(e / NW) * stride + e % NW] = src[e];
-    __syncthreads();
-    const int st = threadIdx.x % CH;
-    for (int cell = threadIdx.x / CH; cell < NC; cell += 256 / CH) {
-        const int a = cell / PB, b = cell % PB;
-        const int i = c.PI * PA + a + 1, j = c.PJ * PB + b + 1, k = c.t0 + st - a - b + 1;
-        if (st >= c.nt || i > c.S.nI || j > c.S.nJ || k < 1 || k > c.S.nK) continue;
-        const long long p = ix(Lv, i, j, k);
-        const T *d = (const T *)(tile + st * stride);
+    constexpr int PA = L::PA, NC = L::NC, R = NC * kRun / 256, NW = L::dq / 16, stride = NW + 1, ST = kRun + PA + PB - 2;
+    __shared__ float4 tile[ST * stride];
+    const int s = blockIdx.y;
+    const WaveSolve S = V.solve[s];
+    const int nr = runs_of(S.nK), p = (int)blockIdx.x / nr, k0 = ((int)blockIdx.x - p * nr) * kRun - PAD;
+    if (p >= S.nPI * S.nPJ) return;
+    const int PI = p / S.nPJ, PJ = p - PI * S.nPJ;
+    const Lvl Lv = B.lv[s];
+    // cells (a, b, k) of the run, at step k - 1 + a + b
+    const int kk = k0 + (int)threadIdx.x % kRun, c0 = (int)threadIdx.x / kRun;
+    bool in[R];
+    long long at[R];
+    double o[R][5];
 #pragma unroll
-        for (int n = 0; n < 4; n++) W.dq[n][p] = d[4 * cell + n];
-        W.dq[4][p] = d[4 * NC + cell];
+    for (int r = 0; r < R; r++) {
+        const int cell = c0 + r * (256 / kRun), i = PI * PA + cell / PB + 1, j = PJ * PB + cell % PB + 1;
+        in[r] = i <= S.nI && j <= S.nJ && kk >= 1 && kk <= S.nK;
+        at[r] = ix(Lv, i, j, kk);
+#pragma unroll
+        for (int n = 0; n < 5; n++) o[r][n] = in[r] ? W.cv[n][at[r]] : 0.0;
     }
+    const int t0 = max(0, k0 - 1), t1 = min(S.T, k0 - 1 + ST);
+    const float4 *src = (const float4 *)(V.dq + (S.step0 + (long long)p * S.T + t0) * L::dq);
+    for (int e = threadIdx.x; e < (t1 - t0) * NW; e += 256) tile[(e / NW) * stride + e % NW] = src[e];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        if (!in[r]) continue;
+        const int cell = c0 + r * (256 / kRun), a = cell / PB, b = cell % PB;
+        const T *d = (const T *)(tile + (kk - 1 + a + b - t0) * stride);
+        double cv[5];
+#pragma unroll
+        for (int n = 0; n < 5; n++) {
+            const T dq = n < 4 ? d[4 * cell + n] : d[4 * NC + cell];
+            W.dq[n][at[r]] = dq;
+            W.cvold[n][at[r]] = o[r][n];
+            cv[n] = o[r][n] + to_f64<T>(dq);
+            W.cv[n][at[r]] = cv[n];
+        }
+        T v[6];
+        prim_from_cons<T>(P, cv, v);
+#pragma unroll
+        for (int n = 0; n < 6; n++) W.pv[n][at[r]] = v[n];
+        limit_flag<T>(P, q, Lv, s, PI * PA + a + 1, PJ * PB + b + 1, kk, v);
+    }
+    limit_done<T>(B, P, W, level, q, s, (unsigned)(S.nPI * S.nPJ * nr));
 }
 
 template <typename T>
@@ -825,7 +860,8 @@ void launch_wave_geometry(const LaunchCtx &ctx, const Geo &G, const WaveTables &
 }
 
 template <typename T>
-void launch_lusgs_sweeps(const LaunchCtx &ctx, const PhysW<T> &P, const Geo &G, Flow<T> W, const WaveTables &V, const WaveTables &VV)
+void launch_lusgs_sweeps(const LaunchCtx &ctx, const Phys &PH, const PhysW<T> &P, const Geo &G, Flow<T> W, const WaveTables &V,
+                         const WaveTables &VV, int level, const LimitLists &q)
 {
     auto chunks = [&](int steps) { return dim3((unsigned)(V.max_tiles * ((V.max_T + steps - 1) / steps)), ctx.batch.nsolve); };
     ctx.mark("sweep_forward", 1, 2);
@@ -849,15 +885,24 @@ void launch_lusgs_sweeps(const LaunchCtx &ctx, const PhysW<T> &P, const Geo &G, 
         k_wave_scatter_var<T><<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, W, VV);
         ctx.mark("sa_sweeps", 0, 3);
     }
-    ctx.mark("sweep_scatter", 1, 1);
-    k_wave_scatter<T><<<chunks(32), 256, 0, ctx.stream>>>(ctx.batch, W, V);
-    ctx.mark("sweep_scatter", 0, 1);
+    ctx.mark("update_limiter", 1, 1);
+    k_wave_update<T><<<dim3((unsigned)(V.max_tiles * runs_of(ctx.maxKM - 1)), ctx.batch.nsolve), 256, 0, ctx.stream>>>(ctx.batch, PH, W, V, level, q);
+    if (W.ev) {
+        // the variable's update and Limit_SA after the mean flow's (source/LU_SGS_Marching.cpp:275-277,
+        // source/ComputeAllBlockVars.cpp:257-266); the limiter's list is reused
+        launch_sa_update<T>(ctx, PH, W, q.list, q.cap, q.count);
+        if (PH.limiter) {
+            launch_sa_limit<T>(ctx, W, q.list, q.cap, q.count);
+            cudaMemsetAsync(q.count, 0, sizeof(int) * ctx.batch.nsolve, ctx.stream);
+        }
+    }
+    ctx.mark("update_limiter", 0, 1);
 }
 
 #define GBT_WAVE_INST(T)                                                                                              \
     template void launch_wave_geometry<T>(const LaunchCtx &, const Geo &, const WaveTables &);                        \
-    template void launch_lusgs_sweeps<T>(const LaunchCtx &, const PhysW<T> &, const Geo &, Flow<T>, const WaveTables &, \
-                                         const WaveTables &);
+    template void launch_lusgs_sweeps<T>(const LaunchCtx &, const Phys &, const PhysW<T> &, const Geo &, Flow<T>,     \
+                                         const WaveTables &, const WaveTables &, int, const LimitLists &);
 GBT_WAVE_INST(double)
 GBT_WAVE_INST(float)
 
