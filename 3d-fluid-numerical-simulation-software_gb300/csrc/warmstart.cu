@@ -5,8 +5,9 @@
 //   forward        Z[cells x N]   = H[cells x K] . W[N x K]^T        (+ bias, SiLU in the epilogue)
 //   backward data  dH[cells x K]  = dZ[cells x N] . W[N x K]          (x SiLU'(Z) in the epilogue)
 //   weight grad    dW[N x K]      = dZ^T . H  (the cells are the reduction dimension)
-// Operands are staged in shared memory in the canonical K-major layout without swizzle (core
-// matrices of 8 rows x 16 bytes, 128 contiguous bytes each), one elected thread issues
+// Operands are staged in shared memory by TMA in the 128-byte swizzle (boxes of 64 columns, a row of 128
+// bytes; operands of 16 columns and the activations of the fused inference in core matrices of 8 rows x
+// 16 bytes, without swizzle), one elected thread issues
 // tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M = 128), tcgen05.commit arrives on an mbarrier
 // that every thread waits on (bounded), and the epilogue reads the accumulator rows with
 // tcgen05.ld (warp w owns TMEM lanes 32w..32w+31, i.e. rows 32w..32w+31 of the tile).
@@ -37,6 +38,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+}
+// the same for an operand in the 128-byte swizzle (bits 61-63 = 2; 1024-byte groups of eight 128-byte rows).
+// K-major: sbo is the distance of groups adjacent along M/N, lbo is not read. MN-major (a row is 64 elements
+// of M/N): lbo is the distance of blocks of 64 along M/N, sbo that of groups adjacent along K.
+__device__ __forceinline__ uint64_t smem_desc_sw(uint32_t addr, uint32_t lbo, uint32_t sbo)
+{
+    return smem_desc(addr, lbo, sbo) | (2ull << 61);
 }
 // instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1),
 // both K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
@@ -107,27 +115,46 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16])
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// the same for 32 columns
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32])
+{
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+
 // ---------------------------------------------------------------- operand staging
 __device__ __forceinline__ float sigmoidf_(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
 
 // ---------------------------------------------------------------- the row product
-// D[128 x N] = A[128 x K] . B[N x K]^T per tile of 128 rows (cells); N, K multiples of 16, N <= 256,
-// K <= 256. Warp-specialised and persistent over the row tiles:
-//   warp 16: TMA producer. For every K chunk of up to 64 elements it loads, into one stage of a
-//     4-deep shared-memory ring, the A chunk (128 rows) and the B chunk (N rows) as boxes of
-//     8 elements x rows from 2D tensor maps; a box lands as rows x 16 bytes, i.e. a column of core
-//     matrices of the K-major layout (M/N neighbours 128 bytes apart, K neighbours one box apart).
-//     Rows past M read as zeros.
+// D[128 x N] = A[128 x K] . B[N x K]^T per tile of 128 rows (cells); K 16 or a multiple of 64, N and K <= 256.
+// Warp-specialised and persistent over the row tiles:
+//   warp 16: TMA producer. Loads B once, it stays for every tile of the CTA, and streams A, a chunk of
+//     128 rows x 64 columns at a time, through a 4-deep ring. Both land in the 128-byte swizzle: a
+//     row of a box is 128 bytes. Rows past M read as zeros. (K = 16: boxes of 8 columns, no swizzle.)
 //   warp 17: MMA issuer. Waits for a stage, issues its tcgen05.mma (K = 16 each) into one of two TMEM
 //     accumulators (256 columns each), and tcgen05.commit frees the stage when they complete;
 //     after a tile's last chunk a commit marks the accumulator full.
 //   warps 0-15: epilogue. Read the full accumulator (warp w: TMEM lanes 32(w%4)..32(w%4)+31, the
 //     (w/4)-th quarter of the columns), apply the epilogue, store, and hand the accumulator back,
-//     while the next tile accumulates in the other.
+//     while the next tile accumulates in the other. Rows of 32 BF16 columns pass through 2 KB of shared
+//     memory per warp, so that a store or load covers 8 rows x 64 bytes instead of 32 rows x 16.
+// Bound by the epilogue (two MUFU operations an element, 32768 elements a tile) once the loads are wide: with
+// boxes of 8 columns a tile took 12288 rows of 16 bytes, about one a clock, and 32768 x 256 x 256 29 us;
+// now 16 us.
 // Epilogues:
-//   0: z = D + bias -> Z (BF16), H = SiLU(z) (BF16)
+//   0: z = D + bias -> Z (BF16), H = SiLU(z) (BF16)      N = 256
 //   1: y = D + bias -> Y (FP32)
-//   2: dZ = D * SiLU'(Zp) (BF16)
+//   2: dZ = D * SiLU'(Zp) (BF16)                           N = 256
 struct GemmArgs {
     long long M; int N, K;
     const float *bias;
@@ -136,10 +163,12 @@ struct GemmArgs {
     int *err;
 };
 
-constexpr int kTcSmem = 200 * 1024;              // one CTA per SM (and so at most 512 TMEM columns in use)
 constexpr int kStages = 4, kChunk = 64;
 constexpr int kEpiWarps = 16;                    // four per TMEM lane quadrant
 constexpr int kStageA = 128 * kChunk * 2, kStageB = 256 * kChunk * 2;
+constexpr int kMaxChunks = kWsHidden / kChunk;
+constexpr int kEpiStage = 32 * 64;               // 32 rows x 32 BF16 columns per epilogue warp
+constexpr int kTcSmem = kMaxChunks * kStageB + kStages * kStageA + kEpiWarps * kEpiStage + 256;
 
 __host__ __device__ inline int tmem_cols(int n) { int c = 32; while (c < n) c <<= 1; return c; }
 
@@ -159,51 +188,76 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
+// 32 rows x 32 BF16 columns (one row per lane in v) to rows row0.. of dst through the warp's 2 KB
+__device__ __forceinline__ void store_rows32(unsigned char *st, int lane, const bf16 v[32], bf16 *dst, long long row0, long long M, long long ld)
+{
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        *reinterpret_cast<uint4 *>(st + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = reinterpret_cast<const uint4 *>(v)[c];
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int r = q * 8 + (lane >> 2), c = lane & 3;
+        const uint4 w = *reinterpret_cast<const uint4 *>(st + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+        if (row0 + r < M) *reinterpret_cast<uint4 *>(dst + (row0 + r) * ld + c * 8) = w;
+    }
+    __syncwarp();
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_gemm(const __grid_constant__ CUtensorMap tmA,
                                                      const __grid_constant__ CUtensorMap tmB, GemmArgs g)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    unsigned char *ring = sm;                                           // kStages x (A | B)
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + kStages * (kStageA + kStageB));
-    // bars: full[kStages], empty[kStages], acc_full[2], acc_empty[2]
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2 * kStages + 4);
+    unsigned char *wsm = sm, *ring = sm + kMaxChunks * kStageB, *epi = ring + kStages * kStageA;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(epi + kEpiWarps * kEpiStage);
+    // bars: full[kStages], empty[kStages], acc_full[2], acc_empty[2], b_full[kMaxChunks]
+    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2 * kStages + 4 + kMaxChunks);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t bar0 = smem_u32(bars);
     auto full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
     auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(kStages + s); };
     auto accf = [&](int a) { return bar0 + 8u * (uint32_t)(2 * kStages + a); };
     auto acce = [&](int a) { return bar0 + 8u * (uint32_t)(2 * kStages + 2 + a); };
+    auto bfull = [&](int c) { return bar0 + 8u * (uint32_t)(2 * kStages + 4 + c); };
     if (warp == kEpiWarps) tmem_alloc(smem_u32(slot), 512);
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
         for (int a = 0; a < 2; a++) { mbar_init(accf(a), 1); mbar_init(acce(a), kEpiWarps); }
+        for (int c = 0; c < kMaxChunks; c++) mbar_init(bfull(c), 1);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *slot;
-    const int chunk = g.K < kChunk ? g.K : kChunk, nchunk = g.K / chunk, nk8 = chunk / 8;
+    const bool sw = g.K >= kChunk;
+    const int chunk = sw ? kChunk : g.K, nchunk = g.K / chunk, nbox = sw ? 1 : chunk / 8, wbox = sw ? kChunk : 8;
     const long long tiles = (g.M + 127) / 128;
     bool failed = false;
     if (warp == kEpiWarps) {
         if (lane == 0) {
-            const uint32_t bytes = (uint32_t)nk8 * (128u + (uint32_t)g.N) * 16u;
             long long it = 0;
             for (long long t = blockIdx.x; t < tiles && !failed; t += gridDim.x)
                 for (int kc = 0; kc < nchunk; kc++, it++) {
                     const int s = (int)(it % kStages);
-                    const uint32_t ph = (uint32_t)((it / kStages) & 1);
-                    if (!mbar_wait_bounded(empty(s), ph ^ 1u)) { failed = true; break; }
-                    mbar_expect_tx(full(s), bytes);
-                    const uint32_t a_s = smem_u32(ring + (size_t)s * (kStageA + kStageB));
-                    const uint32_t b_s = a_s + kStageA;
-                    for (int k8 = 0; k8 < nk8; k8++) {
-                        const int x = kc * chunk + k8 * 8;
-                        tma_load_2d(a_s + (uint32_t)k8 * 128u * 16u, &tmA, x, (int)(t * 128), full(s));
-                        tma_load_2d(b_s + (uint32_t)k8 * (uint32_t)g.N * 16u, &tmB, x, 0, full(s));
+                    if (it < nchunk) {
+                        mbar_expect_tx(bfull(kc), (uint32_t)chunk * (uint32_t)g.N * 2u);
+                        for (int b = 0; b < nbox; b++)
+                            tma_load_2d(smem_u32(wsm + (size_t)kc * kStageB) + (uint32_t)b * (uint32_t)g.N * 16u, &tmB, kc * chunk + b * wbox, 0,
+                                        bfull(kc));
                     }
+                    if (!mbar_wait_bounded(empty(s), (uint32_t)((it / kStages) & 1) ^ 1u)) { failed = true; break; }
+                    mbar_expect_tx(full(s), (uint32_t)chunk * 128u * 2u);
+                    for (int b = 0; b < nbox; b++)
+                        tma_load_2d(smem_u32(ring + (size_t)s * kStageA) + (uint32_t)b * 128u * 16u, &tmA, kc * chunk + b * wbox, (int)(t * 128),
+                                    full(s));
                 }
+            // nothing of a tile that was given up on may still be on its way when the CTA ends
+            if (failed) {
+                for (int c = 0; c < nchunk && c < it; c++) mbar_wait_bounded(bfull(c), 0u);
+                for (long long q = it < kStages ? 0 : it - kStages; q < it; q++)
+                    mbar_wait_bounded(full((int)(q % kStages)), (uint32_t)((q / kStages) & 1));
+            }
         }
     } else if (warp == kEpiWarps + 1) {
         if (lane == 0) {
@@ -215,14 +269,16 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_gemm(const __gr
                 tc_fence_after();
                 for (int kc = 0; kc < nchunk; kc++, it++) {
                     const int s = (int)(it % kStages);
+                    if (it < nchunk && !mbar_wait_bounded(bfull(kc), 0u)) { failed = true; break; }
                     if (!mbar_wait_bounded(full(s), (uint32_t)((it / kStages) & 1))) { failed = true; break; }
                     tc_fence_after();
-                    const uint32_t a_s = smem_u32(ring + (size_t)s * (kStageA + kStageB));
-                    const uint32_t b_s = a_s + kStageA;
+                    const uint32_t a_s = smem_u32(ring + (size_t)s * kStageA), b_s = smem_u32(wsm + (size_t)kc * kStageB);
                     for (int ks = 0; ks < chunk / 16; ks++)
-                        mma_bf16(tmem + (uint32_t)(a * 256), smem_desc(a_s + (uint32_t)ks * 2u * 2048u, 2048u, 128u),
-                                 smem_desc(b_s + (uint32_t)ks * 2u * (uint32_t)g.N * 16u, (uint32_t)g.N * 16u, 128u), idesc,
-                                 (kc > 0 || ks > 0) ? 1u : 0u);
+                        mma_bf16(tmem + (uint32_t)(a * 256),
+                                 sw ? smem_desc_sw(a_s + (uint32_t)ks * 32u, 16u, 1024u) : smem_desc(a_s + (uint32_t)ks * 4096u, 2048u, 128u),
+                                 sw ? smem_desc_sw(b_s + (uint32_t)ks * 32u, 16u, 1024u)
+                                    : smem_desc(b_s + (uint32_t)ks * 2u * (uint32_t)g.N * 16u, (uint32_t)g.N * 16u, 128u),
+                                 idesc, (kc > 0 || ks > 0) ? 1u : 0u);
                     mma_commit(empty(s));
                 }
                 if (failed) break;
@@ -231,51 +287,82 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_gemm(const __gr
         }
     } else {
         long long ai = 0;
+        unsigned char *st = epi + warp * kEpiStage;
         for (long long t = blockIdx.x; t < tiles; t += gridDim.x, ai++) {
             const int a = (int)(ai & 1);
-            const bool ok = mbar_wait_bounded(accf(a), (uint32_t)((ai >> 1) & 1));
-            tc_fence_after();
-            if (!ok) { failed = true; break; }
             const int quad = warp & 3;
-            const int cols = g.N >= 64 ? g.N / 4 : 16;        // a quarter of the columns, at least 16
-            const int cbeg = (warp >> 2) * cols, cend = cbeg + cols < g.N ? cbeg + cols : g.N;
-            const long long row = t * 128 + quad * 32 + lane;
-            const bool live = row < g.M;
-            for (int c0 = cbeg; c0 < cend; c0 += 16) {
-                float v[16];
-                tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * 256 + c0), v);
-                if (!live) continue;
-                if constexpr (EPI == 0) {
-                    alignas(16) bf16 zo[16], ho[16];
-#pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const float z = v[i] + g.bias[c0 + i];
-                        zo[i] = __float2bfloat16_rn(z);
-                        ho[i] = __float2bfloat16_rn(z * sigmoidf_(z));
-                    }
-                    uint4 *zp = reinterpret_cast<uint4 *>(g.Z + row * g.ldo + c0);
-                    uint4 *hp = reinterpret_cast<uint4 *>(g.H + row * g.ldo + c0);
-                    zp[0] = reinterpret_cast<uint4 *>(zo)[0]; zp[1] = reinterpret_cast<uint4 *>(zo)[1];
-                    hp[0] = reinterpret_cast<uint4 *>(ho)[0]; hp[1] = reinterpret_cast<uint4 *>(ho)[1];
-                } else if constexpr (EPI == 1) {
+            const long long row0 = t * 128 + quad * 32, row = row0 + lane;
+            const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * 256);
+            if constexpr (EPI == 1) {
+                const bool ok = mbar_wait_bounded(accf(a), (uint32_t)((ai >> 1) & 1));
+                tc_fence_after();
+                if (!ok) { failed = true; break; }
+                for (int c0 = (warp >> 2) * 16; c0 < g.N; c0 += 64) {
+                    float v[16];
+                    tmem_ld16(acc + (uint32_t)c0, v);
+                    if (row >= g.M) continue;
                     float4 *yp = reinterpret_cast<float4 *>(g.Y + row * g.ldo + c0);
 #pragma unroll
                     for (int i = 0; i < 4; i++)
                         yp[i] = make_float4(v[4 * i] + g.bias[c0 + 4 * i], v[4 * i + 1] + g.bias[c0 + 4 * i + 1],
                                             v[4 * i + 2] + g.bias[c0 + 4 * i + 2], v[4 * i + 3] + g.bias[c0 + 4 * i + 3]);
-                } else {
-                    alignas(16) bf16 zi[16], dz[16];
-                    const uint4 *zs = reinterpret_cast<const uint4 *>(g.Zp + row * g.ldo + c0);
-                    reinterpret_cast<uint4 *>(zi)[0] = zs[0];
-                    reinterpret_cast<uint4 *>(zi)[1] = zs[1];
+                }
+            } else {
+                const int cbeg = (warp >> 2) * 64;
+                uint4 zl[2][4];                          // Z of the warp's 64 columns, asked for before the wait
+                if constexpr (EPI == 2) {
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const float z = __bfloat162float(zi[i]);
-                        const float sg = sigmoidf_(z);
-                        dz[i] = __float2bfloat16_rn(v[i] * (sg * (1.0f + z * (1.0f - sg))));
+                    for (int h = 0; h < 2; h++)
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const long long r = row0 + q * 8 + (lane >> 2);
+                            zl[h][q] = r < g.M ? *reinterpret_cast<const uint4 *>(g.Zp + r * g.ldo + cbeg + h * 32 + (lane & 3) * 8)
+                                               : make_uint4(0u, 0u, 0u, 0u);
+                        }
+                }
+                const bool ok = mbar_wait_bounded(accf(a), (uint32_t)((ai >> 1) & 1));
+                tc_fence_after();
+                if (!ok) { failed = true; break; }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int c0 = cbeg + h * 32;
+                    float v[32];
+                    tmem_ld32(acc + (uint32_t)c0, v);
+                    if constexpr (EPI == 0) {
+                        alignas(16) bf16 zo[32], ho[32];
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4) {
+                            const float4 b = *reinterpret_cast<const float4 *>(g.bias + c0 + i);
+                            const float bb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                            for (int n = 0; n < 4; n++) {
+                                const float z = v[i + n] + bb[n];
+                                zo[i + n] = __float2bfloat16_rn(z);
+                                ho[i + n] = __float2bfloat16_rn(z * sigmoidf_(z));
+                            }
+                        }
+                        store_rows32(st, lane, zo, g.Z + c0, row0, g.M, g.ldo);
+                        store_rows32(st, lane, ho, g.H + c0, row0, g.M, g.ldo);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const int r = q * 8 + (lane >> 2), c = lane & 3;
+                            *reinterpret_cast<uint4 *>(st + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) = zl[h][q];
+                        }
+                        __syncwarp();
+                        alignas(16) bf16 zi[32], dz[32];
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            reinterpret_cast<uint4 *>(zi)[c] = *reinterpret_cast<const uint4 *>(st + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4));
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < 32; i++) {
+                            const float z = __bfloat162float(zi[i]);
+                            const float sg = sigmoidf_(z);
+                            dz[i] = __float2bfloat16_rn(v[i] * (sg * (1.0f + z * (1.0f - sg))));
+                        }
+                        store_rows32(st, lane, dz, g.dZ + c0, row0, g.M, g.ldo);
                     }
-                    uint4 *dp = reinterpret_cast<uint4 *>(g.dZ + row * g.ldo + c0);
-                    dp[0] = reinterpret_cast<uint4 *>(dz)[0]; dp[1] = reinterpret_cast<uint4 *>(dz)[1];
                 }
             }
             tc_fence_before();
@@ -292,20 +379,22 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_gemm(const __gr
 }
 
 // ---------------------------------------------------------------- inference, all layers fused
-// Y[rows x 16] = the whole network on X[rows x 64], per tile of 128 rows, the activations kept on
-// chip: the tile's activations live in one shared-memory buffer in the K-major core-matrix layout
-// (8-column groups 2 KB apart, rows 16 B apart), each layer's accumulator in TMEM. Roles as in
-// k_mlp_gemm, persistent over the tiles:
-//   warp 16: TMA producer. Loads the tile's features into the activation buffer once the previous
-//     tile's last layer has read it, and streams the weights, 64-column chunk by chunk, layer by
-//     layer, through a 3-stage ring (the same chunks for every tile; they stay in L2).
-//   warp 17: MMA issuer. Per layer: waits for the epilogue of the layer before (its outputs are this
-//     layer's inputs, and it has read the accumulator out), issues the layer's MMAs with A from the
-//     activation buffer, commits the accumulator; after the last layer it frees the buffer.
-//   warps 0-15: epilogue. Per layer: bias and SiLU of the accumulator, rounded to BF16 and written
+// Y[rows x 16] = the whole network on X[rows x 64], the activations kept on chip. A CTA works on two tiles of
+// 128 rows in turn, so that the tensor cores run a layer of one while the epilogue warps are on the
+// other: each has a shared-memory buffer of activations (K-major core matrices: 8-column groups 2 KB
+// apart, rows 16 B apart) and a TMEM accumulator. Roles as in k_mlp_gemm, persistent over the tiles:
+//   warp 16: TMA producer. Loads a tile's features into its activation buffer once the last layer of the
+//     buffer's previous tile has read it, and streams the weights, 64-column chunk by chunk in the
+//     128-byte swizzle, layer by layer and tile by tile, through a 3-stage ring (they stay in L2).
+//   warp 17: MMA issuer. Per layer and tile: waits for the tile's epilogue of the layer before (its
+//     outputs are this layer's inputs, and it has read the accumulator out), issues the layer's MMAs with A
+//     from the activation buffer, commits the accumulator; after the last layer it frees the buffer.
+//   warps 0-15: epilogue. Per layer and tile: bias and SiLU of the accumulator, rounded to BF16 and written
 //     over the activation buffer (hidden layers), or bias and FP32 rows of Y (the output layer).
-// The arithmetic is the layer-by-layer forward's (same MMA order, same epilogue), so the outputs
-// are the same bits; nothing but X and Y crosses HBM.
+// The arithmetic is the layer-by-layer forward's (same MMA order, same epilogue), so the outputs are the
+// same bits; nothing but X and Y crosses HBM. Bound by the epilogue's MUFU operations (two an
+// element, 16 a clock: 144 us for 262144 rows); with boxes of 8 columns (about one row of 16 bytes a
+// clock) and one tile at a time 375 us, now 196 us.
 struct InferArgs {
     long long M;
     const float *bias[kWsLayers];
@@ -314,7 +403,7 @@ struct InferArgs {
 };
 constexpr int kInfStages = 3;
 constexpr int kInfH = 128 * kWsHidden * 2;                  // 64 KB of activations
-constexpr int kInfSmem = kInfH + kInfStages * kStageB + 256;
+constexpr int kInfSmem = 2 * kInfH + kInfStages * kStageB + 256;
 __host__ __device__ constexpr int inf_n(int l) { return l == kWsLayers - 1 ? kWsOut : kWsHidden; }
 __host__ __device__ constexpr int inf_chunks(int l) { return l == 0 ? kWsIn / kChunk : kWsHidden / kChunk; }
 
@@ -324,123 +413,160 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_infer(
     const __grid_constant__ CUtensorMap tw5, InferArgs g)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    unsigned char *hbuf = sm;                                           // activations
-    unsigned char *ring = sm + kInfH;                                   // weight chunks
-    uint64_t *bars = reinterpret_cast<uint64_t *>(ring + kInfStages * kStageB);
-    // bars: full[3], empty[3], x_full, h_free, acc_full, h_ready
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2 * kInfStages + 4);
+    unsigned char *ring = sm;                                           // weight chunks
+    unsigned char *hbuf = sm + kInfStages * kStageB;                    // activations of two tiles
+    uint64_t *bars = reinterpret_cast<uint64_t *>(hbuf + 2 * kInfH);
+    // bars: full[3], empty[3]; of each tile x_full, h_free, acc_full, h_ready
+    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2 * kInfStages + 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t bar0 = smem_u32(bars);
     auto full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
     auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(kInfStages + s); };
-    const uint32_t x_full = bar0 + 8u * (2 * kInfStages), h_free = x_full + 8u, acc_full = x_full + 16u,
-                   h_ready = x_full + 24u;
-    const uint32_t hb = smem_u32(hbuf);
-    if (warp == kEpiWarps) tmem_alloc(smem_u32(slot), 256);
+    auto x_full = [&](int h) { return bar0 + 8u * (uint32_t)(2 * kInfStages + 4 * h); };
+    auto h_free = [&](int h) { return x_full(h) + 8u; };
+    auto acc_full = [&](int h) { return x_full(h) + 16u; };
+    auto h_ready = [&](int h) { return x_full(h) + 24u; };
+    if (warp == kEpiWarps) tmem_alloc(smem_u32(slot), 512);
     if (threadIdx.x == 0) {
         for (int s = 0; s < kInfStages; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        mbar_init(x_full, 1);
-        mbar_init(h_free, 1);
-        mbar_init(acc_full, 1);
-        mbar_init(h_ready, kEpiWarps);
+        for (int h = 0; h < 2; h++) {
+            mbar_init(x_full(h), 1);
+            mbar_init(h_free(h), 1);
+            mbar_init(acc_full(h), 1);
+            mbar_init(h_ready(h), kEpiWarps);
+        }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *slot;
-    const long long tiles = (g.M + 127) / 128;
+    const long long tiles = (g.M + 127) / 128, step = 2 * (long long)gridDim.x;
     bool failed = false;
+    // pair p of the CTA's tiles: blockIdx.x + 2 p gridDim.x and, where there is one, the tile gridDim.x further
     if (warp == kEpiWarps) {
         if (lane == 0) {
-            long long it = 0, ti = 0;
-            for (long long t = blockIdx.x; t < tiles && !failed; t += gridDim.x, ti++) {
-                if (!mbar_wait_bounded(h_free, (uint32_t)((ti & 1) ^ 1))) { failed = true; break; }
-                mbar_expect_tx(x_full, (uint32_t)(kWsIn / 8) * 128u * 16u);
-                for (int k8 = 0; k8 < kWsIn / 8; k8++) tma_load_2d(hb + (uint32_t)k8 * 2048u, &tmX, k8 * 8, (int)(t * 128), x_full);
+            long long it = 0, p = 0;
+            int xs[2] = {0, 0};                                         // feature loads issued
+            for (long long t = blockIdx.x; t < tiles && !failed; t += step, p++) {
+                const int nh = t + gridDim.x < tiles ? 2 : 1;
                 for (int l = 0; l < kWsLayers && !failed; l++) {
                     const CUtensorMap *wm = l == 0 ? &tw0 : l == 1 ? &tw1 : l == 2 ? &tw2 : l == 3 ? &tw3 : l == 4 ? &tw4 : &tw5;
                     const int n = inf_n(l);
-                    for (int kc = 0; kc < inf_chunks(l); kc++, it++) {
-                        const int s = (int)(it % kInfStages);
-                        if (!mbar_wait_bounded(empty(s), (uint32_t)(((it / kInfStages) & 1) ^ 1))) { failed = true; break; }
-                        mbar_expect_tx(full(s), 8u * (uint32_t)n * 16u);
-                        const uint32_t b_s = smem_u32(ring + (size_t)s * kStageB);
-                        for (int k8 = 0; k8 < 8; k8++) tma_load_2d(b_s + (uint32_t)k8 * (uint32_t)n * 16u, wm, kc * kChunk + k8 * 8, 0, full(s));
+                    for (int h = 0; h < nh && !failed; h++) {
+                        if (l == 0) {
+                            if (!mbar_wait_bounded(h_free(h), (uint32_t)((p & 1) ^ 1))) { failed = true; break; }
+                            mbar_expect_tx(x_full(h), (uint32_t)(kWsIn / 8) * 128u * 16u);
+                            const uint32_t hb = smem_u32(hbuf + (size_t)h * kInfH);
+                            for (int k8 = 0; k8 < kWsIn / 8; k8++)
+                                tma_load_2d(hb + (uint32_t)k8 * 2048u, &tmX, k8 * 8, (int)((t + h * (long long)gridDim.x) * 128), x_full(h));
+                            xs[h]++;
+                        }
+                        for (int kc = 0; kc < inf_chunks(l); kc++, it++) {
+                            const int s = (int)(it % kInfStages);
+                            if (!mbar_wait_bounded(empty(s), (uint32_t)(((it / kInfStages) & 1) ^ 1))) { failed = true; break; }
+                            mbar_expect_tx(full(s), (uint32_t)(kChunk * n) * 2u);
+                            tma_load_2d(smem_u32(ring + (size_t)s * kStageB), wm, kc * kChunk, 0, full(s));
+                        }
                     }
                 }
+            }
+            // nothing of a tile that was given up on may still be on its way when the CTA ends
+            if (failed) {
+                for (int h = 0; h < 2; h++)
+                    if (xs[h] > 0) mbar_wait_bounded(x_full(h), (uint32_t)((xs[h] - 1) & 1));
+                for (long long q = it < kInfStages ? 0 : it - kInfStages; q < it; q++)
+                    mbar_wait_bounded(full((int)(q % kInfStages)), (uint32_t)((q / kInfStages) & 1));
             }
         }
     } else if (warp == kEpiWarps + 1) {
         if (lane == 0) {
-            long long it = 0, ti = 0, hu = 0;
-            for (long long t = blockIdx.x; t < tiles && !failed; t += gridDim.x, ti++) {
-                if (!mbar_wait_bounded(x_full, (uint32_t)(ti & 1))) { failed = true; break; }
+            long long it = 0, p = 0;
+            uint32_t hu[2] = {0u, 0u};                                  // epilogues waited for
+            for (long long t = blockIdx.x; t < tiles && !failed; t += step, p++) {
+                const int nh = t + gridDim.x < tiles ? 2 : 1;
                 for (int l = 0; l < kWsLayers && !failed; l++) {
-                    // the epilogue of the layer before has written this layer's inputs and read the accumulator
-                    if (ti > 0 || l > 0) {
-                        if (!mbar_wait_bounded(h_ready, (uint32_t)(hu & 1))) { failed = true; break; }
-                        hu++;
-                    }
-                    tc_fence_after();
                     const int n = inf_n(l);
                     const uint32_t idesc = idesc_bf16(128, n);
-                    for (int kc = 0; kc < inf_chunks(l); kc++, it++) {
-                        const int s = (int)(it % kInfStages);
-                        if (!mbar_wait_bounded(full(s), (uint32_t)((it / kInfStages) & 1))) { failed = true; break; }
+                    for (int h = 0; h < nh && !failed; h++) {
+                        if (l == 0 && !mbar_wait_bounded(x_full(h), (uint32_t)(p & 1))) { failed = true; break; }
+                        // the epilogue of the layer before has written this layer's inputs and read the accumulator
+                        if (p > 0 || l > 0) {
+                            if (!mbar_wait_bounded(h_ready(h), hu[h] & 1u)) { failed = true; break; }
+                            hu[h]++;
+                        }
                         tc_fence_after();
-                        const uint32_t b_s = smem_u32(ring + (size_t)s * kStageB);
-                        for (int ks = 0; ks < kChunk / 16; ks++)
-                            mma_bf16(tmem, smem_desc(hb + (uint32_t)(kc * (kChunk / 16) + ks) * 2u * 2048u, 2048u, 128u),
-                                     smem_desc(b_s + (uint32_t)ks * 2u * (uint32_t)n * 16u, (uint32_t)n * 16u, 128u), idesc,
-                                     (kc > 0 || ks > 0) ? 1u : 0u);
-                        mma_commit(empty(s));
+                        const uint32_t hb = smem_u32(hbuf + (size_t)h * kInfH);
+                        for (int kc = 0; kc < inf_chunks(l); kc++, it++) {
+                            const int s = (int)(it % kInfStages);
+                            if (!mbar_wait_bounded(full(s), (uint32_t)((it / kInfStages) & 1))) { failed = true; break; }
+                            tc_fence_after();
+                            const uint32_t b_s = smem_u32(ring + (size_t)s * kStageB);
+                            for (int ks = 0; ks < kChunk / 16; ks++)
+                                mma_bf16(tmem + (uint32_t)(h * 256),
+                                         smem_desc(hb + (uint32_t)(kc * (kChunk / 16) + ks) * 2u * 2048u, 2048u, 128u),
+                                         smem_desc_sw(b_s + (uint32_t)ks * 32u, 16u, 1024u), idesc, (kc > 0 || ks > 0) ? 1u : 0u);
+                            mma_commit(empty(s));
+                        }
+                        if (failed) break;
+                        mma_commit(acc_full(h));
+                        if (l == kWsLayers - 1) mma_commit(h_free(h));
                     }
-                    if (failed) break;
-                    mma_commit(acc_full);
-                    if (l == kWsLayers - 1) mma_commit(h_free);
                 }
             }
         }
     } else {
-        long long au = 0;
+        uint32_t au[2] = {0u, 0u};                                     // accumulators waited for
         const int quad = warp & 3;
         const int r = quad * 32 + lane;                                // the TMEM lane = row of the tile
-        for (long long t = blockIdx.x; t < tiles && !failed; t += gridDim.x) {
-            const long long row = t * 128 + r;
-            for (int l = 0; l < kWsLayers; l++, au++) {
-                const bool ok = mbar_wait_bounded(acc_full, (uint32_t)(au & 1));
-                tc_fence_after();
-                if (!ok) { failed = true; break; }
-                const int n = inf_n(l);
-                const int cols = n >= 64 ? n / 4 : 16;
-                const int cbeg = (warp >> 2) * cols, cend = cbeg + cols < n ? cbeg + cols : n;
+        for (long long t = blockIdx.x; t < tiles && !failed; t += step) {
+            const int nh = t + gridDim.x < tiles ? 2 : 1;
+            for (int l = 0; l < kWsLayers && !failed; l++) {
                 const float *bias = g.bias[l];
-                for (int c0 = cbeg; c0 < cend; c0 += 16) {
-                    float v[16];
-                    tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+                for (int h = 0; h < nh; h++) {
+                    const bool ok = mbar_wait_bounded(acc_full(h), au[h] & 1u);
+                    au[h]++;
+                    tc_fence_after();
+                    if (!ok) { failed = true; break; }
+                    const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(h * 256);
                     if (l < kWsLayers - 1) {
-                        alignas(16) bf16 ho[16];
+                        const int cbeg = (warp >> 2) * (kWsHidden / 4);
+                        unsigned char *hb = hbuf + (size_t)h * kInfH + (size_t)r * 16;
 #pragma unroll
-                        for (int i = 0; i < 16; i++) {
-                            const float z = v[i] + bias[c0 + i];
-                            ho[i] = __float2bfloat16_rn(z * sigmoidf_(z));
+                        for (int c0 = cbeg; c0 < cbeg + kWsHidden / 4; c0 += 32) {
+                            float v[32];
+                            tmem_ld32(acc + (uint32_t)c0, v);
+                            alignas(16) bf16 ho[32];
+#pragma unroll
+                            for (int i = 0; i < 32; i += 4) {
+                                const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + i);
+                                const float bb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                                for (int n = 0; n < 4; n++) {
+                                    const float z = v[i + n] + bb[n];
+                                    ho[i + n] = __float2bfloat16_rn(z * sigmoidf_(z));
+                                }
+                            }
+#pragma unroll
+                            for (int c = 0; c < 4; c++)
+                                *reinterpret_cast<uint4 *>(hb + (size_t)(c0 / 8 + c) * 2048) = reinterpret_cast<uint4 *>(ho)[c];
                         }
-                        uint4 *h0 = reinterpret_cast<uint4 *>(hbuf + (size_t)(c0 / 8) * 2048 + (size_t)r * 16);
-                        uint4 *h1 = reinterpret_cast<uint4 *>(hbuf + (size_t)(c0 / 8 + 1) * 2048 + (size_t)r * 16);
-                        *h0 = reinterpret_cast<uint4 *>(ho)[0];
-                        *h1 = reinterpret_cast<uint4 *>(ho)[1];
-                    } else if (row < g.M) {
-                        float4 *yp = reinterpret_cast<float4 *>(g.Y + row * kWsOut + c0);
+                    } else if (warp < 4) {
+                        float v[16];
+                        tmem_ld16(acc, v);
+                        const long long row = (t + h * (long long)gridDim.x) * 128 + r;
+                        if (row < g.M) {
+                            float4 *yp = reinterpret_cast<float4 *>(g.Y + row * kWsOut);
 #pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            yp[i] = make_float4(v[4 * i] + bias[c0 + 4 * i], v[4 * i + 1] + bias[c0 + 4 * i + 1],
-                                                v[4 * i + 2] + bias[c0 + 4 * i + 2], v[4 * i + 3] + bias[c0 + 4 * i + 3]);
+                            for (int i = 0; i < 4; i++)
+                                yp[i] = make_float4(v[4 * i] + bias[4 * i], v[4 * i + 1] + bias[4 * i + 1],
+                                                    v[4 * i + 2] + bias[4 * i + 2], v[4 * i + 3] + bias[4 * i + 3]);
+                        }
                     }
+                    fence_proxy_async();                               // the activations, for the tensor cores
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(h_ready(h));
                 }
-                fence_proxy_async();                                   // the activations, for the tensor cores
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(h_ready);
             }
         }
     }
@@ -449,41 +575,45 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_infer(
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == kEpiWarps) tmem_dealloc(tmem, 256);
+    if (warp == kEpiWarps) tmem_dealloc(tmem, 512);
 }
 
-// ---------------------------------------------------------------- the weight gradient
-// part[(ay * gridDim.x + bx)][a][b] = sum over the CTA's cells of Xa[cell][128 ay + a] Xb[cell][b]
-// (a < 128, b < Nb): the cells are the product's K. Both operands are MN-major: a TMA box of 8
-// features x 64 cells lands as 64 rows of 16 bytes, i.e. eight core matrices of the MN-major
-// no-swizzle layout stacked along K (128 bytes apart), the next 8 features one box (1024 bytes)
-// further. Warp 4 loads (4-stage ring), warp 5 issues the MMAs into one accumulator, warps 0-3
-// write it out once the CTA's cells are done.
+// ---------------------------------------------------------------- the gradients
+// Of layer l: part[(ay * gridDim.x + bx)][b][a] = sum over the CTA's cells of Xa[cell][128 ay + a] Xb[cell][b]
+// (a < 128, b < Nb): the cells are the product's K, split over blockIdx.x; blockIdx.z is the layer, so that one
+// launch covers the network. Both operands are MN-major: a TMA box of 64 features x 64 cells lands in the
+// 128-byte swizzle as 64 rows of 128 bytes, 8 KB from the next 64 features. (Xb of 16 features: two boxes of
+// 8, core matrices stacked along K.) Warp 4 loads (2-stage ring), warp 5 issues the MMAs into one
+// accumulator, warps 0-3 write it out once the CTA's cells are done, in its own order (lanes along a,
+// so that a store is one line); two CTAs per SM, so that one loads while the other writes.
+// Bound by the loads from L2: with boxes of 8 features (3072 rows of 16 bytes a stage) and stores along b
+// 190 us for the six layers of 32768 cells, now 41.
 struct WgradArgs {
-    long long M; int Nb; long long chunk;
-    float *part;
+    CUtensorMap a[kWsLayers], b[kWsLayers];
+    long long M; int Nb[kWsLayers]; long long chunk;
+    float *part[kWsLayers];
     int *err;
 };
 
-constexpr int kWgCells = 64;
+constexpr int kWgCells = 64, kWgStages = 2;
 constexpr int kWgStageA = 128 * kWgCells * 2, kWgStageB = 256 * kWgCells * 2;
+constexpr int kWgSmem = kWgStages * (kWgStageA + kWgStageB) + 256;
 
-__global__ void __launch_bounds__(192, 1) k_mlp_wgrad(const __grid_constant__ CUtensorMap tmA,
-                                                      const __grid_constant__ CUtensorMap tmB, WgradArgs g)
+__global__ void __launch_bounds__(192, 2) k_mlp_wgrad(const __grid_constant__ WgradArgs g)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     unsigned char *ring = sm;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + kStages * (kWgStageA + kWgStageB));
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2 * kStages + 1);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + kWgStages * (kWgStageA + kWgStageB));
+    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2 * kWgStages + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, layer = blockIdx.z, Nb = g.Nb[layer];
     const uint32_t bar0 = smem_u32(bars);
     auto full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
-    auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(kStages + s); };
-    const uint32_t accf = bar0 + 8u * (uint32_t)(2 * kStages);
-    const uint32_t ncols = (uint32_t)tmem_cols(g.Nb);
+    auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(kWgStages + s); };
+    const uint32_t accf = bar0 + 8u * (uint32_t)(2 * kWgStages);
+    const uint32_t ncols = (uint32_t)tmem_cols(Nb);
     if (warp == 4) tmem_alloc(smem_u32(slot), ncols);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (int s = 0; s < kWgStages; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
         mbar_init(accf, 1);
     }
     tc_fence_before();
@@ -494,41 +624,47 @@ __global__ void __launch_bounds__(192, 1) k_mlp_wgrad(const __grid_constant__ CU
     const long long c_end = c_begin + g.chunk < g.M ? c_begin + g.chunk : g.M;
     const int nch = c_end > c_begin ? (int)((c_end - c_begin + kWgCells - 1) / kWgCells) : 0;
     const int a0 = (int)blockIdx.y * 128;
+    const bool sw = Nb >= 64;
+    const int wb = sw ? 64 : 8;                              // features of a box of Xb
     bool failed = false;
     if (warp == 4) {
         if (lane == 0) {
-            const uint32_t bytes = (uint32_t)(16 + g.Nb / 8) * 1024u;
-            for (int it = 0; it < nch; it++) {
-                const int s = it % kStages;
-                if (!mbar_wait_bounded(empty(s), (uint32_t)(((it / kStages) & 1) ^ 1))) { failed = true; break; }
+            const uint32_t bytes = (uint32_t)(128 + Nb) * kWgCells * 2u;
+            int it = 0;
+            for (; it < nch; it++) {
+                const int s = it % kWgStages;
+                if (!mbar_wait_bounded(empty(s), (uint32_t)(((it / kWgStages) & 1) ^ 1))) { failed = true; break; }
                 mbar_expect_tx(full(s), bytes);
                 const uint32_t a_s = smem_u32(ring + (size_t)s * (kWgStageA + kWgStageB));
                 const uint32_t b_s = a_s + kWgStageA;
                 const int y = (int)(c_begin + (long long)it * kWgCells);
-                for (int a8 = 0; a8 < 16; a8++) tma_load_2d(a_s + (uint32_t)a8 * 1024u, &tmA, a0 + a8 * 8, y, full(s));
-                for (int b8 = 0; b8 < g.Nb / 8; b8++) tma_load_2d(b_s + (uint32_t)b8 * 1024u, &tmB, b8 * 8, y, full(s));
+                for (int q = 0; q < 2; q++) tma_load_2d(a_s + (uint32_t)q * 8192u, &g.a[layer], a0 + q * 64, y, full(s));
+                for (int q = 0; q < Nb / wb; q++) tma_load_2d(b_s + (uint32_t)(q * wb) * 128u, &g.b[layer], q * wb, y, full(s));
             }
+            if (failed)                                       // no copy of its own may outlive the CTA
+                for (int q = it < kWgStages ? 0 : it - kWgStages; q < it; q++)
+                    mbar_wait_bounded(full(q % kWgStages), (uint32_t)((q / kWgStages) & 1));
         }
     } else if (warp == 5) {
         if (lane == 0 && nch > 0) {
-            // MN-major A and B (bits 15 and 16); in 16-byte units LBO = K step (128 B), SBO = MN step (1024 B)
-            const uint32_t idesc = idesc_bf16(128, g.Nb) | (1u << 15) | (1u << 16);
+            const uint32_t idesc = idesc_bf16(128, Nb) | (1u << 15) | (1u << 16);      // both MN-major
             for (int it = 0; it < nch && !failed; it++) {
-                const int s = it % kStages;
-                if (!mbar_wait_bounded(full(s), (uint32_t)((it / kStages) & 1))) { failed = true; break; }
+                const int s = it % kWgStages;
+                if (!mbar_wait_bounded(full(s), (uint32_t)((it / kWgStages) & 1))) { failed = true; break; }
                 tc_fence_after();
                 const uint32_t a_s = smem_u32(ring + (size_t)s * (kWgStageA + kWgStageB));
                 const uint32_t b_s = a_s + kWgStageA;
+                // 16 cells further: two groups of eight rows; without swizzle lbo = K step (128 B), sbo = MN step (1 KB)
                 for (int ks = 0; ks < kWgCells / 16; ks++)
-                    mma_bf16(tmem, smem_desc(a_s + (uint32_t)ks * 256u, 128u, 1024u), smem_desc(b_s + (uint32_t)ks * 256u, 128u, 1024u),
+                    mma_bf16(tmem, smem_desc_sw(a_s + (uint32_t)ks * 2048u, 8192u, 1024u),
+                             sw ? smem_desc_sw(b_s + (uint32_t)ks * 2048u, 8192u, 1024u) : smem_desc(b_s + (uint32_t)ks * 256u, 128u, 1024u),
                              idesc, (it > 0 || ks > 0) ? 1u : 0u);
                 mma_commit(empty(s));
             }
             if (!failed) mma_commit(accf);
         }
     } else {
-        float *out = g.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 128 * g.Nb;
-        const int a = warp * 32 + lane;
+        float *out = g.part[layer] + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 128 * Nb + warp * 32 + lane;
         bool ok = true;
         if (nch > 0) {
             ok = mbar_wait_bounded(accf, 0u);
@@ -536,11 +672,11 @@ __global__ void __launch_bounds__(192, 1) k_mlp_wgrad(const __grid_constant__ CU
         }
         if (!ok) failed = true;
         else
-            for (int c0 = 0; c0 < g.Nb; c0 += 16) {
+            for (int c0 = 0; c0 < Nb; c0 += 16) {
                 float v[16];
                 tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
-                for (int i = 0; i < 16; i++) out[(size_t)a * g.Nb + c0 + i] = nch > 0 ? v[i] : 0.0f;
+                for (int i = 0; i < 16; i++) out[(size_t)(c0 + i) * 128] = nch > 0 ? v[i] : 0.0f;
             }
     }
     if (failed) atomicOr(g.err, 1);
@@ -551,34 +687,37 @@ __global__ void __launch_bounds__(192, 1) k_mlp_wgrad(const __grid_constant__ CU
     if (warp == 4) tmem_dealloc(tmem, ncols);
 }
 
-// dst = scale * sum over the CTAs (fixed order); trans stores element (a, b) at b * Wa + a
-__global__ void k_wgrad_reduce(const float *part, int gx, int Wa, int Nb, float scale, int trans, float *dst)
+// column sums of the layers' X[M x W] (W <= 256; layer = blockIdx.y): per block the sum of its rows in their
+// order, two columns a thread, 32 rows asked for at a time
+struct ColsumArgs {
+    const bf16 *X[kWsLayers];
+    int W[kWsLayers];
+    float *part[kWsLayers];
+    long long M, rows;
+};
+__global__ void __launch_bounds__(128) k_colsum_partial(ColsumArgs g)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= Wa * Nb) return;
-    const int a = t / Nb, b = t - a * Nb, ay = a >> 7, al = a & 127;
-    float s = 0.0f;
-    for (int bx = 0; bx < gx; bx++) s += part[((size_t)ay * gx + bx) * 128 * Nb + (size_t)al * Nb + b];
-    dst[trans ? (size_t)b * Wa + a : (size_t)a * Nb + b] = scale * s;
-}
-
-// column sums of X[M x W] (W <= 256): per block partial sums, then a fixed-order reduction
-__global__ void __launch_bounds__(256) k_colsum_partial(const bf16 *X, long long M, int W, long long rows_per, float *part)
-{
-    const int c = threadIdx.x;
+    const int W = g.W[blockIdx.y], c = 2 * threadIdx.x;
     if (c >= W) return;
-    const long long r0 = (long long)blockIdx.x * rows_per, r1 = std::min(M, r0 + rows_per);
-    float s = 0.0f;
-    for (long long r = r0; r < r1; r++) s += __bfloat162float(X[r * W + c]);
-    part[(size_t)blockIdx.x * W + c] = s;
-}
-__global__ void k_colsum_reduce(const float *part, int nb, int W, float scale, float *dst)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= W) return;
-    float s = 0.0f;
-    for (int b = 0; b < nb; b++) s += part[(size_t)b * W + c];
-    dst[c] = scale * s;
+    const bf16 *X = g.X[blockIdx.y] + c;
+    const long long r0 = (long long)blockIdx.x * g.rows, r1 = r0 + g.rows < g.M ? r0 + g.rows : g.M;
+    float s0 = 0.0f, s1 = 0.0f;
+    long long r = r0;
+    for (; r + 32 <= r1; r += 32) {
+        __nv_bfloat162 x[32];
+#pragma unroll
+        for (int q = 0; q < 32; q++) x[q] = *reinterpret_cast<const __nv_bfloat162 *>(X + (r + q) * W);
+#pragma unroll
+        for (int q = 0; q < 32; q++) { s0 += __low2float(x[q]); s1 += __high2float(x[q]); }
+    }
+    for (; r < r1; r++) {
+        const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162 *>(X + r * W);
+        s0 += __low2float(x);
+        s1 += __high2float(x);
+    }
+    float *dst = g.part[blockIdx.y] + (size_t)blockIdx.x * W + c;
+    dst[0] = s0;
+    dst[1] = s1;
 }
 
 // ---------------------------------------------------------------- features, loss, optimiser
@@ -666,16 +805,106 @@ __global__ void __launch_bounds__(256) k_ws_loss(const float *Y, const float *T,
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-__global__ void k_adam(float *p, const float *g, float *m, float *v, long long n, float lr, float b1, float b2, float eps,
-                       float c1, float c2)
+__device__ __forceinline__ void adam(float *p, float gi, float *m, float *v, float lr, float b1, float b2, float eps, float c1, float c2)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi, vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float mi = b1 * *m + (1.0f - b1) * gi, vi = b2 * *v + (1.0f - b2) * gi * gi;
+    *m = mi;
+    *v = vi;
+    *p -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+}
+
+// The end of a step in one launch: every gradient as scale * the sum of its partial sums in their order, and
+// ADAM: the optimiser step and the BF16 weights, as stored [N x K] and transposed [K x N]; else: the
+// gradients to G. Blocks 0 .. nw-1 take 32 x 32 weights of a layer (partials read along a, parameters along
+// their rows), the last six the biases of a layer. Bound by the partials (84 MB for 32768 cells on
+// 152 SMs); as 19 launches with one load in flight a thread 150 us, now 25 us.
+struct StepArgs {
+    float *P, *G, *Mo, *Vo;
+    long long w_off[kWsLayers], b_off[kWsLayers];
+    const float *part[kWsLayers], *cpart[kWsLayers];
+    bf16 *Wb[kWsLayers], *Wt[kWsLayers];
+    int Nb[kWsLayers], trans[kWsLayers], W[kWsLayers], first[kWsLayers + 1];       // blocks of a layer
+    int gx, nb;
+    float scale, lr, b1, b2, eps, c1, c2;
+};
+template <bool ADAM>
+__global__ void __launch_bounds__(256) k_ws_step(StepArgs g)
+{
+    const int nw = g.first[kWsLayers];
+    if ((int)blockIdx.x >= nw) {
+        const int l = (int)blockIdx.x - nw, W = g.W[l], c = threadIdx.x;
+        if (c >= W) return;
+        const float *q = g.cpart[l] + c;
+        float s = 0.0f;
+        int b = 0;
+        for (; b + 32 <= g.nb; b += 32) {
+            float x[32];
+#pragma unroll
+            for (int n = 0; n < 32; n++) x[n] = q[(size_t)(b + n) * W];
+#pragma unroll
+            for (int n = 0; n < 32; n++) s += x[n];
+        }
+        for (; b < g.nb; b++) s += q[(size_t)b * W];
+        const long long i = g.b_off[l] + c;
+        if constexpr (ADAM) adam(g.P + i, g.scale * s, g.Mo + i, g.Vo + i, g.lr, g.b1, g.b2, g.eps, g.c1, g.c2);
+        else g.G[i] = g.scale * s;
+        return;
+    }
+    __shared__ float tile[32][33];                         // [b][a]
+    int l = 0;
+    while ((int)blockIdx.x >= g.first[l + 1]) l++;
+    const int Nb = g.Nb[l], tb = (Nb + 31) / 32, at = ((int)blockIdx.x - g.first[l]) / tb, bt = ((int)blockIdx.x - g.first[l]) - at * tb;
+    const int a = at * 32 + (threadIdx.x & 31), w = threadIdx.x >> 5;
+    const float *q = g.part[l] + (size_t)(a >> 7) * g.gx * 128 * Nb + (a & 127);
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    bool in[4];
+#pragma unroll
+    for (int n = 0; n < 4; n++) in[n] = bt * 32 + w + 8 * n < Nb;
+    int bx = 0;
+    for (; bx + 8 <= g.gx; bx += 8) {
+        float x[8][4];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+#pragma unroll
+            for (int n = 0; n < 4; n++) x[u][n] = in[n] ? q[((size_t)(bx + u) * Nb + bt * 32 + w + 8 * n) * 128] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+#pragma unroll
+            for (int n = 0; n < 4; n++) s[n] += x[u][n];
+    }
+    for (; bx < g.gx; bx++)
+#pragma unroll
+        for (int n = 0; n < 4; n++) s[n] += in[n] ? q[((size_t)bx * Nb + bt * 32 + w + 8 * n) * 128] : 0.0f;
+#pragma unroll
+    for (int n = 0; n < 4; n++) tile[w + 8 * n][threadIdx.x & 31] = s[n];
+    __syncthreads();
+    // the layer's matrix is [a][b], or [b][a] where it is stored transposed
+    const int Wa = kWsHidden, trans = g.trans[l], K = trans ? Wa : Nb, N = trans ? Nb : Wa;
+#pragma unroll
+    for (int n = 0; n < 4; n++) {
+        const int f = threadIdx.x & 31, r = w + 8 * n;     // along a row of the matrix, row
+        const int ai = at * 32 + (trans ? f : r), bi = bt * 32 + (trans ? r : f);
+        if (bi >= Nb) continue;
+        float &e = tile[trans ? r : f][trans ? f : r];
+        const int row = trans ? bi : ai, col = trans ? ai : bi;
+        const long long i = g.w_off[l] + (long long)row * K + col;
+        if constexpr (ADAM) {
+            adam(g.P + i, g.scale * e, g.Mo + i, g.Vo + i, g.lr, g.b1, g.b2, g.eps, g.c1, g.c2);
+            e = g.P[i];
+            g.Wb[l][(size_t)row * K + col] = __float2bfloat16_rn(e);
+        } else g.G[i] = g.scale * e;
+    }
+    if constexpr (ADAM) {
+        __syncthreads();
+#pragma unroll
+        for (int n = 0; n < 4; n++) {
+            const int f = threadIdx.x & 31, r = w + 8 * n; // along a column of the matrix, column
+            const int ai = at * 32 + (trans ? r : f), bi = bt * 32 + (trans ? f : r);
+            if (bi >= Nb) continue;
+            const int row = trans ? bi : ai, col = trans ? ai : bi;
+            g.Wt[l][(size_t)col * N + row] = __float2bfloat16_rn(tile[trans ? f : r][trans ? r : f]);
+        }
+    }
 }
 
 // BF16 copies of a layer's weights, as stored [N x K] and transposed [K x N]
@@ -797,8 +1026,9 @@ __global__ void __launch_bounds__(256) k_ws_stats(const float *set, long long n,
 
 // ---------------------------------------------------------------- host side
 // 2D tensor map of a row-major BF16 matrix [rows x cols] (row stride ld elements) read in boxes
-// of 8 columns (16 bytes) x box_rows rows; rows past the end read as zeros
-static CUtensorMap tensor_map_rows(const bf16 *base, long long rows, int cols, long long ld, int box_rows)
+// of 64 columns (128 bytes, in the 128-byte swizzle) x box_rows rows, or of 8 without swizzle where it has
+// fewer than 64 or wide is false; rows past the end read as zeros
+static CUtensorMap tensor_map_rows(const bf16 *base, long long rows, int cols, long long ld, int box_rows, bool wide = true)
 {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
@@ -808,15 +1038,17 @@ static CUtensorMap tensor_map_rows(const bf16 *base, long long rows, int cols, l
         if (!f || q != cudaDriverEntryPointSuccess) throw std::runtime_error("cuTensorMapEncodeTiled is not available");
         encode = (PFN_cuTensorMapEncodeTiled_v12000)f;
     }
+    wide = wide && cols >= kChunk;
     if (((uintptr_t)base & 15) || ((ld * 2) & 15) || (cols & 7) || box_rows < 1 || box_rows > 256)
         throw std::runtime_error("tensor map: misaligned matrix or box");
     CUtensorMap m;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {8u, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {wide ? (cuuint32_t)kChunk : 8u, (cuuint32_t)box_rows};
     const cuuint32_t es[2] = {1u, 1u};
     const CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)base, dims, strides, box, es,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, wide ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed");
     return m;
@@ -831,6 +1063,7 @@ static size_t w_off(int l)
     for (int q = 0; q < l; q++) o += (size_t)kN[q] * kK[q] + kN[q];
     return o;
 }
+constexpr int kLossKept = 20;                    // steps whose loss train() averages
 static size_t b_off(int l) { return w_off(l) + (size_t)kN[l] * kK[l]; }
 
 struct WarmStart::Impl {
@@ -843,9 +1076,9 @@ struct WarmStart::Impl {
     float nrm[kWsNorm] = {};
     bool have_norm = false;
     int adam_t = 0;
-    // activations for up to cap rows
-    long long cap = 0;
-    bf16 *X0 = nullptr, *Z[5] = {}, *H[5] = {}, *dY = nullptr, *dZa = nullptr, *dZb = nullptr;
+    // rows in and out for up to cap rows, activations, targets and gradients for up to tcap
+    long long cap = 0, tcap = 0;
+    bf16 *X0 = nullptr, *Z[5] = {}, *H[5] = {}, *dY = nullptr, *dZ[5] = {};
     float *Y = nullptr, *T = nullptr, *part = nullptr, *cpart = nullptr, *lpart = nullptr;
     size_t part_n = 0;
     // training set
@@ -853,28 +1086,44 @@ struct WarmStart::Impl {
     long long set_cap = 0;
     unsigned long long rng = 0;
 
+    static bf16 *abf(long long n) { bf16 *p; WCK(cudaMalloc(&p, sizeof(bf16) * n)); return p; }
+    static float *af(long long n) { float *p; WCK(cudaMalloc(&p, sizeof(float) * n)); return p; }
     void ensure(long long M)
     {
         if (M <= cap) return;
-        release_acts();
-        cap = std::max(M, (long long)4096);
-        auto abf = [&](long long n) { bf16 *p; WCK(cudaMalloc(&p, sizeof(bf16) * n)); return p; };
-        auto af = [&](long long n) { float *p; WCK(cudaMalloc(&p, sizeof(float) * n)); return p; };
-        X0 = abf(cap * kWsIn);
-        for (int l = 0; l < 5; l++) { Z[l] = abf(cap * kWsHidden); H[l] = abf(cap * kWsHidden); }
-        dY = abf(cap * kWsOut);
-        dZa = abf(cap * kWsHidden);
-        dZb = abf(cap * kWsHidden);
-        Y = af(cap * kWsOut);
-        T = af(cap * 8);
-        lpart = af((cap + 255) / 256);
+        cudaFree(X0); cudaFree(Y);
+        X0 = nullptr; Y = nullptr;
+        cap = 0;
+        const long long n = std::max(M, (long long)4096);
+        X0 = abf(n * kWsIn);
+        Y = af(n * kWsOut);
+        cap = n;
+    }
+    void ensure_train(long long M)
+    {
+        ensure(M);
+        if (M <= tcap) return;
+        release_train();
+        const long long n = std::max(M, (long long)4096);
+        for (int l = 0; l < 5; l++) { Z[l] = abf(n * kWsHidden); H[l] = abf(n * kWsHidden); dZ[l] = abf(n * kWsHidden); }
+        dY = abf(n * kWsOut);
+        T = af(n * 8);
+        lpart = af(kLossKept * ((n + 255) / 256));
+        if (!cpart) cpart = af(kWsLayers * 512 * kWsHidden);
+        tcap = n;
+    }
+    void release_train()
+    {
+        for (int l = 0; l < 5; l++) { cudaFree(Z[l]); cudaFree(H[l]); cudaFree(dZ[l]); Z[l] = H[l] = dZ[l] = nullptr; }
+        cudaFree(dY); cudaFree(T); cudaFree(lpart);
+        dY = nullptr; T = lpart = nullptr;
+        tcap = 0;
     }
     void release_acts()
     {
-        cudaFree(X0); X0 = nullptr;
-        for (int l = 0; l < 5; l++) { cudaFree(Z[l]); cudaFree(H[l]); Z[l] = H[l] = nullptr; }
-        cudaFree(dY); cudaFree(dZa); cudaFree(dZb); cudaFree(Y); cudaFree(T); cudaFree(lpart);
-        dY = dZa = dZb = nullptr; Y = T = lpart = nullptr;
+        release_train();
+        cudaFree(X0); cudaFree(Y);
+        X0 = nullptr; Y = nullptr;
         cap = 0;
     }
 
@@ -894,37 +1143,6 @@ struct WarmStart::Impl {
         WCK(cudaGetLastError());
     }
 
-    void wgrad(const bf16 *Xa, long long lda, const bf16 *Xb, int Nb, long long M, float scale, int trans, float *dst)
-    {
-        const int Wa = kWsHidden;                           // every weight gradient has 256 rows on one side
-        const int gy = Wa / 128;
-        int gx = std::max(1, n_sm / gy);
-        long long chunk = ((M + gx - 1) / gx + 63) / 64 * 64;
-        gx = (int)((M + chunk - 1) / chunk);
-        const size_t need = (size_t)gy * gx * 128 * Nb;
-        if (need > part_n) {
-            cudaFree(part);
-            WCK(cudaMalloc(&part, sizeof(float) * need));
-            part_n = need;
-        }
-        WgradArgs g{};
-        g.M = M; g.Nb = Nb; g.chunk = chunk; g.part = part; g.err = err;
-        const CUtensorMap ta = tensor_map_rows(Xa, M, Wa, lda, kWgCells);
-        const CUtensorMap tb = tensor_map_rows(Xb, M, Nb, Nb, kWgCells);
-        k_mlp_wgrad<<<dim3(gx, gy), 192, kTcSmem, st>>>(ta, tb, g);
-        WCK(cudaGetLastError());
-        k_wgrad_reduce<<<(Wa * Nb + 255) / 256, 256, 0, st>>>(part, gx, Wa, Nb, scale, trans, dst);
-    }
-
-    void colsum(const bf16 *X, long long M, int W, float scale, float *dst)
-    {
-        const int nb = (int)std::min<long long>(std::max<long long>(1, (M + 255) / 256), 512);
-        const long long rows = (M + nb - 1) / nb;
-        if (!cpart) WCK(cudaMalloc(&cpart, sizeof(float) * 512 * 256));
-        k_colsum_partial<<<nb, 256, 0, st>>>(X, M, W, rows, cpart);
-        k_colsum_reduce<<<1, 256, 0, st>>>(cpart, nb, W, scale, dst);
-    }
-
     void refresh_bf16()
     {
         for (int l = 0; l < kWsLayers; l++)
@@ -938,7 +1156,7 @@ struct WarmStart::Impl {
         InferArgs g{};
         g.M = M; g.Y = Y; g.err = err;
         for (int l = 0; l < kWsLayers; l++) g.bias[l] = P + b_off(l);
-        const CUtensorMap tx = tensor_map_rows(X0, M, kWsIn, kWsIn, 128);
+        const CUtensorMap tx = tensor_map_rows(X0, M, kWsIn, kWsIn, 128, false);
         CUtensorMap tw[kWsLayers];
         for (int l = 0; l < kWsLayers; l++) tw[l] = tensor_map_rows(Wb[l], kN[l], kK[l], kK[l], kN[l]);
         const long long tiles = (M + 127) / 128;
@@ -960,35 +1178,75 @@ struct WarmStart::Impl {
         gemm<1>(in, ld, 5, false, M, kWsOut, kWsHidden, P + b_off(5), nullptr, nullptr, Y, kWsOut, nullptr, nullptr);
     }
 
-    // from dY: every gradient into G (mean over the M rows)
-    void backward(long long M)
+    // from dY: every gradient (mean over the M rows) into G, or with adam the optimiser step
+    void backward(long long M, const StepArgs *adam = nullptr)
     {
-        const float sc = 1.0f / (float)M;
-        wgrad(H[4], kWsHidden, dY, kWsOut, M, sc, 1, G + w_off(5));             // dW6 (stored transposed)
-        colsum(dY, M, kWsOut, sc, G + b_off(5));
-        // dZ5 = (dY . W6) * SiLU'(Z5)
-        gemm<2>(dY, kWsOut, 5, true, M, kWsHidden, kWsOut, nullptr, nullptr, nullptr, nullptr, kWsHidden, Z[4], dZa);
-        bf16 *cur = dZa, *nxt = dZb;
-        for (int l = 4; l >= 1; l--) {
-            wgrad(cur, kWsHidden, H[l - 1], kWsHidden, M, sc, 0, G + w_off(l));
-            colsum(cur, M, kWsHidden, sc, G + b_off(l));
-            gemm<2>(cur, kWsHidden, l, true, M, kWsHidden, kWsHidden, nullptr, nullptr, nullptr, nullptr, kWsHidden, Z[l - 1], nxt);
-            std::swap(cur, nxt);
+        // dZ5 = (dY . W6) * SiLU'(Z5), and so on down to dZ1
+        gemm<2>(dY, kWsOut, 5, true, M, kWsHidden, kWsOut, nullptr, nullptr, nullptr, nullptr, kWsHidden, Z[4], dZ[4]);
+        for (int l = 4; l >= 1; l--)
+            gemm<2>(dZ[l], kWsHidden, l, true, M, kWsHidden, kWsHidden, nullptr, nullptr, nullptr, nullptr, kWsHidden, Z[l - 1], dZ[l - 1]);
+        // dW[l] = dZ^T . inputs, with 256 rows on the a side: of the last layer the transposed, H5^T . dY
+        const int gy = kWsHidden / 128;
+        int gx = std::max(1, n_sm / gy);
+        const long long chunk = ((M + gx - 1) / gx + 63) / 64 * 64;
+        gx = (int)((M + chunk - 1) / chunk);
+        const int nb = (int)std::min<long long>(std::max<long long>(1, (M + 255) / 256), 512);
+        size_t need = 0;
+        for (int l = 0; l < kWsLayers; l++) need += (size_t)gy * gx * 128 * (l == kWsLayers - 1 ? kWsOut : kK[l]);
+        if (need > part_n) {
+            cudaFree(part);
+            part = nullptr;
+            part_n = 0;
+            part = af((long long)need);
+            part_n = need;
         }
-        wgrad(cur, kWsHidden, X0, kWsIn, M, sc, 0, G + w_off(0));
-        colsum(cur, M, kWsHidden, sc, G + b_off(0));
+        WgradArgs w{};
+        ColsumArgs c{};
+        StepArgs t{};
+        if (adam) t = *adam;
+        w.M = c.M = M; w.chunk = chunk; w.err = err;
+        c.rows = (M + nb - 1) / nb;
+        t.P = P; t.G = G; t.Mo = Mo; t.Vo = Vo; t.gx = gx; t.nb = nb; t.scale = 1.0f / (float)M;
+        float *at = part;
+        for (int l = 0; l < kWsLayers; l++) {
+            const bool last = l == kWsLayers - 1;
+            const bf16 *in = l == 0 ? X0 : H[l - 1], *d = last ? dY : dZ[l];
+            w.Nb[l] = t.Nb[l] = last ? kWsOut : kK[l];
+            w.a[l] = tensor_map_rows(last ? in : d, M, kWsHidden, kWsHidden, kWgCells);
+            w.b[l] = tensor_map_rows(last ? d : in, M, w.Nb[l], w.Nb[l], kWgCells);
+            w.part[l] = at;
+            t.part[l] = at;
+            at += (size_t)gy * gx * 128 * w.Nb[l];
+            c.X[l] = d; c.W[l] = t.W[l] = kN[l];
+            c.part[l] = cpart + (size_t)l * 512 * kWsHidden;
+            t.cpart[l] = c.part[l];
+            t.w_off[l] = (long long)w_off(l); t.b_off[l] = (long long)b_off(l);
+            t.Wb[l] = Wb[l]; t.Wt[l] = Wt[l]; t.trans[l] = last;
+            t.first[l + 1] = t.first[l] + kWsHidden / 32 * ((t.Nb[l] + 31) / 32);
+        }
+        k_mlp_wgrad<<<dim3(gx, gy, kWsLayers), 192, kWgSmem, st>>>(w);
+        k_colsum_partial<<<dim3(nb, kWsLayers), 128, 0, st>>>(c);
+        if (adam) k_ws_step<true><<<t.first[kWsLayers] + kWsLayers, 256, 0, st>>>(t);
+        else k_ws_step<false><<<t.first[kWsLayers] + kWsLayers, 256, 0, st>>>(t);
+        WCK(cudaGetLastError());
     }
 
-    float loss(long long M)
+    // dY of the loss; its sums per block stay in slot (step % kLossKept) until losses() reads them
+    void loss(long long M, int step) { k_ws_loss<<<loss_blocks(M), 256, 0, st>>>(Y, T, M, dY, lpart + (size_t)(step % kLossKept) * loss_blocks(M)); }
+    static int loss_blocks(long long M) { return (int)((M + 255) / 256); }
+    // the losses of steps first .. first + n - 1, n <= kLossKept
+    std::vector<float> losses(long long M, int first, int n)
     {
-        const int nb = (int)((M + 255) / 256);
-        k_ws_loss<<<nb, 256, 0, st>>>(Y, T, M, dY, lpart);
-        std::vector<float> h(nb);
-        WCK(cudaMemcpyAsync(h.data(), lpart, sizeof(float) * nb, cudaMemcpyDeviceToHost, st));
+        const int nb = loss_blocks(M);
+        std::vector<float> h((size_t)kLossKept * nb), out;
+        WCK(cudaMemcpyAsync(h.data(), lpart, sizeof(float) * h.size(), cudaMemcpyDeviceToHost, st));
         WCK(cudaStreamSynchronize(st));
-        double s = 0.0;
-        for (float v : h) s += v;
-        return (float)(s / ((double)M * kWsOutUsed));
+        for (int q = first; q < first + n; q++) {
+            double s = 0.0;
+            for (int b = 0; b < nb; b++) s += h[(size_t)(q % kLossKept) * nb + b];
+            out.push_back((float)(s / ((double)M * kWsOutUsed)));
+        }
+        return out;
     }
 };
 
@@ -1003,7 +1261,7 @@ WarmStart::WarmStart(unsigned seed) : d(new Impl)
     WCK(cudaFuncSetAttribute(k_mlp_gemm<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
     WCK(cudaFuncSetAttribute(k_mlp_gemm<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
     WCK(cudaFuncSetAttribute(k_mlp_gemm<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
-    WCK(cudaFuncSetAttribute(k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
+    WCK(cudaFuncSetAttribute(k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem));
     WCK(cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfSmem));
     const size_t np = n_params();
     WCK(cudaMalloc(&d->P, sizeof(float) * np));
@@ -1153,22 +1411,22 @@ float WarmStart::train(int steps, int batch, float lr)
         WCK(cudaMemcpy(m.nrm_d, m.nrm, sizeof(m.nrm), cudaMemcpyHostToDevice));
         m.have_norm = true;
     }
-    m.ensure(batch);
-    const size_t np = n_params();
-    double acc = 0.0;
-    int nacc = 0;
+    m.ensure_train(batch);
+    StepArgs adam{};
+    adam.lr = lr; adam.b1 = 0.9f; adam.b2 = 0.999f; adam.eps = 1e-8f;
     for (int it = 0; it < steps; it++) {
         m.rng = m.rng * 6364136223846793005ull + 1442695040888963407ull;
-        k_ws_gather<<<(batch + 255) / 256, 256, 0, m.st>>>(m.set, n_set, m.rng, batch, m.nrm_d, m.X0, m.T);
+        k_ws_gather<<<(batch + 63) / 64, 64, 0, m.st>>>(m.set, n_set, m.rng, batch, m.nrm_d, m.X0, m.T);
         m.forward(batch);
-        const float l = m.loss(batch);
-        m.backward(batch);
+        m.loss(batch, it);
         m.adam_t++;
-        const float c1 = 1.0f - std::pow(0.9f, (float)m.adam_t), c2 = 1.0f - std::pow(0.999f, (float)m.adam_t);
-        k_adam<<<(unsigned)((np + 255) / 256), 256, 0, m.st>>>(m.P, m.G, m.Mo, m.Vo, (long long)np, lr, 0.9f, 0.999f, 1e-8f, c1, c2);
-        m.refresh_bf16();
-        if (it >= steps - 20) { acc += l; nacc++; }
+        adam.c1 = 1.0f - std::pow(0.9f, (float)m.adam_t);
+        adam.c2 = 1.0f - std::pow(0.999f, (float)m.adam_t);
+        m.backward(batch, &adam);
     }
+    const int nacc = std::max(0, std::min(steps, kLossKept));
+    double acc = 0.0;
+    for (float l : m.losses(batch, steps - nacc, nacc)) acc += l;
     WCK(cudaStreamSynchronize(m.st));
     WCK(cudaGetLastError());
     if (error_flag()) throw std::runtime_error("a tensor-core wait of the warm-start network ran out");
@@ -1263,7 +1521,7 @@ void WarmStart::forward(const float *feat, int M, float *y)
 float WarmStart::forward_backward(const float *feat, const float *target, int M, float *grad)
 {
     Impl &m = *d;
-    m.ensure(M);
+    m.ensure_train(M);
     DevBuf f;
     f.bytes = sizeof(float) * (size_t)M * kWsIn;
     WCK(cudaMalloc(&f.p, f.bytes));
@@ -1274,8 +1532,9 @@ float WarmStart::forward_backward(const float *feat, const float *target, int M,
         for (int o = 0; o < kWsOutUsed; o++) t8[(size_t)r * 8 + o] = target[(size_t)r * kWsOutUsed + o];
     WCK(cudaMemcpyAsync(m.T, t8.data(), sizeof(float) * t8.size(), cudaMemcpyHostToDevice, m.st));
     m.forward(M);
-    const float l = m.loss(M);
+    m.loss(M, 0);
     m.backward(M);
+    const float l = m.losses(M, 0, 1)[0];
     WCK(cudaMemcpyAsync(grad, m.G, sizeof(float) * n_params(), cudaMemcpyDeviceToHost, m.st));
     WCK(cudaStreamSynchronize(m.st));
     if (error_flag()) throw std::runtime_error("a tensor-core wait of the warm-start network ran out");
@@ -1300,7 +1559,7 @@ void WarmStart::benchmark(long long M, int iters, float *ms_forward, float *ms_s
 {
     if (M < 128 || iters < 1) throw std::invalid_argument("benchmark: at least 128 rows and one iteration");
     Impl &m = *d;
-    m.ensure(M);
+    m.ensure_train(M);
     k_ws_random_rows<<<(unsigned)((M + 255) / 256), 256, 0, m.st>>>(M, 12345ull, m.X0, m.T);
     cudaEvent_t e0, e1;
     WCK(cudaEventCreate(&e0));
@@ -1331,11 +1590,10 @@ void WarmStart::benchmark(long long M, int iters, float *ms_forward, float *ms_s
         dmax = (dq > dmax || dq != dq) ? dq : dmax;
     }
     if (max_diff) *max_diff = dmax;
-    const int nb = (int)((M + 255) / 256);
     WCK(cudaEventRecord(e0, m.st));
     for (int i = 0; i < iters; i++) {
         m.forward(M);
-        k_ws_loss<<<nb, 256, 0, m.st>>>(m.Y, m.T, M, m.dY, m.lpart);
+        m.loss(M, 0);
         m.backward(M);
     }
     WCK(cudaEventRecord(e1, m.st));
