@@ -135,40 +135,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32])
 // ---------------------------------------------------------------- operand staging
 __device__ __forceinline__ float sigmoidf_(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
 
-// ---------------------------------------------------------------- the row product
-// D[128 x N] = A[128 x K] . B[N x K]^T per tile of 128 rows (cells); K 16 or a multiple of 64, N and K <= 256.
-// Warp-specialised and persistent over the row tiles:
-//   warp 16: TMA producer. Loads B once, it stays for every tile of the CTA, and streams A, a chunk of
-//     128 rows x 64 columns at a time, through a 4-deep ring. Both land in the 128-byte swizzle: a
-//     row of a box is 128 bytes. Rows past M read as zeros. (K = 16: boxes of 8 columns, no swizzle.)
-//   warp 17: MMA issuer. Waits for a stage, issues its tcgen05.mma (K = 16 each) into one of two TMEM
-//     accumulators (256 columns each), and tcgen05.commit frees the stage when they complete;
-//     after a tile's last chunk a commit marks the accumulator full.
-//   warps 0-15: epilogue. Read the full accumulator (warp w: TMEM lanes 32(w%4)..32(w%4)+31, the
-//     (w/4)-th quarter of the columns), apply the epilogue, store, and hand the accumulator back,
-//     while the next tile accumulates in the other. Rows of 32 BF16 columns pass through 2 KB of shared
-//     memory per warp, so that a store or load covers 8 rows x 64 bytes instead of 32 rows x 16.
-// Bound by the epilogue (two MUFU operations an element, 32768 elements a tile) once the loads are wide: with
-// boxes of 8 columns a tile took 12288 rows of 16 bytes, about one a clock, and 32768 x 256 x 256 29 us;
-// now 16 us.
-// Epilogues:
-//   0: z = D + bias -> Z (BF16), H = SiLU(z) (BF16)      N = 256
-//   1: y = D + bias -> Y (FP32)
-//   2: dZ = D * SiLU'(Zp) (BF16)                           N = 256
-struct GemmArgs {
-    long long M; int N, K;
-    const float *bias;
-    bf16 *Z, *H; float *Y; long long ldo;
-    const bf16 *Zp; bf16 *dZ;
-    int *err;
-};
-
-constexpr int kStages = 4, kChunk = 64;
+constexpr int kChunk = 64;
 constexpr int kEpiWarps = 16;                    // four per TMEM lane quadrant
-constexpr int kStageA = 128 * kChunk * 2, kStageB = 256 * kChunk * 2;
-constexpr int kMaxChunks = kWsHidden / kChunk;
 constexpr int kEpiStage = 32 * 64;               // 32 rows x 32 BF16 columns per epilogue warp
-constexpr int kTcSmem = kMaxChunks * kStageB + kStages * kStageA + kEpiWarps * kEpiStage + 256;
 
 __host__ __device__ inline int tmem_cols(int n) { int c = 32; while (c < n) c <<= 1; return c; }
 
@@ -204,231 +173,91 @@ __device__ __forceinline__ void store_rows32(unsigned char *st, int lane, const 
     __syncwarp();
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_gemm(const __grid_constant__ CUtensorMap tmA,
-                                                     const __grid_constant__ CUtensorMap tmB, GemmArgs g)
+// ---------------------------------------------------------------- the row products, all layers fused
+// The products of rows (cells) with the layers' matrices, D[128 x N] = A[128 x K] . B[N x K]^T per tile of 128
+// rows and layer, a tile's activations kept on chip from layer to layer:
+//   PASS_INFER     Y[rows x 16] = the whole network on X[rows x 64]; nothing but X and Y crosses HBM
+//   PASS_FORWARD   the same, and Z = D + bias, H = SiLU(Z) of every hidden layer stored (BF16) for the gradients
+//   PASS_BACKWARD  from dY[rows x 16]: dZ5 = (dY . W6) * SiLU'(Z5), ..., dZ1 = (dZ2 . W2) * SiLU'(Z1), stored (BF16)
+// A CTA works on two tiles in turn, so that the tensor cores run a layer of one while the epilogue warps are
+// on the other: each has a shared-memory buffer of activations (K-major core matrices: 8-column groups
+// 2 KB apart, rows 16 B apart) and a TMEM accumulator. Persistent over the tiles:
+//   warp 16: TMA producer. Loads a tile's input rows into its activation buffer once the last layer of the
+//     buffer's previous tile has read it, and streams the weights, 64-column chunk by chunk in the
+//     128-byte swizzle, layer by layer and tile by tile, through a ring (they stay in L2). Rows past M read
+//     as zeros. (16 columns: boxes of 8, no swizzle.)
+//   warp 17: MMA issuer. Per layer and tile: waits for the tile's epilogue of the layer before (its
+//     outputs are this layer's inputs, and it has read the accumulator out), issues the layer's MMAs with A
+//     from the activation buffer, commits the accumulator; after the last layer it frees the buffer.
+//   warps 0-15: epilogue (warp w: TMEM lanes 32(w%4)..32(w%4)+31, the (w/4)-th quarter of the columns).
+//     Bias and SiLU of the accumulator, or the product with SiLU', rounded to BF16, written over the
+//     activation buffer, and stored; or bias and FP32 rows of Y (the output layer). Rows of 32 BF16 columns
+//     go to and come from HBM through 2 KB of shared memory per warp, so that an access covers 8 rows x
+//     64 bytes instead of 32 rows x 16.
+// Inference and forward pass have the same MMA order and arithmetic, so the same bits in Y. Bound by the
+// epilogue's MUFU operations (two an element, 16 a clock: 144 us for the inference of 262144 rows). Inference of
+// 262144 rows with boxes of 8 columns (about one row of 16 bytes a clock) and one tile at a time 371 us,
+// now 196 us. On 32768 rows a launch per layer took 90 us forward and 76 us backward, now 52 and 50.
+enum { PASS_INFER, PASS_FORWARD, PASS_BACKWARD };
+struct ChainArgs {
+    long long M;
+    const float *bias[kWsLayers];
+    float *Y;
+    bf16 *Z[kWsLayers - 1], *H[kWsLayers - 1], *dZ[kWsLayers - 1];
+    int *err;
+};
+constexpr int kStageB = kWsHidden * kChunk * 2;
+constexpr int kActs = 128 * kWsHidden * 2;                  // 64 KB of activations
+__host__ __device__ constexpr int chain_stages(int pass) { return pass == PASS_INFER ? 3 : 2; }
+__host__ __device__ constexpr int chain_smem(int pass)
 {
+    return chain_stages(pass) * kStageB + 2 * kActs + (pass == PASS_INFER ? 0 : kEpiWarps * kEpiStage) + 256;
+}
+__host__ __device__ constexpr int chain_layers(int pass) { return pass == PASS_BACKWARD ? kWsLayers - 1 : kWsLayers; }
+__host__ __device__ constexpr int chain_n(int pass, int l) { return pass != PASS_BACKWARD && l == kWsLayers - 1 ? kWsOut : kWsHidden; }
+__host__ __device__ constexpr int chain_k(int pass, int l) { return l > 0 ? kWsHidden : pass == PASS_BACKWARD ? kWsOut : kWsIn; }
+
+// 32 rows x 32 BF16 columns (one row per lane in v) to rows row0.. of dst through the warp's 2 KB
+__device__ __forceinline__ void store_rows32(unsigned char *st, int lane, const bf16 v[32], bf16 *dst, long long row0, long long M)
+{
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        *reinterpret_cast<uint4 *>(st + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = reinterpret_cast<const uint4 *>(v)[c];
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int r = q * 8 + (lane >> 2), c = lane & 3;
+        const uint4 w = *reinterpret_cast<const uint4 *>(st + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+        if (row0 + r < M) *reinterpret_cast<uint4 *>(dst + (row0 + r) * kWsHidden + c * 8) = w;
+    }
+    __syncwarp();
+}
+
+template <int PASS>
+__global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_chain(
+    const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tw0, const __grid_constant__ CUtensorMap tw1,
+    const __grid_constant__ CUtensorMap tw2, const __grid_constant__ CUtensorMap tw3, const __grid_constant__ CUtensorMap tw4,
+    const __grid_constant__ CUtensorMap tw5, const __grid_constant__ ChainArgs g)
+{
+    constexpr int kStages = chain_stages(PASS), NL = chain_layers(PASS), KX = chain_k(PASS, 0);
     extern __shared__ __align__(1024) unsigned char sm[];
-    unsigned char *wsm = sm, *ring = sm + kMaxChunks * kStageB, *epi = ring + kStages * kStageA;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(epi + kEpiWarps * kEpiStage);
-    // bars: full[kStages], empty[kStages], acc_full[2], acc_empty[2], b_full[kMaxChunks]
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2 * kStages + 4 + kMaxChunks);
+    unsigned char *ring = sm;                                           // weight chunks
+    unsigned char *hbuf = sm + kStages * kStageB;                    // activations of two tiles
+    unsigned char *epi = hbuf + 2 * kActs;                               // rows on their way, per epilogue warp
+    uint64_t *bars = reinterpret_cast<uint64_t *>(epi + (PASS == PASS_INFER ? 0 : kEpiWarps * kEpiStage));
+    // bars: full[], empty[]; of each tile x_full, h_free, acc_full, h_ready
+    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2 * kStages + 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t bar0 = smem_u32(bars);
     auto full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
     auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(kStages + s); };
-    auto accf = [&](int a) { return bar0 + 8u * (uint32_t)(2 * kStages + a); };
-    auto acce = [&](int a) { return bar0 + 8u * (uint32_t)(2 * kStages + 2 + a); };
-    auto bfull = [&](int c) { return bar0 + 8u * (uint32_t)(2 * kStages + 4 + c); };
-    if (warp == kEpiWarps) tmem_alloc(smem_u32(slot), 512);
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        for (int a = 0; a < 2; a++) { mbar_init(accf(a), 1); mbar_init(acce(a), kEpiWarps); }
-        for (int c = 0; c < kMaxChunks; c++) mbar_init(bfull(c), 1);
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *slot;
-    const bool sw = g.K >= kChunk;
-    const int chunk = sw ? kChunk : g.K, nchunk = g.K / chunk, nbox = sw ? 1 : chunk / 8, wbox = sw ? kChunk : 8;
-    const long long tiles = (g.M + 127) / 128;
-    bool failed = false;
-    if (warp == kEpiWarps) {
-        if (lane == 0) {
-            long long it = 0;
-            for (long long t = blockIdx.x; t < tiles && !failed; t += gridDim.x)
-                for (int kc = 0; kc < nchunk; kc++, it++) {
-                    const int s = (int)(it % kStages);
-                    if (it < nchunk) {
-                        mbar_expect_tx(bfull(kc), (uint32_t)chunk * (uint32_t)g.N * 2u);
-                        for (int b = 0; b < nbox; b++)
-                            tma_load_2d(smem_u32(wsm + (size_t)kc * kStageB) + (uint32_t)b * (uint32_t)g.N * 16u, &tmB, kc * chunk + b * wbox, 0,
-                                        bfull(kc));
-                    }
-                    if (!mbar_wait_bounded(empty(s), (uint32_t)((it / kStages) & 1) ^ 1u)) { failed = true; break; }
-                    mbar_expect_tx(full(s), (uint32_t)chunk * 128u * 2u);
-                    for (int b = 0; b < nbox; b++)
-                        tma_load_2d(smem_u32(ring + (size_t)s * kStageA) + (uint32_t)b * 128u * 16u, &tmA, kc * chunk + b * wbox, (int)(t * 128),
-                                    full(s));
-                }
-            // nothing of a tile that was given up on may still be on its way when the CTA ends
-            if (failed) {
-                for (int c = 0; c < nchunk && c < it; c++) mbar_wait_bounded(bfull(c), 0u);
-                for (long long q = it < kStages ? 0 : it - kStages; q < it; q++)
-                    mbar_wait_bounded(full((int)(q % kStages)), (uint32_t)((q / kStages) & 1));
-            }
-        }
-    } else if (warp == kEpiWarps + 1) {
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16(128, g.N);
-            long long it = 0, ai = 0;
-            for (long long t = blockIdx.x; t < tiles && !failed; t += gridDim.x, ai++) {
-                const int a = (int)(ai & 1);
-                if (!mbar_wait_bounded(acce(a), (uint32_t)(((ai >> 1) & 1) ^ 1))) { failed = true; break; }
-                tc_fence_after();
-                for (int kc = 0; kc < nchunk; kc++, it++) {
-                    const int s = (int)(it % kStages);
-                    if (it < nchunk && !mbar_wait_bounded(bfull(kc), 0u)) { failed = true; break; }
-                    if (!mbar_wait_bounded(full(s), (uint32_t)((it / kStages) & 1))) { failed = true; break; }
-                    tc_fence_after();
-                    const uint32_t a_s = smem_u32(ring + (size_t)s * kStageA), b_s = smem_u32(wsm + (size_t)kc * kStageB);
-                    for (int ks = 0; ks < chunk / 16; ks++)
-                        mma_bf16(tmem + (uint32_t)(a * 256),
-                                 sw ? smem_desc_sw(a_s + (uint32_t)ks * 32u, 16u, 1024u) : smem_desc(a_s + (uint32_t)ks * 4096u, 2048u, 128u),
-                                 sw ? smem_desc_sw(b_s + (uint32_t)ks * 32u, 16u, 1024u)
-                                    : smem_desc(b_s + (uint32_t)ks * 2u * (uint32_t)g.N * 16u, (uint32_t)g.N * 16u, 128u),
-                                 idesc, (kc > 0 || ks > 0) ? 1u : 0u);
-                    mma_commit(empty(s));
-                }
-                if (failed) break;
-                mma_commit(accf(a));
-            }
-        }
-    } else {
-        long long ai = 0;
-        unsigned char *st = epi + warp * kEpiStage;
-        for (long long t = blockIdx.x; t < tiles; t += gridDim.x, ai++) {
-            const int a = (int)(ai & 1);
-            const int quad = warp & 3;
-            const long long row0 = t * 128 + quad * 32, row = row0 + lane;
-            const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * 256);
-            if constexpr (EPI == 1) {
-                const bool ok = mbar_wait_bounded(accf(a), (uint32_t)((ai >> 1) & 1));
-                tc_fence_after();
-                if (!ok) { failed = true; break; }
-                for (int c0 = (warp >> 2) * 16; c0 < g.N; c0 += 64) {
-                    float v[16];
-                    tmem_ld16(acc + (uint32_t)c0, v);
-                    if (row >= g.M) continue;
-                    float4 *yp = reinterpret_cast<float4 *>(g.Y + row * g.ldo + c0);
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        yp[i] = make_float4(v[4 * i] + g.bias[c0 + 4 * i], v[4 * i + 1] + g.bias[c0 + 4 * i + 1],
-                                            v[4 * i + 2] + g.bias[c0 + 4 * i + 2], v[4 * i + 3] + g.bias[c0 + 4 * i + 3]);
-                }
-            } else {
-                const int cbeg = (warp >> 2) * 64;
-                uint4 zl[2][4];                          // Z of the warp's 64 columns, asked for before the wait
-                if constexpr (EPI == 2) {
-#pragma unroll
-                    for (int h = 0; h < 2; h++)
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const long long r = row0 + q * 8 + (lane >> 2);
-                            zl[h][q] = r < g.M ? *reinterpret_cast<const uint4 *>(g.Zp + r * g.ldo + cbeg + h * 32 + (lane & 3) * 8)
-                                               : make_uint4(0u, 0u, 0u, 0u);
-                        }
-                }
-                const bool ok = mbar_wait_bounded(accf(a), (uint32_t)((ai >> 1) & 1));
-                tc_fence_after();
-                if (!ok) { failed = true; break; }
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int c0 = cbeg + h * 32;
-                    float v[32];
-                    tmem_ld32(acc + (uint32_t)c0, v);
-                    if constexpr (EPI == 0) {
-                        alignas(16) bf16 zo[32], ho[32];
-#pragma unroll
-                        for (int i = 0; i < 32; i += 4) {
-                            const float4 b = *reinterpret_cast<const float4 *>(g.bias + c0 + i);
-                            const float bb[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-                            for (int n = 0; n < 4; n++) {
-                                const float z = v[i + n] + bb[n];
-                                zo[i + n] = __float2bfloat16_rn(z);
-                                ho[i + n] = __float2bfloat16_rn(z * sigmoidf_(z));
-                            }
-                        }
-                        store_rows32(st, lane, zo, g.Z + c0, row0, g.M, g.ldo);
-                        store_rows32(st, lane, ho, g.H + c0, row0, g.M, g.ldo);
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const int r = q * 8 + (lane >> 2), c = lane & 3;
-                            *reinterpret_cast<uint4 *>(st + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) = zl[h][q];
-                        }
-                        __syncwarp();
-                        alignas(16) bf16 zi[32], dz[32];
-#pragma unroll
-                        for (int c = 0; c < 4; c++)
-                            reinterpret_cast<uint4 *>(zi)[c] = *reinterpret_cast<const uint4 *>(st + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4));
-                        __syncwarp();
-#pragma unroll
-                        for (int i = 0; i < 32; i++) {
-                            const float z = __bfloat162float(zi[i]);
-                            const float sg = sigmoidf_(z);
-                            dz[i] = __float2bfloat16_rn(v[i] * (sg * (1.0f + z * (1.0f - sg))));
-                        }
-                        store_rows32(st, lane, dz, g.dZ + c0, row0, g.M, g.ldo);
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acce(a));
-        }
-    }
-    if (failed) atomicOr(g.err, 1);
-    __syncwarp();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (warp == kEpiWarps) tmem_dealloc(tmem, 512);
-}
-
-// ---------------------------------------------------------------- inference, all layers fused
-// Y[rows x 16] = the whole network on X[rows x 64], the activations kept on chip. A CTA works on two tiles of
-// 128 rows in turn, so that the tensor cores run a layer of one while the epilogue warps are on the
-// other: each has a shared-memory buffer of activations (K-major core matrices: 8-column groups 2 KB
-// apart, rows 16 B apart) and a TMEM accumulator. Roles as in k_mlp_gemm, persistent over the tiles:
-//   warp 16: TMA producer. Loads a tile's features into its activation buffer once the last layer of the
-//     buffer's previous tile has read it, and streams the weights, 64-column chunk by chunk in the
-//     128-byte swizzle, layer by layer and tile by tile, through a 3-stage ring (they stay in L2).
-//   warp 17: MMA issuer. Per layer and tile: waits for the tile's epilogue of the layer before (its
-//     outputs are this layer's inputs, and it has read the accumulator out), issues the layer's MMAs with A
-//     from the activation buffer, commits the accumulator; after the last layer it frees the buffer.
-//   warps 0-15: epilogue. Per layer and tile: bias and SiLU of the accumulator, rounded to BF16 and written
-//     over the activation buffer (hidden layers), or bias and FP32 rows of Y (the output layer).
-// The arithmetic is the layer-by-layer forward's (same MMA order, same epilogue), so the outputs are the
-// same bits; nothing but X and Y crosses HBM. Bound by the epilogue's MUFU operations (two an
-// element, 16 a clock: 144 us for 262144 rows); with boxes of 8 columns (about one row of 16 bytes a
-// clock) and one tile at a time 375 us, now 196 us.
-struct InferArgs {
-    long long M;
-    const float *bias[kWsLayers];
-    float *Y;
-    int *err;
-};
-constexpr int kInfStages = 3;
-constexpr int kInfH = 128 * kWsHidden * 2;                  // 64 KB of activations
-constexpr int kInfSmem = 2 * kInfH + kInfStages * kStageB + 256;
-__host__ __device__ constexpr int inf_n(int l) { return l == kWsLayers - 1 ? kWsOut : kWsHidden; }
-__host__ __device__ constexpr int inf_chunks(int l) { return l == 0 ? kWsIn / kChunk : kWsHidden / kChunk; }
-
-__global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_infer(
-    const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tw0, const __grid_constant__ CUtensorMap tw1,
-    const __grid_constant__ CUtensorMap tw2, const __grid_constant__ CUtensorMap tw3, const __grid_constant__ CUtensorMap tw4,
-    const __grid_constant__ CUtensorMap tw5, InferArgs g)
-{
-    extern __shared__ __align__(1024) unsigned char sm[];
-    unsigned char *ring = sm;                                           // weight chunks
-    unsigned char *hbuf = sm + kInfStages * kStageB;                    // activations of two tiles
-    uint64_t *bars = reinterpret_cast<uint64_t *>(hbuf + 2 * kInfH);
-    // bars: full[3], empty[3]; of each tile x_full, h_free, acc_full, h_ready
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2 * kInfStages + 8);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t bar0 = smem_u32(bars);
-    auto full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
-    auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(kInfStages + s); };
-    auto x_full = [&](int h) { return bar0 + 8u * (uint32_t)(2 * kInfStages + 4 * h); };
+    auto x_full = [&](int h) { return bar0 + 8u * (uint32_t)(2 * kStages + 4 * h); };
     auto h_free = [&](int h) { return x_full(h) + 8u; };
     auto acc_full = [&](int h) { return x_full(h) + 16u; };
     auto h_ready = [&](int h) { return x_full(h) + 24u; };
     if (warp == kEpiWarps) tmem_alloc(smem_u32(slot), 512);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kInfStages; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (int s = 0; s < kStages; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
         for (int h = 0; h < 2; h++) {
             mbar_init(x_full(h), 1);
             mbar_init(h_free(h), 1);
@@ -446,26 +275,29 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_infer(
     if (warp == kEpiWarps) {
         if (lane == 0) {
             long long it = 0, p = 0;
-            int xs[2] = {0, 0};                                         // feature loads issued
+            int xs[2] = {0, 0};                                         // input loads issued
             for (long long t = blockIdx.x; t < tiles && !failed; t += step, p++) {
                 const int nh = t + gridDim.x < tiles ? 2 : 1;
-                for (int l = 0; l < kWsLayers && !failed; l++) {
+                for (int l = 0; l < NL && !failed; l++) {
                     const CUtensorMap *wm = l == 0 ? &tw0 : l == 1 ? &tw1 : l == 2 ? &tw2 : l == 3 ? &tw3 : l == 4 ? &tw4 : &tw5;
-                    const int n = inf_n(l);
+                    const int n = chain_n(PASS, l), k = chain_k(PASS, l), w = k < kChunk ? k : kChunk;
                     for (int h = 0; h < nh && !failed; h++) {
                         if (l == 0) {
                             if (!mbar_wait_bounded(h_free(h), (uint32_t)((p & 1) ^ 1))) { failed = true; break; }
-                            mbar_expect_tx(x_full(h), (uint32_t)(kWsIn / 8) * 128u * 16u);
-                            const uint32_t hb = smem_u32(hbuf + (size_t)h * kInfH);
-                            for (int k8 = 0; k8 < kWsIn / 8; k8++)
+                            mbar_expect_tx(x_full(h), (uint32_t)(KX / 8) * 128u * 16u);
+                            const uint32_t hb = smem_u32(hbuf + (size_t)h * kActs);
+                            for (int k8 = 0; k8 < KX / 8; k8++)
                                 tma_load_2d(hb + (uint32_t)k8 * 2048u, &tmX, k8 * 8, (int)((t + h * (long long)gridDim.x) * 128), x_full(h));
                             xs[h]++;
                         }
-                        for (int kc = 0; kc < inf_chunks(l); kc++, it++) {
-                            const int s = (int)(it % kInfStages);
-                            if (!mbar_wait_bounded(empty(s), (uint32_t)(((it / kInfStages) & 1) ^ 1))) { failed = true; break; }
-                            mbar_expect_tx(full(s), (uint32_t)(kChunk * n) * 2u);
-                            tma_load_2d(smem_u32(ring + (size_t)s * kStageB), wm, kc * kChunk, 0, full(s));
+                        for (int kc = 0; kc < k / w; kc++, it++) {
+                            const int s = (int)(it % kStages);
+                            if (!mbar_wait_bounded(empty(s), (uint32_t)(((it / kStages) & 1) ^ 1))) { failed = true; break; }
+                            mbar_expect_tx(full(s), (uint32_t)(w * n) * 2u);
+                            const uint32_t b_s = smem_u32(ring + (size_t)s * kStageB);
+                            if (w == kChunk) tma_load_2d(b_s, wm, kc * kChunk, 0, full(s));
+                            else
+                                for (int k8 = 0; k8 < w / 8; k8++) tma_load_2d(b_s + (uint32_t)(k8 * n) * 16u, wm, k8 * 8, 0, full(s));
                         }
                     }
                 }
@@ -474,8 +306,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_infer(
             if (failed) {
                 for (int h = 0; h < 2; h++)
                     if (xs[h] > 0) mbar_wait_bounded(x_full(h), (uint32_t)((xs[h] - 1) & 1));
-                for (long long q = it < kInfStages ? 0 : it - kInfStages; q < it; q++)
-                    mbar_wait_bounded(full((int)(q % kInfStages)), (uint32_t)((q / kInfStages) & 1));
+                for (long long q = it < kStages ? 0 : it - kStages; q < it; q++)
+                    mbar_wait_bounded(full((int)(q % kStages)), (uint32_t)((q / kStages) & 1));
             }
         }
     } else if (warp == kEpiWarps + 1) {
@@ -484,8 +316,8 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_infer(
             uint32_t hu[2] = {0u, 0u};                                  // epilogues waited for
             for (long long t = blockIdx.x; t < tiles && !failed; t += step, p++) {
                 const int nh = t + gridDim.x < tiles ? 2 : 1;
-                for (int l = 0; l < kWsLayers && !failed; l++) {
-                    const int n = inf_n(l);
+                for (int l = 0; l < NL && !failed; l++) {
+                    const int n = chain_n(PASS, l), k = chain_k(PASS, l), w = k < kChunk ? k : kChunk;
                     const uint32_t idesc = idesc_bf16(128, n);
                     for (int h = 0; h < nh && !failed; h++) {
                         if (l == 0 && !mbar_wait_bounded(x_full(h), (uint32_t)(p & 1))) { failed = true; break; }
@@ -495,21 +327,23 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_infer(
                             hu[h]++;
                         }
                         tc_fence_after();
-                        const uint32_t hb = smem_u32(hbuf + (size_t)h * kInfH);
-                        for (int kc = 0; kc < inf_chunks(l); kc++, it++) {
-                            const int s = (int)(it % kInfStages);
-                            if (!mbar_wait_bounded(full(s), (uint32_t)((it / kInfStages) & 1))) { failed = true; break; }
+                        const uint32_t hb = smem_u32(hbuf + (size_t)h * kActs);
+                        for (int kc = 0; kc < k / w; kc++, it++) {
+                            const int s = (int)(it % kStages);
+                            if (!mbar_wait_bounded(full(s), (uint32_t)((it / kStages) & 1))) { failed = true; break; }
                             tc_fence_after();
                             const uint32_t b_s = smem_u32(ring + (size_t)s * kStageB);
-                            for (int ks = 0; ks < kChunk / 16; ks++)
+                            for (int ks = 0; ks < w / 16; ks++)
                                 mma_bf16(tmem + (uint32_t)(h * 256),
                                          smem_desc(hb + (uint32_t)(kc * (kChunk / 16) + ks) * 2u * 2048u, 2048u, 128u),
-                                         smem_desc_sw(b_s + (uint32_t)ks * 32u, 16u, 1024u), idesc, (kc > 0 || ks > 0) ? 1u : 0u);
+                                         w == kChunk ? smem_desc_sw(b_s + (uint32_t)ks * 32u, 16u, 1024u)
+                                                     : smem_desc(b_s + (uint32_t)(2 * ks * n) * 16u, (uint32_t)n * 16u, 128u),
+                                         idesc, (kc > 0 || ks > 0) ? 1u : 0u);
                             mma_commit(empty(s));
                         }
                         if (failed) break;
                         mma_commit(acc_full(h));
-                        if (l == kWsLayers - 1) mma_commit(h_free(h));
+                        if (l == NL - 1) mma_commit(h_free(h));
                     }
                 }
             }
@@ -517,43 +351,86 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_infer(
     } else {
         uint32_t au[2] = {0u, 0u};                                     // accumulators waited for
         const int quad = warp & 3;
+        unsigned char *st = epi + warp * kEpiStage;
         const int r = quad * 32 + lane;                                // the TMEM lane = row of the tile
         for (long long t = blockIdx.x; t < tiles && !failed; t += step) {
             const int nh = t + gridDim.x < tiles ? 2 : 1;
-            for (int l = 0; l < kWsLayers && !failed; l++) {
-                const float *bias = g.bias[l];
+            for (int l = 0; l < NL && !failed; l++) {
                 for (int h = 0; h < nh; h++) {
+                    const long long row0 = (t + h * (long long)gridDim.x) * 128 + quad * 32;
+                    const int cbeg = (warp >> 2) * (kWsHidden / 4);
+                    uint4 zl[2][4];                          // Z of the warp's 64 columns, asked for before the wait
+                    if constexpr (PASS == PASS_BACKWARD) {
+                        const bf16 *Z = g.Z[NL - 1 - l] + cbeg + (lane & 3) * 8;
+#pragma unroll
+                        for (int c = 0; c < 2; c++)
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {
+                                const long long zr = row0 + q * 8 + (lane >> 2);
+                                zl[c][q] = zr < g.M ? *reinterpret_cast<const uint4 *>(Z + zr * kWsHidden + c * 32) : make_uint4(0u, 0u, 0u, 0u);
+                            }
+                    }
                     const bool ok = mbar_wait_bounded(acc_full(h), au[h] & 1u);
                     au[h]++;
                     tc_fence_after();
                     if (!ok) { failed = true; break; }
                     const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(h * 256);
-                    if (l < kWsLayers - 1) {
-                        const int cbeg = (warp >> 2) * (kWsHidden / 4);
-                        unsigned char *hb = hbuf + (size_t)h * kInfH + (size_t)r * 16;
+                    if (PASS == PASS_BACKWARD || l < NL - 1) {
+                        const float *bias = g.bias[l];
+                        unsigned char *hb = hbuf + (size_t)h * kActs + (size_t)r * 16;
 #pragma unroll
-                        for (int c0 = cbeg; c0 < cbeg + kWsHidden / 4; c0 += 32) {
+                        for (int c = 0; c < 2; c++) {
+                            const int c0 = cbeg + c * 32;
                             float v[32];
                             tmem_ld32(acc + (uint32_t)c0, v);
                             alignas(16) bf16 ho[32];
+                            if constexpr (PASS == PASS_BACKWARD) {
 #pragma unroll
-                            for (int i = 0; i < 32; i += 4) {
-                                const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + i);
-                                const float bb[4] = {b.x, b.y, b.z, b.w};
+                                for (int q = 0; q < 4; q++) {
+                                    const int zr = q * 8 + (lane >> 2), zc = lane & 3;
+                                    *reinterpret_cast<uint4 *>(st + zr * 64 + ((zc ^ ((zr >> 1) & 3)) << 4)) = zl[c][q];
+                                }
+                                __syncwarp();
+                                alignas(16) bf16 zi[32];
 #pragma unroll
-                                for (int n = 0; n < 4; n++) {
-                                    const float z = v[i + n] + bb[n];
-                                    ho[i + n] = __float2bfloat16_rn(z * sigmoidf_(z));
+                                for (int q = 0; q < 4; q++)
+                                    reinterpret_cast<uint4 *>(zi)[q] = *reinterpret_cast<const uint4 *>(st + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4));
+                                __syncwarp();
+#pragma unroll
+                                for (int i = 0; i < 32; i++) {
+                                    const float z = __bfloat162float(zi[i]);
+                                    const float sg = sigmoidf_(z);
+                                    ho[i] = __float2bfloat16_rn(v[i] * (sg * (1.0f + z * (1.0f - sg))));
+                                }
+                                store_rows32(st, lane, ho, g.dZ[NL - 1 - l] + c0, row0, g.M);
+                            } else {
+                                alignas(16) bf16 zo[32];
+#pragma unroll
+                                for (int i = 0; i < 32; i += 4) {
+                                    const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + i);
+                                    const float bb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                                    for (int n = 0; n < 4; n++) {
+                                        const float z = v[i + n] + bb[n];
+                                        zo[i + n] = __float2bfloat16_rn(z);
+                                        ho[i + n] = __float2bfloat16_rn(z * sigmoidf_(z));
+                                    }
+                                }
+                                if constexpr (PASS == PASS_FORWARD) {
+                                    store_rows32(st, lane, zo, g.Z[l] + c0, row0, g.M);
+                                    store_rows32(st, lane, ho, g.H[l] + c0, row0, g.M);
                                 }
                             }
+                            if (l < NL - 1)
 #pragma unroll
-                            for (int c = 0; c < 4; c++)
-                                *reinterpret_cast<uint4 *>(hb + (size_t)(c0 / 8 + c) * 2048) = reinterpret_cast<uint4 *>(ho)[c];
+                                for (int q = 0; q < 4; q++)
+                                    *reinterpret_cast<uint4 *>(hb + (size_t)(c0 / 8 + q) * 2048) = reinterpret_cast<uint4 *>(ho)[q];
                         }
                     } else if (warp < 4) {
+                        const float *bias = g.bias[l];
                         float v[16];
                         tmem_ld16(acc, v);
-                        const long long row = (t + h * (long long)gridDim.x) * 128 + r;
+                        const long long row = row0 + lane;
                         if (row < g.M) {
                             float4 *yp = reinterpret_cast<float4 *>(g.Y + row * kWsOut);
 #pragma unroll
@@ -1067,7 +944,8 @@ constexpr int kLossKept = 20;                    // steps whose loss train() ave
 static size_t b_off(int l) { return w_off(l) + (size_t)kN[l] * kK[l]; }
 
 struct WarmStart::Impl {
-    cudaStream_t st = nullptr;
+    cudaStream_t st = nullptr, st2 = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     int n_sm = 0;
     float *P = nullptr, *G = nullptr, *Mo = nullptr, *Vo = nullptr;
     bf16 *Wb[kWsLayers] = {}, *Wt[kWsLayers] = {};
@@ -1127,64 +1005,39 @@ struct WarmStart::Impl {
         cap = 0;
     }
 
-    template <int EPI>
-    void gemm(const bf16 *A, long long lda, int l_w, bool transposed, long long M, int N, int K, const float *bias, bf16 *Zo,
-              bf16 *Ho, float *Yo, long long ldo, const bf16 *Zp, bf16 *dZ)
-    {
-        if (M <= 0) return;
-        GemmArgs g{};
-        g.M = M; g.N = N; g.K = K;
-        g.bias = bias; g.Z = Zo; g.H = Ho; g.Y = Yo; g.ldo = ldo; g.Zp = Zp; g.dZ = dZ; g.err = err;
-        const CUtensorMap ta = tensor_map_rows(A, M, K, lda, 128);
-        const CUtensorMap tb = tensor_map_rows(transposed ? Wt[l_w] : Wb[l_w], N, K, K, N);
-        const long long tiles = (M + 127) / 128;
-        const int grid = (int)std::min<long long>(tiles, n_sm);
-        k_mlp_gemm<EPI><<<grid, 32 * (kEpiWarps + 2), kTcSmem, st>>>(ta, tb, g);
-        WCK(cudaGetLastError());
-    }
-
     void refresh_bf16()
     {
         for (int l = 0; l < kWsLayers; l++)
             k_ws_weights_bf16<<<(kN[l] * kK[l] + 255) / 256, 256, 0, st>>>(P + w_off(l), kN[l], kK[l], Wb[l], Wt[l]);
     }
 
-    // rows of X0 -> Y with every layer fused in one kernel (inference: no activations kept)
-    void infer(long long M)
+    template <int PASS>
+    void chain(long long M)
     {
         if (M <= 0) return;
-        InferArgs g{};
+        ChainArgs g{};
         g.M = M; g.Y = Y; g.err = err;
         for (int l = 0; l < kWsLayers; l++) g.bias[l] = P + b_off(l);
-        const CUtensorMap tx = tensor_map_rows(X0, M, kWsIn, kWsIn, 128, false);
-        CUtensorMap tw[kWsLayers];
-        for (int l = 0; l < kWsLayers; l++) tw[l] = tensor_map_rows(Wb[l], kN[l], kK[l], kK[l], kN[l]);
-        const long long tiles = (M + 127) / 128;
-        const int grid = (int)std::min<long long>(tiles, n_sm);
-        k_mlp_infer<<<grid, 32 * (kEpiWarps + 2), kInfSmem, st>>>(tx, tw[0], tw[1], tw[2], tw[3], tw[4], tw[5], g);
+        for (int l = 0; l < kWsLayers - 1; l++) { g.Z[l] = Z[l]; g.H[l] = H[l]; g.dZ[l] = dZ[l]; }
+        const bool back = PASS == PASS_BACKWARD;
+        const int kx = chain_k(PASS, 0);
+        const CUtensorMap tx = tensor_map_rows(back ? dY : X0, M, kx, kx, 128, false);
+        CUtensorMap tw[kWsLayers] = {};
+        for (int l = 0; l < chain_layers(PASS); l++)
+            tw[l] = tensor_map_rows(back ? Wt[kWsLayers - 1 - l] : Wb[l], chain_n(PASS, l), chain_k(PASS, l), chain_k(PASS, l), chain_n(PASS, l));
+        const int grid = (int)std::min<long long>((M + 127) / 128, n_sm);
+        k_mlp_chain<PASS><<<grid, 32 * (kEpiWarps + 2), chain_smem(PASS), st>>>(tx, tw[0], tw[1], tw[2], tw[3], tw[4], tw[5], g);
         WCK(cudaGetLastError());
     }
-
-    // rows of X0 -> Y (and the hidden activations, which training needs)
-    void forward(long long M)
-    {
-        const bf16 *in = X0;
-        long long ld = kWsIn;
-        for (int l = 0; l < 5; l++) {
-            gemm<0>(in, ld, l, false, M, kN[l], kK[l], P + b_off(l), Z[l], H[l], nullptr, kWsHidden, nullptr, nullptr);
-            in = H[l];
-            ld = kWsHidden;
-        }
-        gemm<1>(in, ld, 5, false, M, kWsOut, kWsHidden, P + b_off(5), nullptr, nullptr, Y, kWsOut, nullptr, nullptr);
-    }
+    // rows of X0 -> Y (inference: no activations kept)
+    void infer(long long M) { chain<PASS_INFER>(M); }
+    // rows of X0 -> Y and the hidden activations, which training needs
+    void forward(long long M) { chain<PASS_FORWARD>(M); }
 
     // from dY: every gradient (mean over the M rows) into G, or with adam the optimiser step
     void backward(long long M, const StepArgs *adam = nullptr)
     {
-        // dZ5 = (dY . W6) * SiLU'(Z5), and so on down to dZ1
-        gemm<2>(dY, kWsOut, 5, true, M, kWsHidden, kWsOut, nullptr, nullptr, nullptr, nullptr, kWsHidden, Z[4], dZ[4]);
-        for (int l = 4; l >= 1; l--)
-            gemm<2>(dZ[l], kWsHidden, l, true, M, kWsHidden, kWsHidden, nullptr, nullptr, nullptr, nullptr, kWsHidden, Z[l - 1], dZ[l - 1]);
+        chain<PASS_BACKWARD>(M);
         // dW[l] = dZ^T . inputs, with 256 rows on the a side: of the last layer the transposed, H5^T . dY
         const int gy = kWsHidden / 128;
         int gx = std::max(1, n_sm / gy);
@@ -1224,8 +1077,13 @@ struct WarmStart::Impl {
             t.Wb[l] = Wb[l]; t.Wt[l] = Wt[l]; t.trans[l] = last;
             t.first[l + 1] = t.first[l] + kWsHidden / 32 * ((t.Nb[l] + 31) / 32);
         }
+        // the column sums need no shared memory, so they run beside the weight gradients
+        WCK(cudaEventRecord(fork, st));
+        WCK(cudaStreamWaitEvent(st2, fork, 0));
+        k_colsum_partial<<<dim3(nb, kWsLayers), 128, 0, st2>>>(c);
         k_mlp_wgrad<<<dim3(gx, gy, kWsLayers), 192, kWgSmem, st>>>(w);
-        k_colsum_partial<<<dim3(nb, kWsLayers), 128, 0, st>>>(c);
+        WCK(cudaEventRecord(join, st2));
+        WCK(cudaStreamWaitEvent(st, join, 0));
         if (adam) k_ws_step<true><<<t.first[kWsLayers] + kWsLayers, 256, 0, st>>>(t);
         else k_ws_step<false><<<t.first[kWsLayers] + kWsLayers, 256, 0, st>>>(t);
         WCK(cudaGetLastError());
@@ -1258,11 +1116,13 @@ WarmStart::WarmStart(unsigned seed) : d(new Impl)
     WCK(cudaGetDevice(&dev));
     WCK(cudaDeviceGetAttribute(&d->n_sm, cudaDevAttrMultiProcessorCount, dev));
     WCK(cudaStreamCreateWithFlags(&d->st, cudaStreamNonBlocking));
-    WCK(cudaFuncSetAttribute(k_mlp_gemm<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
-    WCK(cudaFuncSetAttribute(k_mlp_gemm<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
-    WCK(cudaFuncSetAttribute(k_mlp_gemm<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
+    WCK(cudaStreamCreateWithFlags(&d->st2, cudaStreamNonBlocking));
+    WCK(cudaEventCreateWithFlags(&d->fork, cudaEventDisableTiming));
+    WCK(cudaEventCreateWithFlags(&d->join, cudaEventDisableTiming));
+    WCK(cudaFuncSetAttribute(k_mlp_chain<PASS_INFER>, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_smem(PASS_INFER)));
+    WCK(cudaFuncSetAttribute(k_mlp_chain<PASS_FORWARD>, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_smem(PASS_FORWARD)));
+    WCK(cudaFuncSetAttribute(k_mlp_chain<PASS_BACKWARD>, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_smem(PASS_BACKWARD)));
     WCK(cudaFuncSetAttribute(k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem));
-    WCK(cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfSmem));
     const size_t np = n_params();
     WCK(cudaMalloc(&d->P, sizeof(float) * np));
     WCK(cudaMalloc(&d->G, sizeof(float) * np));
@@ -1307,6 +1167,10 @@ WarmStart::~WarmStart()
     for (int l = 0; l < kWsLayers; l++) { cudaFree(d->Wb[l]); cudaFree(d->Wt[l]); }
     cudaFree(d->err); cudaFree(d->nrm_d); cudaFree(d->part); cudaFree(d->cpart); cudaFree(d->set);
     cudaStreamDestroy(d->st);
+    cudaStreamSynchronize(d->st2);
+    cudaStreamDestroy(d->st2);
+    cudaEventDestroy(d->fork);
+    cudaEventDestroy(d->join);
     delete d;
 }
 
