@@ -804,10 +804,34 @@ __global__ void k_ws_weights_bf16(const float *w, int N, int K, bf16 *wb, bf16 *
     wt[(size_t)k * N + n] = b;
 }
 
-__global__ void k_f32_to_bf16(const float *x, long long n, bf16 *y)
+// n values to BF16; V = 4 values a load (x 16-byte aligned), 4 loads in flight a thread. x may be the caller's
+// host memory: 262144 rows of 64 read over the link to the CPU at 200 GB/s, 0.34 ms, where a copy to
+// the device takes 0.50 ms and the conversion from there 0.04.
+template <int V>
+__global__ void __launch_bounds__(256) k_f32_to_bf16(const float *x, long long n, bf16 *y)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = __float2bfloat16_rn(x[i]);
+    const long long i0 = ((long long)blockIdx.x * 1024 + threadIdx.x) * V;
+    float v[4][V];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const long long i = i0 + q * 256 * V;
+        if (i + V <= n) {
+            if constexpr (V == 4) {
+                const float4 t = *reinterpret_cast<const float4 *>(x + i);
+                v[q][0] = t.x; v[q][1] = t.y; v[q][2] = t.z; v[q][3] = t.w;
+            } else v[q][0] = x[i];
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const long long i = i0 + q * 256 * V;
+        if (i + V > n) continue;
+        alignas(8) bf16 o[V];
+#pragma unroll
+        for (int u = 0; u < V; u++) o[u] = __float2bfloat16_rn(v[q][u]);
+        if constexpr (V == 4) *reinterpret_cast<uint2 *>(y + i) = *reinterpret_cast<uint2 *>(o);
+        else y[i] = o[0];
+    }
 }
 
 // ---------------------------------------------------------------- cells of a solver's fine level
@@ -949,12 +973,13 @@ static size_t w_off(int l)
     for (int q = 0; q < l; q++) o += (size_t)kN[q] * kK[q] + kN[q];
     return o;
 }
+constexpr long long kPiece = 32768;              // rows of a piece of a call on host rows (a multiple of 128)
 constexpr int kLossKept = 20;                    // steps whose loss train() averages
 static size_t b_off(int l) { return w_off(l) + (size_t)kN[l] * kK[l]; }
 
 struct WarmStart::Impl {
-    cudaStream_t st = nullptr, st2 = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t st = nullptr, st2 = nullptr, st3 = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, asked[3] = {}, made[2] = {};
     int n_sm = 0;
     float *P = nullptr, *G = nullptr, *Mo = nullptr, *Vo = nullptr;
     bf16 *Wb[kWsLayers] = {}, *Wt[kWsLayers] = {};
@@ -966,6 +991,8 @@ struct WarmStart::Impl {
     // rows in and out for up to cap rows, activations, targets and gradients for up to tcap
     long long cap = 0, tcap = 0;
     bf16 *X0 = nullptr, *Z[5] = {}, *H[5] = {}, *dY = nullptr, *dZ[5] = {};
+    float *F = nullptr;                              // host rows on their way, where the device cannot read them
+    bool host_rows = false;
     float *Y = nullptr, *T = nullptr, *part = nullptr, *cpart = nullptr, *lpart = nullptr;
     size_t part_n = 0;
     // training set
@@ -1020,17 +1047,33 @@ struct WarmStart::Impl {
             k_ws_weights_bf16<<<(kN[l] * kK[l] + 255) / 256, 256, 0, st>>>(P + w_off(l), kN[l], kK[l], Wb[l], Wt[l]);
     }
 
+    // features of M host rows from row r0 on into X0, on stream q: read by the kernel where the device reaches
+    // pageable memory through the host's page tables, copied first where it does not
+    void features(const float *feat, long long r0, long long M, cudaStream_t q)
+    {
+        const float *x = feat + r0 * kWsIn;
+        if (!host_rows) {
+            if (!F) F = af(kPiece * kWsIn);
+            WCK(cudaMemcpyAsync(F, x, sizeof(float) * (size_t)M * kWsIn, cudaMemcpyHostToDevice, q));
+            x = F;
+        }
+        const long long n = M * kWsIn;
+        if (((uintptr_t)x & 15) == 0) k_f32_to_bf16<4><<<(unsigned)((n + 4095) / 4096), 256, 0, q>>>(x, n, X0 + r0 * kWsIn);
+        else k_f32_to_bf16<1><<<(unsigned)((n + 1023) / 1024), 256, 0, q>>>(x, n, X0 + r0 * kWsIn);
+        WCK(cudaGetLastError());
+    }
+
     template <int PASS>
-    void chain(long long M)
+    void chain(long long M, long long r0 = 0)
     {
         if (M <= 0) return;
         ChainArgs g{};
-        g.M = M; g.Y = Y; g.err = err;
+        g.M = M; g.Y = Y + r0 * kWsOut; g.err = err;
         for (int l = 0; l < kWsLayers; l++) g.bias[l] = P + b_off(l);
         for (int l = 0; l < kWsLayers - 1; l++) { g.Z[l] = Z[l]; g.H[l] = H[l]; g.dZ[l] = dZ[l]; }
         const bool back = PASS == PASS_BACKWARD;
         const int kx = chain_k(PASS, 0);
-        const CUtensorMap tx = tensor_map_rows(back ? dY : X0, M, kx, kx, 128, false);
+        const CUtensorMap tx = tensor_map_rows(back ? dY : X0 + r0 * kWsIn, M, kx, kx, 128, false);
         CUtensorMap tw[kWsLayers] = {};
         for (int l = 0; l < chain_layers(PASS); l++)
             tw[l] = tensor_map_rows(back ? Wt[kWsLayers - 1 - l] : Wb[l], chain_n(PASS, l), chain_k(PASS, l), chain_k(PASS, l), chain_n(PASS, l));
@@ -1038,8 +1081,8 @@ struct WarmStart::Impl {
         k_mlp_chain<PASS><<<grid, 32 * (kEpiWarps + 2), chain_smem(PASS), st>>>(tx, tw[0], tw[1], tw[2], tw[3], tw[4], tw[5], g);
         WCK(cudaGetLastError());
     }
-    // rows of X0 -> Y (inference: no activations kept)
-    void infer(long long M) { chain<PASS_INFER>(M); }
+    // rows r0 .. r0 + M - 1 of X0 -> Y (inference: no activations kept)
+    void infer(long long M, long long r0 = 0) { chain<PASS_INFER>(M, r0); }
     // rows of X0 -> Y and the hidden activations, which training needs
     void forward(long long M) { chain<PASS_FORWARD>(M); }
 
@@ -1126,8 +1169,15 @@ WarmStart::WarmStart(unsigned seed) : d(new Impl)
     WCK(cudaDeviceGetAttribute(&d->n_sm, cudaDevAttrMultiProcessorCount, dev));
     WCK(cudaStreamCreateWithFlags(&d->st, cudaStreamNonBlocking));
     WCK(cudaStreamCreateWithFlags(&d->st2, cudaStreamNonBlocking));
+    int reach = 0, tables = 0;
+    WCK(cudaDeviceGetAttribute(&reach, cudaDevAttrPageableMemoryAccess, dev));
+    WCK(cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev));
+    d->host_rows = reach && tables;
     WCK(cudaEventCreateWithFlags(&d->fork, cudaEventDisableTiming));
     WCK(cudaEventCreateWithFlags(&d->join, cudaEventDisableTiming));
+    WCK(cudaStreamCreateWithFlags(&d->st3, cudaStreamNonBlocking));
+    for (auto &e : d->made) WCK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (auto &e : d->asked) WCK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     WCK(cudaFuncSetAttribute(k_mlp_chain<PASS_INFER>, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_smem(PASS_INFER)));
     WCK(cudaFuncSetAttribute(k_mlp_chain<PASS_FORWARD>, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_smem(PASS_FORWARD)));
     WCK(cudaFuncSetAttribute(k_mlp_chain<PASS_BACKWARD>, cudaFuncAttributeMaxDynamicSharedMemorySize, chain_smem(PASS_BACKWARD)));
@@ -1174,12 +1224,15 @@ WarmStart::~WarmStart()
     d->release_acts();
     cudaFree(d->P); cudaFree(d->G); cudaFree(d->Mo); cudaFree(d->Vo);
     for (int l = 0; l < kWsLayers; l++) { cudaFree(d->Wb[l]); cudaFree(d->Wt[l]); }
-    cudaFree(d->err); cudaFree(d->nrm_d); cudaFree(d->part); cudaFree(d->cpart); cudaFree(d->set);
+    cudaFree(d->err); cudaFree(d->nrm_d); cudaFree(d->part); cudaFree(d->cpart); cudaFree(d->set); cudaFree(d->F);
     cudaStreamDestroy(d->st);
     cudaStreamSynchronize(d->st2);
     cudaStreamDestroy(d->st2);
     cudaEventDestroy(d->fork);
     cudaEventDestroy(d->join);
+    for (auto e : d->asked) cudaEventDestroy(e);
+    for (auto e : d->made) cudaEventDestroy(e);
+    cudaStreamDestroy(d->st3);
     delete d;
 }
 
@@ -1380,14 +1433,41 @@ void WarmStart::forward(const float *feat, int M, float *y)
 {
     Impl &m = *d;
     m.ensure(M);
-    DevBuf f;
-    f.bytes = sizeof(float) * (size_t)M * kWsIn;
-    WCK(cudaMalloc(&f.p, f.bytes));
-    WCK(cudaMemcpy(f.p, feat, f.bytes, cudaMemcpyHostToDevice));
-    k_f32_to_bf16<<<(unsigned)(((size_t)M * kWsIn + 255) / 256), 256, 0, m.st>>>((const float *)f.p, (long long)M * kWsIn, m.X0);
-    m.infer(M);
-    WCK(cudaMemcpyAsync(y, m.Y, sizeof(float) * (size_t)M * kWsOut, cudaMemcpyDeviceToHost, m.st));
-    WCK(cudaStreamSynchronize(m.st));
+    // nothing of the call may outlive it, also where it ends in an error: the kernels read the caller's rows
+    struct Done {
+        Impl &m;
+        ~Done() { cudaStreamSynchronize(m.st2); cudaStreamSynchronize(m.st); cudaStreamSynchronize(m.st3); }
+    } done{m};
+    // Piece by piece: features on st2 up to two pieces ahead of the network on st, the copy to the caller (which
+    // the host waits for) a piece behind it on st3. A caller whose y lies in its features gets one copy at the end.
+    const uintptr_t fa = (uintptr_t)feat, ya = (uintptr_t)y;
+    const bool apart = ya + sizeof(float) * (size_t)M * kWsOut <= fa || fa + sizeof(float) * (size_t)M * kWsIn <= ya;
+    const long long np = (M + kPiece - 1) / kPiece;
+    auto rows = [&](long long p) { return std::min(kPiece, M - p * kPiece); };
+    auto ask = [&](long long p) {
+        if (p >= np) return;
+        m.features(feat, p * kPiece, rows(p), m.st2);
+        WCK(cudaEventRecord(m.asked[p % 3], m.st2));
+    };
+    if (np == 1) m.features(feat, 0, M, m.st);
+    else for (long long p = 0; p < 2; p++) ask(p);
+    auto give = [&](long long p) {
+        const long long o = apart ? p * kPiece * kWsOut : 0, n = apart ? rows(p) : p == np - 1 ? M : 0;
+        if (n <= 0) return;
+        WCK(cudaStreamWaitEvent(m.st3, m.made[p % 2], 0));
+        WCK(cudaMemcpyAsync(y + o, m.Y + o, sizeof(float) * (size_t)n * kWsOut, cudaMemcpyDeviceToHost, m.st3));
+    };
+    for (long long p = 0; p < np; p++) {
+        if (np > 1) {
+            ask(p + 2);
+            WCK(cudaStreamWaitEvent(m.st, m.asked[p % 3], 0));
+        }
+        m.infer(rows(p), p * kPiece);
+        WCK(cudaEventRecord(m.made[p % 2], m.st));
+        if (p > 0) give(p - 1);
+    }
+    give(np - 1);
+    WCK(cudaStreamSynchronize(m.st3));
     if (error_flag()) throw std::runtime_error("a tensor-core wait of the warm-start network ran out");
 }
 
@@ -1395,12 +1475,12 @@ float WarmStart::forward_backward(const float *feat, const float *target, int M,
 {
     Impl &m = *d;
     m.ensure_train(M);
-    DevBuf f;
-    f.bytes = sizeof(float) * (size_t)M * kWsIn;
-    WCK(cudaMalloc(&f.p, f.bytes));
-    WCK(cudaMemcpy(f.p, feat, f.bytes, cudaMemcpyHostToDevice));
-    k_f32_to_bf16<<<(unsigned)(((size_t)M * kWsIn + 255) / 256), 256, 0, m.st>>>((const float *)f.p, (long long)M * kWsIn, m.X0);
     std::vector<float> t8((size_t)M * 8, 0.0f);
+    struct Done {
+        Impl &m;
+        ~Done() { cudaStreamSynchronize(m.st); }
+    } done{m};                                            // the kernels read the caller's rows
+    for (long long r0 = 0; r0 < M; r0 += kPiece) m.features(feat, r0, std::min<long long>(kPiece, M - r0), m.st);
     for (int r = 0; r < M; r++)
         for (int o = 0; o < kWsOutUsed; o++) t8[(size_t)r * 8 + o] = target[(size_t)r * kWsOutUsed + o];
     WCK(cudaMemcpyAsync(m.T, t8.data(), sizeof(float) * t8.size(), cudaMemcpyHostToDevice, m.st));

@@ -476,7 +476,7 @@ class WarmStart:
     def forward(self, feat) -> np.ndarray:
         f = np.ascontiguousarray(np.asarray(feat, dtype=np.float32))
         n = f.shape[0]
-        y = np.zeros((n, WS_OUT), dtype=np.float32)
+        y = np.empty((n, WS_OUT), dtype=np.float32)
         self._check(self._L.gb_ws_forward(self.h, _fptr(f), n, _fptr(y)))
         return y
 
