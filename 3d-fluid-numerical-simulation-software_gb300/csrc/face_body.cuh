@@ -51,7 +51,7 @@ __device__ __forceinline__ T tan_diff(const T *__restrict__ c, int p, int sn, in
     // away from the corners both means hold the two cells across the face, which cancel: in exact
     // arithmetic the reference's difference of means is 1/4 of the difference of the remaining
     // pairs, which is formed here without the rounding of the cancelled terms
-    if (!((lo_n || hi_n) && (lo_t || hi_t))) return (T)0.25 * ((c0p + cmp) - (cmm + c0m));
+    if (!((lo_n || hi_n) && (lo_t || hi_t))) return scale_down<2>((c0p + cmp) - (cmm + c0m));
     const T third = (T)(1.0 / 3.0);
     T plus, minus;
     if (lo_n && hi_t) plus = (c00 + c0p + cm0) * third;                // no (-1,+1)
@@ -129,7 +129,8 @@ __device__ __forceinline__ void face_body(const Phys &P, const PhysW<T> &PC, con
             C5<T> fp = sw_half(gamma, QL, qe, (T)1), fm = sw_half(gamma, QR, qe, (T)-1);
             Fc.d = fp.d + fm.d; Fc.mx = fp.mx + fm.mx; Fc.my = fp.my + fm.my; Fc.mz = fp.mz + fm.mz; Fc.e = fp.e + fm.e;
         }
-        const T sa = g.s[g.q];
+        T sa = g.s[g.q];
+        if (scheme == 300) sa = scale_down<1>(sa);
         f0 = Fc.d * sa;
         f1 = (Fc.mx * nx + Fc.my * ax + Fc.mz * bx) * sa;
         f2 = (Fc.mx * ny + Fc.my * ay + Fc.mz * by) * sa;
@@ -172,13 +173,12 @@ __device__ __forceinline__ void face_body(const Phys &P, const PhysW<T> &PC, con
         gz[q] = dk[q] * m2 + de[q] * m5 + dz[q] * m8;
     }
     const int m = p - sn;
-    const T h = (T)0.5;
-    const T uf = h * (C.pv[PU][p] + C.pv[PU][m]), vf = h * (C.pv[PV][p] + C.pv[PV][m]);
-    const T wf = h * (C.pv[PW][p] + C.pv[PW][m]), tf = h * (C.pv[PT][p] + C.pv[PT][m]);
+    const T uf = scale_down<1>(C.pv[PU][p] + C.pv[PU][m]), vf = scale_down<1>(C.pv[PV][p] + C.pv[PV][m]);
+    const T wf = scale_down<1>(C.pv[PW][p] + C.pv[PW][m]), tf = scale_down<1>(C.pv[PT][p] + C.pv[PT][m]);
     const T mul = sutherland_face(PC, tf);
     T mu = mul, cond = mul * PC.cond_lam;
     if (P.turb_bl || P.turb_sa) {
-        const T mt = (C.mut[m] + C.mut[p]) / (T)2;
+        const T mt = scale_down<1>(C.mut[m] + C.mut[p]);
         mu = mul + mt;
         cond = cond + mt * PC.cond_tur;
     }

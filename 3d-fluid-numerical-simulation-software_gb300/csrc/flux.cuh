@@ -47,15 +47,40 @@ __device__ __forceinline__ void recon1(int type, T eta, T FF, T F, T B, T BB, T 
         f = max2t((T)0, min3t((T)2, f1, (T)2 * r1));
         R = B - ((T)0.5 * f) * (B - F);
     } else if (type == 500) {               // MUSCL3 with the smooth (van Albada-type) limiter
-        T a = F - FF, b = B - F, c = BB - B;
-        T SL = fdiv<T>((T)2 * a * b + eps, a * a + b * b + eps);
-        T SR = fdiv<T>((T)2 * c * b + eps, c * c + b * b + eps);
+        const T a = F - FF, b = B - F, c = BB - B;
+        // a quarter of the limiter S = (2 a b + eps) / (a^2 + b^2 + eps): powers of two move through products and
+        // FMAs without a rounding, so the bits are those of S * 0.25 with fewer multiplications
+        const T b2 = scale_down<1>(b), eps4 = (T)0.25 * eps;
+        // (FP64: which product of a sum is the exact one of the FMA is written out, so that rewording what is
+        // around cannot change the bits; the compiler's choice is kept in FP32)
+        T SL, SR;
+        if constexpr (sizeof(T) == 8) {
+            SL = fdiv<T>(fma(a, b2, eps4), fma(a, a, __dmul_rn(b, b)) + eps);
+            SR = fdiv<T>(fma(c, b2, eps4), fma(b, b, __dmul_rn(c, c)) + eps);
+        } else {
+            SL = fdiv<T>(a * b2 + eps4, a * a + b * b + eps);
+            SR = fdiv<T>(c * b2 + eps4, c * c + b * b + eps);
+        }
         // S/3 as a product with 1/3 (the FP64 divide is the costly instruction here; within rounding)
-        const T third = (T)(1.0 / 3.0);
+        const T third = (T)4 * (T)(1.0 / 3.0);
         const T sl3 = SL * third, sr3 = SR * third;
-        L = F + SL * (T)0.25 * (((T)1 - sl3) * a + (sl3 + (T)1) * b);
-        R = B - SR * (T)0.25 * (((T)1 - sr3) * c + (sr3 + (T)1) * b);
+        if constexpr (sizeof(T) == 8) {
+            L = fma(SL, fma(1.0 - sl3, a, __dmul_rn(sl3 + 1.0, b)), F);
+            R = fma(-SR, fma(1.0 - sr3, c, __dmul_rn(sr3 + 1.0, b)), B);
+        } else {
+            L = F + SL * (((T)1 - sl3) * a + (sl3 + (T)1) * b);
+            R = B - SR * (((T)1 - sr3) * c + (sr3 + (T)1) * b);
+        }
     }
+}
+
+template <typename T>
+__device__ __forceinline__ void cons_state(T rgm1, const P6<T> &v, C5<T> &c)
+{
+    c.d = v.d; c.mx = v.d * v.u; c.my = v.d * v.v; c.mz = v.d * v.w;
+    if constexpr (sizeof(T) == 8)
+        c.e = fma(v.p, rgm1, __dmul_rn(scale_down<1>(v.d), fma(v.w, v.w, fma(v.u, v.u, __dmul_rn(v.v, v.v)))));
+    else c.e = v.p * rgm1 + v.d * (v.u * v.u + v.v * v.v + v.w * v.w) * (T)0.5;
 }
 
 // primitive reconstruction + positivity fallback + conversion to conserved variables
@@ -70,12 +95,10 @@ __device__ __forceinline__ void recon_prim(int type, T rgm1, const P6<T> &FF, co
     recon1(type, eta, FF.v, F.v, B.v, BB.v, l.v, r.v);
     recon1(type, eta, FF.w, F.w, B.w, BB.w, l.w, r.w);
     recon1(type, eta, FF.p, F.p, B.p, BB.p, l.p, r.p);
-    if (l.d <= lz || l.p <= lz) l = F;
-    if (r.d <= lz || r.p <= lz) r = B;
-    cl.d = l.d; cl.mx = l.d * l.u; cl.my = l.d * l.v; cl.mz = l.d * l.w;
-    cl.e = l.p * rgm1 + l.d * (l.u * l.u + l.v * l.v + l.w * l.w) * (T)0.5;
-    cr.d = r.d; cr.mx = r.d * r.u; cr.my = r.d * r.v; cr.mz = r.d * r.w;
-    cr.e = r.p * rgm1 + r.d * (r.u * r.u + r.v * r.v + r.w * r.w) * (T)0.5;
+    if (at_most(l.d, lz) || at_most(l.p, lz)) l = F;
+    if (at_most(r.d, lz) || at_most(r.p, lz)) r = B;
+    cons_state(rgm1, l, cl);
+    cons_state(rgm1, r, cr);
 }
 
 template <typename T>
@@ -95,13 +118,20 @@ __device__ __forceinline__ void recon_cons(int type, T gamma, const C5<T> &FF, c
     if (cr.d <= lz || pR <= lz) cr = B;
 }
 
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fadd_rn(a, -b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dadd_rn(a, -b); }
 // Harten's entropy fix z > d ? z : 0.5 (z^2 + d^2) / d at the Roe flux's d = 0.5, where it is
 // z^2 + 0.25 bit for bit (the halving and the division by one half are exact)
-template <typename T>
-__device__ __forceinline__ T entropy_corr_half(T z) { return z > (T)0.5 ? z : z * z + (T)0.25; }
+// (z = |x|; in FP64 compared as integers)
+__device__ __forceinline__ float entropy_corr_half(float x) { const float z = fabsf(x); return z > 0.5f ? z : z * z + 0.25f; }
+__device__ __forceinline__ double entropy_corr_half(double x)
+{
+    const double z = fabs(x);
+    return __double_as_longlong(z) > 0x3fe0000000000000ll ? z : z * z + 0.25;
+}
 
-// Roe flux in the face frame with Harten's fix (delta fixed at 0.5) and the reference's wave
-// strengths arr[2], arr[3] divided by (v+1e-8), (w+1e-8)
+// Twice the Roe flux in the face frame (the caller halves |S| instead of five components), with
+// Harten's fix (delta fixed at 0.5) and the reference's wave strengths arr[2], arr[3] divided by (v+1e-8), (w+1e-8)
 template <typename T>
 __device__ __forceinline__ C5<T> roe(T gamma, const C5<T> &QL, const C5<T> &QR, T qe)
 {
@@ -120,7 +150,7 @@ __device__ __forceinline__ C5<T> roe(T gamma, const C5<T> &QL, const C5<T> &QR, 
     T q2 = ua * ua + va * va + wa * wa;
     T ca = fsqrt<T>(g1 * (Ha - (T)0.5 * q2));
     T una = ua - qe;
-    T l1 = entropy_corr_half(tabs(una - ca)), l2 = entropy_corr_half(tabs(una)), l5 = entropy_corr_half(tabs(una + ca));
+    T l1 = entropy_corr_half(una - ca), l2 = entropy_corr_half(una), l5 = entropy_corr_half(una + ca);
     T dd = dR - dL, dmx = QR.mx - QL.mx, dmy = QR.my - QL.my, dmz = QR.mz - QL.mz, de = QR.e - QL.e;
     T a2, a3;
     if constexpr (sizeof(T) == 8) {
@@ -143,14 +173,12 @@ __device__ __forceinline__ C5<T> roe(T gamma, const C5<T> &QL, const C5<T> &QR, 
     T a1 = ((ua + ca) * dd - dmx - ca * a4) * ((T)0.5 * rca);
     T a5 = dd - (a1 + a4);
     C5<T> F;
-    F.d = (T)0.5 * (QL.d * unL + QR.d * unR) - (T)0.5 * (l1 * a1 + l2 * a4 + l5 * a5);
-    F.mx = (T)0.5 * ((QL.mx * unL + pL) + (QR.mx * unR + pR)) -
-           (T)0.5 * (l1 * a1 * (ua - ca) + l2 * a4 * ua + l5 * a5 * (ua + ca));
-    F.my = (T)0.5 * (QL.my * unL + QR.my * unR) - (T)0.5 * (l1 * a1 * va + l2 * a2 * va + l2 * a4 * va + l5 * a5 * va);
-    F.mz = (T)0.5 * (QL.mz * unL + QR.mz * unR) - (T)0.5 * (l1 * a1 * wa + l2 * a3 * wa + l2 * a4 * wa + l5 * a5 * wa);
-    F.e = (T)0.5 * (((QL.e + pL) * unL + qe * pL) + ((QR.e + pR) * unR + qe * pR)) -
-          (T)0.5 * (l1 * a1 * (Ha - ua * ca) + l2 * a2 * va * va + l2 * a3 * wa * wa + l2 * a4 * (T)0.5 * q2 +
-                    l5 * a5 * (Ha + ua * ca));
+    F.d = sub_rn(QL.d * unL + QR.d * unR, l1 * a1 + l2 * a4 + l5 * a5);
+    F.mx = sub_rn((QL.mx * unL + pL) + (QR.mx * unR + pR), l1 * a1 * (ua - ca) + l2 * a4 * ua + l5 * a5 * (ua + ca));
+    F.my = sub_rn(QL.my * unL + QR.my * unR, l1 * a1 * va + l2 * a2 * va + l2 * a4 * va + l5 * a5 * va);
+    F.mz = sub_rn(QL.mz * unL + QR.mz * unR, l1 * a1 * wa + l2 * a3 * wa + l2 * a4 * wa + l5 * a5 * wa);
+    F.e = sub_rn(((QL.e + pL) * unL + qe * pL) + ((QR.e + pR) * unR + qe * pR),
+                 l1 * a1 * (Ha - ua * ca) + l2 * a2 * va * va + l2 * a3 * wa * wa + l2 * a4 * (T)0.5 * q2 + l5 * a5 * (Ha + ua * ca));
     return F;
 }
 

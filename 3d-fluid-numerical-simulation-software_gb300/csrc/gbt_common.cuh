@@ -223,6 +223,22 @@ __device__ __forceinline__ double sqrt_nr(double x)
     s = fma(fma(-s, s, x), h, s);
     return fma(fma(-s, s, x), h, s);
 }
+// x * 2^-K (K 1 or 2). In FP64 by integer operations on the exponent, eight against an instruction that holds the
+// pipe for 76 cycles; what would leave the normal range is multiplied.
+template <int K> __device__ __forceinline__ float scale_down(float x) { return x * (K == 1 ? 0.5f : 0.25f); }
+template <int K> __device__ __forceinline__ double scale_down(double x)
+{
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    if (((unsigned)hi & 0x7ff00000u) - ((K + 1u) << 20) < 0x7ff00000u - ((K + 1u) << 20)) return __hiloint2double(hi - (K << 20), lo);
+    if (((unsigned)hi << 1 | (unsigned)lo) == 0u) return x;
+    return x * (K == 1 ? 0.5 : 0.25);
+}
+// x <= c for a positive c, false for NaN; in FP64 on the bits (an FP64 comparison holds the pipe as an addition does)
+__device__ __forceinline__ bool at_most(float x, float c) { return x <= c; }
+__device__ __forceinline__ bool at_most(double x, double c)
+{
+    return __double_as_longlong(x) <= __double_as_longlong(c) && (unsigned)__double2hiint(x) <= 0xfff00000u;
+}
 template <typename T> __device__ __forceinline__ T frcp(T b);
 template <> __device__ __forceinline__ double frcp<double>(double b) { return rcp_nr(b); }
 template <> __device__ __forceinline__ float frcp<float>(float b)

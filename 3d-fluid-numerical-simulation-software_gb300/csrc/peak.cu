@@ -89,7 +89,11 @@ __global__ void k_arith(int op, const double *__restrict__ x, const double *__re
     // FP64 conversions by integer operations against the conversion instructions
     case 5: { const gbt::dfloat d = gbt::df_from(a); v = (double)d.hi + (double)d.lo; } break;
     case 6: v = gbt::f32_to_f64(gbt::f64_to_f32_rn(a)); break;
-    default: v = (double)__double2float_rn(a); break;
+    case 7: v = (double)__double2float_rn(a); break;
+    // halves, quarters and comparisons by integer operations
+    case 8: v = gbt::scale_down<1>(a); break;
+    case 9: v = gbt::scale_down<2>(a); break;
+    default: v = gbt::at_most(a, b) ? 1.0 : 0.0; break;
     }
     out[t] = v;
 }
@@ -98,8 +102,8 @@ __global__ void k_arith(int op, const double *__restrict__ x, const double *__re
 
 extern "C" int gb_fp64_arith_check(int op, const double *x, const double *y, long long n, double *out)
 {
-    const bool binary = op == 0 || op == 3;
-    if (op < 0 || op > 7 || !x || !out || n < 1 || (binary && !y)) return GB_ERR_ARG;
+    const bool binary = op == 0 || op == 3 || op == 10;
+    if (op < 0 || op > 10 || !x || !out || n < 1 || (binary && !y)) return GB_ERR_ARG;
     double *d = nullptr;
     const size_t bytes = sizeof(double) * (size_t)n;
     if (cudaMalloc(&d, 3 * bytes) != cudaSuccess) return GB_ERR_CUDA;

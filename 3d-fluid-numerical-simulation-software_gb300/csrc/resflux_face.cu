@@ -57,7 +57,8 @@ __device__ __forceinline__ void face_one(const Batch &B, const Phys &P, const Ph
 // The three families in one launch: the blocks of one fill the SMs that the last wave of the one before
 // leaves idle, and a solve's cells (blockIdx.z) are still in L2 for its next family (blockIdx.y; all solves' I
 // faces first cost 12 solves on three meshes 3%, the families in turn block by block 5%). In FP64 bound by
-// its pipe (520 instructions a face). In FP32 by the latency of its loads: nine blocks of 128
+// its pipe (470 instructions a face; 520 with halves, quarters and comparisons on it, 1.74 ms on
+// 49 x 49 x 129 against 1.64 now). In FP32 by the latency of its loads: nine blocks of 128
 // threads per SM in 56 registers, against eight in 64, 7%.
 // Per cycle as three launches and as one: FP64 9 x 9 x 33 0.085/0.033, 33 x 33 x 65 0.252/0.216,
 // 49 x 49 x 129 1.82/1.74 ms; mixed 49 x 49 x 129 0.117/0.095, 12 solves on three meshes 1.285/1.215 ms.

@@ -157,8 +157,8 @@ int gb_fp64_rate(double *flop_per_s);
  * they can be checked against the IEEE operations: op 0 x / y, 1 sqrt(x), 2 1 / x; op 3 and 4 are
  * the device's IEEE x / y and sqrt(x). Also the mixed form's integer operations: op 5 splits x into
  * a pair of FP32 numbers (returned as their FP64 sum), op 6 rounds x to FP32 and widens it back by
- * integer operations, op 7 does the same by the conversion instructions. x, y (y only for ops 0
- * and 3) and out are host arrays. No counterpart in the reference. */
+ * integer operations, op 7 does the same by the conversion instructions; and the FP64 form's: op 8
+ * x / 2, op 9 x / 4, op 10 x <= y (1 or 0) for a positive y. x, y (y only for ops 0, 3 and 10) and out are host arrays. No counterpart in the reference. */
 int gb_fp64_arith_check(int op, const double *x, const double *y, long long n, double *out);
 
 /* Residual norm of gb_res_calculate (same arguments, same values in out and in the solve states)
