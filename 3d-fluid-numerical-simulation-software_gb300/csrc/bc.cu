@@ -246,20 +246,21 @@ void launch_periodic_trig(const LaunchCtx &ctx, double *trig)
 // turned into a mixed-out state by the quadratic for the pressure (the pitch sums are formed as a
 // warp reduction, not in the reference's sequential order)
 template <typename T>
-__global__ void __launch_bounds__(32) k_mix_average(Batch B, Phys P, Geo G, Flow<T> W, const DevMix *mix, int max_rows, double *avg)
+__device__ __forceinline__ void bc_mix_average(const Batch &B, const Phys &P, const Geo &G, const Flow<T> &W, const BcTables &bc, int unit)
 {
-    const DevMix m = mix[blockIdx.y];
-    const int r = blockIdx.x, side = blockIdx.z;
-    if (r > m.ie - m.is) return;
+    // unit: row, mixing plane, side
+    const int r = unit % bc.max_mix_rows, mi = unit / bc.max_mix_rows % bc.n_mix, side = unit / bc.max_mix_rows / bc.n_mix, lane = threadIdx.x & 31;
+    const DevMix m = bc.mix[mi];
+    if (side > 1 || r > m.ie - m.is) return;
     const int i = m.is + r;
     const double g = P.gamma, R = P.rgas;
-    double *o = avg + ((long long)blockIdx.y * max_rows + r) * kMixVals;
+    double *o = bc.mix_avg + ((long long)mi * bc.max_mix_rows + r) * kMixVals;
     const int s = side ? m.s2 : m.s1;
     const Lvl L = B.lv[s];
     const int kf = side ? 1 : L.KM, kc = side ? 1 : L.KM - 1;
     const int j0 = side ? m.js2 : m.js1, j1 = side ? m.je2 : m.je1;
     double acc[10] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // I1..I6, n*s (3), s
-    for (int j = j0 + (int)threadIdx.x; j <= j1; j += 32) {
+    for (int j = j0 + lane; j <= j1; j += 32) {
         const long long f = ix(L, i, j, kf), c = ix(L, i, j, kc);
         const double sa = G.s[2][f];
         const double nx = G.S[2][0][f] / sa, ny = G.S[2][1][f] / sa, nz = G.S[2][2][f] / sa;
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(32) k_mix_average(Batch B, Phys P, Geo G, Flow
 #pragma unroll
     for (int q = 0; q < 10; q++)
         for (int off = 16; off > 0; off >>= 1) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], off);
-    if (threadIdx.x != 0) return;
+    if (lane != 0) return;
     const double ss = acc[9];
     const double I1 = acc[0] / ss, I2 = acc[1] / ss, I3 = acc[2] / ss, I4 = acc[3] / ss, I5 = acc[4] / ss;
     if (side == 0) o[12] = W.ev ? (acc[5] / ss) / I1 : 0.0;
@@ -296,16 +297,17 @@ __global__ void __launch_bounds__(32) k_mix_average(Batch B, Phys P, Geo G, Flow
 // ghost and reconstruction layers of both sides from the other side's mixed-out state and the
 // outgoing characteristics (:431-518); the SA variable of both ghosts is the upstream average
 template <typename T>
-__global__ void k_mix_fill(Batch B, Phys P, Flow<T> W, const DevMix *mix, int max_rows, int max_j, const double *avg)
+__device__ __forceinline__ void bc_mix_fill(const Batch &B, const Phys &P, Flow<T> &W, const BcTables &bc, long long unit)
 {
-    const DevMix m = mix[blockIdx.y];
-    const int side = blockIdx.z;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    // unit: cell of the side, mixing plane, side
+    const int most = bc.max_mix_rows * bc.max_mix_j, t = (int)(unit % most), mi = (int)(unit / most % bc.n_mix), side = (int)(unit / most / bc.n_mix);
+    if (side > 1) return;
+    const DevMix m = bc.mix[mi];
     const int j0 = side ? m.js2 : m.js1, nj = (side ? m.je2 : m.je1) - j0 + 1;
     const int nr = m.ie - m.is + 1;
     if (t >= nr * nj) return;
     const int r = t / nj, i = m.is + r, j = j0 + t % nj;
-    const double *o = avg + ((long long)blockIdx.y * max_rows + r) * kMixVals;
+    const double *o = bc.mix_avg + ((long long)mi * bc.max_mix_rows + r) * kMixVals;
     const double *pu = o, *pd = o + 6;                         // d u v w p c of the upstream / downstream average
     const double g = P.gamma, R = P.rgas;
     const Lvl L = B.lv[side ? m.s2 : m.s1];
@@ -344,12 +346,14 @@ __global__ void k_mix_fill(Batch B, Phys P, Flow<T> W, const DevMix *mix, int ma
     for (int nd = 1; nd <= P.ndummy; nd++) st_state(W, gp + step * nd, c, q);
 }
 
-// The fills in two launches, each block with one part of the work: first the outlets' swirl, the walls and the
-// periodic and interface copies, then the inlets and the outlets' lines. None of them reads what another
-// one writes (they read interior cells, and an outlet's line its own ghost's density), so they can run
-// side by side as long as no cell belongs to two of them (BcTables::apart; the parts come one after
-// another, as in the reference, where one does). Bound by the latency of the FP64 chains of the inlet's
-// state: as six launches in a row 69 us per evaluation of the 129x49x49 passage, as two 35.
+// The fills in two launches, each block with one part of the work: first the mixing planes' averages, the outlets'
+// swirl, the walls and the periodic and interface copies, then the outlets' lines and the mixing planes'
+// ghosts; the inlets beside both on the second stream. None of them reads what another one of its launch
+// writes (they read interior cells, and an outlet's line its own ghost's density), so they can run side by
+// side as long as no cell belongs to two of them (BcTables::apart; the parts come one after another, as in
+// the reference, where one does). Bound by the latency of the FP64 chains of the inlet's state and of a mixing
+// plane's: per evaluation of the 129x49x49 passage 69 us as six launches in a row, 35 as two, 30 so; of the
+// stage of 33x33x97 blocks 74 with the planes in two launches of their own, and 52.
 constexpr int kBcThreads = 128;
 struct BcParts { unsigned first[3]; };              // blocks of the first parts of a launch, summed up
 template <typename T>
@@ -358,15 +362,18 @@ __global__ void __launch_bounds__(kBcThreads) k_bc_first(Batch B, Phys P, Geo G,
 {
     unsigned b = blockIdx.x;
     if (b < n.first[0]) {
+        bc_mix_average<T>(B, P, G, W, bc, (int)(b * (kBcThreads / 32) + (threadIdx.x >> 5)));
+    } else if (b < n.first[1]) {
+        b -= n.first[0];
         const unsigned o = b / per_outlet;
         bc_swirl<T>(B, G, W, bc.outlet[o], bc.outlet_trig + o * bc.outlet_trig_stride, bc.outlet_cu + (long long)o * (bc.max_outlet_im + 1),
                     1 + (int)((b - o * per_outlet) * (kBcThreads / 32) + (threadIdx.x >> 5)));
-    } else if (b < n.first[1]) {
-        b -= n.first[0];
+    } else if (b < n.first[2]) {
+        b -= n.first[1];
         const unsigned o = b / per_wall;
         bc_wall<T>(B, P, G, W, bc.wall[o], (b - o * per_wall) * kBcThreads + threadIdx.x);
     } else {
-        const long long t = (long long)(b - n.first[1]) * kBcThreads + threadIdx.x;
+        const long long t = (long long)(b - n.first[2]) * kBcThreads + threadIdx.x;
         if (t < bc.n_per) bc_periodic<T>(B, W, bc.per_dst, bc.per_src, bc.per_meta, bc.per_trig, t);
     }
 }
@@ -378,8 +385,10 @@ __global__ void __launch_bounds__(kBcThreads) k_bc_second(Batch B, Phys P, Geo G
     if (b < n.first[0]) {
         const unsigned o = b / per_inlet;
         bc_inlet<T>(B, P, G, W, bc.inlet[o], (int)((b - o * per_inlet) * kBcThreads + threadIdx.x));
+    } else if (b < n.first[1]) {
+        bc_mix_fill<T>(B, P, W, bc, (long long)(b - n.first[0]) * kBcThreads + threadIdx.x);
     } else {
-        b -= n.first[0];
+        b -= n.first[1];
         const unsigned o = b / per_outlet;
         bc_outlet_line<T>(B, P, G, W, bc.outlet[o], bc.outlet_cu + (long long)o * (bc.max_outlet_im + 1),
                           1 + (int)((b - o * per_outlet) * (kBcThreads / 32) + (threadIdx.x >> 5)));
@@ -402,27 +411,39 @@ void launch_boundary(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> 
                    pline = (unsigned)(bc.max_outlet_jm + w - 1) / w, pwall = (unsigned)(bc.max_wall + kBcThreads - 1) / kBcThreads;
     const unsigned nin = pin * bc.n_inlet, nrow = prow * bc.n_outlet, nline = pline * bc.n_outlet, nwall = pwall * bc.n_wall,
                    nper = (unsigned)((bc.n_per + kBcThreads - 1) / kBcThreads);
-    auto first = [&](unsigned a, unsigned b, unsigned c) {
-        if (a + b + c) k_bc_first<T><<<a + b + c, kBcThreads, 0, ctx.stream>>>(B, P, G, W, bc, BcParts{{a, a + b, a + b + c}}, prow, pwall);
+    const unsigned navg = ((unsigned)(bc.max_mix_rows * bc.n_mix * 2) + w - 1) / w,
+                   nmix = (unsigned)(((long long)bc.max_mix_rows * bc.max_mix_j * bc.n_mix * 2 + kBcThreads - 1) / kBcThreads);
+    auto first = [&](unsigned m, unsigned a, unsigned b, unsigned c) {
+        if (m + a + b + c)
+            k_bc_first<T><<<m + a + b + c, kBcThreads, 0, ctx.stream>>>(B, P, G, W, bc, BcParts{{m, m + a, m + a + b}}, prow, pwall);
     };
-    auto second = [&](unsigned a, unsigned b) {
-        if (a + b) k_bc_second<T><<<a + b, kBcThreads, 0, ctx.stream>>>(B, P, G, W, bc, BcParts{{a, a + b, a + b}}, pin, pline);
+    auto second = [&](unsigned a, unsigned m, unsigned b, cudaStream_t on) {
+        if (a + m + b) k_bc_second<T><<<a + m + b, kBcThreads, 0, on>>>(B, P, G, W, bc, BcParts{{a, a + m, a + m + b}}, pin, pline);
     };
+    // (with the Spalart-Allmaras variable the mixing planes come after its own fill)
+    const bool mixed = bc.n_mix && bc.mix_apart && !W.ev;
     if (bc.apart) {
-        first(nrow, nwall, nper);
-        second(nin, nline);
+        const bool beside = ctx.side && nin;
+        if (beside) {
+            cudaEventRecord(ctx.fork, ctx.stream);
+            cudaStreamWaitEvent(ctx.side, ctx.fork, 0);
+            second(nin, 0, 0, ctx.side);
+            cudaEventRecord(ctx.join, ctx.side);
+        }
+        first(mixed ? navg : 0, nrow, nwall, nper);
+        second(beside ? 0 : nin, mixed ? nmix : 0, nline, ctx.stream);
+        if (beside) cudaStreamWaitEvent(ctx.stream, ctx.join, 0);
     } else {
-        second(nin, 0);
-        first(nrow, 0, 0);
-        second(0, nline);
-        first(0, nwall, 0);
-        first(0, 0, nper);
+        second(nin, 0, 0, ctx.stream);
+        first(0, nrow, 0, 0);
+        second(0, 0, nline, ctx.stream);
+        first(0, 0, nwall, 0);
+        first(0, 0, 0, nper);
     }
     if (W.ev) launch_sa_boundary<T>(ctx, P, W, bc);
-    if (bc.n_mix) {
-        k_mix_average<T><<<dim3(bc.max_mix_rows, bc.n_mix, 2), 32, 0, ctx.stream>>>(B, P, G, W, bc.mix, bc.max_mix_rows, bc.mix_avg);
-        k_mix_fill<T><<<dim3((bc.max_mix_rows * bc.max_mix_j + 127) / 128, bc.n_mix, 2), 128, 0, ctx.stream>>>(
-            B, P, W, bc.mix, bc.max_mix_rows, bc.max_mix_j, bc.mix_avg);
+    if (bc.n_mix && !(mixed && bc.apart)) {
+        first(navg, 0, 0, 0);
+        second(0, nmix, 0, ctx.stream);
     }
 }
 

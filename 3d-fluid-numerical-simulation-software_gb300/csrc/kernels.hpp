@@ -17,6 +17,9 @@ struct LaunchCtx {
     void (*hook)(void *user, const char *stage, int begin, int launches, int level) = nullptr;
     void *hook_user = nullptr;
     int level = 0;                            // grid level of these launches (1 = fine)
+    // a second stream for what may run beside the launches of the first, and the events between the two (null: none)
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     const void *face_tma = nullptr;           // tables of the TMA-staged face stage (mixed form), or null
     const void *face_tma_host = nullptr;      // their header, on the host
     void mark(const char *stage, int begin, int launches = 1) const { if (hook) hook(hook_user, stage, begin, launches, level); }
@@ -53,6 +56,7 @@ struct BcTables {
     double2 *outlet_trig = nullptr;               // per outlet patch and face: sine and cosine of its polar angle
     long long outlet_trig_stride = 0;
     bool apart = false;                           // no ghost cell belongs to two of inlet, outlet, wall and periodic fills
+    bool mix_apart = false;                       // nor one of a mixing plane to any of them
     double *integ_part = nullptr;                 // per solve and section: kIntegralBlocks partial sums of 3
     unsigned *integ_count = nullptr;              // per solve: blocks of a launch that are done
     // Baldwin-Lomax wall distances (fine level): record w holds, for point n0 = 1..N-1 of each of
@@ -71,7 +75,9 @@ struct BcTables {
 };
 
 // where the integrals put an iteration's row of the history (12 values per case): row iter - *base
-struct HistorySink { double *out; const int *base; int rows, ncase; };
+// With both (per slot, zero between iterations) the norm and the integrals may finish in either order, and the
+// later one writes the row; without, the integrals, which then come after the norm.
+struct HistorySink { double *out; const int *base; int rows, ncase; unsigned *both; };
 
 // out-of-range cells of every slot (update.cuh): their list, its length, blocks of a launch that are done
 struct LimitLists { int *list, cap, *count; unsigned *done; };
@@ -140,7 +146,7 @@ void launch_wave_geometry(const LaunchCtx &ctx, const Geo &G, const WaveTables &
 
 template <typename T>
 void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> F, const double *totalvol, double *partials,
-                     int nblk, unsigned *count);
+                     int nblk, unsigned *count, const HistorySink &hist);
 
 // residual norm with scratch in a static device array; copies the norms to host_out if given
 template <typename T>

@@ -61,9 +61,31 @@ __host__ __device__ inline int norm_blocks(const Lvl &L, int most)
     return n < most ? n : most;
 }
 
+// the iteration's row of the history, by the case's first slot
+__device__ __forceinline__ void history_row(const SolveState *state, const SolveConst &sc, const HistorySink &hist)
+{
+    const volatile SolveState &st = state[sc.lead];
+    const int row = st.iter - *hist.base;
+    if (row < 0 || row >= hist.rows) return;
+    double *r = hist.out + ((long long)row * hist.ncase + sc.cix) * 12;
+    r[0] = st.iter;
+    for (int c = 0; c < 5; c++) r[1 + c] = st.res[c];
+    r[6] = st.m_in; r[7] = st.m_out; r[8] = st.pr; r[9] = st.eff; r[10] = st.m_ratio;
+    r[11] = st.cfl;
+}
+// one of the six values' groups a row waits for (five components of the norm, the integrals) is in the state
+__device__ __forceinline__ void history_arrive(const SolveState *state, const SolveConst &sc, const HistorySink &hist)
+{
+    __threadfence();
+    if (atomicAdd(hist.both + sc.lead, 1u) != 5u) return;
+    hist.both[sc.lead] = 0;
+    __threadfence();
+    history_row(state, sc, hist);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kNormThreads) k_norm(Batch B, Geo G, Flow<T> W, double *partials, int nblk, const double *totalvol,
-                                                       unsigned *count)
+                                                       unsigned *count, HistorySink hist)
 {
     const int s = blockIdx.y;
     const Lvl L = B.lv[s];
@@ -113,17 +135,19 @@ __global__ void __launch_bounds__(kNormThreads) k_norm(Batch B, Geo G, Flow<T> W
     for (int q = sc.lead; q < sc.lead + sc.nblk; q++) {
         const double w = v / totalvol[q];
         B.st[q].res[m] = w;
-        if (m == 0 && !isfinite(w)) B.st[q].status |= GBT_STATUS_NAN;
+        if (m == 0 && !isfinite(w)) atomicOr(&B.st[q].status, GBT_STATUS_NAN);
     }
+    if (hist.both) history_arrive(B.st, sc, hist);
 }
 
 template <typename T>
-void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> W, const double *totalvol, double *partials, int nblk, unsigned *count)
+void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> W, const double *totalvol, double *partials, int nblk, unsigned *count,
+                     const HistorySink &hist)
 {
     const Batch &B = ctx.batch;
     ctx.mark("res_norm", 1, 1);
     const Lvl most = {ctx.maxIM, ctx.maxJM, ctx.maxKM, 0, 0, 0};
-    k_norm<T><<<dim3(norm_blocks(most, nblk), B.nsolve), kNormThreads, 0, ctx.stream>>>(B, G, W, partials, nblk, totalvol, count);
+    k_norm<T><<<dim3(norm_blocks(most, nblk), B.nsolve), kNormThreads, 0, ctx.stream>>>(B, G, W, partials, nblk, totalvol, count, hist);
     ctx.mark("res_norm", 0, 1);
 }
 
@@ -197,16 +221,11 @@ __global__ void __launch_bounds__(128) k_integrals(Batch B, Phys P, Geo G, Flow<
     SolveState &st = B.st[s];
     st.m_in = mi; st.m_out = mo; st.pr = PR; st.eff = Ladk / Lk;
     st.m_ratio = fabs((mi - mo) / mi);
-    if (!isfinite(mi) || !isfinite(mo)) st.status |= GBT_STATUS_NAN;
-    // the iteration's row of the history, by the case's first slot
+    if (!isfinite(mi) || !isfinite(mo)) atomicOr(&st.status, GBT_STATUS_NAN);
     const SolveConst &sc = B.sc[s];
-    const int row = st.iter - *hist.base;
-    if (sc.lead != s || row < 0 || row >= hist.rows) return;
-    double *r = hist.out + ((long long)row * hist.ncase + sc.cix) * 12;
-    r[0] = st.iter;
-    for (int c = 0; c < 5; c++) r[1 + c] = st.res[c];
-    r[6] = mi; r[7] = mo; r[8] = PR; r[9] = st.eff; r[10] = st.m_ratio;
-    r[11] = st.cfl;
+    if (sc.lead != s) return;
+    if (hist.both) history_arrive(B.st, sc, hist);
+    else history_row(B.st, sc, hist);
 }
 
 template <typename T>
@@ -239,7 +258,7 @@ void launch_cfl_ramp(const LaunchCtx &ctx, int iter)
 #define GBT_INST(T)                                                                                                   \
     template void launch_primitive<T>(const LaunchCtx &, const Phys &, Flow<T>);                                       \
     template void launch_limiter<T>(const LaunchCtx &, const Phys &, Flow<T>, int, const LimitLists &);                 \
-    template void launch_res_norm<T>(const LaunchCtx &, const Geo &, Flow<T>, const double *, double *, int, unsigned *);          \
+    template void launch_res_norm<T>(const LaunchCtx &, const Geo &, Flow<T>, const double *, double *, int, unsigned *, const HistorySink &);          \
     template void launch_integrals<T>(const LaunchCtx &, const Phys &, const Geo &, Flow<T>, const BcTables &, const HistorySink &);
 GBT_INST(double)
 GBT_INST(float)

@@ -193,7 +193,7 @@ template <typename T>
 void launch_resflux(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC, const Geo &G, const GeoW<T> &GW, Flow<T> W,
                     const BcTables &bc, int level, T *scratch)
 {
-    const int nbc = bc.apart ? 2 : 5;
+    const int nbc = (bc.apart ? (ctx.side && bc.n_inlet ? 3 : 2) : 5) + (bc.n_mix && (W.ev || !bc.mix_apart) ? 2 : 0);
     ctx.mark("boundary", 1, nbc);
     launch_boundary<T>(ctx, P, G, W, bc);
     ctx.mark("boundary", 0, nbc);

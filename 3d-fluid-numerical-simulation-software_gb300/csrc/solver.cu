@@ -343,6 +343,10 @@ public:
     T *dtmin = nullptr;
     DevBuf hist_mem;                      // rows of the history since *hist.base, brought back when they are full
     HistorySink hist{};
+    unsigned *both = nullptr;             // of the history's rows (HistorySink::both)
+    // second streams: [0] of the boundary fill, [1] of the residual norm
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t forks[2] = {nullptr, nullptr}, joins[2] = {nullptr, nullptr};
     cudaGraphExec_t graphs[3] = {nullptr, nullptr, nullptr};
     int phase_runs[3] = {0, 0, 0};        // iterations run in each driver phase (graphs: see iterate)
 
@@ -428,8 +432,23 @@ public:
         LaunchCtx c = lev[l].ctx(batch(l), stream);
         if (profiling) { c.hook = &SolverT::hook_fn; c.hook_user = (void *)this; }
         c.level = l;
+        c.side = side[0]; c.fork = forks[0]; c.join = joins[0];
         return c;
     }
+    // launches that f makes on its context beside what follows on the solver's stream until meet(); in line while
+    // the stages are profiled
+    template <typename F> void beside(int l, F f)
+    {
+        LaunchCtx c = ctx(l);
+        if (!profiling) {
+            CK(cudaEventRecord(forks[1], stream));
+            CK(cudaStreamWaitEvent(side[1], forks[1], 0));
+            c.stream = side[1];
+        }
+        f(c);
+        if (!profiling) CK(cudaEventRecord(joins[1], side[1]));
+    }
+    void meet() { if (!profiling) CK(cudaStreamWaitEvent(stream, joins[1], 0)); }
 
     PhaseTimer timer;
     explicit SolverT(const std::vector<std::string> &dirs, int prec, int max_levels)
@@ -510,6 +529,11 @@ public:
         PC = phys_working<T>(P);
 
         CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        for (int q = 0; q < 2; q++) {
+            CK(cudaStreamCreateWithFlags(&side[q], cudaStreamNonBlocking));
+            CK(cudaEventCreateWithFlags(&forks[q], cudaEventDisableTiming));
+            CK(cudaEventCreateWithFlags(&joins[q], cudaEventDisableTiming));
+        }
         // per-solve state
         st_mem.bytes = sizeof(SolveState) * nsolve;
         CK(cudaMalloc(&st_mem.p, st_mem.bytes));
@@ -524,7 +548,7 @@ public:
         CK(cudaMemcpy(st_d, st.data(), st_mem.bytes, cudaMemcpyHostToDevice));
         // scratch: limiter lists, norm partials, global-dt minima
         size_t sb = sizeof(int) * (size_t)nsolve * (limits.cap + 2) + sizeof(double) * (size_t)nsolve * (norm_blk + 1) * 5 +
-                    sizeof(unsigned) * nsolve + sizeof(T) * nsolve + 256;
+                    2 * sizeof(unsigned) * nsolve + sizeof(T) * nsolve + 256;
         scratch_mem.bytes = sb;
         CK(cudaMalloc(&scratch_mem.p, sb));
         char *q = (char *)scratch_mem.p;
@@ -535,7 +559,8 @@ public:
         limits.done = (unsigned *)q; q += sizeof(unsigned) * nsolve;
         CK(cudaMemset(limits.count, 0, 2 * sizeof(int) * nsolve));
         norm_count = (unsigned *)q; q += sizeof(unsigned) * nsolve;
-        CK(cudaMemset(norm_count, 0, sizeof(unsigned) * nsolve));
+        both = (unsigned *)q; q += sizeof(unsigned) * nsolve;
+        CK(cudaMemset(norm_count, 0, 2 * sizeof(unsigned) * nsolve));
         dtmin = (T *)(((uintptr_t)q + 15) & ~(uintptr_t)15);
         // 256 rows of history, fewer for very large batches (about 4 MB)
         hist.ncase = ncase;
@@ -556,6 +581,11 @@ public:
         for (auto &e : pin_done) if (e) cudaEventDestroy(e);
         if (pin) cudaFreeHost(pin);
         if (stream) { cudaStreamSynchronize(stream); cudaStreamDestroy(stream); }
+        for (int q = 0; q < 2; q++) {
+            if (side[q]) { cudaStreamSynchronize(side[q]); cudaStreamDestroy(side[q]); }
+            if (forks[q]) cudaEventDestroy(forks[q]);
+            if (joins[q]) cudaEventDestroy(joins[q]);
+        }
     }
 
     void build_level(int l)
@@ -1014,6 +1044,21 @@ public:
                 }
             }
         }
+        // mixing planes of every case (applied last, source/BoundaryCondition.cpp:59-62)
+        std::vector<DevMix> mixes;
+        for (int cix = 0; cix < ncase; cix++) {
+            const int s0 = case_first[cix];
+            for (auto mp : cases[s0].mixing) {
+                const PeriodicIO q = level_pair(mp, l);
+                DevMix m{s0 + q.b1 - 1, s0 + q.b2 - 1, q.r1[0], q.r1[1], q.r1[2], q.r1[3], q.r2[2], q.r2[3]};
+                const Lvl &v1 = Lv.lv[m.s1], &v2 = Lv.lv[m.s2];
+                if (m.is < 1 || m.ie > v1.IM - 1 || m.ie > v2.IM - 1 || m.js1 < 1 || m.je1 > v1.JM - 1 || m.js2 < 1 || m.je2 > v2.JM - 1)
+                    throw std::runtime_error("mixing plane range outside its blocks (rows of the first block are used on both sides)");
+                mixes.push_back(m);
+                bc.max_mix_rows = std::max(bc.max_mix_rows, m.ie - m.is + 1);
+                bc.max_mix_j = std::max(bc.max_mix_j, std::max(m.je1 - m.js1 + 1, m.je2 - m.js2 + 1));
+            }
+        }
         // whether the ghost cells of inlets, outlets, walls and the gather list are all different ones (then
         // the fills need no order among each other)
         {
@@ -1057,21 +1102,20 @@ public:
             for (long long d : pdst) claim(d, 251);
             // (nor may the gather list read a cell that one of the fills writes)
             for (long long p : psrc) if (owner[p]) bc.apart = false;
-        }
-        // mixing planes of every case (applied last, source/BoundaryCondition.cpp:59-62)
-        std::vector<DevMix> mixes;
-        for (int cix = 0; cix < ncase; cix++) {
-            const int s0 = case_first[cix];
-            for (auto mp : cases[s0].mixing) {
-                const PeriodicIO q = level_pair(mp, l);
-                DevMix m{s0 + q.b1 - 1, s0 + q.b2 - 1, q.r1[0], q.r1[1], q.r1[2], q.r1[3], q.r2[2], q.r2[3]};
-                const Lvl &v1 = Lv.lv[m.s1], &v2 = Lv.lv[m.s2];
-                if (m.is < 1 || m.ie > v1.IM - 1 || m.ie > v2.IM - 1 || m.js1 < 1 || m.je1 > v1.JM - 1 || m.js2 < 1 || m.je2 > v2.JM - 1)
-                    throw std::runtime_error("mixing plane range outside its blocks (rows of the first block are used on both sides)");
-                mixes.push_back(m);
-                bc.max_mix_rows = std::max(bc.max_mix_rows, m.ie - m.is + 1);
-                bc.max_mix_j = std::max(bc.max_mix_j, std::max(m.je1 - m.js1 + 1, m.je2 - m.js2 + 1));
-            }
+            // the mixing planes' ghosts: written by nothing else and read by no copy of the gather list
+            bc.mix_apart = bc.apart;
+            for (const DevMix &m : mixes)
+                for (int side = 0; side < 2; side++) {
+                    const Lvl &v = Lv.lv[side ? m.s2 : m.s1];
+                    for (int i = m.is; i <= m.ie; i++)
+                        for (int j = side ? m.js2 : m.js1; j <= (side ? m.je2 : m.je1); j++)
+                            for (int nd = 0; nd <= P.ndummy; nd++) {
+                                unsigned char &o = owner[ix(v, i, j, side ? -nd : v.KM + nd)];
+                                if (o) bc.mix_apart = false;
+                                o = 252;
+                            }
+                }
+            for (long long p : psrc) if (owner[p] == 252) bc.mix_apart = false;
         }
         // upload everything into one table buffer
         auto bytes = [](size_t n, size_t sz) { return (n * sz + 255) & ~(size_t)255; };
@@ -1195,7 +1239,13 @@ public:
         { Mark m(this, "mg_forcing"); launch_forcing_keep<T>(ctx(l), lev[l].W); }
         sweep_update(l);
     }
-    void res_calculate(int l) override { launch_res_norm<T>(ctx(l), lev[l].G, lev[l].W, lev[l].totalvol, norm_part, norm_blk, norm_count); }
+    void res_norm(const LaunchCtx &c, int l, bool pair)
+    {
+        HistorySink h = hist;
+        h.both = pair ? both : nullptr;
+        launch_res_norm<T>(c, lev[l].G, lev[l].W, lev[l].totalvol, norm_part, norm_blk, norm_count, h);
+    }
+    void res_calculate(int l) override { res_norm(ctx(l), l, false); }
     void sweep_shape(int, int out[2]) const override { out[0] = 10; out[1] = 1; }
     bool face_staged(int l) const override
     {
@@ -1221,7 +1271,14 @@ public:
         launch_interpolate<T>(ctx(1), ctx(2), lev[1].W, lev[2].W, init);
     }
     void delta_cons() override { need_mg(); Mark m(this, "mg_delta"); launch_delta<T>(ctx(2), lev[2].W); }
-    void integrals(int l) override { Mark m(this, "integrals", 1); launch_integrals<T>(ctx(l), P, lev[l].G, lev[l].W, lev[l].bc, hist); }
+    void integrals(int l) override { integrals(l, false); }
+    void integrals(int l, bool pair)
+    {
+        Mark m(this, "integrals", 1);
+        HistorySink h = hist;
+        h.both = pair ? both : nullptr;
+        launch_integrals<T>(ctx(l), P, lev[l].G, lev[l].W, lev[l].bc, h);
+    }
     void set_use_force(int l, bool on) override { lev[l].use_force = on; }
     void need_mg() const { if (ng < 2) throw std::runtime_error("the case runs on a single grid level"); }
 
@@ -1241,14 +1298,20 @@ public:
     void step_body()
     {
         if (ng == 1) { time_marching(1); res_calculate(1); return; }
+        // (the norm reads the interior, which nothing writes until the restriction and what comes after it)
+        auto fine_norm_and_residual = [&] {
+            beside(1, [&](const LaunchCtx &c) { res_norm(c, 1, false); });
+            resflux(1);
+            meet();
+        };
         if (!reuse && iter < coarse_iter) { time_marching(2); res_calculate(2); }
         else if (!reuse && iter == coarse_iter) {
             time_marching(2); res_calculate(2); corner_treatment(2);
             interpolate_primitive(1, 1);
         } else if (ng == 2) {
             lev[2].use_force = true;
-            time_marching(1); res_calculate(1);
-            resflux(1);
+            time_marching(1);
+            fine_norm_and_residual();
             restrict_primitive(1);
             time_marching(2);
             delta_cons();
@@ -1257,8 +1320,8 @@ public:
         } else {
             // three-level V-cycle (extension): the fine step as in the two-level cycle, then FAS
             // on levels 2 and 3 with the coarse residuals evaluated at the restricted states
-            time_marching(1); res_calculate(1);
-            resflux(1);
+            time_marching(1);
+            fine_norm_and_residual();
             restrict_primitive(1);
             smooth_fas(2);
             resflux(2);
@@ -1284,6 +1347,22 @@ public:
         if (ng == 1) return 0;
         if (reuse) return 2;
         return iter < coarse_iter ? 1 : (iter == coarse_iter ? -1 : 2);
+    }
+
+    // an iteration of the driver: step and integrals; on a single grid the norm runs beside the integrals
+    void iteration()
+    {
+        begin_iteration();
+        if (ng == 1) {
+            time_marching(1);
+            beside(1, [&](const LaunchCtx &c) { res_norm(c, 1, true); });
+            integrals(1, true);
+            meet();
+        } else {
+            step_body();
+            integrals(report_level());
+        }
+        mass_flow_imposed();
     }
 
     void solver_step() override
@@ -1324,21 +1403,13 @@ public:
                 if (!graphs[ph]) {
                     cudaGraph_t g;
                     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-                    begin_iteration();
-                    step_body();
-                    integrals(report_level());
-                    mass_flow_imposed();
+                    iteration();
                     CK(cudaStreamEndCapture(stream, &g));
                     CK(cudaGraphInstantiate(&graphs[ph], g, 0));
                     cudaGraphDestroy(g);
                 }
                 CK(cudaGraphLaunch(graphs[ph], stream));
-            } else {
-                begin_iteration();
-                step_body();
-                integrals(report_level());
-                mass_flow_imposed();
-            }
+            } else iteration();
             if (hist_out && ++kept == hist.rows) bring(q + 1);
         }
         bring(n);
