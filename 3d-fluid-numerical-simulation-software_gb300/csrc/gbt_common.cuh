@@ -131,6 +131,8 @@ template <typename T>
 struct GeoW {
     T *S[3][3], *s[3], *c[3][2], *nrm[3][3], *t1[3][3], *t2[3][3], *qe[3], *m[3][9];   // faces
     T *vol, *cc[2], *sb[3][3], *cm[9];                                                 // cells
+    // FP64 form: |sb|^2, |sb| and 1 / vol (0 where vol is out of div_by's range), which cost its narrow pipe more than memory
+    T *sb2[3], *sbn[3], *rvol;
 };
 
 // Physical constants in the working precision, converted (and the reciprocal Reynolds number
@@ -141,6 +143,7 @@ struct PhysW {
     // formed once in FP64 on the host: 1 / (gamma - 1) and the conductivity factors
     // gamma R / (gamma - 1) / Pr of the laminar and turbulent parts
     T rgm1, cond_lam, cond_tur;
+    T r_pr_lam, r_pr_tur;                            // 1 / pr_lam, 1 / pr_tur
 };
 
 template <typename T>
@@ -161,6 +164,8 @@ inline PhysW<T> phys_working(const Phys &P)
     w.rgm1 = (T)(1.0 / g1);
     w.cond_lam = (T)(cp / (double)w.pr_lam);
     w.cond_tur = (T)(cp / (double)w.pr_tur);
+    w.r_pr_lam = (T)1 / w.pr_lam;
+    w.r_pr_tur = (T)1 / w.pr_tur;
     return w;
 }
 
@@ -239,6 +244,32 @@ __device__ __forceinline__ bool at_most(double x, double c)
 {
     return __double_as_longlong(x) <= __double_as_longlong(c) && (unsigned)__double2hiint(x) <= 0xfff00000u;
 }
+// a > b for b >= 0 or NaN, false where either is NaN; in FP64 on the bits
+__device__ __forceinline__ bool larger(float a, float b) { return a > b; }
+__device__ __forceinline__ bool larger(double a, double b)
+{
+    const long long x = __double_as_longlong(a);
+    return x > __double_as_longlong(b) && x <= 0x7ff0000000000000ll;
+}
+// |x| without a comparison
+__device__ __forceinline__ float mag(float x) { return fabsf(x); }
+__device__ __forceinline__ double mag(double x) { return fabs(x); }
+// Whether b or 1 / b may take the place of a division by b below
+__host__ __device__ inline bool div_range(double b) { return b > 1e-150 && b < 1e150; }
+// a / b as the IEEE division rounds it, from r = 1 / b rounded: P. Markstein's theorem (IBM J. Res. Dev. 34(1),
+// 1990): with r the rounded reciprocal and q within an ulp of a / b, q + r (a - b q) rounds to the quotient; one step
+// of the same kind brings a r within the ulp. Five FP64 instructions instead of a division's, for several
+// quotients by one b. r = 0 marks a b out of div_range.
+__device__ __forceinline__ double div_by(double a, double b, double r)
+{
+    if (((unsigned)__double2hiint(a) & 0x7ff00000u) - (200u << 20) > (1600u << 20) || __double2hiint(r) == 0) {
+        if (__double_as_longlong(a) == 0 && __double2hiint(r) != 0) return a;
+        return a / b;
+    }
+    const double q = a * r, p = fma(fma(-b, q, a), r, q);
+    return fma(fma(-b, p, a), r, p);
+}
+__device__ __forceinline__ float div_by(float a, float b, float) { return a / b; }
 template <typename T> __device__ __forceinline__ T frcp(T b);
 template <> __device__ __forceinline__ double frcp<double>(double b) { return rcp_nr(b); }
 template <> __device__ __forceinline__ float frcp<float>(float b)

@@ -138,6 +138,7 @@ template <typename T>
 void launch_wall_distances(const LaunchCtx &ctx, const Geo &G, const BcTables &bc);
 
 // FP32 copies of the geometry the working-precision kernels read (mixed form; once per level)
+void launch_cell_norms(const LaunchCtx &ctx, const GeoW<double> &G);
 void launch_geometry_working(const LaunchCtx &ctx, const Geo &G, const GeoW<float> &GW);
 
 // the sweeps' geometry in step order (once per level, after the geometry kernels)

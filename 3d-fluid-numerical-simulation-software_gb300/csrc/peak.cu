@@ -93,7 +93,9 @@ __global__ void k_arith(int op, const double *__restrict__ x, const double *__re
     // halves, quarters and comparisons by integer operations
     case 8: v = gbt::scale_down<1>(a); break;
     case 9: v = gbt::scale_down<2>(a); break;
-    default: v = gbt::at_most(a, b) ? 1.0 : 0.0; break;
+    case 10: v = gbt::at_most(a, b) ? 1.0 : 0.0; break;
+    case 11: v = gbt::larger(a, b) ? 1.0 : 0.0; break;
+    default: v = gbt::div_by(a, b, gbt::div_range(b) ? 1.0 / b : 0.0); break;
     }
     out[t] = v;
 }
@@ -102,8 +104,8 @@ __global__ void k_arith(int op, const double *__restrict__ x, const double *__re
 
 extern "C" int gb_fp64_arith_check(int op, const double *x, const double *y, long long n, double *out)
 {
-    const bool binary = op == 0 || op == 3 || op == 10;
-    if (op < 0 || op > 10 || !x || !out || n < 1 || (binary && !y)) return GB_ERR_ARG;
+    const bool binary = op == 0 || op == 3 || op >= 10;
+    if (op < 0 || op > 12 || !x || !out || n < 1 || (binary && !y)) return GB_ERR_ARG;
     double *d = nullptr;
     const size_t bytes = sizeof(double) * (size_t)n;
     if (cudaMalloc(&d, 3 * bytes) != cudaSuccess) return GB_ERR_CUDA;

@@ -8,6 +8,23 @@
 
 namespace gbt {
 
+// the cells' |sb|^2, |sb| and 1 / vol of the FP64 form
+__global__ void __launch_bounds__(256) k_cell_norms(GeoW<double> G, long long n)
+{
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    for (int d = 0; d < 3; d++) {
+        const double x = G.sb[d][0][p], y = G.sb[d][1][p], z = G.sb[d][2][p], q = fma(z, z, fma(x, x, __dmul_rn(y, y)));
+        G.sb2[d][p] = q;
+        G.sbn[d][p] = sqrt(q);
+    }
+    G.rvol[p] = div_range(G.vol[p]) ? 1.0 / G.vol[p] : 0.0;
+}
+void launch_cell_norms(const LaunchCtx &ctx, const GeoW<double> &G)
+{
+    k_cell_norms<<<(unsigned)((ctx.pool_n + 255) / 256), 256, 0, ctx.stream>>>(G, ctx.pool_n);
+}
+
 // lambda_c per direction and |curl V| (needs ghosts of the velocity)
 template <typename T, bool NS>   // NS: Navier-Stokes (the curl is needed), else Euler
 __global__ void __launch_bounds__(256) k_cell_a(Batch B, PhysW<T> PC, GeoW<T> G, Flow<T> W)
@@ -26,7 +43,8 @@ __global__ void __launch_bounds__(256) k_cell_a(Batch B, PhysW<T> PC, GeoW<T> G,
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         T sx = G.sb[d][0][p], sy = G.sb[d][1][p], sz = G.sb[d][2][p];
-        lam[d] = tabs(ur * sx + vr * sy + w * sz) + cs * tsqrt(sx * sx + sy * sy + sz * sz);
+        const T sn = sizeof(T) == 8 ? G.sbn[d][p] : tsqrt(sx * sx + sy * sy + sz * sz);
+        lam[d] = mag(ur * sx + vr * sy + w * sz) + cs * sn;
     }
     if constexpr (!NS) {
 #pragma unroll
@@ -34,16 +52,16 @@ __global__ void __launch_bounds__(256) k_cell_a(Batch B, PhysW<T> PC, GeoW<T> G,
         return;
     }
     const long long sI = (long long)L.NJ * L.NK, sJ = L.NK;
-    const T h = (T)0.5;
-    T uk = h * (W.pv[PU][p + sI] - W.pv[PU][p - sI]), vk = h * (W.pv[PV][p + sI] - W.pv[PV][p - sI]), wk = h * (W.pv[PW][p + sI] - W.pv[PW][p - sI]);
-    T ue = h * (W.pv[PU][p + sJ] - W.pv[PU][p - sJ]), ve = h * (W.pv[PV][p + sJ] - W.pv[PV][p - sJ]), we = h * (W.pv[PW][p + sJ] - W.pv[PW][p - sJ]);
-    T uz = h * (W.pv[PU][p + 1] - W.pv[PU][p - 1]), vz = h * (W.pv[PV][p + 1] - W.pv[PV][p - 1]), wz = h * (W.pv[PW][p + 1] - W.pv[PW][p - 1]);
+    auto diff = [&](int c, long long o) { return scale_down<1>(W.pv[c][p + o] - W.pv[c][p - o]); };
+    T uk = diff(PU, sI), vk = diff(PV, sI), wk = diff(PW, sI);
+    T ue = diff(PU, sJ), ve = diff(PV, sJ), we = diff(PW, sJ);
+    T uz = diff(PU, 1), vz = diff(PV, 1), wz = diff(PW, 1);
     T m0 = G.cm[0][p], m1 = G.cm[1][p], m2 = G.cm[2][p], m3 = G.cm[3][p], m4 = G.cm[4][p],
       m5 = G.cm[5][p], m6 = G.cm[6][p], m7 = G.cm[7][p], m8 = G.cm[8][p];
     T v_x = vk * m0 + ve * m3 + vz * m6, w_x = wk * m0 + we * m3 + wz * m6;
     T u_y = uk * m1 + ue * m4 + uz * m7, w_y = wk * m1 + we * m4 + wz * m7;
     T u_z = uk * m2 + ue * m5 + uz * m8, v_z = vk * m2 + ve * m5 + vz * m8;
-    const T om = tsqrt(h * ((w_y - v_z) * (w_y - v_z) + (u_z - w_x) * (u_z - w_x) + (v_x - u_y) * (v_x - u_y)));
+    const T om = tsqrt(scale_down<1>((w_y - v_z) * (w_y - v_z) + (u_z - w_x) * (u_z - w_x) + (v_x - u_y) * (v_x - u_y)));
 #pragma unroll
     for (int d = 0; d < 3; d++) W.lamc[d][p] = lam[d];
     W.omega[p] = om;
@@ -157,9 +175,9 @@ __global__ void __launch_bounds__(32 * BL_WARPS) k_bl(Batch B, PhysW<T> PC, Flow
     bool any = false;
     if (live) {
         auto p1 = [&](int n0, T ml, T om) {
-            const T tw = tabs(om * ml);
+            const T tw = mag(om * ml);
             if (n0 == 1) { sh_d1[lane] = W.pv[PD][CELL(1)]; sh_m1[lane] = ml; }   // first cell: density, mu_l
-            if (!any || tw > tmax) tmax = tw;
+            if (!any || larger(tw, tmax)) tmax = tw;
             any = true;
         };
 #pragma unroll
@@ -193,19 +211,21 @@ __global__ void __launch_bounds__(32 * BL_WARPS) k_bl(Batch B, PhysW<T> PC, Flow
     __syncthreads();
     const T Ret = sh_ret[lane];
     const T Aplus = (T)26.0, kap = (T)(double)0.4f, Ckleb = (T)(double)0.3f;
+    const T rAplus = (T)(1.0 / 26.0);
     const T aCcp = (T)((double)0.0168f * (double)1.6f);
     // pass 2: largest speed, and F = y |omega| (1 - exp(-y+/A+)) with its first maximiser
-    T Fmax = (T)0, ymax = (T)0, Udif = (T)0;
+    // (the root of the largest squared speed is the largest speed: rounding keeps the order)
+    T Fmax = (T)0, ymax = (T)0, V2max = (T)0;
     int nmax = 0x7fffffff;
     // van Driest damping of this thread's first BL_CACHE points, reused by pass 3
     T c_damp[BL_CACHE];
     if (live) {
         auto p2 = [&](int n0, T dis, T u, T v, T w, T om) -> T {
-            const T V = tsqrt(u * u + v * v + w * w);
-            if (V > Udif) Udif = V;
-            const T damp = (T)1 - exp(-(dis * Ret) / Aplus);
-            const T F = dis * tabs(om) * damp;
-            if (F > Fmax) { Fmax = F; ymax = dis; nmax = n0; }
+            const T V2 = u * u + v * v + w * w;
+            if (larger(V2, V2max)) V2max = V2;
+            const T damp = (T)1 - exp(div_by(-(dis * Ret), Aplus, rAplus));
+            const T F = dis * mag(om) * damp;
+            if (larger(F, Fmax)) { Fmax = F; ymax = dis; nmax = n0; }
             return damp;
         };
 #pragma unroll
@@ -233,7 +253,7 @@ __global__ void __launch_bounds__(32 * BL_WARPS) k_bl(Batch B, PhysW<T> PC, Flow
     sh_a[wp][lane] = Fmax;
     sh_b[wp][lane] = ymax;
     sh_n[wp][lane] = nmax;
-    sh_u[wp][lane] = Udif;
+    sh_u[wp][lane] = tsqrt(V2max);
     __syncthreads();
     if (wp == 0 && live) {
         T F = (T)0, y = (T)0, U = (T)0;
@@ -251,17 +271,18 @@ __global__ void __launch_bounds__(32 * BL_WARPS) k_bl(Batch B, PhysW<T> PC, Flow
     __syncthreads();
     if (!live) return;
     const T ym = sh_ymax[lane], Fwake = sh_fwake[lane];
+    const T rym = sizeof(T) == 8 && div_range(ym) ? (T)1 / ym : (T)0;
     // (Ret * dis) equals (dis * Ret) exactly, so the cached damping is the value pass 3 would form
     // pass 3: inner and outer viscosity, the smaller one merged into mu_t
     auto p3 = [&](int n0, T dis, T damp, T om, T rho) {
         const long long p = CELL(n0);
         const T bL = kap * dis * damp;
         const T m_in = rho * bL * bL * om;
-        const T r = Ckleb * dis / ym;
+        const T r = div_by(Ckleb * dis, ym, rym);
         const T r2 = r * r;
         const T Fk = (T)1 / ((T)1 + (T)5.5 * (r2 * r2 * r2));
         const T m_out = aCcp * rho * Fwake * Fk;
-        const T mt = (tabs(m_in) > tabs(m_out)) ? m_out : m_in;
+        const T mt = larger(mag(m_in), mag(m_out)) ? m_out : m_in;
         if (n0 == 1) {
             atomicMin(&W.blmin[p], 0ull);                      // wall-adjacent cell: mu_t = 0
             W.mut[p0 + (long long)(lo ? 0 : N) * sn] = (T)0;   // its ghost
@@ -291,7 +312,7 @@ __global__ void __launch_bounds__(32 * BL_WARPS) k_bl(Batch B, PhysW<T> PC, Flow
     for (int n0 = 1 + wp + BL_CACHE * BL_WARPS; n0 < N; n0 += BL_WARPS) {
         const long long p = CELL(n0);
         const T dis = DIST(n0);
-        p3(n0, dis, (T)1 - exp(-(Ret * dis) / Aplus), W.omega[p], W.pv[PD][p]);
+        p3(n0, dis, (T)1 - exp(div_by(-(Ret * dis), Aplus, rAplus)), W.omega[p], W.pv[PD][p]);
     }
 #undef CELL
 #undef DIST
@@ -358,13 +379,25 @@ __global__ void __launch_bounds__(256) k_cell_b(Batch B, PhysW<T> PC, GeoW<T> G,
         const T ml = sizeof(T) == 8 ? W.mul[p] : sutherland(PC, W.pv[PT][p]);   // FP64: formed by k_cell_a
         const T mt = W.mut[p];
         const T rho = W.pv[PD][p];
-        const T a = (T)(double)(4.0f / 3.0f) / rho, b = PC.gamma / rho;
-        const T coef = (a > b ? a : b) * (ml / PC.pr_lam + mt / PC.pr_tur);
+        const T c43 = (T)(double)(4.0f / 3.0f);
+        T big;                                      // the larger one of 4/3 / rho and gamma / rho
+        if constexpr (sizeof(T) == 8) {
+            // (one division: rounding keeps the order, which a negative rho turns round)
+            const bool swap = larger(PC.gamma, c43) == (__double2hiint(rho) >= 0);
+            big = (swap ? PC.gamma : c43) / rho;
+        } else {
+            const T a = c43 / rho, b = PC.gamma / rho;
+            big = a > b ? a : b;
+        }
+        const T coef = big * (div_by(ml, PC.pr_lam, PC.r_pr_lam) + div_by(mt, PC.pr_tur, PC.r_pr_tur));
         T l[3];
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            T sx = G.sb[d][0][p], sy = G.sb[d][1][p], sz = G.sb[d][2][p];
-            l[d] = coef * (sx * sx + sy * sy + sz * sz) / vol;
+            if constexpr (sizeof(T) == 8) l[d] = div_by(coef * G.sb2[d][p], vol, G.rvol[p]);
+            else {
+                T sx = G.sb[d][0][p], sy = G.sb[d][1][p], sz = G.sb[d][2][p];
+                l[d] = coef * (sx * sx + sy * sy + sz * sz) / vol;
+            }
         }
 #pragma unroll
         for (int d = 0; d < 3; d++) W.lamv[d][p] = l[d];

@@ -817,6 +817,13 @@ public:
             W.vol = G.vol;
             for (int c = 0; c < 2; c++) W.cc[c] = G.cc[c];
             for (int c = 0; c < 9; c++) W.cm[c] = G.cm[c];
+            const long long N = Lv.pool_n;
+            Lv.geow_mem.bytes = sizeof(double) * (size_t)N * 7;
+            CK(cudaMalloc(&Lv.geow_mem.p, Lv.geow_mem.bytes));
+            double *g = (double *)Lv.geow_mem.p;
+            for (int f = 0; f < 3; f++) { W.sb2[f] = g + f * N; W.sbn[f] = g + (3 + f) * N; }
+            W.rvol = g + 6 * N;
+            launch_cell_norms(ctx(l), W);
         } else {
             const long long N = Lv.pool_n;
             const int NW = 3 * (5 * 3 + 2 + 1 + 1 + 9) + 1 + 2 + 9;

@@ -156,8 +156,8 @@ def fp64_arith_check(op: int, x: np.ndarray, y: Optional[np.ndarray] = None) -> 
     """the device's FP64 arithmetic on host arrays: op 0 x / y, 1 sqrt(x), 2 1 / x as the FP64 form's
     kernels compute them (Newton-refined), 3 and 4 the IEEE x / y and sqrt(x); 5 x split into a
     pair of FP32 numbers and summed back, 6 and 7 x rounded to FP32 and widened back by integer
-    operations / by the conversion instructions; 8 x / 2, 9 x / 4 and 10 x <= y for a positive y by
-    integer operations"""
+    operations / by the conversion instructions; 8 x / 2, 9 x / 4, 10 x <= y for a positive y
+    and 11 x > y for a y that is not negative by integer operations; 12 x / y from the rounded reciprocal"""
     L = load()
     x = np.ascontiguousarray(x, dtype=np.float64)
     yy = None if y is None else np.ascontiguousarray(y, dtype=np.float64)

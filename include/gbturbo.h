@@ -158,7 +158,8 @@ int gb_fp64_rate(double *flop_per_s);
  * the device's IEEE x / y and sqrt(x). Also the mixed form's integer operations: op 5 splits x into
  * a pair of FP32 numbers (returned as their FP64 sum), op 6 rounds x to FP32 and widens it back by
  * integer operations, op 7 does the same by the conversion instructions; and the FP64 form's: op 8
- * x / 2, op 9 x / 4, op 10 x <= y (1 or 0) for a positive y. x, y (y only for ops 0, 3 and 10) and out are host arrays. No counterpart in the reference. */
+ * x / 2, op 9 x / 4, op 10 x <= y (1 or 0) for a positive y, op 11 x > y for a y that is not negative; op 12
+ * x / y from the rounded reciprocal of y. x, y (y only for ops 0, 3 and from 10 on) and out are host arrays. No counterpart in the reference. */
 int gb_fp64_arith_check(int op, const double *x, const double *y, long long n, double *out);
 
 /* Residual norm of gb_res_calculate (same arguments, same values in out and in the solve states)

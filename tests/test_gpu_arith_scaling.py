@@ -1,5 +1,5 @@
-"""Halves, quarters and the comparison with a positive bound, which the FP64 face flux forms by integer
-operations, against numpy: bit for bit over all exponents, with zeros, subnormal numbers, infinities and NaN."""
+"""Halves, quarters and comparisons, which the FP64 form takes by integer operations, and quotients from a rounded
+reciprocal, against numpy: bit for bit over all exponents, with zeros, subnormal numbers, infinities and NaN."""
 import numpy as np
 import pytest
 
@@ -27,3 +27,19 @@ def test_scaled_by_powers_of_two(gpu_lib, op, factor):
 def test_comparison(gpu_lib, bound):
     x = _values()
     assert np.array_equal(gpu_lib.fp64_arith_check(10, x, np.full_like(x, bound)), (x <= bound).astype(np.float64))
+
+
+@pytest.mark.parametrize("bound", [0.0, 1e-300, 1.0, np.inf, np.nan])
+def test_larger(gpu_lib, bound):
+    x = _values()
+    assert np.array_equal(gpu_lib.fp64_arith_check(11, x, np.full_like(x, bound)), (x > bound).astype(np.float64))
+
+
+@pytest.mark.parametrize("divisor", [26.0, 0.72, 0.9, 1.0, np.nextafter(2.0, 0), 3e-7, 1e-200, 0.0, None])
+def test_quotient_from_the_reciprocal(gpu_lib, divisor):
+    # (the sign of a zero quotient is not kept where it is minus zero over a positive number: it equals plus zero)
+    x = np.concatenate([_values(), np.random.default_rng(5).normal(size=1 << 18)])
+    y = np.full_like(x, divisor) if divisor is not None else np.abs(np.random.default_rng(6).normal(size=x.size)) + 1e-3
+    with np.errstate(all="ignore"):
+        want = x / y
+    assert np.array_equal(gpu_lib.fp64_arith_check(12, x, y), want, equal_nan=True)
