@@ -12,11 +12,12 @@
 // What a step costs is the number of instructions one warp issues (a lone warp of a sub-partition issues
 // one every three to four cycles, and an FP64 instruction holds its sub-partition for some 70): with a
 // lane per cell a step took 337 instructions and 1.3k cycles in FP32. So four lanes share a cell (eight in
-// FP64, 26 FP64 instructions a step where four lanes took 38), four warps a step, and everything that is
-// not the cell's arithmetic is done by two further warps of the block:
-//   a cell's lanes     receive a component each (FP32: and the fifth); lanes 0..2 form the terms of a direction
-//                      each (FP64: with lanes 4..6, which take its last two components), and lane 3 the
-//                      pressure, with the instructions with which the others form their V_n
+// FP64, 22 FP64 instructions a step where four lanes took 38; 26 with three terms to a lane, 0.193 and 0.177 ms
+// a sweep of the 65x33x33 duct), four warps a step, and everything that is not the cell's arithmetic is
+// done by two further warps of the block:
+//   a cell's lanes     receive a component each (FP32: and the fifth); lanes 0..2 form V_n of a direction each, and
+//                      lane 3 the pressure with the same instructions; the fifteen terms are formed by
+//                      direction on lanes 0..2 (FP64: two to a lane of eight)
 //   the incoming warp  reads the terms that cross into the tile and puts them beside the tile's own
 //   the outgoing warp  sends the terms that leave it and fetches the inputs of later steps
 //
@@ -245,37 +246,36 @@ template <int DIR> struct CellStep<double, DIR, MEAN> {
                                                int w_off4, bool active, double gm1, char *dq_out)
     {
         const int d = q & 3, c = q < 4 ? q : 4, e = 3 * cell + (d < 3 ? d : 0);     // direction, component received
-        const bool low = q < 4;                      // components 1..3 of the direction's term, or 4 and 5
+        const bool low = q < 4;
+        const int d0 = q / 5, c0 = q % 5, t1 = min(q + 8, 14), d1 = t1 / 5, c1 = t1 % 5;      // the two terms
         const double2 *g = (const double2 *)in + e;
         const char *own = in + L::geo + (DIR > 0 ? 0 : L::flow_in - L::ends), *mid = in + L::geo + (DIR > 0 ? L::ends : 0);
-        const double *f = (const double *)mid + (low ? 0 : 9 * NC) + e, *oc = (const double *)mid + 15 * NC + (low ? 4 * cell + c : 4 * NC + cell),
+        const double *oc = (const double *)mid + 15 * NC + (low ? 4 * cell + c : 4 * NC + cell),
                      *rc = (const double *)(in + L::geo + L::flow_in) + (low ? 4 * cell + c : 4 * NC + cell);
-        const double2 g0 = g[0], g1 = g[3 * NC], hc = ((const double2 *)own)[e];
-        const double fa = f[0], fb = f[3 * NC], fc = low ? f[6 * NC] : 0.0, o = *oc, r = *rc;
+        const double2 g0 = g[0], g1 = g[3 * NC], ha = ((const double2 *)own)[3 * cell + d0], hb = ((const double2 *)own)[3 * cell + d1];
+        auto coef = [&](int dir, int cc) { return ((const double *)in)[(cc > 2 ? 6 * NC : 0) + 2 * (3 * cell + dir) + ((cc - 1) & 1)]; };
+        const double fa = ((const double *)mid)[3 * (NC * c0 + cell) + d0], fb = ((const double *)mid)[3 * (NC * c1 + cell) + d1], o = *oc, r = *rc,
+                     ka = coef(d0, c0), kb = coef(d1, c1);
         // received
         const double s = __dadd_rn(__dadd_rn(*(const double *)(rd + r_off[0]), *(const double *)(rd + r_off[1])), *(const double *)(rd + r_off[2]));
         const double x = __dadd_rn(r, DIR > 0 ? s : -s), dq = active ? x : 0.0, nq = __dadd_rn(o, dq);
         const unsigned oct = (threadIdx.x & 31) & ~7u;
         auto from = [&](double v, int lane) { return __shfl_sync(0xffffffffu, v, oct + lane); };
         const double n0 = from(nq, 0), n1 = from(nq, 1), n2 = from(nq, 2), n3 = from(nq, 3), n4 = from(nq, 4);
-        const double da = from(dq, low ? 0 : 3), db = from(dq, low ? 1 : 4), dc = from(dq, 2);
+        const double va = from(dq, c0), vb = from(dq, c1), na = from(nq, c0), nb = from(nq, c1);
         const double inv = rcp_nr(n0);
         // lanes 0..2 of a half: V_n - ve; lane 3: p = (gamma - 1)(rho E - |m|^2 / (2 rho))
         const double mm = fma(n3, d < 3 ? g1.x : n3, fma(n1, d < 3 ? g0.x : n1, __dmul_rn(n2, d < 3 ? g0.y : n2)));
         const double dn = fma(mm, inv, d < 3 ? -g1.y : -0.0);
         const double pn = from(__dmul_rn(gm1, fma(-0.5, dn, n4)), 3), ep = __dadd_rn(n4, pn);
-        auto term = [&](double n, double y, double v) {
-            const double w = __dmul_rn(hc.y, v);
-            return fma(hc.x, fma(n, dn, y), DIR > 0 ? w : -w);
+        auto term = [&](double n, double dv, double y, double v, const double2 &h) {
+            const double w = __dmul_rn(h.y, v);
+            return fma(h.x, fma(n, dv, y), DIR > 0 ? w : -w);
         };
-        const double y = fma(pn, g1.x, -fa);
-        const double ta = term(low ? n0 : n3, low ? -fa : y, da), tb = term(low ? n1 : ep, fma(pn, low ? g0.x : g1.y, -fb), db),
-                     tc = term(n2, fma(pn, g0.y, -fc), dc);
-        if (d < 3) {
-            double *w = (double *)(wr + w_off);
-            if (low) { *(double2 *)w = make_double2(ta, tb); w[2] = tc; }
-            else { w[3] = ta; *(double *)(wr + w_off4) = tb; }
-        }
+        const double ya = fma(pn, ka, -fa), yb = fma(pn, kb, -fb);
+        const double ta = term(c0 < 4 ? na : ep, from(dn, d0), c0 > 0 ? ya : -fa, va, ha), tb = term(c1 < 4 ? nb : ep, from(dn, d1), c1 > 0 ? yb : -fb, vb, hb);
+        *(double *)(wr + w_off) = ta;
+        if (q < 7) *(double *)(wr + w_off4) = tb;
         if (q < 5) ((double *)dq_out)[low ? 4 * cell + c : 4 * NC + cell] = dq;
     }
 };
@@ -342,9 +342,14 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
             r_off[1] = low ? r_off[2] + 8 * q : r_off[3];
             r_off[2] = low ? L::KA + 8 * (4 * cell + q) : L::KB + 8 * cell;
         }
-        const int dir = sizeof(T) == 8 ? q & 3 : q;
-        const int w_off = dir == 0 ? off_ia<L>(a + F, b) : dir == 1 ? off_ja<L>(a, b + F) : L::KA + L::CA * cell * L::B;
-        const int w_off4 = dir == 0 ? off_ib<L>(a + F, b) : dir == 1 ? off_jb<L>(a, b + F) : L::KB + L::CB * cell * L::B;
+        auto to_a = [&](int dir) { return dir == 0 ? off_ia<L>(a + F, b) : dir == 1 ? off_ja<L>(a, b + F) : L::KA + L::CA * cell * L::B; };
+        auto to_b = [&](int dir) { return dir == 0 ? off_ib<L>(a + F, b) : dir == 1 ? off_jb<L>(a, b + F) : L::KB + L::CB * cell * L::B; };
+        int w_off = to_a(q), w_off4 = to_b(q);
+        if (sizeof(T) == 8 && K == MEAN) {             // terms written: q and q + 8 of the fifteen
+            auto to = [&](int t) { return t % 5 < 4 ? to_a(t / 5) + 8 * (t % 5) : to_b(t / 5); };
+            w_off = to(q);
+            w_off4 = to(min(q + 8, 14));
+        }
         char *dq = V.dq + (w.step0 + (DIR > 0 ? 0 : T_ - 1)) * L::dq;
         int k = (DIR > 0 ? 0 : T_ - 1) - a - b;
         unsigned ph = 0;
