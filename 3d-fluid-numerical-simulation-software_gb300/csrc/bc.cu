@@ -422,8 +422,8 @@ void launch_boundary(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> 
     };
     // (with the Spalart-Allmaras variable the mixing planes come after its own fill)
     const bool mixed = bc.n_mix && bc.mix_apart && !W.ev;
+    const bool beside = bc.apart && ctx.side && nin;
     if (bc.apart) {
-        const bool beside = ctx.side && nin;
         if (beside) {
             cudaEventRecord(ctx.fork, ctx.stream);
             cudaStreamWaitEvent(ctx.side, ctx.fork, 0);
@@ -432,7 +432,6 @@ void launch_boundary(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> 
         }
         first(mixed ? navg : 0, nrow, nwall, nper);
         second(beside ? 0 : nin, mixed ? nmix : 0, nline, ctx.stream);
-        if (beside) cudaStreamWaitEvent(ctx.stream, ctx.join, 0);
     } else {
         second(nin, 0, 0, ctx.stream);
         first(0, nrow, 0, 0);
@@ -441,6 +440,7 @@ void launch_boundary(const LaunchCtx &ctx, const Phys &P, const Geo &G, Flow<T> 
         first(0, 0, 0, nper);
     }
     if (W.ev) launch_sa_boundary<T>(ctx, P, W, bc);
+    if (beside) cudaStreamWaitEvent(ctx.stream, ctx.join, 0);
     if (bc.n_mix && !(mixed && bc.apart)) {
         first(navg, 0, 0, 0);
         second(0, nmix, 0, ctx.stream);

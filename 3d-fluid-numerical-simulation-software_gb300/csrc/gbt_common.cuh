@@ -144,6 +144,7 @@ struct PhysW {
     // gamma R / (gamma - 1) / Pr of the laminar and turbulent parts
     T rgm1, cond_lam, cond_tur;
     T r_pr_lam, r_pr_tur;                            // 1 / pr_lam, 1 / pr_tur
+    T re;                                            // the reference Reynolds number
 };
 
 template <typename T>
@@ -165,6 +166,7 @@ inline PhysW<T> phys_working(const Phys &P)
     w.cond_lam = (T)(cp / (double)w.pr_lam);
     w.cond_tur = (T)(cp / (double)w.pr_tur);
     w.r_pr_lam = (T)1 / w.pr_lam;
+    w.re = (T)P.re_ref;
     w.r_pr_tur = (T)1 / w.pr_tur;
     return w;
 }

@@ -195,7 +195,7 @@ void launch_sa_init(const LaunchCtx &ctx, double *ev, double ev_ratio);
 template <typename T>
 void launch_sa_boundary(const LaunchCtx &ctx, const Phys &P, Flow<T> W, const BcTables &bc);
 template <typename T>
-void launch_sa_model(const LaunchCtx &ctx, const Phys &P, const GeoW<T> &GW, Flow<T> W);
+void launch_sa_model(const LaunchCtx &ctx, const PhysW<T> &P, const GeoW<T> &GW, Flow<T> W);
 template <typename T>
 void launch_sa_update(const LaunchCtx &ctx, const Phys &P, Flow<T> W, int *bad_list, int bad_cap, int *bad_count);
 template <typename T>

@@ -462,7 +462,7 @@ void launch_cell_stages(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC,
         k_bl<T><<<g, 32 * BL_WARPS, 0, ctx.stream>>>(B, PC, W, bc.wall, 0, bc.wall_dist_off, (const T *)bc.wall_dist);
         k_bl_merge<T><<<(unsigned)((ctx.pool_n + 255) / 256), 256, 0, ctx.stream>>>(W, ctx.pool_n);
     }
-    if (level == 1 && P.turb_sa && W.ev) launch_sa_model<T>(ctx, P, GW, W);
+    if (level == 1 && P.turb_sa && W.ev) launch_sa_model<T>(ctx, PC, GW, W);
     ctx.mark("baldwin_lomax", 0, 2);
     ctx.mark("time_step", 1, 1);
     dim3 g = ctx.grid_cells(256);

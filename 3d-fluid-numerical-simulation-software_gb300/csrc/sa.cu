@@ -19,6 +19,7 @@
 // source/SA_Model.cpp:19-29).
 #include "gbt_common.cuh"
 #include "kernels.hpp"
+#include <algorithm>
 
 namespace gbt {
 
@@ -175,17 +176,17 @@ void launch_sa_boundary(const LaunchCtx &ctx, const Phys &P, Flow<T> W, const Bc
 // ---------------------------------------------------------------------------------------------
 // mu_t from the variable, then the clipping of mu_t and of the variable (source/SA_Model.cpp:44-83)
 template <typename T>
-__global__ void __launch_bounds__(256) k_sa_mut(Batch B, Phys P, Flow<T> W)
+__global__ void __launch_bounds__(256) k_sa_mut(Batch B, PhysW<T> P, Flow<T> W)
 {
     const Lvl L = B.lv[blockIdx.y];
     int i, j, k;
     if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
     const long long p = ix(L, i, j, k);
     const SAConst C = sa_const();
-    const T Re = (T)P.re_ref, Cv1 = (T)C.Cv1;
+    const T Re = P.re, Cv1 = (T)C.Cv1;
     const T d = W.pv[PD][p], tt = W.pv[PT][p];
-    T ev = (T)W.ev[p];
-    const T mlam = sutherland<T>(P, tt);
+    T ev = to_work<T>(W.ev[p]);
+    const T mlam = sutherland(P, tt);
     T ev_lam = Re * mlam / d;
     const T X = ev / ev_lam;
     T mt = fv1_of<T>(X, Cv1) * d * ev / Re;
@@ -206,8 +207,8 @@ template <typename T, int F, int DT>
 __device__ __forceinline__ T sa_tan_diff(const double *__restrict__ c, long long p, long long sn, long long st, int a,
                                          int NN, int b, int TT)
 {
-    const T c00 = (T)c[p], cm0 = (T)c[p - sn];
-    const T c0p = (T)c[p + st], cmp = (T)c[p - sn + st], c0m = (T)c[p - st], cmm = (T)c[p - sn - st];
+    const T c00 = to_work<T>(c[p]), cm0 = to_work<T>(c[p - sn]);
+    const T c0p = to_work<T>(c[p + st]), cmp = to_work<T>(c[p - sn + st]), c0m = to_work<T>(c[p - st]), cmm = to_work<T>(c[p - sn - st]);
     T plus, minus;
     const bool lo_n = (a == 1), hi_n = (a == NN), lo_t = (b == 1), hi_t = (b == TT - 1);
     if (lo_n && hi_t) plus = (c00 + c0p + cm0) / (T)3;
@@ -225,9 +226,9 @@ __device__ __forceinline__ T sa_tan_diff(const double *__restrict__ c, long long
 // (zero on wall faces, source/WallFlux.cpp:104-105), viscous flux and the gradient flux of the
 // cross-diffusion term
 template <typename T, int F>
-__global__ void __launch_bounds__(128) k_sa_face(Batch B, Phys P, GeoW<T> G, Flow<T> W)
+__device__ __forceinline__ void sa_face(const Batch &B, const PhysW<T> &P, const GeoW<T> &G, const Flow<T> &W)
 {
-    const int s = blockIdx.y;
+    const int s = blockIdx.z;
     const Lvl L = B.lv[s];
     int ni, nj, nk, i, j, k;
     face_extent(L, F, ni, nj, nk);
@@ -239,13 +240,13 @@ __global__ void __launch_bounds__(128) k_sa_face(Batch B, Phys P, GeoW<T> G, Flo
     const int a = F == 0 ? i : (F == 1 ? j : k);
     const long long m = p - sn;
     const SAConst C = sa_const();
-    const T Re = (T)P.re_ref;
+    const T Re = P.re;
     // face gradient of the variable before the clipping (W.evg)
     const int iD1 = F == 0 ? 1 : 0, iD2 = F == 2 ? 1 : 2;
     const long long st1 = iD1 == 0 ? sI : sJ, st2 = iD2 == 1 ? sJ : sK;
     const int b1 = iD1 == 0 ? i : j, T1 = iD1 == 0 ? L.IM : L.JM;
     const int b2 = iD2 == 1 ? j : k, T2 = iD2 == 1 ? L.JM : L.KM;
-    const T dn = (T)W.evg[p] - (T)W.evg[m];
+    const T dn = to_work<T>(W.evg[p]) - to_work<T>(W.evg[m]);
     const T d1 = sa_tan_diff<T, F, (F == 0 ? 1 : 0)>(W.evg, p, sn, st1, a, NN, b1, T1);
     const T d2 = sa_tan_diff<T, F, (F == 2 ? 1 : 2)>(W.evg, p, sn, st2, a, NN, b2, T2);
     T dk, de, dz;
@@ -261,9 +262,9 @@ __global__ void __launch_bounds__(128) k_sa_face(Batch B, Phys P, GeoW<T> G, Flo
     const T h = (T)0.5;
     const T densf = h * (W.pv[PD][p] + W.pv[PD][m]);
     const T tempf = h * (W.pv[PT][p] + W.pv[PT][m]);
-    const T evp = (T)W.ev[p], evm = (T)W.ev[m];
+    const T evp = to_work<T>(W.ev[p]), evm = to_work<T>(W.ev[m]);
     const T evf = h * (evp + evm);
-    const T ev_lam = Re * sutherland<T>(P, tempf) / densf;
+    const T ev_lam = Re * sutherland(P, tempf) / densf;
     const T cf = (T)((1.0 + C.Cb2) / C.sigma) * (ev_lam + evf);
     const T tx = cf * ux, ty = cf * uy, tz = cf * uz;
     const T Sx = G.S[F][0][p], Sy = G.S[F][1][p], Sz = G.S[F][2][p], sa = G.s[F][p];
@@ -276,11 +277,20 @@ __global__ void __launch_bounds__(128) k_sa_face(Batch B, Phys P, GeoW<T> G, Flo
     W.Fvt[F][p] = (tx * Sx + ty * Sy + tz * Sz) / Re;
     W.Fv1t[F][p] = ux * Sx + uy * Sy + uz * Sz;
 }
+// the three families (blockIdx.y) in one launch. The mixed form was bound by the FP64 pipe, which conversions
+// and a constant's division took 21 times a face: 53 us on 129 x 49 x 49 as three launches, TODOS now.
+template <typename T>
+__global__ void __launch_bounds__(128) k_sa_face(Batch B, PhysW<T> P, GeoW<T> G, Flow<T> W)
+{
+    if (blockIdx.y == 0) sa_face<T, 0>(B, P, G, W);
+    else if (blockIdx.y == 1) sa_face<T, 1>(B, P, G, W);
+    else sa_face<T, 2>(B, P, G, W);
+}
 
 // source term, cell sums and the residual of the variable (source/SA_Model.cpp:182-205,
 // source/ComputeAllBlockVars.cpp:109-113, 245-248)
 template <typename T>
-__global__ void __launch_bounds__(256) k_sa_cell(Batch B, Phys P, GeoW<T> G, Flow<T> W)
+__global__ void __launch_bounds__(256) k_sa_cell(Batch B, PhysW<T> P, GeoW<T> G, Flow<T> W)
 {
     const Lvl L = B.lv[blockIdx.y];
     int i, j, k;
@@ -288,16 +298,16 @@ __global__ void __launch_bounds__(256) k_sa_cell(Batch B, Phys P, GeoW<T> G, Flo
     const long long p = ix(L, i, j, k);
     const long long pI = p + (long long)L.NJ * L.NK, pJ = p + L.NK, pK = p + 1;
     const SAConst C = sa_const();
-    const T Re = (T)P.re_ref, Cv1 = (T)C.Cv1, kv = (T)C.kavf, Cb1 = (T)C.Cb1, Cb2 = (T)C.Cb2, sigma = (T)C.sigma;
+    const T Re = P.re, Cv1 = (T)C.Cv1, kv = (T)C.kavf, Cb1 = (T)C.Cb1, Cb2 = (T)C.Cb2, sigma = (T)C.sigma;
     const T Cw1 = (T)C.Cw1, Cw2 = (T)C.Cw2, Cw3 = (T)C.Cw3, Ct3 = (T)C.Ct3, Ct4 = (T)C.Ct4;
-    const T ev = (T)W.ev[p];
-    const T ev_lam = Re * sutherland<T>(P, W.pv[PT][p]) / W.pv[PD][p];
+    const T ev = to_work<T>(W.ev[p]);
+    const T ev_lam = Re * sutherland(P, W.pv[PT][p]) / W.pv[PD][p];
     const T X = ev / ev_lam;
     const T fv1 = fv1_of<T>(X, Cv1);
     const T fv2 = (T)1 - X / ((T)1 + X * fv1);
     const T ft2 = Ct3 * exp((T)0 - Ct4 * X * X);
     const T om = W.omega[p];
-    const T dw = (T)W.dwall[p];
+    const T dw = to_work<T>(W.dwall[p]);
     const T Sbar = fmax(om + ev * fv2 / (pow(kv * dw, (T)2) * Re), (T)(double)0.3f * om);
     const T r = fmin(ev / (Sbar * kv * kv * dw * dw * Re), (T)10);
     const T g = r + Cw2 * (pow(r, (T)6) - r);
@@ -315,7 +325,7 @@ __global__ void __launch_bounds__(256) k_sa_cell(Batch B, Phys P, GeoW<T> G, Flo
 // mu_t of the ghost layer from its variable (source/SA_Model.cpp:208-256): threads over the six
 // faces' interior ranges
 template <typename T>
-__global__ void k_sa_ghost_mut(Batch B, Phys P, Flow<T> W)
+__global__ void k_sa_ghost_mut(Batch B, PhysW<T> P, Flow<T> W)
 {
     const Lvl L = B.lv[blockIdx.y];
     const int nI = L.IM - 1, nJ = L.JM - 1, nK = L.KM - 1;
@@ -336,22 +346,21 @@ __global__ void k_sa_ghost_mut(Batch B, Phys P, Flow<T> W)
     }
     const long long p = ix(L, i, j, k);
     const SAConst C = sa_const();
-    const T Re = (T)P.re_ref;
-    const T d = W.pv[PD][p], ev = (T)W.ev[p];
-    const T ev_lam = Re * sutherland<T>(P, W.pv[PT][p]) / d;
+    const T Re = P.re;
+    const T d = W.pv[PD][p], ev = to_work<T>(W.ev[p]);
+    const T ev_lam = Re * sutherland(P, W.pv[PT][p]) / d;
     W.mut[p] = fv1_of<T>(ev / ev_lam, (T)C.Cv1) * d * ev / Re;
 }
 
 template <typename T>
-void launch_sa_model(const LaunchCtx &ctx, const Phys &P, const GeoW<T> &GW, Flow<T> W)
+void launch_sa_model(const LaunchCtx &ctx, const PhysW<T> &P, const GeoW<T> &GW, Flow<T> W)
 {
     const Batch &B = ctx.batch;
     // the gradients of the variable are those of the state before the model clips it
     cudaMemcpyAsync(W.evg, W.ev, sizeof(double) * (size_t)ctx.pool_n, cudaMemcpyDeviceToDevice, ctx.stream);
     k_sa_mut<T><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, P, W);
-    k_sa_face<T, 0><<<ctx.grid_faces(0, 128), 128, 0, ctx.stream>>>(B, P, GW, W);
-    k_sa_face<T, 1><<<ctx.grid_faces(1, 128), 128, 0, ctx.stream>>>(B, P, GW, W);
-    k_sa_face<T, 2><<<ctx.grid_faces(2, 128), 128, 0, ctx.stream>>>(B, P, GW, W);
+    k_sa_face<T><<<dim3(std::max({ctx.grid_faces(0, 128).x, ctx.grid_faces(1, 128).x, ctx.grid_faces(2, 128).x}), 3, B.nsolve), 128, 0, ctx.stream>>>(
+        B, P, GW, W);
     k_sa_cell<T><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, P, GW, W);
     const long long ng = 2LL * ((long long)(ctx.maxJM - 1) * (ctx.maxKM - 1) + (long long)(ctx.maxIM - 1) * (ctx.maxKM - 1) +
                                 (long long)(ctx.maxIM - 1) * (ctx.maxJM - 1));
@@ -451,7 +460,7 @@ void launch_sa_limit(const LaunchCtx &ctx, Flow<T> W, int *bad_list, int bad_cap
 
 #define GBT_SA_INST(T)                                                                                                 \
     template void launch_sa_boundary<T>(const LaunchCtx &, const Phys &, Flow<T>, const BcTables &);                  \
-    template void launch_sa_model<T>(const LaunchCtx &, const Phys &, const GeoW<T> &, Flow<T>);                      \
+    template void launch_sa_model<T>(const LaunchCtx &, const PhysW<T> &, const GeoW<T> &, Flow<T>);                    \
     template void launch_sa_update<T>(const LaunchCtx &, const Phys &, Flow<T>, int *, int, int *);                    \
     template void launch_sa_limit<T>(const LaunchCtx &, Flow<T>, int *, int, int *);
 GBT_SA_INST(double)

@@ -692,16 +692,21 @@ __global__ void __launch_bounds__(256) k_wave_var(Batch B, PhysW<T> P, Geo G, Fl
     const long long p = ix(Lv, i, j, k);
     const T *dq = (const T *)(V.dq + (c.step + st) * Lay<T, MEAN>::dq) + 4 * cell;
     const double o0 = W.cv[0][p], o1 = W.cv[1][p], o2 = W.cv[2][p], o3 = W.cv[3][p];
-    const T dn0 = (T)(o0 + (double)dq[0]), dn1 = (T)(o1 + (double)dq[1]), dn2 = (T)(o2 + (double)dq[2]), dn3 = (T)(o3 + (double)dq[3]);
-    const T evo = (T)W.ev[p];
+    auto next = [&](double o, T q) { return to_work<T>(o + to_f64<T>(q)); };
+    const T dn0 = next(o0, dq[0]), dn1 = next(o1, dq[1]), dn2 = next(o2, dq[2]), dn3 = next(o3, dq[3]);
+    const T evo = to_work<T>(W.ev[p]);
+    // the normals and areas as the mean flow's sweep has them
+    const T *geo = (const T *)(V.geo + (c.step + st) * Lay<T, MEAN>::geo), *area = (const T *)V.area + (c.step + st) * (3 * Lay<T, MEAN>::NC) + 3 * cell;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        const T nx = (T)G.cn[d][0][p], ny = (T)G.cn[d][1][p], nz = (T)G.cn[d][2][p];
+        const int g = 3 * cell + d;
+        const T nx = geo[sizeof(T) == 4 ? 4 * g : 2 * g], ny = geo[sizeof(T) == 4 ? 4 * g + 1 : 2 * g + 1],
+                nz = geo[sizeof(T) == 4 ? 4 * g + 2 : 6 * NC + 2 * g];
         fd[d] = dn1 / dn0 * nx + dn2 / dn0 * ny + dn3 / dn0 * nz;
         if (DIR > 0) {
-            const T Vold = (T)o1 / (T)o0 * nx + (T)o2 / (T)o0 * ny + (T)o3 / (T)o0 * nz;
+            const T q0 = to_work<T>(o0), Vold = to_work<T>(o1) / q0 * nx + to_work<T>(o2) / q0 * ny + to_work<T>(o3) / q0 * nz;
             fd[3 * NC + d] = evo * Vold;
-            fd[6 * NC + d] = (T)G.cs[d][p];
+            fd[6 * NC + d] = area[d];
             fd[9 * NC + d] = P.relax * W.lamc[d][p];
             fd[12 * NC + d] = W.lamv[d][p];
         }
@@ -710,7 +715,7 @@ __global__ void __launch_bounds__(256) k_wave_var(Batch B, PhysW<T> P, Geo G, Fl
         const T lc = W.lamc[0][p] + W.lamc[1][p] + W.lamc[2][p];
         const T lv = W.lamv[0][p] + W.lamv[1][p] + W.lamv[2][p];
         f[15 * NC + cell] = evo;
-        f[16 * NC + cell] = (T)G.vol[p] / W.dt[p] + P.relax * lc + (T)3 * lv;
+        f[16 * NC + cell] = to_work<T>(G.vol[p]) / W.dt[p] + P.relax * lc + (T)3 * lv;
         ((T *)(VV.dq + (c.step + st) * L::dq))[cell] = -W.res_ev[p];
     }
 }
@@ -874,10 +879,24 @@ void launch_lusgs_sweeps(const LaunchCtx &ctx, const Phys &PH, const PhysW<T> &P
     else k_wave_gather64<<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, P, W, V);
     march<T, 1, MEAN>(ctx, V, P.gm1);
     ctx.mark("sweep_forward", 0, 2);
+    // The variable's sweep of a direction needs the mean flow's dQ of that direction and nothing of the other one,
+    // nor of the update: its march, as the mean flow's bound by the chain of planes, runs beside them on the
+    // second stream once its inputs are formed.
+    LaunchCtx second = ctx;
+    if (ctx.side) second.stream = ctx.side;
+    auto beside = [&](auto launches) {
+        if (ctx.side) {
+            cudaEventRecord(ctx.fork, ctx.stream);
+            cudaStreamWaitEvent(ctx.side, ctx.fork, 0);
+        }
+        launches();
+        if (ctx.side) cudaEventRecord(ctx.join, ctx.side);
+    };
+    auto meet = [&] { if (ctx.side) cudaStreamWaitEvent(ctx.stream, ctx.join, 0); };
     if (W.ev) {
         ctx.mark("sa_sweeps", 1, 2);
         k_wave_var<T, 1><<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
-        march<T, 1, VAR>(ctx, VV, (T)0);
+        beside([&] { march<T, 1, VAR>(second, VV, (T)0); });
         ctx.mark("sa_sweeps", 0, 2);
     }
     ctx.mark("sweep_backward", 1, 1);
@@ -885,14 +904,18 @@ void launch_lusgs_sweeps(const LaunchCtx &ctx, const Phys &PH, const PhysW<T> &P
     ctx.mark("sweep_backward", 0, 1);
     if (W.ev) {
         ctx.mark("sa_sweeps", 1, 3);
+        meet();
         k_wave_var<T, -1><<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
-        march<T, -1, VAR>(ctx, VV, (T)0);
-        k_wave_scatter_var<T><<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, W, VV);
+        beside([&] {
+            march<T, -1, VAR>(second, VV, (T)0);
+            k_wave_scatter_var<T><<<chunks(kSteps<T>), 256, 0, second.stream>>>(ctx.batch, W, VV);
+        });
         ctx.mark("sa_sweeps", 0, 3);
     }
     ctx.mark("update_limiter", 1, 1);
     k_wave_update<T><<<dim3((unsigned)(V.max_tiles * runs_of(ctx.maxKM - 1)), ctx.batch.nsolve), 256, 0, ctx.stream>>>(ctx.batch, PH, W, V, level, q);
     if (W.ev) {
+        meet();
         // the variable's update and Limit_SA after the mean flow's (source/LU_SGS_Marching.cpp:275-277,
         // source/ComputeAllBlockVars.cpp:257-266); the limiter's list is reused
         launch_sa_update<T>(ctx, PH, W, q.list, q.cap, q.count);
