@@ -159,10 +159,12 @@ __global__ void __launch_bounds__(64) k_corners(Batch B, Flow<T> W)
     W.dq2h[c][dst] = d;
 }
 
+// Bound by the latency of its gathers: FP32 eight blocks per SM in 32 registers, 0.203 and 0.158 ms per cycle of
+// 12 solves on three meshes.
 // fine Q (+)= sum of 27/64, 9/64, 3/64, 1/64 weighted coarse values around the fine cell; the
 // first call after the coarse start-up phase interpolates Q itself, later calls the correction
 template <typename T, bool PRIM>
-__global__ void __launch_bounds__(256) k_interpolate(Batch Bf, Batch Bc, Phys P, Flow<T> Wf, Flow<T> Wc, int init, int level,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 1) k_interpolate(Batch Bf, Batch Bc, Phys P, Flow<T> Wf, Flow<T> Wc, int init, int level,
                                                      LimitLists lists)
 {
     const int s = blockIdx.y;

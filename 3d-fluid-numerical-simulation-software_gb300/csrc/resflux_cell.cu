@@ -26,8 +26,9 @@ void launch_cell_norms(const LaunchCtx &ctx, const GeoW<double> &G)
 }
 
 // lambda_c per direction and |curl V| (needs ghosts of the velocity)
+// (FP32: eight blocks per SM; two registers more cost 10% on large batches)
 template <typename T, bool NS>   // NS: Navier-Stokes (the curl is needed), else Euler
-__global__ void __launch_bounds__(256) k_cell_a(Batch B, PhysW<T> PC, GeoW<T> G, Flow<T> W)
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 1) k_cell_a(Batch B, PhysW<T> PC, GeoW<T> G, Flow<T> W)
 {
     const int s = blockIdx.y;
     const Lvl L = B.lv[s];
@@ -147,8 +148,10 @@ template <typename T> __device__ __forceinline__ T bl_value(unsigned long long b
 template <> __device__ __forceinline__ double bl_value<double>(unsigned long long b) { return __longlong_as_double((long long)b); }
 template <> __device__ __forceinline__ float bl_value<float>(unsigned long long b) { return __uint_as_float((unsigned)b); }
 
+// (FP32: five blocks per SM in 48 registers; four in 64 took 0.348 ms per cycle of 12 solves on three meshes,
+// six or eight, with spills, 0.309 and 0.324, five 0.315, and six cost single solves what they gain)
 template <typename T>
-__global__ void __launch_bounds__(32 * BL_WARPS) k_bl(Batch B, PhysW<T> PC, Flow<T> W, const DevWall *walls, int off,
+__global__ void __launch_bounds__(32 * BL_WARPS, sizeof(T) == 4 ? 5 : 1) k_bl(Batch B, PhysW<T> PC, Flow<T> W, const DevWall *walls, int off,
                                                       const long long *dist_off, const T *dist_all)
 {
     __shared__ T sh_a[BL_WARPS][32], sh_b[BL_WARPS][32], sh_u[BL_WARPS][32];

@@ -278,7 +278,7 @@ __device__ __forceinline__ void sa_face(const Batch &B, const PhysW<T> &P, const
     W.Fv1t[F][p] = ux * Sx + uy * Sy + uz * Sz;
 }
 // the three families (blockIdx.y) in one launch. The mixed form was bound by the FP64 pipe, which conversions
-// and a constant's division took 21 times a face: 53 us on 129 x 49 x 49 as three launches, TODOS now.
+// and a constant's division took 21 times a face: 53 us on 129 x 49 x 49 as three launches.
 template <typename T>
 __global__ void __launch_bounds__(128) k_sa_face(Batch B, PhysW<T> P, GeoW<T> G, Flow<T> W)
 {
