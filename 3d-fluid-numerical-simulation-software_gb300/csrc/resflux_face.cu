@@ -50,8 +50,9 @@ __device__ __forceinline__ void face_one(const Batch &B, const Phys &P, const Ph
 #pragma unroll
     for (int c = 0; c < NQ; c++) W.Ff[F][c][p] = out[c];
     if (!P.equation_ns) return;
+    // (no viscous flux of mass: its pool stays the zeros it was allocated with)
 #pragma unroll
-    for (int c = 0; c < NQ; c++) W.Vf[F][c][p] = out[5 + c];
+    for (int c = 1; c < NQ; c++) W.Vf[F][c][p] = out[5 + c];
 }
 
 // The three families in one launch: the blocks of one fill the SMs that the last wave of the one before
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(256) k_cell_sum(Batch B, GeoW<T> G, Flow<T> W,
     for (int c = 0; c < NQ; c++) {
         T fc = W.Ff[0][c][pI] - W.Ff[0][c][p] + W.Ff[1][c][pJ] - W.Ff[1][c][p] + W.Ff[2][c][pK] - W.Ff[2][c][p] - src[c];
         T fv = (T)0;
-        if constexpr (NS)
+        if (NS && c > 0)
             fv = W.Vf[0][c][pI] - W.Vf[0][c][p] + W.Vf[1][c][pJ] - W.Vf[1][c][p] + W.Vf[2][c][pK] - W.Vf[2][c][p];
         r[c] = fc - fv;
         if constexpr (JST)
