@@ -157,7 +157,8 @@ void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> W, const double
 // FP64 power per point instead of two, and Ma^2 needs no roots. The last block of a solve adds its
 // blocks' sums up in their order and forms the reported values, a lane per section where they are powers.
 // Bound by the latency of the FP64 chains: 48 us per evaluation of the 129x49x49 passage as two kernels
-// with two powers per point, sums and powers of a solve on one thread, now 26.
+// with two powers per point, sums and powers of a solve on one thread; 27 with a third power in a row at the end,
+// 25 now.
 template <typename T>
 __global__ void __launch_bounds__(128) k_integrals(Batch B, Phys P, Geo G, Flow<T> W, const DevInOut *inl, const DevInOut *outl,
                                                    double *part, unsigned *count, HistorySink hist)
@@ -201,8 +202,13 @@ __global__ void __launch_bounds__(128) k_integrals(Batch B, Phys P, Geo G, Flow<
     // lanes 0..2: the inlet's sums, 3..5: the outlet's
     const int lane = threadIdx.x;
     double sum = 0;
-    if (lane < 6)
-        for (int b = 0; b < kIntegralBlocks; b++) sum += __ldcg(&part[(((long long)s * 2 + lane / 3) * kIntegralBlocks + b) * 3 + lane % 3]);
+    if (lane < 6) {
+        double v[kIntegralBlocks];
+#pragma unroll
+        for (int b = 0; b < kIntegralBlocks; b++) v[b] = __ldcg(&part[(((long long)s * 2 + lane / 3) * kIntegralBlocks + b) * 3 + lane % 3]);
+#pragma unroll
+        for (int b = 0; b < kIntegralBlocks; b++) sum += v[b];
+    }
     double a[3], b[3];
     for (int c = 0; c < 3; c++) {
         a[c] = __shfl_sync(0xffffffffu, sum, c);
@@ -211,11 +217,13 @@ __global__ void __launch_bounds__(128) k_integrals(Batch B, Phys P, Geo G, Flow<
     // blade count of the inlet's and of the outlet's block (source/Ouput.cpp:288,294)
     const double mi = a[0] * P.dens_ref * P.vel_ref * B.sc[inl[s].solve].nblade;
     const double mo = b[0] * P.dens_ref * P.vel_ref * B.sc[outl[s].solve].nblade;
-    const double pt = pow(lane == 0 ? a[1] / a[0] : b[1] / b[0], g / g1) * P.dens_ref * P.vel_ref * P.vel_ref;
+    const double fa = a[1] / a[0], fb = b[1] / b[0];
+    const double pt = pow(lane == 0 ? fa : fb, g / g1) * P.dens_ref * P.vel_ref * P.vel_ref;
     const double pti = __shfl_sync(0xffffffffu, pt, 0), pto = __shfl_sync(0xffffffffu, pt, 1);
     const double tti = a[2] / a[0] * P.temp_ref, tto = b[2] / b[0] * P.temp_ref;
     const double PR = pto / pti;
-    const double Ladk = g / g1 * R * tti * (pow(PR, g1 / g) - 1.0);
+    // (PR^((g-1)/g) is the quotient of the two bases)
+    const double Ladk = g / g1 * R * tti * ((isnan(PR) ? PR : fb / fa) - 1.0);
     const double Lk = g / g1 * R * tti * (tto / tti - 1.0);
     if (lane != 0) return;
     SolveState &st = B.st[s];
