@@ -183,6 +183,8 @@ void launch_add_forcing(const LaunchCtx &cc, Flow<T> Fc);
 template <typename T>
 void launch_corner(const LaunchCtx &cc, Flow<T> Fc);
 template <typename T>
+void launch_delta_corner(const LaunchCtx &cc, Flow<T> Fc);
+template <typename T>
 void launch_interpolate(const LaunchCtx &cf, const LaunchCtx &cc, Flow<T> Ff, Flow<T> Fc, int init_from_coarse);
 
 // per-solve scalar stages

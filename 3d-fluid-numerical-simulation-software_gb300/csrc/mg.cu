@@ -9,7 +9,8 @@
 
 namespace gbt {
 
-// PRIM: the coarse level's primitive variables and limiter with it (a launch each otherwise)
+// PRIM: the coarse level's primitive variables and limiter with it (a launch each otherwise). (The forcing with it
+// as well saved single solves 3 us and cost 12 solves on three meshes 10, in 98 registers.)
 template <typename T, bool PRIM>
 __global__ void __launch_bounds__(256) k_restrict(Batch Bf, Batch Bc, Phys P, Geo Gf, Geo Gc, Flow<T> Wf, Flow<T> Wc, int level,
                                                   LimitLists lists)
@@ -93,59 +94,45 @@ __global__ void __launch_bounds__(256) k_add_forcing(Batch B, Flow<T> W)
     for (int c = 0; c < NQ; c++) W.res[c][p] = W.res[c][p] + W.res2h[c][p];
 }
 
+// 12 edges then 8 corners of the ghost layer, for Q and for the coarse correction (source/Corner_Treatment.cpp),
+// by the threads of one block: first the edges, one cell after another of all twelve, then the corners, which
+// read the edges
 template <typename T>
-__global__ void __launch_bounds__(256) k_delta(Batch B, Flow<T> W)
+__device__ __forceinline__ void edges_and_corners(const Lvl &L, Flow<T> &W)
 {
-    const Lvl L = B.lv[blockIdx.y];
-    int i, j, k;
-    if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
-    const long long p = ix(L, i, j, k);
+    const int IM = L.IM, JM = L.JM, KM = L.KM, nI = IM - 1, nJ = JM - 1, nK = KM - 1;
+    for (int t = threadIdx.x; t < 4 * (nI + nJ + nK); t += blockDim.x) {
+        int e, n;
+        if (t < 4 * nI) { e = t / nI; n = 1 + t % nI; }
+        else if (t < 4 * (nI + nJ)) { e = 4 + (t - 4 * nI) / nJ; n = 1 + (t - 4 * nI) % nJ; }
+        else { e = 8 + (t - 4 * (nI + nJ)) / nK; n = 1 + (t - 4 * (nI + nJ)) % nK; }
+        long long dst, a, b;
+        switch (e) {
+        case 0: dst = ix(L, n, 0, 0); a = ix(L, n, 1, 0); b = ix(L, n, 0, 1); break;
+        case 1: dst = ix(L, n, JM, 0); a = ix(L, n, JM - 1, 0); b = ix(L, n, JM, 1); break;
+        case 2: dst = ix(L, n, 0, KM); a = ix(L, n, 0, KM - 1); b = ix(L, n, 1, KM); break;
+        case 3: dst = ix(L, n, JM, KM); a = ix(L, n, JM - 1, KM); b = ix(L, n, JM, KM - 1); break;
+        case 4: dst = ix(L, 0, n, 0); a = ix(L, 1, n, 0); b = ix(L, 0, n, 1); break;
+        case 5: dst = ix(L, 0, n, KM); a = ix(L, 1, n, KM); b = ix(L, 0, n, KM - 1); break;
+        case 6: dst = ix(L, IM, n, KM); a = ix(L, IM - 1, n, KM); b = ix(L, IM, n, KM - 1); break;
+        case 7: dst = ix(L, IM, n, 0); a = ix(L, IM - 1, n, 0); b = ix(L, IM, n, 1); break;
+        case 8: dst = ix(L, 0, 0, n); a = ix(L, 1, 0, n); b = ix(L, 0, 1, n); break;
+        case 9: dst = ix(L, IM, 0, n); a = ix(L, IM, 1, n); b = ix(L, IM - 1, 0, n); break;
+        case 10: dst = ix(L, 0, JM, n); a = ix(L, 1, JM, n); b = ix(L, 0, JM - 1, n); break;
+        default: dst = ix(L, IM, JM, n); a = ix(L, IM - 1, JM, n); b = ix(L, IM, JM - 1, n); break;
+        }
+        double qa[NQ], qb[NQ];
+        T da[NQ], db[NQ];
 #pragma unroll
-    for (int c = 0; c < NQ; c++) W.dq2h[c][p] = to_work<T>(W.cv[c][p] - W.cv2h[c][p]);
-}
-
-// 12 edges then 8 corners of the ghost layer, for Q and for the coarse correction
-// (source/Corner_Treatment.cpp): edges in one launch (one thread per edge cell, all values read
-// before any is written), then the corners, which read the edges, in a second one
-template <typename T>
-__global__ void __launch_bounds__(64) k_edges(Batch B, Flow<T> W)
-{
-    const Lvl L = B.lv[blockIdx.z];
-    const int IM = L.IM, JM = L.JM, KM = L.KM;
-    const int e = blockIdx.y, n = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    long long dst, a, b;
-    switch (e) {
-    case 0: if (n > IM - 1) return; dst = ix(L, n, 0, 0); a = ix(L, n, 1, 0); b = ix(L, n, 0, 1); break;
-    case 1: if (n > IM - 1) return; dst = ix(L, n, JM, 0); a = ix(L, n, JM - 1, 0); b = ix(L, n, JM, 1); break;
-    case 2: if (n > IM - 1) return; dst = ix(L, n, 0, KM); a = ix(L, n, 0, KM - 1); b = ix(L, n, 1, KM); break;
-    case 3: if (n > IM - 1) return; dst = ix(L, n, JM, KM); a = ix(L, n, JM - 1, KM); b = ix(L, n, JM, KM - 1); break;
-    case 4: if (n > JM - 1) return; dst = ix(L, 0, n, 0); a = ix(L, 1, n, 0); b = ix(L, 0, n, 1); break;
-    case 5: if (n > JM - 1) return; dst = ix(L, 0, n, KM); a = ix(L, 1, n, KM); b = ix(L, 0, n, KM - 1); break;
-    case 6: if (n > JM - 1) return; dst = ix(L, IM, n, KM); a = ix(L, IM - 1, n, KM); b = ix(L, IM, n, KM - 1); break;
-    case 7: if (n > JM - 1) return; dst = ix(L, IM, n, 0); a = ix(L, IM - 1, n, 0); b = ix(L, IM, n, 1); break;
-    case 8: if (n > KM - 1) return; dst = ix(L, 0, 0, n); a = ix(L, 1, 0, n); b = ix(L, 0, 1, n); break;
-    case 9: if (n > KM - 1) return; dst = ix(L, IM, 0, n); a = ix(L, IM, 1, n); b = ix(L, IM - 1, 0, n); break;
-    case 10: if (n > KM - 1) return; dst = ix(L, 0, JM, n); a = ix(L, 1, JM, n); b = ix(L, 0, JM - 1, n); break;
-    default: if (n > KM - 1) return; dst = ix(L, IM, JM, n); a = ix(L, IM - 1, JM, n); b = ix(L, IM, JM - 1, n); break;
+        for (int c = 0; c < NQ; c++) { qa[c] = W.cv[c][a]; qb[c] = W.cv[c][b]; da[c] = W.dq2h[c][a]; db[c] = W.dq2h[c][b]; }
+#pragma unroll
+        for (int c = 0; c < NQ; c++) {
+            W.cv[c][dst] = 0.5 * (qa[c] + qb[c]);
+            W.dq2h[c][dst] = (T)0.5 * (da[c] + db[c]);
+        }
     }
-    double qa[NQ], qb[NQ];
-    T da[NQ], db[NQ];
-#pragma unroll
-    for (int c = 0; c < NQ; c++) { qa[c] = W.cv[c][a]; qb[c] = W.cv[c][b]; da[c] = W.dq2h[c][a]; db[c] = W.dq2h[c][b]; }
-#pragma unroll
-    for (int c = 0; c < NQ; c++) {
-        W.cv[c][dst] = 0.5 * (qa[c] + qb[c]);
-        W.dq2h[c][dst] = (T)0.5 * (da[c] + db[c]);
-    }
-}
-
-// corner (ci,cj,ck) from its three edge neighbours and three face-diagonal neighbours; thread
-// corner * NQ + c of the block of its solve
-template <typename T>
-__global__ void __launch_bounds__(64) k_corners(Batch B, Flow<T> W)
-{
-    const Lvl L = B.lv[blockIdx.x];
-    const int IM = L.IM, JM = L.JM, KM = L.KM;
+    __syncthreads();
+    // corner (ci,cj,ck) from its three edge neighbours and three face-diagonal neighbours: thread corner * NQ + c
     if (threadIdx.x >= 8 * NQ) return;
     const int corner = threadIdx.x / NQ, c = threadIdx.x % NQ;
     const int ci = (corner & 1) ? IM : 0, cj = (corner & 2) ? JM : 0, ck = (corner & 4) ? KM : 0;
@@ -157,6 +144,21 @@ __global__ void __launch_bounds__(64) k_corners(Batch B, Flow<T> W)
     const T d = ((T)2 * (W.dq2h[c][e1] + W.dq2h[c][e2] + W.dq2h[c][e3]) - (W.dq2h[c][d1] + W.dq2h[c][d2] + W.dq2h[c][d3])) / (T)3;
     W.cv[c][dst] = q;
     W.dq2h[c][dst] = d;
+}
+
+// the coarse correction of the cells (cell_blocks blocks of a solve), and the ghost layer's edges and corners by a
+// further block: they read ghost cells, the correction writes the others. As three launches 22 us per
+// cycle of a single solve, as one 8.
+template <typename T>
+__global__ void __launch_bounds__(256) k_delta_corner(Batch B, Flow<T> W, unsigned cell_blocks)
+{
+    const Lvl L = B.lv[blockIdx.y];
+    if (blockIdx.x >= cell_blocks) { edges_and_corners<T>(L, W); return; }
+    int i, j, k;
+    if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
+    const long long p = ix(L, i, j, k);
+#pragma unroll
+    for (int c = 0; c < NQ; c++) W.dq2h[c][p] = to_work<T>(W.cv[c][p] - W.cv2h[c][p]);
 }
 
 // Bound by the latency of its gathers: FP32 eight blocks per SM in 32 registers, 0.203 and 0.158 ms per cycle of
@@ -247,14 +249,19 @@ void launch_add_forcing(const LaunchCtx &cc, Flow<T> Fc)
 template <typename T>
 void launch_delta(const LaunchCtx &cc, Flow<T> Fc)
 {
-    k_delta<T><<<cc.grid_cells(256), 256, 0, cc.stream>>>(cc.batch, Fc);
+    const dim3 g = cc.grid_cells(256);
+    k_delta_corner<T><<<g, 256, 0, cc.stream>>>(cc.batch, Fc, g.x);
 }
 template <typename T>
 void launch_corner(const LaunchCtx &cc, Flow<T> Fc)
 {
-    const int mx = std::max(cc.maxIM, std::max(cc.maxJM, cc.maxKM));
-    k_edges<T><<<dim3((mx + 63) / 64, 12, cc.batch.nsolve), 64, 0, cc.stream>>>(cc.batch, Fc);
-    k_corners<T><<<cc.batch.nsolve, 64, 0, cc.stream>>>(cc.batch, Fc);
+    k_delta_corner<T><<<dim3(1, cc.batch.nsolve), 256, 0, cc.stream>>>(cc.batch, Fc, 0);
+}
+template <typename T>
+void launch_delta_corner(const LaunchCtx &cc, Flow<T> Fc)
+{
+    const dim3 g = cc.grid_cells(256);
+    k_delta_corner<T><<<dim3(g.x + 1, g.y), 256, 0, cc.stream>>>(cc.batch, Fc, g.x);
 }
 template <typename T>
 void launch_interpolate(const LaunchCtx &cf, const LaunchCtx &cc, Flow<T> Ff, Flow<T> Fc, int init)
@@ -275,6 +282,7 @@ void launch_interpolate_primitive(const LaunchCtx &cf, const LaunchCtx &cc, cons
     template void launch_add_forcing<T>(const LaunchCtx &, Flow<T>);                                                     \
     template void launch_delta<T>(const LaunchCtx &, Flow<T>);                                                           \
     template void launch_corner<T>(const LaunchCtx &, Flow<T>);                                                          \
+    template void launch_delta_corner<T>(const LaunchCtx &, Flow<T>);                                                    \
     template void launch_interpolate<T>(const LaunchCtx &, const LaunchCtx &, Flow<T>, Flow<T>, int);                    \
     template void launch_restrict_primitive<T>(const LaunchCtx &, const LaunchCtx &, const Phys &, const Geo &, const Geo &, Flow<T>, \
                                                Flow<T>, int, const LimitLists &);                                        \

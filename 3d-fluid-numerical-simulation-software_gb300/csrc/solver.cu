@@ -1237,7 +1237,7 @@ public:
         Mark m(this, "mg_prolong");
         launch_interpolate_primitive<T>(ctx(lf), ctx(lf + 1), P, lev[lf].W, lev[lf + 1].W, init, lf, limits);
     }
-    void delta_lv(int lc) { Mark m(this, "mg_delta"); launch_delta<T>(ctx(lc), lev[lc].W); }
+    void delta_corner(int lc) { Mark m(this, "mg_delta"); launch_delta_corner<T>(ctx(lc), lev[lc].W); }
     // FAS smoothing of coarse level l (three-level extension): residual at the restricted state,
     // forcing kept, sweeps and update
     void smooth_fas(int l)
@@ -1264,7 +1264,7 @@ public:
     }
     void primitive_vars(int l) override { Mark m(this, "primitive"); launch_primitive<T>(ctx(l), P, lev[l].W); }
     void limit_vars(int l) override { Mark m(this, "limiter", 1); launch_limiter<T>(ctx(l), P, lev[l].W, l, limits); }
-    void corner_treatment(int l) override { Mark m(this, "mg_corner", 2); launch_corner<T>(ctx(l), lev[l].W); }
+    void corner_treatment(int l) override { Mark m(this, "mg_corner", 1); launch_corner<T>(ctx(l), lev[l].W); }
     void restrict_to_coarse() override
     {
         need_mg();
@@ -1321,8 +1321,7 @@ public:
             fine_norm_and_residual();
             restrict_primitive(1);
             time_marching(2);
-            delta_cons();
-            corner_treatment(2);
+            delta_corner(2);
             interpolate_primitive(1, 0);
         } else {
             // three-level V-cycle (extension): the fine step as in the two-level cycle, then FAS
@@ -1335,11 +1334,9 @@ public:
             { Mark m(this, "mg_forcing"); launch_add_forcing<T>(ctx(2), lev[2].W); }
             restrict_primitive(2);
             smooth_fas(3);
-            delta_lv(3);
-            corner_treatment(3);
+            delta_corner(3);
             interpolate_primitive(2, 0);
-            delta_lv(2);
-            corner_treatment(2);
+            delta_corner(2);
             interpolate_primitive(1, 0);
         }
     }
