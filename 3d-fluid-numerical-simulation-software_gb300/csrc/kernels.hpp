@@ -93,7 +93,7 @@ struct WaveBytes { int geo, flow, dq, pkt, area, var_flow, var_dq, var_pkt; };  
 struct WaveTables {
     const WaveSolve *solve = nullptr;              // per slot
     const int2 *item = nullptr;                    // {slot, PI << 16 | PJ}: every tile, after the two it reads from
-    int n_item = 0;
+    int n_item = 0, narrow = 0;
     int max_tiles = 0, max_T = 0;                  // largest of a slot: tiles, steps of a tile
     long long max_steps = 0;                       // and steps of all its tiles
     WaveCtl *ctl = nullptr;
@@ -101,10 +101,10 @@ struct WaveTables {
     void *area = nullptr;                          // mean area per cell and direction
     uint4 *pkt = nullptr;                          // terms that cross from tile to tile
 };
-// columns of a tile in i and j; bytes of a step's blocks (fp64: working type; sa: with the
-// Spalart-Allmaras variable)
-void wave_patch(int fp64, int &pa, int &pb);
-void wave_bytes(int fp64, int sa, WaveBytes &w);
+// columns of a tile in i and j; bytes of a step's blocks (fp64: working type; narrow: half as wide in j, FP64 only;
+// sa: with the Spalart-Allmaras variable)
+void wave_patch(int fp64, int narrow, int &pa, int &pb);
+void wave_bytes(int fp64, int narrow, int sa, WaveBytes &w);
 
 void launch_geometry(const LaunchCtx &ctx, const Geo &G, double *totalvol);
 // the periodic rotation's cosines and sines per solve (BcTables::per_trig), once at create

@@ -17,7 +17,8 @@
 // done by two further warps of the block:
 //   a cell's lanes     receive a component each (FP32: and the fifth); lanes 0..2 form V_n of a direction each, and
 //                      lane 3 the pressure with the same instructions; the fifteen terms are formed by
-//                      direction on lanes 0..2 (FP64: two to a lane of eight)
+//                      direction on lanes 0..2 (FP64: two to a lane of eight, or one to a lane of sixteen
+//                      in narrow tiles, where there is an SM for each of them)
 //   the incoming warp  reads the terms that cross into the tile and puts them beside the tile's own
 //   the outgoing warp  sends the terms that leave it and fetches the inputs of later steps
 //
@@ -49,16 +50,18 @@
 #include "kernels.hpp"
 #include "flux.cuh"
 #include "update.cuh"
+#include <type_traits>
 
 namespace gbt {
 
 namespace {
 
-// columns of a tile in i and j, lanes of a cell: 128 lanes a step in both precisions
-constexpr int PB = 8;
+// columns of a tile in i and j, lanes of a cell: 128 lanes a step in both precisions. N = 1 (FP64): narrow tiles of
+// 2 x 4 columns with sixteen lanes a cell, one term to a lane (18 FP64 instructions a step instead of 22).
 template <typename T> constexpr int kPA = sizeof(T) == 4 ? 4 : 2;
-template <typename T> constexpr int kCells = kPA<T> * PB;
-template <typename T> constexpr int kLanes = 128 / kCells<T>;
+template <typename T, int N> constexpr int kPB = N ? 4 : 8;
+template <typename T, int N> constexpr int kCells = kPA<T> * kPB<T, N>;
+template <typename T, int N> constexpr int kLanes = 128 / kCells<T, N>;
 constexpr int kGroup = 2, kStages = 3;          // steps of a stage of the input ring, stages
 constexpr int kSlots = kGroup * kStages;        // steps whose terms are kept: the outgoing warp fetches a stage
                                                 // after it has sent the steps that used it, so a step's terms
@@ -69,7 +72,7 @@ constexpr int kAhead = 2;                       // steps that the incoming warp 
                                                 // 129x49x49 passage in FP32 with 2, 3, 4, 8)
 constexpr unsigned kWaitLimit = 1u << 21;       // polls of a wait before it gives up (seconds)
 constexpr int kSteps32 = 16;                    // steps of a block of the FP32 gather kernel
-template <typename T> constexpr int kSteps = 256 / kCells<T>;                   // of the kernels with a thread per cell
+template <typename T, int N> constexpr int kSteps = 256 / kCells<T, N>;                   // of the kernels with a thread per cell
 
 // bytes of a step's blocks, packets of an edge cell and of a step
 //   FP32: geo {n_d, V_entrainment,d} at 3 cell + d; flow {h_d, c_d} at 3 cell + d of the forward sweep, {rho, m},
@@ -81,8 +84,8 @@ template <typename T> constexpr int kSteps = 256 / kCells<T>;                   
 //   the variable's sweep: flow V_d, ev V_old,d, |S_d|, relax lambda_c,d, lambda_v,d at 3 cell + d, ev, alpha per cell;
 //         dq one value per cell; packets {A term, V term, 0, tag} in FP32, one {value, tag} each in FP64
 enum Kind { MEAN, VAR };
-template <typename T, Kind K> struct Lay {
-    static constexpr int PA = kPA<T>, NC = kCells<T>;
+template <typename T, Kind K, int N = 0> struct Lay {
+    static constexpr int PA = kPA<T>, PB = kPB<T, N>, NC = kCells<T, N>;
     static constexpr int B = sizeof(T), CA = K == VAR ? 2 : 4, CB = K == VAR ? 0 : 1, NV = CA + CB;   // values of a term
     static constexpr int geo = K == VAR ? 0 : 12 * NC * B;
     static constexpr int ends = K == MEAN ? 6 * NC * B : 0;                  // of the flow block, one sweep's own
@@ -177,16 +180,16 @@ __device__ __forceinline__ Where tile_of(const WaveTables &V, unsigned ticket)
 
 // byte offsets in a slot of the first and the second group of a term's components: halo cells sit before the
 // first column (row) in the forward sweep and after the last one in the backward sweep
-template <class L> __device__ __forceinline__ int off_ia(int row, int b) { return L::IA + L::CA * (row * PB + b) * L::B; }
-template <class L> __device__ __forceinline__ int off_ib(int row, int b) { return L::IB + L::CB * (row * PB + b) * L::B; }
-template <class L> __device__ __forceinline__ int off_ja(int a, int col) { return L::JA + L::CA * (a * (PB + 1) + col) * L::B; }
-template <class L> __device__ __forceinline__ int off_jb(int a, int col) { return L::JB + L::CB * (a * (PB + 1) + col) * L::B; }
+template <class L> __device__ __forceinline__ int off_ia(int row, int b) { return L::IA + L::CA * (row * L::PB + b) * L::B; }
+template <class L> __device__ __forceinline__ int off_ib(int row, int b) { return L::IB + L::CB * (row * L::PB + b) * L::B; }
+template <class L> __device__ __forceinline__ int off_ja(int a, int col) { return L::JA + L::CA * (a * (L::PB + 1) + col) * L::B; }
+template <class L> __device__ __forceinline__ int off_jb(int a, int col) { return L::JB + L::CB * (a * (L::PB + 1) + col) * L::B; }
 
 // a step's cell on its quad of lanes: what it receives -> dQ -> what it sends. in: the step's inputs;
 // rd: the slot of the last step, wr: this step's
-template <typename T, int DIR, Kind K> struct CellStep;
+template <typename T, int DIR, Kind K, int N> struct CellStep;
 
-template <int DIR> struct CellStep<float, DIR, MEAN> {
+template <int DIR> struct CellStep<float, DIR, MEAN, 0> {
     using L = Lay<float, MEAN>;
     static __device__ __forceinline__ float dot(float a0, float a1, float a2, float b0, float b1, float b2)
     {
@@ -239,30 +242,33 @@ template <int DIR> struct CellStep<float, DIR, MEAN> {
     }
 };
 
-template <int DIR> struct CellStep<double, DIR, MEAN> {
-    using L = Lay<double, MEAN>;
+template <int DIR, int N> struct CellStep<double, DIR, MEAN, N> {
+    using L = Lay<double, MEAN, N>;
+    static constexpr int lanes = kLanes<double, N>;
     static constexpr int NC = L::NC;
     static __device__ __forceinline__ void run(const char *in, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
                                                int w_off4, bool active, double gm1, char *dq_out)
     {
         const int d = q & 3, c = q < 4 ? q : 4, e = 3 * cell + (d < 3 ? d : 0);     // direction, component received
         const bool low = q < 4;
-        const int d0 = q / 5, c0 = q % 5, t1 = min(q + 8, 14), d1 = t1 / 5, c1 = t1 % 5;      // the two terms
+        const int t0 = min(q, 14), d0 = t0 / 5, c0 = t0 % 5, t1 = min(q + 8, 14), d1 = t1 / 5, c1 = t1 % 5;   // the terms
         const double2 *g = (const double2 *)in + e;
         const char *own = in + L::geo + (DIR > 0 ? 0 : L::flow_in - L::ends), *mid = in + L::geo + (DIR > 0 ? L::ends : 0);
         const double *oc = (const double *)mid + 15 * NC + (low ? 4 * cell + c : 4 * NC + cell),
                      *rc = (const double *)(in + L::geo + L::flow_in) + (low ? 4 * cell + c : 4 * NC + cell);
-        const double2 g0 = g[0], g1 = g[3 * NC], ha = ((const double2 *)own)[3 * cell + d0], hb = ((const double2 *)own)[3 * cell + d1];
+        const double2 g0 = g[0], g1 = g[3 * NC], ha = ((const double2 *)own)[3 * cell + d0];
         auto coef = [&](int dir, int cc) { return ((const double *)in)[(cc > 2 ? 6 * NC : 0) + 2 * (3 * cell + dir) + ((cc - 1) & 1)]; };
-        const double fa = ((const double *)mid)[3 * (NC * c0 + cell) + d0], fb = ((const double *)mid)[3 * (NC * c1 + cell) + d1], o = *oc, r = *rc,
-                     ka = coef(d0, c0), kb = coef(d1, c1);
+        const double fa = ((const double *)mid)[3 * (NC * c0 + cell) + d0], o = *oc, r = *rc, ka = coef(d0, c0);
+        double2 hb = make_double2(0.0, 0.0);
+        double fb = 0.0, kb = 0.0;
+        if (lanes == 8) { hb = ((const double2 *)own)[3 * cell + d1]; fb = ((const double *)mid)[3 * (NC * c1 + cell) + d1]; kb = coef(d1, c1); }
         // received
         const double s = __dadd_rn(__dadd_rn(*(const double *)(rd + r_off[0]), *(const double *)(rd + r_off[1])), *(const double *)(rd + r_off[2]));
         const double x = __dadd_rn(r, DIR > 0 ? s : -s), dq = active ? x : 0.0, nq = __dadd_rn(o, dq);
-        const unsigned oct = (threadIdx.x & 31) & ~7u;
-        auto from = [&](double v, int lane) { return __shfl_sync(0xffffffffu, v, oct + lane); };
+        const unsigned first = (threadIdx.x & 31) & ~(unsigned)(lanes - 1);
+        auto from = [&](double v, int lane) { return __shfl_sync(0xffffffffu, v, first + lane); };
         const double n0 = from(nq, 0), n1 = from(nq, 1), n2 = from(nq, 2), n3 = from(nq, 3), n4 = from(nq, 4);
-        const double va = from(dq, c0), vb = from(dq, c1), na = from(nq, c0), nb = from(nq, c1);
+        const double va = from(dq, c0), na = from(nq, c0);
         const double inv = rcp_nr(n0);
         // lanes 0..2 of a half: V_n - ve; lane 3: p = (gamma - 1)(rho E - |m|^2 / (2 rho))
         const double mm = fma(n3, d < 3 ? g1.x : n3, fma(n1, d < 3 ? g0.x : n1, __dmul_rn(n2, d < 3 ? g0.y : n2)));
@@ -272,17 +278,20 @@ template <int DIR> struct CellStep<double, DIR, MEAN> {
             const double w = __dmul_rn(h.y, v);
             return fma(h.x, fma(n, dv, y), DIR > 0 ? w : -w);
         };
-        const double ya = fma(pn, ka, -fa), yb = fma(pn, kb, -fb);
-        const double ta = term(c0 < 4 ? na : ep, from(dn, d0), c0 > 0 ? ya : -fa, va, ha), tb = term(c1 < 4 ? nb : ep, from(dn, d1), c1 > 0 ? yb : -fb, vb, hb);
-        *(double *)(wr + w_off) = ta;
-        if (q < 7) *(double *)(wr + w_off4) = tb;
+        const double ya = fma(pn, ka, -fa), ta = term(c0 < 4 ? na : ep, from(dn, d0), c0 > 0 ? ya : -fa, va, ha);
+        if (q < 15) *(double *)(wr + w_off) = ta;
+        if constexpr (lanes == 8) {
+            const double vb = from(dq, c1), nb = from(nq, c1), yb = fma(pn, kb, -fb);
+            const double tb = term(c1 < 4 ? nb : ep, from(dn, d1), c1 > 0 ? yb : -fb, vb, hb);
+            if (q < 7) *(double *)(wr + w_off4) = tb;
+        }
         if (q < 5) ((double *)dq_out)[low ? 4 * cell + c : 4 * NC + cell] = dq;
     }
 };
 
 // the variable's sweep: A terms of the three directions, then V terms, then the division
-template <typename T, int DIR> struct CellStep<T, DIR, VAR> {
-    using L = Lay<T, VAR>;
+template <typename T, int DIR, int N> struct CellStep<T, DIR, VAR, N> {
+    using L = Lay<T, VAR, N>;
     static constexpr int NC = L::NC;
     static __device__ __forceinline__ T add(T a, T b) { if constexpr (sizeof(T) == 4) return __fadd_rn(a, b); else return __dadd_rn(a, b); }
     static __device__ __forceinline__ T mul(T a, T b) { if constexpr (sizeof(T) == 4) return __fmul_rn(a, b); else return __dmul_rn(a, b); }
@@ -306,11 +315,11 @@ template <typename T, int DIR> struct CellStep<T, DIR, VAR> {
     }
 };
 
-template <typename T, int DIR, Kind K>
+template <typename T, int DIR, Kind K, int N>
 __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, WaveTables V, T gm1)
 {
-    using L = Lay<T, K>;
-    constexpr int PA = L::PA, NC = L::NC;
+    using L = Lay<T, K, N>;
+    constexpr int PA = L::PA, PB = L::PB, NC = L::NC;
     extern __shared__ __align__(128) char smem[];
     __shared__ unsigned s_take[2];
     const unsigned base = (unsigned)__cvta_generic_to_shared(smem);
@@ -331,7 +340,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
     const bool edges = w.has_i || w.has_j;
     bool ok = true;
     if (warp < 4) {
-        const int cell = threadIdx.x / kLanes<T>, q = threadIdx.x % kLanes<T>, a = cell / PB, b = cell % PB;
+        const int cell = threadIdx.x / kLanes<T, N>, q = threadIdx.x % kLanes<T, N>, a = cell / PB, b = cell % PB;
         const bool column = w.PI * PA + a < w.S.nI && w.PJ * PB + b < w.S.nJ;
         constexpr int F = DIR > 0 ? 1 : 0;          // forward: halo first
         // terms read: FP64, component q (or the fifth) of the three directions; otherwise both groups of I and J
@@ -347,7 +356,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
         int w_off = to_a(q), w_off4 = to_b(q);
         if (sizeof(T) == 8 && K == MEAN) {             // terms written: q and q + 8 of the fifteen
             auto to = [&](int t) { return t % 5 < 4 ? to_a(t / 5) + 8 * (t % 5) : to_b(t / 5); };
-            w_off = to(q);
+            w_off = to(min(q, 14));
             w_off4 = to(min(q + 8, 14));
         }
         char *dq = V.dq + (w.step0 + (DIR > 0 ? 0 : T_ - 1)) * L::dq;
@@ -365,7 +374,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
                 if (u >= cnt) break;
                 if (edges) bar_wait(edge + 8 * slot, ph, ok);
                 char *wr = terms + slot * L::slot;
-                CellStep<T, DIR, K>::run(in + (DIR > 0 ? u : cnt - 1 - u) * L::step, rd, wr, cell, q, r_off, w_off, w_off4,
+                CellStep<T, DIR, K, N>::run(in + (DIR > 0 ? u : cnt - 1 - u) * L::step, rd, wr, cell, q, r_off, w_off, w_off4,
                                          column && (unsigned)k < (unsigned)w.S.nK, gm1, dq);
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (threadIdx.x == 0) bar_arrive(done + 8 * slot);
@@ -557,10 +566,10 @@ __device__ __forceinline__ void next_sweep(const WaveTables &V)
 // shared memory. Bound by the latency of its loads, some 30 per cell: with 32 steps and four cells per
 // thread one after another it took 43 us on the 129x49x49 passage and 168 us per cycle on 32 solves of
 // 25x25x65 nodes, one cell per thread 15 and 64 (40 for the bytes of the latter).
-__global__ void __launch_bounds__(kCells<float> * kSteps32) k_wave_gather32(Batch B, PhysW<float> P, Flow<float> W, WaveTables V)
+__global__ void __launch_bounds__(kCells<float, 0> * kSteps32) k_wave_gather32(Batch B, PhysW<float> P, Flow<float> W, WaveTables V)
 {
     using L = Lay<float, MEAN>;
-    constexpr int PA = L::PA, NC = L::NC;
+    constexpr int PA = L::PA, PB = L::PB, NC = L::NC;
     constexpr int NF = L::flow / 16, ND = L::dq / 16, stride = NF + ND + 1;      // quads per step, and in shared memory
     extern __shared__ __align__(128) char smem[];
     float4 *tile = (float4 *)smem;
@@ -618,12 +627,13 @@ __global__ void __launch_bounds__(kCells<float> * kSteps32) k_wave_gather32(Batc
 }
 
 // FP64: one thread per cell and step, 16 steps per block (a line of a column's row serves them from L1). Bound by its FP64 instructions, some 75 per cell.
+template <int N>
 __global__ void __launch_bounds__(256) k_wave_gather64(Batch B, PhysW<double> P, Flow<double> W, WaveTables V)
 {
-    using L = Lay<double, MEAN>;
-    constexpr int PA = L::PA, NC = L::NC;
+    using L = Lay<double, MEAN, N>;
+    constexpr int PA = L::PA, PB = L::PB, NC = L::NC;
     next_sweep(V);
-    const Chunk c = chunk_of(V, kSteps<double>);
+    const Chunk c = chunk_of(V, kSteps<double, N>);
     const int cell = threadIdx.x % NC, st = threadIdx.x / NC, a = cell / PB, b = cell % PB;
     if (!c.live || st >= c.nt) return;
     const Lvl Lv = B.lv[blockIdx.y];
@@ -673,13 +683,13 @@ __global__ void __launch_bounds__(256) k_wave_gather64(Batch B, PhysW<double> P,
 
 // inputs of the variable's sweep of one direction, from the mean flow's dQ of that direction: everything
 // that does not depend on the variable's own update
-template <typename T, int DIR>
+template <typename T, int DIR, int N>
 __global__ void __launch_bounds__(256) k_wave_var(Batch B, PhysW<T> P, Geo G, Flow<T> W, WaveTables V, WaveTables VV)
 {
-    using L = Lay<T, VAR>;
-    constexpr int PA = L::PA, NC = L::NC;
+    using L = Lay<T, VAR, N>;
+    constexpr int PA = L::PA, PB = L::PB, NC = L::NC;
     next_sweep(VV);
-    const Chunk c = chunk_of(V, kSteps<T>);
+    const Chunk c = chunk_of(V, kSteps<T, N>);
     const int cell = threadIdx.x % NC, st = threadIdx.x / NC, a = cell / PB, b = cell % PB;
     if (!c.live || st >= c.nt) return;
     const Lvl Lv = B.lv[blockIdx.y];
@@ -690,13 +700,13 @@ __global__ void __launch_bounds__(256) k_wave_var(Batch B, PhysW<T> P, Geo G, Fl
         return;
     }
     const long long p = ix(Lv, i, j, k);
-    const T *dq = (const T *)(V.dq + (c.step + st) * Lay<T, MEAN>::dq) + 4 * cell;
+    const T *dq = (const T *)(V.dq + (c.step + st) * Lay<T, MEAN, N>::dq) + 4 * cell;
     const double o0 = W.cv[0][p], o1 = W.cv[1][p], o2 = W.cv[2][p], o3 = W.cv[3][p];
     auto next = [&](double o, T q) { return to_work<T>(o + to_f64<T>(q)); };
     const T dn0 = next(o0, dq[0]), dn1 = next(o1, dq[1]), dn2 = next(o2, dq[2]), dn3 = next(o3, dq[3]);
     const T evo = to_work<T>(W.ev[p]);
     // the normals and areas as the mean flow's sweep has them
-    const T *geo = (const T *)(V.geo + (c.step + st) * Lay<T, MEAN>::geo), *area = (const T *)V.area + (c.step + st) * (3 * Lay<T, MEAN>::NC) + 3 * cell;
+    const T *geo = (const T *)(V.geo + (c.step + st) * Lay<T, MEAN, N>::geo), *area = (const T *)V.area + (c.step + st) * (3 * Lay<T, MEAN, N>::NC) + 3 * cell;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         const int g = 3 * cell + d;
@@ -721,10 +731,10 @@ __global__ void __launch_bounds__(256) k_wave_var(Batch B, PhysW<T> P, Geo G, Fl
 }
 
 // geometry of the steps (once per level): the mean normal, entrainment speed and area of each direction
-template <typename T>
+template <typename T, int N>
 __global__ void __launch_bounds__(256) k_wave_geometry(Batch B, Geo G, WaveTables V)
 {
-    constexpr int PA = kPA<T>, NC = kCells<T>;
+    constexpr int PA = kPA<T>, PB = kPB<T, N>, NC = kCells<T, N>;
     const WaveSolve S = V.solve[blockIdx.y];
     const Lvl Lv = B.lv[blockIdx.y];
     const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -735,7 +745,7 @@ __global__ void __launch_bounds__(256) k_wave_geometry(Batch B, Geo G, WaveTable
     const int i = (p / S.nPJ) * PA + a + 1, j = (p % S.nPJ) * PB + b + 1, k = t - a - b + 1;
     if (i > S.nI || j > S.nJ || k < 1 || k > S.nK) return;            // (the pool is zeroed)
     const long long x = ix(Lv, i, j, k);
-    char *o = V.geo + (S.step0 + st) * Lay<T, MEAN>::geo;
+    char *o = V.geo + (S.step0 + st) * Lay<T, MEAN, N>::geo;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         const T n0 = (T)G.cn[d][0][x], n1 = (T)G.cn[d][1][x], n2 = (T)G.cn[d][2][x], ve = (T)G.cve[d][x];
@@ -755,11 +765,11 @@ __global__ void __launch_bounds__(256) k_wave_geometry(Batch B, Geo G, WaveTable
 // and update, 0.214 as one; with runs of 16 or 32 k that start anywhere, 0.352 and 0.285.
 constexpr int kRun = 32;
 __host__ __device__ inline int runs_of(int nK) { return (nK + PAD) / kRun + 1; }
-template <typename T>
+template <typename T, int N>
 __global__ void __launch_bounds__(256) k_wave_update(Batch B, Phys P, Flow<T> W, WaveTables V, int level, LimitLists q)
 {
-    using L = Lay<T, MEAN>;
-    constexpr int PA = L::PA, NC = L::NC, R = NC * kRun / 256, NW = L::dq / 16, stride = NW + 1, ST = kRun + PA + PB - 2;
+    using L = Lay<T, MEAN, N>;
+    constexpr int PA = L::PA, PB = L::PB, NC = L::NC, R = NC * kRun / 256, NW = L::dq / 16, stride = NW + 1, ST = kRun + PA + PB - 2;
     __shared__ float4 tile[ST * stride];
     const int s = blockIdx.y;
     const WaveSolve S = V.solve[s];
@@ -807,16 +817,16 @@ __global__ void __launch_bounds__(256) k_wave_update(Batch B, Phys P, Flow<T> W,
     limit_done<T>(B, P, W, level, q, s, (unsigned)(S.nPI * S.nPJ * nr));
 }
 
-template <typename T>
+template <typename T, int N>
 __global__ void __launch_bounds__(256) k_wave_scatter_var(Batch B, Flow<T> W, WaveTables VV)
 {
-    constexpr int PA = kPA<T>, NC = kCells<T>;
-    const Chunk c = chunk_of(VV, kSteps<T>);
+    constexpr int PA = kPA<T>, PB = kPB<T, N>, NC = kCells<T, N>;
+    const Chunk c = chunk_of(VV, kSteps<T, N>);
     const int cell = threadIdx.x % NC, st = threadIdx.x / NC, a = cell / PB, b = cell % PB;
     if (!c.live || st >= c.nt) return;
     const int i = c.PI * PA + a + 1, j = c.PJ * PB + b + 1, k = c.t0 + st - a - b + 1;
     if (i > c.S.nI || j > c.S.nJ || k < 1 || k > c.S.nK) return;
-    W.dq_ev[ix(B.lv[blockIdx.y], i, j, k)] = ((const T *)(VV.dq + (c.step + st) * Lay<T, VAR>::dq))[cell];
+    W.dq_ev[ix(B.lv[blockIdx.y], i, j, k)] = ((const T *)(VV.dq + (c.step + st) * Lay<T, VAR, N>::dq))[cell];
 }
 
 constexpr unsigned kGatherBytes = kSteps32 * (Lay<float, MEAN>::flow + Lay<float, MEAN>::dq + 16);
@@ -824,31 +834,41 @@ constexpr unsigned kGatherBytes = kSteps32 * (Lay<float, MEAN>::flow + Lay<float
 // Shared memory of a block of the march. FP64: no more than two blocks on an SM, whose FP64 pipes they share:
 // further ones slow the tiles that the others wait for (forward sweep of four 129x49x49 passages 1110 us
 // with four blocks, 903 with two, 1012 with one; of one 161x65x65 passage 751, 751, 709).
-template <typename T, Kind K> constexpr int kMarchShared = sizeof(T) == 8 && Lay<T, K>::smem < 100000 ? 100000 : Lay<T, K>::smem;
+template <typename T, Kind K, int N> constexpr int kMarchShared = sizeof(T) == 8 && Lay<T, K, N>::smem < 100000 ? 100000 : Lay<T, K, N>::smem;
 
 // (shared memory beyond the default limit has to be asked for, once per kernel and device)
-template <typename T, Kind K>
+template <typename T, Kind K, int N>
 void allow_shared()
 {
-    cudaFuncSetAttribute(k_wave<T, 1, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMarchShared<T, K>);
-    cudaFuncSetAttribute(k_wave<T, -1, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMarchShared<T, K>);
+    cudaFuncSetAttribute(k_wave<T, 1, K, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMarchShared<T, K, N>);
+    cudaFuncSetAttribute(k_wave<T, -1, K, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMarchShared<T, K, N>);
 }
 
-template <typename T, int DIR, Kind K>
+template <typename T, int DIR, Kind K, int N>
 void march(const LaunchCtx &ctx, const WaveTables &V, T gm1)
 {
-    k_wave<T, DIR, K><<<V.n_item, 192, kMarchShared<T, K>, ctx.stream>>>(ctx.batch, V, gm1);
+    k_wave<T, DIR, K, N><<<V.n_item, 192, kMarchShared<T, K, N>, ctx.stream>>>(ctx.batch, V, gm1);
+}
+
+// f with the tiles' shape as a constant
+template <typename T, typename F>
+void with_shape(const WaveTables &V, F f)
+{
+    if constexpr (sizeof(T) == 8) {
+        if (V.narrow) return f(std::integral_constant<int, 1>{});
+    }
+    f(std::integral_constant<int, 0>{});
 }
 
 }  // namespace
 
-void wave_patch(int fp64, int &pa, int &pb)
+void wave_patch(int fp64, int narrow, int &pa, int &pb)
 {
     pa = fp64 ? kPA<double> : kPA<float>;
-    pb = PB;
+    pb = fp64 && narrow ? kPB<double, 1> : kPB<float, 0>;
 }
 
-void wave_bytes(int fp64, int sa, WaveBytes &w)
+void wave_bytes(int fp64, int narrow, int sa, WaveBytes &w)
 {
     auto set = [&](auto mean, auto var) {
         using L = decltype(mean);
@@ -856,28 +876,32 @@ void wave_bytes(int fp64, int sa, WaveBytes &w)
         w = {L::geo, L::flow, L::dq, L::pkt * 16, 3 * L::NC * L::B, 0, 0, 0};
         if (sa) { w.var_flow = X::flow; w.var_dq = X::dq; w.var_pkt = X::pkt * 16; }
     };
-    if (fp64) set(Lay<double, MEAN>{}, Lay<double, VAR>{});
+    if (fp64 && narrow) set(Lay<double, MEAN, 1>{}, Lay<double, VAR, 1>{});
+    else if (fp64) set(Lay<double, MEAN>{}, Lay<double, VAR>{});
     else set(Lay<float, MEAN>{}, Lay<float, VAR>{});
 }
 
 template <typename T>
 void launch_wave_geometry(const LaunchCtx &ctx, const Geo &G, const WaveTables &V)
 {
-    allow_shared<T, MEAN>();
-    allow_shared<T, VAR>();
     if (sizeof(T) == 4) cudaFuncSetAttribute(k_wave_gather32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGatherBytes);
-    k_wave_geometry<T><<<ctx.grid_n(V.max_steps * kCells<T>, 256), 256, 0, ctx.stream>>>(ctx.batch, G, V);
+    with_shape<T>(V, [&](auto shape) {
+        constexpr int N = decltype(shape)::value;
+        allow_shared<T, MEAN, N>();
+        allow_shared<T, VAR, N>();
+        k_wave_geometry<T, N><<<ctx.grid_n(V.max_steps * kCells<T, N>, 256), 256, 0, ctx.stream>>>(ctx.batch, G, V);
+    });
 }
 
-template <typename T>
-void launch_lusgs_sweeps(const LaunchCtx &ctx, const Phys &PH, const PhysW<T> &P, const Geo &G, Flow<T> W, const WaveTables &V,
+template <typename T, int N>
+static void sweeps(const LaunchCtx &ctx, const Phys &PH, const PhysW<T> &P, const Geo &G, Flow<T> W, const WaveTables &V,
                          const WaveTables &VV, int level, const LimitLists &q)
 {
     auto chunks = [&](int steps) { return dim3((unsigned)(V.max_tiles * ((V.max_T + steps - 1) / steps)), ctx.batch.nsolve); };
     ctx.mark("sweep_forward", 1, 2);
-    if constexpr (sizeof(T) == 4) k_wave_gather32<<<chunks(kSteps32), kCells<float> * kSteps32, kGatherBytes, ctx.stream>>>(ctx.batch, P, W, V);
-    else k_wave_gather64<<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, P, W, V);
-    march<T, 1, MEAN>(ctx, V, P.gm1);
+    if constexpr (sizeof(T) == 4) k_wave_gather32<<<chunks(kSteps32), kCells<float, 0> * kSteps32, kGatherBytes, ctx.stream>>>(ctx.batch, P, W, V);
+    else k_wave_gather64<N><<<chunks(kSteps<T, N>), 256, 0, ctx.stream>>>(ctx.batch, P, W, V);
+    march<T, 1, MEAN, N>(ctx, V, P.gm1);
     ctx.mark("sweep_forward", 0, 2);
     // The variable's sweep of a direction needs the mean flow's dQ of that direction and nothing of the other one,
     // nor of the update: its march, as the mean flow's bound by the chain of planes, runs beside them on the
@@ -895,25 +919,25 @@ void launch_lusgs_sweeps(const LaunchCtx &ctx, const Phys &PH, const PhysW<T> &P
     auto meet = [&] { if (ctx.side) cudaStreamWaitEvent(ctx.stream, ctx.join, 0); };
     if (W.ev) {
         ctx.mark("sa_sweeps", 1, 2);
-        k_wave_var<T, 1><<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
-        beside([&] { march<T, 1, VAR>(second, VV, (T)0); });
+        k_wave_var<T, 1, N><<<chunks(kSteps<T, N>), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
+        beside([&] { march<T, 1, VAR, N>(second, VV, (T)0); });
         ctx.mark("sa_sweeps", 0, 2);
     }
     ctx.mark("sweep_backward", 1, 1);
-    march<T, -1, MEAN>(ctx, V, P.gm1);
+    march<T, -1, MEAN, N>(ctx, V, P.gm1);
     ctx.mark("sweep_backward", 0, 1);
     if (W.ev) {
         ctx.mark("sa_sweeps", 1, 3);
         meet();
-        k_wave_var<T, -1><<<chunks(kSteps<T>), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
+        k_wave_var<T, -1, N><<<chunks(kSteps<T, N>), 256, 0, ctx.stream>>>(ctx.batch, P, G, W, V, VV);
         beside([&] {
-            march<T, -1, VAR>(second, VV, (T)0);
-            k_wave_scatter_var<T><<<chunks(kSteps<T>), 256, 0, second.stream>>>(ctx.batch, W, VV);
+            march<T, -1, VAR, N>(second, VV, (T)0);
+            k_wave_scatter_var<T, N><<<chunks(kSteps<T, N>), 256, 0, second.stream>>>(ctx.batch, W, VV);
         });
         ctx.mark("sa_sweeps", 0, 3);
     }
     ctx.mark("update_limiter", 1, 1);
-    k_wave_update<T><<<dim3((unsigned)(V.max_tiles * runs_of(ctx.maxKM - 1)), ctx.batch.nsolve), 256, 0, ctx.stream>>>(ctx.batch, PH, W, V, level, q);
+    k_wave_update<T, N><<<dim3((unsigned)(V.max_tiles * runs_of(ctx.maxKM - 1)), ctx.batch.nsolve), 256, 0, ctx.stream>>>(ctx.batch, PH, W, V, level, q);
     if (W.ev) {
         meet();
         // the variable's update and Limit_SA after the mean flow's (source/LU_SGS_Marching.cpp:275-277,
@@ -925,6 +949,13 @@ void launch_lusgs_sweeps(const LaunchCtx &ctx, const Phys &PH, const PhysW<T> &P
         }
     }
     ctx.mark("update_limiter", 0, 1);
+}
+
+template <typename T>
+void launch_lusgs_sweeps(const LaunchCtx &ctx, const Phys &PH, const PhysW<T> &P, const Geo &G, Flow<T> W, const WaveTables &V,
+                         const WaveTables &VV, int level, const LimitLists &q)
+{
+    with_shape<T>(V, [&](auto shape) { sweeps<T, decltype(shape)::value>(ctx, PH, P, G, W, V, VV, level, q); });
 }
 
 #define GBT_WAVE_INST(T)                                                                                              \
