@@ -79,9 +79,9 @@ __device__ __forceinline__ int jst_pos(int c, int NN) { return c <= 0 ? c - 1 : 
 // pressure sensor of every position -1 .. N + 1 of every line of direction F (sensorI/J/K, :5-190);
 // the k-direction sensor's range check compares j with KM, as the reference's does
 template <typename T, int F>
-__global__ void __launch_bounds__(256) k_jst_sensor(Batch B, Flow<T> W)
+__device__ __forceinline__ void jst_sensor(const Batch &B, const Flow<T> &W)
 {
-    const Lvl L = B.lv[blockIdx.y];
+    const Lvl L = B.lv[blockIdx.z];
     const int NN = F == 0 ? L.IM : (F == 1 ? L.JM : L.KM);
     const int n1 = F == 0 ? L.JM - 1 : L.IM - 1, n2 = F == 2 ? L.JM - 1 : L.KM - 1;
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -108,9 +108,9 @@ __global__ void __launch_bounds__(256) k_jst_sensor(Batch B, Flow<T> W)
 // anisotropy-weighted spectral radius phi * lambda of every cell and direction (:198-216); the
 // two other directions in the reference's order of the sum: I faces J, K; J faces I, K; K faces J, I
 template <typename T>
-__global__ void __launch_bounds__(256) k_jst_weights(Batch B, Flow<T> W)
+__device__ __forceinline__ void jst_weights(const Batch &B, const Flow<T> &W)
 {
-    const Lvl L = B.lv[blockIdx.y];
+    const Lvl L = B.lv[blockIdx.z];
     int i, j, k;
     if (!box_index(L.IM - 1, L.JM - 1, L.KM - 1, i, j, k)) return;
     const long long p = ix(L, i, j, k);
@@ -121,11 +121,21 @@ __global__ void __launch_bounds__(256) k_jst_weights(Batch B, Flow<T> W)
     W.jva[2][p] = ((T)1 + pow(l1 / l2, ex) + pow(l0 / l2, ex)) * l2;
 }
 
+// both in one launch, blockIdx.y the direction of the sensor or, first and longest (six FP64 powers a cell), the weights
+template <typename T>
+__global__ void __launch_bounds__(256) k_jst_cells(Batch B, Flow<T> W)
+{
+    if (blockIdx.y == 0) jst_weights<T>(B, W);
+    else if (blockIdx.y == 1) jst_sensor<T, 0>(B, W);
+    else if (blockIdx.y == 2) jst_sensor<T, 1>(B, W);
+    else jst_sensor<T, 2>(B, W);
+}
+
 // dissipation of one face: blended second and fourth differences of Q (:193-413)
 template <typename T, int F>
-__global__ void __launch_bounds__(128) k_jst_dissip(Batch B, Phys P, Flow<T> W)
+__device__ __forceinline__ void jst_dissip(const Batch &B, const Phys &P, const Flow<T> &W)
 {
-    const int s = blockIdx.y;
+    const int s = blockIdx.z;
     const Lvl L = B.lv[s];
     int ni, nj, nk, i, j, k;
     face_extent(L, F, ni, nj, nk);
@@ -152,6 +162,15 @@ __global__ void __launch_bounds__(128) k_jst_dissip(Batch B, Phys P, Flow<T> W)
     }
 #pragma unroll
     for (int c = 0; c < NQ; c++) W.Fd[F][c][p] = d[c];
+}
+// the three families (blockIdx.y); with the sensors and weights seven launches took 0.269 ms per cycle of the 65 x 33 x 25
+// passage on two levels, two take 0.219
+template <typename T>
+__global__ void __launch_bounds__(128) k_jst_dissip(Batch B, Phys P, Flow<T> W)
+{
+    if (blockIdx.y == 0) jst_dissip<T, 0>(B, P, W);
+    else if (blockIdx.y == 1) jst_dissip<T, 1>(B, P, W);
+    else jst_dissip<T, 2>(B, P, W);
 }
 
 // face sums, rotation source, residual R = Fc - Fv (- Fd with JST). The viscous and dissipation
@@ -213,18 +232,14 @@ void launch_resflux(const LaunchCtx &ctx, const Phys &P, const PhysW<T> &PC, con
     }
     ctx.mark("face_flux", 0, staged ? 3 : 1);
     if (P.scheme == 100) {
-        ctx.mark("jst_dissipation", 1, 7);
+        ctx.mark("jst_dissipation", 1, 2);
         const long long ls0 = (long long)(ctx.maxIM + 3) * (ctx.maxJM - 1) * (ctx.maxKM - 1);
         const long long ls1 = (long long)(ctx.maxJM + 3) * (ctx.maxIM - 1) * (ctx.maxKM - 1);
         const long long ls2 = (long long)(ctx.maxKM + 3) * (ctx.maxIM - 1) * (ctx.maxJM - 1);
-        k_jst_sensor<T, 0><<<ctx.grid_n(ls0, 256), 256, 0, ctx.stream>>>(B, W);
-        k_jst_sensor<T, 1><<<ctx.grid_n(ls1, 256), 256, 0, ctx.stream>>>(B, W);
-        k_jst_sensor<T, 2><<<ctx.grid_n(ls2, 256), 256, 0, ctx.stream>>>(B, W);
-        k_jst_weights<T><<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(B, W);
-        k_jst_dissip<T, 0><<<ctx.grid_faces(0, 128), 128, 0, ctx.stream>>>(B, P, W);
-        k_jst_dissip<T, 1><<<ctx.grid_faces(1, 128), 128, 0, ctx.stream>>>(B, P, W);
-        k_jst_dissip<T, 2><<<ctx.grid_faces(2, 128), 128, 0, ctx.stream>>>(B, P, W);
-        ctx.mark("jst_dissipation", 0, 7);
+        const unsigned nf = std::max({ctx.grid_faces(0, 128).x, ctx.grid_faces(1, 128).x, ctx.grid_faces(2, 128).x});
+        k_jst_cells<T><<<dim3(ctx.grid_n(std::max({ls0, ls1, ls2}), 256).x, 4, B.nsolve), 256, 0, ctx.stream>>>(B, W);
+        k_jst_dissip<T><<<dim3(nf, 3, B.nsolve), 128, 0, ctx.stream>>>(B, P, W);
+        ctx.mark("jst_dissipation", 0, 2);
     }
     ctx.mark("cell_sum", 1);
     const bool jst = W.Fd[0][0] != nullptr;
