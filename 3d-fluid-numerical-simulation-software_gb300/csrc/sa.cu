@@ -116,59 +116,60 @@ void launch_sa_init(const LaunchCtx &ctx, double *ev, double ev_ratio)
     k_sa_fill<<<ctx.grid_cells(256), 256, 0, ctx.stream>>>(ctx.batch, ev, ev_ratio);
 }
 
-// inlet: the ghost holds the configured ratio; outlet: the ghost copies the last cell
-__global__ void k_sa_bc_inout(Batch B, double *ev, const DevInOut *pat, int outlet, double ev_ratio)
+// Ghosts of the variable: the inlet's hold the configured ratio, the outlet's copy the last cell, the walls' are
+// zero, interfaces and periodic pairs copy their source. A part of the work per block (b: first block of the
+// outlets, of the walls and of the copies); one launch where no ghost cell belongs to two parts
+// (BcTables::apart), four in the reference's order where one does.
+struct SaParts { unsigned b[3], per_inlet, per_outlet, per_wall; };
+__global__ void __launch_bounds__(128) k_sa_bc(Batch B, double *ev, BcTables bc, SaParts n, double ev_ratio)
 {
-    const DevInOut pt = pat[blockIdx.y];
-    const Lvl L = B.lv[pt.solve];
-    if (outlet) {
-        const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned b = blockIdx.x;
+    if (b < n.b[0]) {
+        const DevInOut pt = bc.inlet[b / n.per_inlet];
+        const Lvl L = B.lv[pt.solve];
+        const int ni = pt.ie - pt.is + 1, nj = pt.je - pt.js + 1, t = (int)(b % n.per_inlet * 128 + threadIdx.x);
+        if (t >= ni * nj) return;
+        ev[ix(L, pt.is + t / nj, pt.js + t % nj, pt.ks == 1 ? 0 : L.KM)] = ev_ratio * (double)1.0f;
+    } else if (b < n.b[1]) {
+        b -= n.b[0];
+        const Lvl L = B.lv[bc.outlet[b / n.per_outlet].solve];
+        const int t = (int)(b % n.per_outlet * 128 + threadIdx.x);
         if (t >= (L.IM - 1) * (L.JM - 1)) return;
         const int i = 1 + t / (L.JM - 1), j = 1 + t % (L.JM - 1);
         ev[ix(L, i, j, L.KM)] = ev[ix(L, i, j, L.KM - 1)];
-        return;
+    } else if (b < n.b[2]) {
+        b -= n.b[1];
+        const DevWall wl = bc.wall[b / n.per_wall];
+        const Lvl L = B.lv[wl.solve];
+        const int ni = wl.ie - wl.is + 1, nj = wl.je - wl.js + 1, nk = wl.ke - wl.ks + 1, t = (int)(b % n.per_wall * 128 + threadIdx.x);
+        if (t >= ni * nj * nk) return;
+        const int f = (wl.face - 1) / 2;
+        const long long sn = f == 0 ? (long long)L.NJ * L.NK : (f == 1 ? (long long)L.NK : 1LL);
+        const long long fp = ix(L, wl.is + t / nk / nj, wl.js + t / nk % nj, wl.ks + t % nk);
+        ev[wl.face % 2 == 1 ? fp - sn : fp] = 0.0;
+    } else {
+        const long long t = (long long)(b - n.b[2]) * 128 + threadIdx.x;
+        if (t < bc.n_sa_gather) ev[bc.sa_dst[t]] = ev[bc.sa_src[t]];
     }
-    const int ni = pt.ie - pt.is + 1, nj = pt.je - pt.js + 1;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ni * nj) return;
-    const int i = pt.is + t / nj, j = pt.js + t % nj;
-    const int kv = pt.ks == 1 ? 0 : L.KM;
-    ev[ix(L, i, j, kv)] = ev_ratio * (double)1.0f;
-}
-
-__global__ void k_sa_bc_wall(Batch B, double *ev, const DevWall *walls)
-{
-    const DevWall wl = walls[blockIdx.y];
-    const Lvl L = B.lv[wl.solve];
-    const int ni = wl.ie - wl.is + 1, nj = wl.je - wl.js + 1, nk = wl.ke - wl.ks + 1;
-    int i, j, k;
-    if (!box_index(ni, nj, nk, i, j, k)) return;
-    i += wl.is - 1; j += wl.js - 1; k += wl.ks - 1;
-    const int f = (wl.face - 1) / 2;
-    const bool lo = wl.face % 2 == 1;
-    const long long sn = f == 0 ? (long long)L.NJ * L.NK : (f == 1 ? (long long)L.NK : 1LL);
-    const long long fp = ix(L, i, j, k);
-    ev[lo ? fp - sn : fp] = 0.0;
-}
-
-__global__ void k_sa_gather(double *ev, const long long *dst, const long long *src, long long n)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) ev[dst[t]] = ev[src[t]];
 }
 
 template <typename T>
 void launch_sa_boundary(const LaunchCtx &ctx, const Phys &P, Flow<T> W, const BcTables &bc)
 {
-    const Batch &B = ctx.batch;
-    if (bc.n_inlet)
-        k_sa_bc_inout<<<dim3((bc.max_inlet + 127) / 128, bc.n_inlet), 128, 0, ctx.stream>>>(B, W.ev, bc.inlet, 0, P.ev_ratio);
-    if (bc.n_outlet)
-        k_sa_bc_inout<<<dim3((bc.max_outlet_im * bc.max_outlet_jm + 127) / 128, bc.n_outlet), 128, 0, ctx.stream>>>(
-            B, W.ev, bc.outlet, 1, P.ev_ratio);
-    if (bc.n_wall) k_sa_bc_wall<<<dim3((bc.max_wall + 127) / 128, bc.n_wall), 128, 0, ctx.stream>>>(B, W.ev, bc.wall);
-    if (bc.n_sa_gather)
-        k_sa_gather<<<(unsigned)((bc.n_sa_gather + 255) / 256), 256, 0, ctx.stream>>>(W.ev, bc.sa_dst, bc.sa_src, bc.n_sa_gather);
+    const unsigned pi = (unsigned)(bc.max_inlet + 127) / 128, po = (unsigned)(bc.max_outlet_im * bc.max_outlet_jm + 127) / 128,
+                   pw = (unsigned)(bc.max_wall + 127) / 128;
+    auto fill = [&](unsigned i, unsigned o, unsigned w, unsigned g) {
+        if (i + o + w + g)
+            k_sa_bc<<<i + o + w + g, 128, 0, ctx.stream>>>(ctx.batch, W.ev, bc, SaParts{{i, i + o, i + o + w}, pi, po, pw}, P.ev_ratio);
+    };
+    const unsigned ni = pi * bc.n_inlet, no = po * bc.n_outlet, nw = pw * bc.n_wall, ng = (unsigned)((bc.n_sa_gather + 127) / 128);
+    if (bc.apart) fill(ni, no, nw, ng);
+    else {
+        fill(ni, 0, 0, 0);
+        fill(0, no, 0, 0);
+        fill(0, 0, nw, 0);
+        fill(0, 0, 0, ng);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
