@@ -134,17 +134,17 @@ def _write_sampled_case(job):
 # ---------------------------------------------------------------------------------------------
 # algorithmic bytes per kernel launch: each input/output element counted once, at the width the
 # kernel reads it ("w": the working precision, 8 B in FP64, 4 B in the mixed form, whose face and
-# sweep kernels read FP32 copies of the geometry; "int": 4 B). unit: "face" (faces of one family,
-# about one per cell), "plane_cell" (cells of one hyperplane)
+# sweep kernels read FP32 copies of the geometry; "int": 4 B). unit: "face" (a face of any family),
+# "cell" (a cell of one sweep)
 # ---------------------------------------------------------------------------------------------
 ALG = {
-    # S(3) s nrm(3) t1(3) t2(3) qe metrics(9) = 23 geometry; prim 6 + mu_t 1 of one cell; 10 fluxes
-    # out; the wall flag
-    "face_flux": {"unit": "face", "w": 40, "int": 1},
-    # plane-order copies: vol dt lamc(3) lamv(3) + res or dq (5) + neighbour cv(5) dq(5) p(1) + mean
-    # normal(3) area entrainment, per direction amortised to one cell: cn 9 cs 3 cve 3; dq out 5
-    "sweep_forward": {"unit": "plane_cell", "w": 45, "int": 0},
-    "sweep_backward": {"unit": "plane_cell", "w": 45, "int": 0},
+    # S(3) s nrm(3) t1(3) t2(3) qe metrics(9) = 23 geometry; prim 6 + mu_t 1 of one cell; 9 fluxes out
+    # (the viscous flux of mass is zero and not stored); the wall flag
+    "face_flux": {"unit": "face", "w": 39, "int": 1},
+    # vol dt lamc(3) lamv(3) + res or dq (5) + neighbour cv(5) dq(5) p(1) + mean normal(3) area
+    # entrainment, per direction amortised to one cell: cn 9 cs 3 cve 3; dq out 5
+    "sweep_forward": {"unit": "cell", "w": 45, "int": 0},
+    "sweep_backward": {"unit": "cell", "w": 45, "int": 0},
 }
 
 
@@ -836,7 +836,6 @@ def run_gpu(args, rank, world, dist):
         s.iterate(nprof, history=False)
         prof = s.profile_end()
         slot_dims = [[s.dims(q, l)[:3] for q in range(s.n_slots)] for l in range(1, s.ng + 1)]
-        tuning = {f"level{l}": list(s.sweep_tuning(l)) for l in range(1, s.ng + 1)}
         total_prof = sum(v[0] for v in prof.values())
         launches_per_step = sum(v[1] for v in prof.values()) / nprof
         dom = max((k for k in prof if k in ALG), key=lambda k: prof[k][0])
@@ -867,7 +866,7 @@ def run_gpu(args, rank, world, dist):
         counts = fp64_ops_per_unit().get(dom) if prec == gbturbo.FP64 else None
         if counts is not None:
             # the FP64 form is bound by the FP64 pipe: counted FP64 operations of the stage (ncu, per
-            # face or plane cell) over its device time, against the FP64 rate measured in this run.
+            # face or cell) over its device time, against the FP64 rate measured in this run.
             # DADD and DMUL hold the pipe as long as an FMA, so beside the FLOP fraction the line
             # gives the pipe's occupancy: FP64 instructions issued per second against the FMA-chain
             # loop's instructions per second (half its FLOP rate).
@@ -929,7 +928,6 @@ def run_gpu(args, rank, world, dist):
                         "h2d_bytes_per_step": int(grid_bytes / n_e2e), "d2h_bytes_per_step": 96 * nsolve},
                 "gpu_launches": int(round(launches_per_step * args.steps)),
                 "roofline": roofline,
-                "sweep_shape_cells_per_warp_warps_per_block": tuning,
                 "stages": stages,
                 "forms": forms,
                 "cpu_baseline": base,
