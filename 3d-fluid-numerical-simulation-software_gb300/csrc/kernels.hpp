@@ -101,7 +101,7 @@ struct WaveTables {
     void *area = nullptr;                          // mean area per cell and direction
     uint4 *pkt = nullptr;                          // terms that cross from tile to tile
 };
-// columns of a tile in i and j; bytes of a step's blocks (fp64: working type; narrow: half as wide in j, FP64 only;
+// columns of a tile in i and j; bytes of a step's blocks (fp64: working type; narrow: the form for small grids, in FP64 half as wide in j;
 // sa: with the Spalart-Allmaras variable)
 void wave_patch(int fp64, int narrow, int &pa, int &pb);
 void wave_bytes(int fp64, int narrow, int sa, WaveBytes &w);

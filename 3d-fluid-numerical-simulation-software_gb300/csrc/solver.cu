@@ -858,16 +858,17 @@ public:
         WaveTables &V = Lv.wave;
         const bool sa = P.turb_sa && l == 1;
         int pa, pb;
-        // FP64: narrow tiles where the GPU has an SM for each of them (a step is what one warp issues, and narrow
-        // tiles spread a cell over twice the lanes: cycle of the 65x33x33 duct, 128 of them, 0.712 and 0.651 ms; two on
-        // an SM share its FP64 pipes: forward sweeps of the 129x49x49 passage, 288 of them, 0.526 and 0.590 ms)
+        // the form for small grids where the GPU has an SM for each tile (a step is what one warp issues: narrow FP64
+        // tiles spread a cell over twice the lanes: cycle of the 65x33x33 duct, 128 of them, 0.712 and 0.651 ms;
+        // two on an SM share its FP64 pipes: forward sweeps of the 129x49x49 passage, 288 of them, 0.526
+        // and 0.590 ms)
         wave_patch(sizeof(T) == 8, 1, pa, pb);
         int dev = 0, n_sm = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
         long long tiles = 0;
         for (int s = 0; s < nsolve; s++) tiles += (long long)((Lv.lv[s].IM - 2 + pa) / pa) * ((Lv.lv[s].JM - 2 + pb) / pb);
-        V.narrow = sizeof(T) == 8 && tiles <= n_sm;
+        V.narrow = tiles <= n_sm;
         wave_patch(sizeof(T) == 8, V.narrow, pa, pb);
         WaveBytes w;
         wave_bytes(sizeof(T) == 8, V.narrow, sa, w);

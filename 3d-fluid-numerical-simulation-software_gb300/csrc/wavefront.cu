@@ -56,10 +56,14 @@ namespace gbt {
 
 namespace {
 
-// columns of a tile in i and j, lanes of a cell: 128 lanes a step in both precisions. N = 1 (FP64): narrow tiles of
-// 2 x 4 columns with sixteen lanes a cell, one term to a lane (18 FP64 instructions a step instead of 22).
+// columns of a tile in i and j, lanes of a cell: 128 lanes a step in both precisions. N = 1 is the form for grids of
+// which every tile has an SM: in FP64 narrow tiles of 2 x 4 columns with sixteen lanes a cell, one term to
+// a lane (18 FP64 instructions a step instead of 22); in FP32 a step's inputs are read, and the old
+// fluxes formed, during the step before, where they fill the gaps of its chain (cycle of the 129x49x49
+// passage 0.672 and 0.660 ms; 12 solves on three meshes, whose SMs have several tiles to fill them with,
+// 3.844 and 3.867).
 template <typename T> constexpr int kPA = sizeof(T) == 4 ? 4 : 2;
-template <typename T, int N> constexpr int kPB = N ? 4 : 8;
+template <typename T, int N> constexpr int kPB = N && sizeof(T) == 8 ? 4 : 8;
 template <typename T, int N> constexpr int kCells = kPA<T> * kPB<T, N>;
 template <typename T, int N> constexpr int kLanes = 128 / kCells<T, N>;
 constexpr int kGroup = 2, kStages = 3;          // steps of a stage of the input ring, stages
@@ -189,15 +193,15 @@ template <class L> __device__ __forceinline__ int off_jb(int a, int col) { retur
 // rd: the slot of the last step, wr: this step's
 template <typename T, int DIR, Kind K, int N> struct CellStep;
 
-template <int DIR> struct CellStep<float, DIR, MEAN, 0> {
-    using L = Lay<float, MEAN>;
+template <int DIR, int FORM> struct CellStep<float, DIR, MEAN, FORM> {
+    using L = Lay<float, MEAN, FORM>;
     static __device__ __forceinline__ float dot(float a0, float a1, float a2, float b0, float b1, float b2)
     {
         return __fmaf_rn(a2, b2, __fmaf_rn(a0, b0, __fmul_rn(a1, b1)));
     }
     static constexpr int NC = L::NC;
-    static __device__ __forceinline__ void run(const char *in, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
-                                               int w_off4, bool active, float gm1, char *dq_out)
+    struct Pre { float4 N, o, x; float2 hc; float rq, r4, f0, f1, f2, f3, f4; };
+    static __device__ __forceinline__ Pre pre(const char *in, int cell, int q)
     {
         const int e = 3 * cell + (q < 3 ? q : 0);
         const float4 N = ((const float4 *)in)[e];
@@ -210,6 +214,14 @@ template <int DIR> struct CellStep<float, DIR, MEAN, 0> {
         const float vo = dot(__fmul_rn(o.y, x.z), __fmul_rn(o.z, x.z), __fmul_rn(o.w, x.z), N.x, N.y, N.z), dv = __fadd_rn(vo, -N.w);
         const float f0 = __fmul_rn(o.x, dv), f1 = __fmaf_rn(o.y, dv, __fmul_rn(x.y, N.x)), f2 = __fmaf_rn(o.z, dv, __fmul_rn(x.y, N.y)),
                     f3 = __fmaf_rn(o.w, dv, __fmul_rn(x.y, N.z)), f4 = __fmaf_rn(x.y, N.w, __fmul_rn(__fadd_rn(x.x, x.y), dv));
+        return {N, o, x, hc, rq, r4, f0, f1, f2, f3, f4};
+    }
+    static __device__ __forceinline__ void run(const Pre &p, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
+                                               int w_off4, bool active, float gm1, char *dq_out)
+    {
+        const float4 N = p.N, o = p.o, x = p.x;
+        const float2 hc = p.hc;
+        const float rq = p.rq, r4 = p.r4, f0 = p.f0, f1 = p.f1, f2 = p.f2, f3 = p.f3, f4 = p.f4;
         // received
         const float sq = __fadd_rn(__fadd_rn(((const float *)(rd + r_off[0]))[q], ((const float *)(rd + r_off[2]))[q]),
                                    ((const float *)(rd + L::KA))[4 * cell + q]);
@@ -246,8 +258,8 @@ template <int DIR, int N> struct CellStep<double, DIR, MEAN, N> {
     using L = Lay<double, MEAN, N>;
     static constexpr int lanes = kLanes<double, N>;
     static constexpr int NC = L::NC;
-    static __device__ __forceinline__ void run(const char *in, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
-                                               int w_off4, bool active, double gm1, char *dq_out)
+    struct Pre { double2 g0, g1, ha, hb; double fa, fb, o, r, ka, kb; };
+    static __device__ __forceinline__ Pre pre(const char *in, int cell, int q)
     {
         const int d = q & 3, c = q < 4 ? q : 4, e = 3 * cell + (d < 3 ? d : 0);     // direction, component received
         const bool low = q < 4;
@@ -262,6 +274,15 @@ template <int DIR, int N> struct CellStep<double, DIR, MEAN, N> {
         double2 hb = make_double2(0.0, 0.0);
         double fb = 0.0, kb = 0.0;
         if (lanes == 8) { hb = ((const double2 *)own)[3 * cell + d1]; fb = ((const double *)mid)[3 * (NC * c1 + cell) + d1]; kb = coef(d1, c1); }
+        return {g0, g1, ha, hb, fa, fb, o, r, ka, kb};
+    }
+    static __device__ __forceinline__ void run(const Pre &p, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
+                                               int w_off4, bool active, double gm1, char *dq_out)
+    {
+        const int d = q & 3, c = q < 4 ? q : 4, t0 = min(q, 14), d0 = t0 / 5, c0 = t0 % 5, t1 = min(q + 8, 14), d1 = t1 / 5, c1 = t1 % 5;
+        const bool low = q < 4;
+        const double2 g0 = p.g0, g1 = p.g1, ha = p.ha, hb = p.hb;
+        const double fa = p.fa, fb = p.fb, o = p.o, r = p.r, ka = p.ka, kb = p.kb;
         // received
         const double s = __dadd_rn(__dadd_rn(*(const double *)(rd + r_off[0]), *(const double *)(rd + r_off[1])), *(const double *)(rd + r_off[2]));
         const double x = __dadd_rn(r, DIR > 0 ? s : -s), dq = active ? x : 0.0, nq = __dadd_rn(o, dq);
@@ -295,12 +316,16 @@ template <typename T, int DIR, int N> struct CellStep<T, DIR, VAR, N> {
     static constexpr int NC = L::NC;
     static __device__ __forceinline__ T add(T a, T b) { if constexpr (sizeof(T) == 4) return __fadd_rn(a, b); else return __dadd_rn(a, b); }
     static __device__ __forceinline__ T mul(T a, T b) { if constexpr (sizeof(T) == 4) return __fmul_rn(a, b); else return __dmul_rn(a, b); }
-    static __device__ __forceinline__ void run(const char *in, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
-                                               int, bool active, T, char *dq_out)
+    struct Pre { T vn, eb, sd, rl, lv, ev, alpha, r; };
+    static __device__ __forceinline__ Pre pre(const char *in, int cell, int q)
     {
         const T *f = (const T *)in, *v = f + 3 * cell + (q < 3 ? q : 0);
-        const T vn = v[0], eb = v[3 * NC], sd = v[6 * NC], rl = v[9 * NC], lv = v[12 * NC], ev = f[15 * NC + cell],
-                alpha = f[16 * NC + cell], r = ((const T *)(in + L::flow_in))[cell];
+        return {v[0], v[3 * NC], v[6 * NC], v[9 * NC], v[12 * NC], f[15 * NC + cell], f[16 * NC + cell], ((const T *)(in + L::flow_in))[cell]};
+    }
+    static __device__ __forceinline__ void run(const Pre &p, const char *rd, char *wr, int cell, int q, const int r_off[4], int w_off,
+                                               int, bool active, T, char *dq_out)
+    {
+        const T vn = p.vn, eb = p.eb, sd = p.sd, rl = p.rl, lv = p.lv, ev = p.ev, alpha = p.alpha, r = p.r;
         const T *i = (const T *)(rd + r_off[0]), *j = (const T *)(rd + r_off[2]), *k = (const T *)(rd + L::KA) + 2 * cell;
         T t = DIR > 0 ? r : mul(alpha, r);
         t = DIR > 0 ? add(add(add(t, i[0]), j[0]), k[0]) : add(add(add(t, -i[0]), -j[0]), -k[0]);
@@ -364,26 +389,57 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
         unsigned ph = 0;
         int slot = 0, stage = 0;
         const char *rd = terms + (kSlots - 1) * L::slot;
-        for (int n = 0; n < T_; n += kGroup) {
-            bar_wait(full + 8 * stage, ph, ok);
-            const char *in = smem + stage * kGroup * L::step;
-            // (a stage holds its steps in order of t; the last one may hold fewer)
-            const int cnt = min(kGroup, T_ - n);
-#pragma unroll
-            for (int u = 0; u < kGroup; u++) {
-                if (u >= cnt) break;
+        using Step = CellStep<T, DIR, K, N>;
+        if constexpr (sizeof(T) == 4 && K == MEAN && N) {
+            auto input = [&](int st, int n) {            // (a stage holds its steps in order of t; the last one may hold fewer)
+                const int u = n % kGroup, cnt = min(kGroup, T_ - (n - u));
+                return smem + st * kGroup * L::step + (DIR > 0 ? u : cnt - 1 - u) * L::step;
+            };
+            bar_wait(full, 0, ok);
+            typename Step::Pre now = Step::pre(input(0, 0), cell, q);
+            for (int n = 0; n < T_; n++) {
+                // the stage of the next step, and its phase
+                const bool turn = (n + 1) % kGroup == 0;
+                int next = stage;
+                unsigned next_ph = ph;
+                if (turn && ++next == kStages) { next = 0; next_ph ^= 1; }
+                if (turn && n + 1 < T_) bar_wait(full + 8 * next, next_ph, ok);
                 if (edges) bar_wait(edge + 8 * slot, ph, ok);
+                const typename Step::Pre then = Step::pre(input(next, min(n + 1, T_ - 1)), cell, q);
                 char *wr = terms + slot * L::slot;
-                CellStep<T, DIR, K, N>::run(in + (DIR > 0 ? u : cnt - 1 - u) * L::step, rd, wr, cell, q, r_off, w_off, w_off4,
-                                         column && (unsigned)k < (unsigned)w.S.nK, gm1, dq);
+                Step::run(now, rd, wr, cell, q, r_off, w_off, w_off4, column && (unsigned)k < (unsigned)w.S.nK, gm1, dq);
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (threadIdx.x == 0) bar_arrive(done + 8 * slot);
+                now = then;
                 rd = wr;
                 k += DIR;
                 dq += DIR * L::dq;
-                slot++;
+                if (++slot == kSlots) slot = 0;
+                stage = next;
+                ph = next_ph;
             }
-            if (++stage == kStages) { stage = slot = 0; ph ^= 1; }
+        } else {
+            for (int n = 0; n < T_; n += kGroup) {
+                bar_wait(full + 8 * stage, ph, ok);
+                const char *in = smem + stage * kGroup * L::step;
+                // (a stage holds its steps in order of t; the last one may hold fewer)
+                const int cnt = min(kGroup, T_ - n);
+#pragma unroll
+                for (int u = 0; u < kGroup; u++) {
+                    if (u >= cnt) break;
+                    if (edges) bar_wait(edge + 8 * slot, ph, ok);
+                    char *wr = terms + slot * L::slot;
+                    Step::run(Step::pre(in + (DIR > 0 ? u : cnt - 1 - u) * L::step, cell, q), rd, wr, cell, q, r_off, w_off, w_off4,
+                              column && (unsigned)k < (unsigned)w.S.nK, gm1, dq);
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    if (threadIdx.x == 0) bar_arrive(done + 8 * slot);
+                    rd = wr;
+                    k += DIR;
+                    dq += DIR * L::dq;
+                    slot++;
+                }
+                if (++stage == kStages) { stage = slot = 0; ph ^= 1; }
+            }
         }
     } else if (warp == 4) {
         if (!edges) return;
@@ -854,10 +910,8 @@ void march(const LaunchCtx &ctx, const WaveTables &V, T gm1)
 template <typename T, typename F>
 void with_shape(const WaveTables &V, F f)
 {
-    if constexpr (sizeof(T) == 8) {
-        if (V.narrow) return f(std::integral_constant<int, 1>{});
-    }
-    f(std::integral_constant<int, 0>{});
+    if (V.narrow) f(std::integral_constant<int, 1>{});
+    else f(std::integral_constant<int, 0>{});
 }
 
 }  // namespace
