@@ -1052,6 +1052,9 @@ struct WarmStart::Impl {
     void features(const float *feat, long long r0, long long M, cudaStream_t q)
     {
         const float *x = feat + r0 * kWsIn;
+        // (a caller's wrong pointer or count ends here, on the host, and not in a kernel that reads it)
+        (void)*(volatile const float *)x;
+        (void)*(volatile const float *)(x + M * kWsIn - 1);
         if (!host_rows) {
             if (!F) F = af(kPiece * kWsIn);
             WCK(cudaMemcpyAsync(F, x, sizeof(float) * (size_t)M * kWsIn, cudaMemcpyHostToDevice, q));
