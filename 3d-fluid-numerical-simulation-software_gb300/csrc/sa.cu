@@ -11,7 +11,7 @@
 //    the source term, the residual Res_ev = Cell_Fc_tur - Cell_Fv_tur
 //    (source/ComputeAllBlockVars.cpp:109-113, 237-249), and mu_t of the ghost layer;
 //  - the variable's LU-SGS sweeps (source/LU_SGS_Marching.cpp:76-258, delt_Fn_up/down :293-419)
-//    as a scalar hyperplane chain after each of the mean-flow sweeps, whose dQ it reads;
+//    as a scalar sweep after each of the mean-flow sweeps, whose dQ it reads;
 //  - its update and limiter (source/LU_SGS_Marching.cpp:262-287, CFluidProps::Limit_SA,
 //    source/Limit_FlowVars.cpp:122-166).
 // The reference's quirks are kept: the I-face viscous flux uses the x derivative for all three
