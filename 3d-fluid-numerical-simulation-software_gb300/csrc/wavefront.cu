@@ -50,6 +50,7 @@
 #include "kernels.hpp"
 #include "flux.cuh"
 #include "update.cuh"
+#include "ring_feed.hpp"
 #include <type_traits>
 
 namespace gbt {
@@ -524,10 +525,11 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
             }
         }
     } else {
-        // inputs of group g of steps into its stage
-        const int groups = (T_ + kGroup - 1) / kGroup;
-        auto fetch = [&](int g) {
-            const int n = g * kGroup, cnt = min(kGroup, T_ - n), stage = g % kStages;
+        // inputs of a group of steps into its stage, on lane 0
+        RingFeed<kStages> feed{(T_ + kGroup - 1) / kGroup};
+        auto landed = [&](int stage, unsigned parity) { bar_wait(full + 8 * stage, parity, ok); return ok; };
+        auto fetch = [&](int g, int stage) {
+            const int n = g * kGroup, cnt = min(kGroup, T_ - n);
             const long long t = w.step0 + (DIR > 0 ? n : T_ - n - cnt);
             const unsigned bar = full + 8 * stage, d = base + stage * kGroup * L::step;
             bar_expect(bar, cnt * L::step);
@@ -539,7 +541,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
             }
         };
         if (lane == 0)
-            for (int g = 0; g < kStages && g < groups; g++) fetch(g);
+            for (int s = 0; s < kStages; s++) feed.next(ok, landed, fetch);
         constexpr int RND = (L::pkt + 31) / 32;
         int from[RND];
         bool mine[RND];
@@ -582,15 +584,17 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
             }
             dst += DIR * L::pkt;
             __syncwarp();
-            if ((n + 1) % kGroup == 0 && lane == 0 && n / kGroup + kStages < groups) fetch(n / kGroup + kStages);
+            if ((n + 1) % kGroup == 0 && lane == 0) feed.next(ok, landed, fetch);
             if (++slot == kSlots) { slot = 0; ph ^= 1; }
         }
-        // no copy is in flight when the block ends, whatever happened
-        bool last = true;
-        for (int g = max(0, groups - kStages); g < groups; g++) bar_wait(full + 8 * (g % kStages), (g / kStages) & 1, last);
-        ok = ok && last;
+        // no copy is in flight when the block ends, also where a wait ran out
+        if (lane == 0) {
+            bool last = true;
+            feed.drain([&](int stage, unsigned parity) { bar_wait(full + 8 * stage, parity, last); });
+            ok = ok && last;
+        }
     }
-    if (!ok && lane == 0) atomicOr(&B.st[w.slot].status, GBT_STATUS_WAIT_TIMEOUT);
+    if (!ok) atomicOr(&B.st[w.slot].status, GBT_STATUS_WAIT_TIMEOUT);
 }
 
 // ---- into step order: everything a cell contributes without its neighbours. Cells outside the solve's
