@@ -171,12 +171,14 @@ inline PhysW<T> phys_working(const Phys &P)
     return w;
 }
 
-// Status bits reported per solve.
+// Status bits reported per solve. Kernels of two streams set them side by side (a march of the Spalart-Allmaras
+// variable beside the update), so they change a status word by atomic operations only.
 enum {
     GBT_STATUS_NAN = 1,          // a residual norm or an integral is not finite
     GBT_STATUS_LIMITER = 2,      // the positivity limiter replaced cells in the last step
     GBT_STATUS_LIMITER_OVF = 4,  // more limited cells than the list holds (processed by a full scan)
-    GBT_STATUS_WAIT_TIMEOUT = 8, // a kernel's bounded wait for its own asynchronous copies ran out
+    GBT_STATUS_WAIT_TIMEOUT = 8, // a kernel's bounded wait ran out: for its own asynchronous copies (staged faces,
+                                 // sweeps) or for another tile's terms (sweeps)
 };
 
 // an FP64 value in the working precision, and a working-precision value in FP64, with the

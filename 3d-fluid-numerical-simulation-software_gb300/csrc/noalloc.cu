@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256) k_norm_onepass(Batch B, Geo G, Flow<T> W,
     for (int q = sc.lead; q < sc.lead + sc.nblk; q++) B.st[q].res[threadIdx.x] = v;
     norms[sc.cix * 5 + threadIdx.x] = v;
     if (threadIdx.x == 0) {
-        if (!isfinite(v)) B.st[sc.lead].status |= GBT_STATUS_NAN;
+        if (!isfinite(v)) atomicOr(&B.st[sc.lead].status, GBT_STATUS_NAN);
         arrivals[sc.lead] = 0u;
     }
 }

@@ -115,7 +115,7 @@ __device__ __noinline__ void limit_cells(const Batch &B, const Phys &P, const Fl
         W.cv[4][p] = pr / (P.gamma - 1.0) + d * (u * u + v * v + w * w) / 2.0;
     }
     B.st[s].flag_low_dt[level] = 10;
-    B.st[s].status |= GBT_STATUS_LIMITER | (full ? GBT_STATUS_LIMITER_OVF : 0);
+    atomicOr(&B.st[s].status, GBT_STATUS_LIMITER | (full ? GBT_STATUS_LIMITER_OVF : 0));
     B.st[s].limiter_hits += n;
 }
 
@@ -134,7 +134,7 @@ __device__ __forceinline__ void limit_done(const Batch &B, const Phys &P, const 
 {
     if (!P.limiter || !last_block(q.done + s, blocks) || threadIdx.x != 0) return;
     const int n = q.count[s];
-    if (n == 0) { B.st[s].status &= ~GBT_STATUS_LIMITER; return; }
+    if (n == 0) { atomicAnd(&B.st[s].status, ~GBT_STATUS_LIMITER); return; }
     q.count[s] = 0;
     limit_cells<T>(B, P, W, level, s, q.list, q.cap, n);
 }
