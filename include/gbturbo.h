@@ -87,7 +87,9 @@ int gb_integrals(gb_solver *h, int level, double *out);
  * iter, Res(dens,xmom,ymom,zmom,ener), m_in, m_out, PR, eta, m_ratio, CFL. */
 int gb_iterate(gb_solver *h, int n, double *hist);
 /* per-solve status words (bit 1: non-finite residual or integral, bit 2: limiter active in the
- * last step, bit 4: limiter list overflow); out[n_solves] */
+ * last step, bit 4: limiter list overflow, bit 8: a kernel's bounded wait for its copies or, in
+ * the sweeps, for another tile's terms ran out: the solve's fields are not to be used from then on.
+ * The calls that iterate return GB_OK all the same; bits 1, 4 and 8 stay set); out[n_solves] */
 int gb_get_status(gb_solver *h, int *out);
 
 /* Copies a named array of one slot (block) and level to out (row-major, components fastest):

@@ -1,10 +1,20 @@
-"""The solves' status words: device code changes them by atomic operations only (kernels of two streams set bits of one
-word side by side)."""
+"""The solves' status words: every bit that a kernel may set is described in the public header, and device code changes
+the words by atomic operations only (kernels of two streams set bits of one word side by side)."""
 import glob
 import os
 import re
 
-from conftest import PKG
+from conftest import PKG, ROOT
+
+
+def test_header_describes_every_bit():
+    common = open(os.path.join(PKG, "csrc", "gbt_common.cuh")).read()
+    bits = re.findall(r"GBT_STATUS_\w+ = (\d+)", common)
+    assert len(bits) == 4
+    header = open(os.path.join(ROOT, "include", "gbturbo.h")).read()
+    text = re.search(r"/\*((?:(?!\*/).)*?)\*/\s*int gb_get_status", header, re.S).group(1)
+    missing = [b for b in bits if not re.search(rf"\bbit {b}\b", text)]
+    assert not missing
 
 
 def test_status_words_are_changed_atomically():
