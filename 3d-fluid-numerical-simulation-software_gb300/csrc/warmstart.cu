@@ -13,6 +13,7 @@
 // tcgen05.ld (warp w owns TMEM lanes 32w..32w+31, i.e. rows 32w..32w+31 of the tile).
 #include "warmstart.hpp"
 #include "gbt_common.cuh"
+#include "host_rows.hpp"
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -1052,9 +1053,7 @@ struct WarmStart::Impl {
     void features(const float *feat, long long r0, long long M, cudaStream_t q)
     {
         const float *x = feat + r0 * kWsIn;
-        // (a caller's wrong pointer or count ends here, on the host, and not in a kernel that reads it)
-        (void)*(volatile const float *)x;
-        (void)*(volatile const float *)(x + M * kWsIn - 1);
+        read_every_page(x, sizeof(float) * (size_t)M * kWsIn);
         if (!host_rows) {
             if (!F) F = af(kPiece * kWsIn);
             WCK(cudaMemcpyAsync(F, x, sizeof(float) * (size_t)M * kWsIn, cudaMemcpyHostToDevice, q));
