@@ -1048,13 +1048,20 @@ struct WarmStart::Impl {
             k_ws_weights_bf16<<<(kN[l] * kK[l] + 255) / 256, 256, 0, st>>>(P + w_off(l), kN[l], kK[l], Wb[l], Wt[l]);
     }
 
-    // features of M host rows from row r0 on into X0, on stream q: read by the kernel where the device reaches
-    // pageable memory through the host's page tables, copied first where it does not
-    void features(const float *feat, long long r0, long long M, cudaStream_t q)
+    // Whether the device is to read the rows at feat where they are: host memory, where it reaches that through the
+    // host's page tables. Rows in device or managed memory are copied, as the host cannot look at them first.
+    bool in_place(const float *feat) const
+    {
+        cudaPointerAttributes a{};
+        WCK(cudaPointerGetAttributes(&a, feat));
+        return host_rows && a.type != cudaMemoryTypeDevice && a.type != cudaMemoryTypeManaged;
+    }
+    // features of the caller's M rows from row r0 on into X0, on stream q
+    void features(const float *feat, long long r0, long long M, bool direct, cudaStream_t q)
     {
         const float *x = feat + r0 * kWsIn;
-        read_every_page(x, sizeof(float) * (size_t)M * kWsIn);
-        if (!host_rows) {
+        if (direct) read_every_page(x, sizeof(float) * (size_t)M * kWsIn);
+        else {
             if (!F) F = af(kPiece * kWsIn);
             WCK(cudaMemcpyAsync(F, x, sizeof(float) * (size_t)M * kWsIn, cudaMemcpyHostToDevice, q));
             x = F;
@@ -1446,12 +1453,13 @@ void WarmStart::forward(const float *feat, int M, float *y)
     const bool apart = ya + sizeof(float) * (size_t)M * kWsOut <= fa || fa + sizeof(float) * (size_t)M * kWsIn <= ya;
     const long long np = (M + kPiece - 1) / kPiece;
     auto rows = [&](long long p) { return std::min(kPiece, M - p * kPiece); };
+    const bool direct = m.in_place(feat);
     auto ask = [&](long long p) {
         if (p >= np) return;
-        m.features(feat, p * kPiece, rows(p), m.st2);
+        m.features(feat, p * kPiece, rows(p), direct, m.st2);
         WCK(cudaEventRecord(m.asked[p % 3], m.st2));
     };
-    if (np == 1) m.features(feat, 0, M, m.st);
+    if (np == 1) m.features(feat, 0, M, direct, m.st);
     else for (long long p = 0; p < 2; p++) ask(p);
     auto give = [&](long long p) {
         const long long o = apart ? p * kPiece * kWsOut : 0, n = apart ? rows(p) : p == np - 1 ? M : 0;
@@ -1482,7 +1490,8 @@ float WarmStart::forward_backward(const float *feat, const float *target, int M,
         Impl &m;
         ~Done() { cudaStreamSynchronize(m.st); }
     } done{m};                                            // the kernels read the caller's rows
-    for (long long r0 = 0; r0 < M; r0 += kPiece) m.features(feat, r0, std::min<long long>(kPiece, M - r0), m.st);
+    const bool direct = m.in_place(feat);
+    for (long long r0 = 0; r0 < M; r0 += kPiece) m.features(feat, r0, std::min<long long>(kPiece, M - r0), direct, m.st);
     for (int r = 0; r < M; r++)
         for (int o = 0; o < kWsOutUsed; o++) t8[(size_t)r * 8 + o] = target[(size_t)r * kWsOutUsed + o];
     WCK(cudaMemcpyAsync(m.T, t8.data(), sizeof(float) * t8.size(), cudaMemcpyHostToDevice, m.st));
