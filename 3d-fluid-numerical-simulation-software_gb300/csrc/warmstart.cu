@@ -980,7 +980,7 @@ static size_t b_off(int l) { return w_off(l) + (size_t)kN[l] * kK[l]; }
 
 struct WarmStart::Impl {
     cudaStream_t st = nullptr, st2 = nullptr, st3 = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr, asked[3] = {}, made[2] = {};
+    cudaEvent_t fork = nullptr, join = nullptr, caller = nullptr, asked[3] = {}, made[2] = {};
     int n_sm = 0;
     float *P = nullptr, *G = nullptr, *Mo = nullptr, *Vo = nullptr;
     bf16 *Wb[kWsLayers] = {}, *Wt[kWsLayers] = {};
@@ -1056,6 +1056,14 @@ struct WarmStart::Impl {
         WCK(cudaPointerGetAttributes(&a, feat));
         return host_rows && a.type != cudaMemoryTypeDevice && a.type != cudaMemoryTypeManaged;
     }
+    // what the caller has under way on the default stream and the streams that it waits for, which may still
+    // write the rows
+    void after_caller(cudaStream_t q)
+    {
+        WCK(cudaEventRecord(caller, cudaStreamLegacy));
+        WCK(cudaStreamWaitEvent(q, caller, 0));
+    }
+
     // features of the caller's M rows from row r0 on into X0, on stream q
     void features(const float *feat, long long r0, long long M, bool direct, cudaStream_t q)
     {
@@ -1184,6 +1192,7 @@ WarmStart::WarmStart(unsigned seed) : d(new Impl)
     d->host_rows = reach && tables;
     WCK(cudaEventCreateWithFlags(&d->fork, cudaEventDisableTiming));
     WCK(cudaEventCreateWithFlags(&d->join, cudaEventDisableTiming));
+    WCK(cudaEventCreateWithFlags(&d->caller, cudaEventDisableTiming));
     WCK(cudaStreamCreateWithFlags(&d->st3, cudaStreamNonBlocking));
     for (auto &e : d->made) WCK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto &e : d->asked) WCK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1239,6 +1248,7 @@ WarmStart::~WarmStart()
     cudaStreamDestroy(d->st2);
     cudaEventDestroy(d->fork);
     cudaEventDestroy(d->join);
+    cudaEventDestroy(d->caller);
     for (auto e : d->asked) cudaEventDestroy(e);
     for (auto e : d->made) cudaEventDestroy(e);
     cudaStreamDestroy(d->st3);
@@ -1459,6 +1469,7 @@ void WarmStart::forward(const float *feat, int M, float *y)
         m.features(feat, p * kPiece, rows(p), direct, m.st2);
         WCK(cudaEventRecord(m.asked[p % 3], m.st2));
     };
+    m.after_caller(np == 1 ? m.st : m.st2);
     if (np == 1) m.features(feat, 0, M, direct, m.st);
     else for (long long p = 0; p < 2; p++) ask(p);
     auto give = [&](long long p) {
@@ -1491,6 +1502,8 @@ float WarmStart::forward_backward(const float *feat, const float *target, int M,
         ~Done() { cudaStreamSynchronize(m.st); }
     } done{m};                                            // the kernels read the caller's rows
     const bool direct = m.in_place(feat);
+    m.after_caller(m.st);
+    WCK(cudaEventSynchronize(m.caller));                  // (the targets are read on the host)
     for (long long r0 = 0; r0 < M; r0 += kPiece) m.features(feat, r0, std::min<long long>(kPiece, M - r0), direct, m.st);
     for (int r = 0; r < M; r++)
         for (int o = 0; o < kWsOutUsed; o++) t8[(size_t)r * 8 + o] = target[(size_t)r * kWsOutUsed + o];
