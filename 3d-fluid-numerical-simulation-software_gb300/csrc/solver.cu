@@ -3,6 +3,7 @@
 // source/ComputeAllBlockVars.cpp:223-255) as kernel launches on one stream, replayed through
 // CUDA graphs.
 #include "solver.hpp"
+#include "host_threads.hpp"
 #include "restart_io.hpp"
 #include <cmath>
 #include <cstring>
@@ -1517,13 +1518,11 @@ public:
     {
         const long per = 1 << 17;                    // a megabyte per thread
         const long nt = std::min<long>({(n + per - 1) / per, 8, (long)std::max(1u, std::thread::hardware_concurrency())});
-        if (nt <= 1) { std::memcpy(dst, src, sizeof(double) * n); return; }
-        std::vector<std::thread> pool;
         const long step = (n + nt - 1) / nt;
-        for (long t = 1; t < nt; t++)
-            pool.emplace_back([=] { std::memcpy(dst + t * step, src + t * step, sizeof(double) * std::max(0L, std::min(step, n - t * step))); });
-        std::memcpy(dst, src, sizeof(double) * std::min(step, n));
-        for (auto &t : pool) t.join();
+        in_parallel((size_t)nt, [=](size_t t) {
+            const long a = std::min(n, (long)t * step);
+            std::memcpy(dst + a, src + a, sizeof(double) * std::min(step, n - a));
+        });
     }
 
     long get_field(int solve, int l, const std::string &name, double *out, long cap) override
