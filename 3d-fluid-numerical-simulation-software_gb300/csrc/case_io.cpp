@@ -1,6 +1,7 @@
 // Case-file reader. Follows the reference's positional parsing (source/UserInput.cpp:17-239,
 // 241-334, 336-446, 799-1068; include/fstringIO.h:15-42) so the same files drive both solvers.
 #include "case_io.hpp"
+#include "host_threads.hpp"
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -9,7 +10,6 @@
 #include <system_error>
 #include <algorithm>
 #include <atomic>
-#include <thread>
 #include <vector>
 
 namespace gbt {
@@ -400,17 +400,8 @@ void read_grid(const CaseSpec &c, const std::vector<BlockRow> &rows, std::vector
                 ls = nl + 1;
             }
         };
-        if (nt == 1) {
-            count_range(0);
-            parse_range(0);
-        } else {
-            std::vector<std::thread> pool;
-            for (size_t t = 0; t < nt; t++) pool.emplace_back(count_range, t);
-            for (auto &th : pool) th.join();
-            pool.clear();
-            for (size_t t = 0; t < nt; t++) pool.emplace_back(parse_range, t);
-            for (auto &th : pool) th.join();
-        }
+        in_parallel(nt, count_range);
+        in_parallel(nt, parse_range);
         size_t total_nl = 0;
         for (size_t t = 1; t <= nt; t++) total_nl += nl_count[t];
         const size_t lines = total_nl + ((end > pos0 && base[end - 1] != '\n') ? 1 : 0);

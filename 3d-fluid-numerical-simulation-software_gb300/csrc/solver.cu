@@ -466,14 +466,11 @@ public:
             const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
             const unsigned nt = std::min<unsigned>((unsigned)ncase, hw);
             const int per = (int)std::max(1u, std::min(16u, hw / nt));     // parse threads of each case's grid
-            std::vector<std::thread> pool;
-            for (unsigned t = 0; t < nt; t++)
-                pool.emplace_back([&] {
-                    for (int i = next++; i < ncase; i = next++) {
-                        try { per_case[i] = read_case(dirs[i], per); } catch (...) { errs[i] = std::current_exception(); }
-                    }
-                });
-            for (auto &t : pool) t.join();
+            in_parallel(nt, [&](size_t) {
+                for (int i = next++; i < ncase; i = next++) {
+                    try { per_case[i] = read_case(dirs[i], per); } catch (...) { errs[i] = std::current_exception(); }
+                }
+            });
             for (auto &e : errs) if (e) std::rethrow_exception(e);
             // one slot per block, the blocks of a case consecutive
             for (int c = 0; c < ncase; c++) {
