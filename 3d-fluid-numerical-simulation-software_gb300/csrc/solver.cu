@@ -13,6 +13,7 @@
 #include <atomic>
 #include <chrono>
 #include <exception>
+#include <mutex>
 #include <thread>
 #include <map>
 #include <array>
@@ -1479,6 +1480,7 @@ public:
             if (!cs[c].d && sizeof(T) == 4) a.fp32 |= 1u << c;
         }
         a.i0 = i0; a.j0 = j0; a.k0 = k0; a.nj = j1 - j0 + 1; a.nk = k1 - k0 + 1; a.NJ = v.NJ; a.NK = v.NK;
+        const std::lock_guard<std::mutex> turn(pin_turn);
         pinned();
         const long most = kPinned / 2;
         long got = 0, had = 0;                       // elements packed, copied
@@ -1500,7 +1502,9 @@ public:
         }
         return n;
     }
-    // pinned memory of the downloads (elements), allocated by the first one
+    // pinned memory of the downloads (elements), allocated by the first one; one download at a time uses it, from
+    // whatever thread
+    std::mutex pin_turn;
     static constexpr long kPinned = 2 << 20;
     double *pin = nullptr, *pin_dev = nullptr;
     cudaEvent_t pin_done[2] = {nullptr, nullptr};
