@@ -547,7 +547,7 @@ public:
         CK(cudaMemcpy(st_d, st.data(), st_mem.bytes, cudaMemcpyHostToDevice));
         // scratch: limiter lists, norm partials, global-dt minima
         size_t sb = sizeof(int) * (size_t)nsolve * (limits.cap + 2) + sizeof(double) * (size_t)nsolve * (norm_blk + 1) * 5 +
-                    2 * sizeof(unsigned) * nsolve + sizeof(T) * nsolve + 256;
+                    2 * sizeof(unsigned) * nsolve + sizeof(T) * nsolve + sizeof(double) * kStaged + 512;
         scratch_mem.bytes = sb;
         CK(cudaMalloc(&scratch_mem.p, sb));
         char *q = (char *)scratch_mem.p;
@@ -561,6 +561,7 @@ public:
         both = (unsigned *)q; q += sizeof(unsigned) * nsolve;
         CK(cudaMemset(norm_count, 0, 2 * sizeof(unsigned) * nsolve));
         dtmin = (T *)(((uintptr_t)q + 15) & ~(uintptr_t)15);
+        staged = (double *)(((uintptr_t)(dtmin + nsolve) + 15) & ~(uintptr_t)15);
         // 256 rows of history, fewer for very large batches (about 4 MB)
         hist.ncase = ncase;
         hist.rows = (int)std::max<long long>(1, std::min<long long>(256, (4LL << 20) / (96LL * ncase)));
@@ -577,9 +578,10 @@ public:
     {
         for (auto &g : graphs) if (g) cudaGraphExecDestroy(g);
         for (auto &e : ev_pool) cudaEventDestroy(e);
+        if (stream) cudaStreamSynchronize(stream);            // (a download that ended in an error may still be packing)
         for (auto &e : pin_done) if (e) cudaEventDestroy(e);
         if (pin) cudaFreeHost(pin);
-        if (stream) { cudaStreamSynchronize(stream); cudaStreamDestroy(stream); }
+        if (stream) cudaStreamDestroy(stream);
         for (int q = 0; q < 2; q++) {
             if (side[q]) { cudaStreamSynchronize(side[q]); cudaStreamDestroy(side[q]); }
             if (forks[q]) cudaEventDestroy(forks[q]);
@@ -1481,7 +1483,16 @@ public:
         }
         a.i0 = i0; a.j0 = j0; a.k0 = k0; a.nj = j1 - j0 + 1; a.nk = k1 - k0 + 1; a.NJ = v.NJ; a.NK = v.NK;
         const std::lock_guard<std::mutex> turn(pin_turn);
-        pinned();
+        if (!pinned()) {
+            for (long had = 0; had < n; had += kStaged) {
+                const long m = std::min(kStaged, n - had);
+                k_pack<<<(unsigned)((m + 255) / 256), 256, 0, stream>>>(a, had, m, staged);
+                CK(cudaGetLastError());
+                CK(cudaMemcpyAsync(out + had, staged, sizeof(double) * m, cudaMemcpyDeviceToHost, stream));
+                CK(cudaStreamSynchronize(stream));
+            }
+            return n;
+        }
         const long most = kPinned / 2;
         long got = 0, had = 0;                       // elements packed, copied
         for (int q = 0; had < n; q++) {
@@ -1502,18 +1513,28 @@ public:
         }
         return n;
     }
-    // pinned memory of the downloads (elements), allocated by the first one; one download at a time uses it, from
-    // whatever thread
+    // pinned memory of the downloads (elements), allocated by the first one, and device memory for those that get
+    // none; one download at a time uses them, from whatever thread
     std::mutex pin_turn;
-    static constexpr long kPinned = 2 << 20;
-    double *pin = nullptr, *pin_dev = nullptr;
+    static constexpr long kPinned = 2 << 20, kStaged = 1 << 16;
+    double *pin = nullptr, *pin_dev = nullptr, *staged = nullptr;
     cudaEvent_t pin_done[2] = {nullptr, nullptr};
-    void pinned()
+    bool pinned()
     {
-        if (pin) return;
+        if (pin) return true;
         for (auto &e : pin_done) if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        CK(cudaHostAlloc(&pin, sizeof(double) * kPinned, cudaHostAllocMapped));
-        CK(cudaHostGetDevicePointer(&pin_dev, pin, 0));
+        double *p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(double) * kPinned, cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (cudaHostGetDevicePointer(&pin_dev, p, 0) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFreeHost(p);
+            return false;
+        }
+        pin = p;
+        return true;
     }
     static void copy_out(double *dst, const double *src, long n)
     {
