@@ -1483,7 +1483,7 @@ public:
         }
         a.i0 = i0; a.j0 = j0; a.k0 = k0; a.nj = j1 - j0 + 1; a.nk = k1 - k0 + 1; a.NJ = v.NJ; a.NK = v.NK;
         const std::lock_guard<std::mutex> turn(pin_turn);
-        if (!pinned()) {
+        if (n <= kStaged || !pinned(n)) {
             for (long had = 0; had < n; had += kStaged) {
                 const long m = std::min(kStaged, n - had);
                 k_pack<<<(unsigned)((m + 255) / 256), 256, 0, stream>>>(a, had, m, staged);
@@ -1493,7 +1493,7 @@ public:
             }
             return n;
         }
-        const long most = kPinned / 2;
+        const long most = std::min(n, kPinned / 2);
         long got = 0, had = 0;                       // elements packed, copied
         for (int q = 0; had < n; q++) {
             long m = 0;
@@ -1513,18 +1513,28 @@ public:
         }
         return n;
     }
-    // pinned memory of the downloads (elements), allocated by the first one, and device memory for those that get
-    // none; one download at a time uses them, from whatever thread
+    // Pinned memory of the downloads (elements): one piece for a field that fits in one, two for the others, allocated
+    // by the first download that needs it (0.13 ms for 1 MB, 0.63 for all 16). Small fields, for which that is more than the
+    // download itself, and fields that get none go through device memory. One download at a time uses either,
+    // from whatever thread.
     std::mutex pin_turn;
     static constexpr long kPinned = 2 << 20, kStaged = 1 << 16;
     double *pin = nullptr, *pin_dev = nullptr, *staged = nullptr;
+    long pin_n = 0;
     cudaEvent_t pin_done[2] = {nullptr, nullptr};
-    bool pinned()
+    bool pinned(long n)
     {
-        if (pin) return true;
+        long need = 2 * kStaged;
+        while (need < kPinned && need < n) need *= 2;
+        if (n > kPinned / 2) need = kPinned;
+        if (need <= pin_n) return true;
         for (auto &e : pin_done) if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        CK(cudaStreamSynchronize(stream));
+        if (pin) cudaFreeHost(pin);
+        pin = nullptr;
+        pin_n = 0;
         double *p = nullptr;
-        if (cudaHostAlloc(&p, sizeof(double) * kPinned, cudaHostAllocMapped) != cudaSuccess) {
+        if (cudaHostAlloc(&p, sizeof(double) * need, cudaHostAllocMapped) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
@@ -1534,6 +1544,7 @@ public:
             return false;
         }
         pin = p;
+        pin_n = need;
         return true;
     }
     static void copy_out(double *dst, const double *src, long n)
