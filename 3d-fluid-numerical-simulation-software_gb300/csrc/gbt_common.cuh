@@ -135,6 +135,10 @@ struct GeoW {
     T *sb2[3], *sbn[3], *rvol;
 };
 
+// Whether 1 / b may take the place of a division by b below: with b between 2^-200 and 2^200 and a between 2^-723 and 2^677
+// the quotient, the products on the way to it and their remainders are normal numbers
+__host__ __device__ inline bool div_range(double b) { return b > 1e-60 && b < 1e60; }
+
 // Physical constants in the working precision, converted (and the reciprocal Reynolds number
 // formed) once on the host.
 template <typename T>
@@ -143,7 +147,7 @@ struct PhysW {
     // formed once in FP64 on the host: 1 / (gamma - 1) and the conductivity factors
     // gamma R / (gamma - 1) / Pr of the laminar and turbulent parts
     T rgm1, cond_lam, cond_tur;
-    T r_pr_lam, r_pr_tur;                            // 1 / pr_lam, 1 / pr_tur
+    T r_pr_lam, r_pr_tur;                            // 1 / pr_lam, 1 / pr_tur (0 out of div_by's range)
     T re;                                            // the reference Reynolds number
 };
 
@@ -165,9 +169,9 @@ inline PhysW<T> phys_working(const Phys &P)
     w.rgm1 = (T)(1.0 / g1);
     w.cond_lam = (T)(cp / (double)w.pr_lam);
     w.cond_tur = (T)(cp / (double)w.pr_tur);
-    w.r_pr_lam = (T)1 / w.pr_lam;
+    w.r_pr_lam = div_range((double)w.pr_lam) ? (T)1 / w.pr_lam : (T)0;
     w.re = (T)P.re_ref;
-    w.r_pr_tur = (T)1 / w.pr_tur;
+    w.r_pr_tur = div_range((double)w.pr_tur) ? (T)1 / w.pr_tur : (T)0;
     return w;
 }
 
@@ -258,15 +262,13 @@ __device__ __forceinline__ bool larger(double a, double b)
 // |x| without a comparison
 __device__ __forceinline__ float mag(float x) { return fabsf(x); }
 __device__ __forceinline__ double mag(double x) { return fabs(x); }
-// Whether b or 1 / b may take the place of a division by b below
-__host__ __device__ inline bool div_range(double b) { return b > 1e-150 && b < 1e150; }
 // a / b as the IEEE division rounds it, from r = 1 / b rounded: P. Markstein's theorem (IBM J. Res. Dev. 34(1),
 // 1990): with r the rounded reciprocal and q within an ulp of a / b, q + r (a - b q) rounds to the quotient; one step
 // of the same kind brings a r within the ulp. Five FP64 instructions instead of a division's, for several
 // quotients by one b. r = 0 marks a b out of div_range.
 __device__ __forceinline__ double div_by(double a, double b, double r)
 {
-    if (((unsigned)__double2hiint(a) & 0x7ff00000u) - (200u << 20) > (1600u << 20) || __double2hiint(r) == 0) {
+    if (((unsigned)__double2hiint(a) & 0x7ff00000u) - (300u << 20) > (1400u << 20) || __double2hiint(r) == 0) {
         if (__double_as_longlong(a) == 0 && __double2hiint(r) != 0) return a;
         return a / b;
     }
