@@ -1081,18 +1081,19 @@ public:
         // whether the ghost cells of inlets, outlets, walls and the gather list are all different ones (then
         // the fills need no order among each other)
         {
-            std::vector<unsigned char> owner((size_t)Lv.pool_n, 0);
+            std::vector<unsigned short> owner((size_t)Lv.pool_n, 0);
+            constexpr unsigned short kGathered = 0xffff, kMixed = 0xfffe;
             bc.apart = true;
-            auto claim = [&](long long p, unsigned char who) {
+            auto claim = [&](long long p, unsigned short who) {
                 if (owner[p] && owner[p] != who) bc.apart = false;
                 owner[p] = who;
             };
             // (every inlet, outlet and wall patch its own: two patches of a kind may not share a cell either)
-            unsigned char who = 1;
-            auto next = [&] { who = who == 250 ? 1 : who + 1; };
             for (int s = 0; s < nsolve; s++) {
                 const Lvl &v = Lv.lv[s];
                 const LevelCase &c = lc[s];
+                unsigned short who = 0;
+                auto next = [&] { if (++who == kMixed) { bc.apart = false; who = 1; } };
                 for (auto &p : c.in) {
                     next();
                     for (int i = p.is; i <= p.ie; i++)
@@ -1118,7 +1119,7 @@ public:
                             }
                 }
             }
-            for (long long d : pdst) claim(d, 251);
+            for (long long d : pdst) claim(d, kGathered);
             // (nor may the gather list read a cell that one of the fills writes)
             for (long long p : psrc) if (owner[p]) bc.apart = false;
             // the mixing planes' ghosts: written by nothing else and read by no copy of the gather list
@@ -1129,12 +1130,12 @@ public:
                     for (int i = m.is; i <= m.ie; i++)
                         for (int j = side ? m.js2 : m.js1; j <= (side ? m.je2 : m.je1); j++)
                             for (int nd = 0; nd <= P.ndummy; nd++) {
-                                unsigned char &o = owner[ix(v, i, j, side ? -nd : v.KM + nd)];
+                                unsigned short &o = owner[ix(v, i, j, side ? -nd : v.KM + nd)];
                                 if (o) bc.mix_apart = false;
-                                o = 252;
+                                o = kMixed;
                             }
                 }
-            for (long long p : psrc) if (owner[p] == 252) bc.mix_apart = false;
+            for (long long p : psrc) if (owner[p] == kMixed) bc.mix_apart = false;
         }
         // upload everything into one table buffer
         auto bytes = [](size_t n, size_t sz) { return (n * sz + 255) & ~(size_t)255; };
