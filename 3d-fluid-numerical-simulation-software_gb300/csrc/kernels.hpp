@@ -92,7 +92,7 @@ struct WaveCtl { unsigned epoch, ticket[2]; };     // sweeps started; tiles hand
 struct WaveBytes { int geo, flow, dq, pkt, area, var_flow, var_dq, var_pkt; };      // of a step
 struct WaveTables {
     const WaveSolve *solve = nullptr;              // per slot
-    const int2 *item = nullptr;                    // {slot, PI << 16 | PJ}: every tile, after the two it reads from
+    const int2 *item = nullptr;                    // {slot, PI * nPJ + PJ}: every tile, after the two it reads from
     int n_item = 0, narrow = 0;
     int max_tiles = 0, max_T = 0;                  // largest of a slot: tiles, steps of a tile
     long long max_steps = 0;                       // and steps of all its tiles

@@ -883,7 +883,6 @@ public:
             q.nPI = (q.nI + pa - 1) / pa; q.nPJ = (q.nJ + pb - 1) / pb;
             q.T = q.nK + pa + pb - 2;
             q.step0 = steps;
-            if (q.nPI > 0x7fff || q.nPJ > 0xffff) throw std::runtime_error("a block has too many columns for the sweeps");
             for (int a = 0; a < q.nPI; a++)
                 for (int b = 0; b < q.nPJ; b++) order.push_back({pa * a + pb * b, s, a, b});
             const long long np = (long long)q.nPI * q.nPJ;
@@ -896,7 +895,7 @@ public:
         // every tile after the two it reads from; those that can start together side by side
         std::stable_sort(order.begin(), order.end(), [](const auto &x, const auto &y) { return x[0] < y[0]; });
         std::vector<int2> item;
-        for (auto &o : order) item.push_back(make_int2(o[1], (o[2] << 16) | o[3]));
+        for (auto &o : order) item.push_back(make_int2(o[1], o[2] * sol[o[1]].nPJ + o[3]));
         V.n_item = (int)item.size();
         auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
         const size_t N = (size_t)steps;

@@ -170,9 +170,9 @@ __device__ __forceinline__ Where tile_of(const WaveTables &V, unsigned ticket)
     Where w;
     const int2 it = V.item[DIR > 0 ? ticket : V.n_item - 1 - ticket];
     w.slot = it.x;
-    w.PI = it.y >> 16;
-    w.PJ = it.y & 0xffff;
     w.S = V.solve[it.x];
+    w.PI = it.y / w.S.nPJ;
+    w.PJ = it.y - w.PI * w.S.nPJ;
     w.step0 = w.S.step0 + (long long)(w.PI * w.S.nPJ + w.PJ) * w.S.T;
     w.has_i = DIR > 0 ? w.PI > 0 : w.PI < w.S.nPI - 1;
     w.next_i = DIR > 0 ? w.PI < w.S.nPI - 1 : w.PI > 0;
