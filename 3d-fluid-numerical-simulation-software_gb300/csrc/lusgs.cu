@@ -55,7 +55,7 @@ void launch_limiter(const LaunchCtx &ctx, const Phys &P, Flow<T> W, int level, c
 // shuffled additions per warp, and the blocks' sums added up by five threads of a second kernel it took 62
 // and 46 us, and 195 us for 32 solves of 25x25x65 nodes; now 33, 20 and 48.
 constexpr int kNormThreads = 256, kNormCells = 4 * kNormThreads;
-__host__ __device__ inline int norm_blocks(const Lvl &L, int most)
+__device__ __forceinline__ int norm_blocks(const Lvl &L, int most)
 {
     const int n = ((L.IM - 1) * (L.JM - 1) * (L.KM - 1) + kNormCells - 1) / kNormCells;
     return n < most ? n : most;
@@ -146,8 +146,9 @@ void launch_res_norm(const LaunchCtx &ctx, const Geo &G, Flow<T> W, const double
 {
     const Batch &B = ctx.batch;
     ctx.mark("res_norm", 1, 1);
-    const Lvl most = {ctx.maxIM, ctx.maxJM, ctx.maxKM, 0, 0, 0};
-    k_norm<T><<<dim3(norm_blocks(most, nblk), B.nsolve), kNormThreads, 0, ctx.stream>>>(B, G, W, partials, nblk, totalvol, count, hist);
+    // (the product of a batch's largest extents, which need not be one slot's, may take more than 32 bits)
+    const long long most = ((long long)(ctx.maxIM - 1) * (ctx.maxJM - 1) * (ctx.maxKM - 1) + kNormCells - 1) / kNormCells;
+    k_norm<T><<<dim3((unsigned)(most < nblk ? most : nblk), B.nsolve), kNormThreads, 0, ctx.stream>>>(B, G, W, partials, nblk, totalvol, count, hist);
     ctx.mark("res_norm", 0, 1);
 }
 
