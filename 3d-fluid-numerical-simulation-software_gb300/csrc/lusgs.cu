@@ -181,7 +181,9 @@ __global__ void __launch_bounds__(128) k_integrals(Batch B, Phys P, Geo G, Flow<
         const double w = 0.5 * ((double)W.pv[PW][p] + (double)W.pv[PW][q]);
         const double mc = d * (u * G.S[2][0][p] + v * G.S[2][1][p] + w * G.S[2][2][p]);
         const double tf = 0.5 * ((double)W.pv[PT][p] + (double)W.pv[PT][q]);
-        const double fac = 1.0 + g1 / 2.0 * ((u * u + v * v + w * w) / (g * R * tf));
+        // (no speed of sound, and no total state, at a negative temperature)
+        const double c2 = g * R * tf, Ma2 = c2 < 0.0 ? nan("") : (u * u + v * v + w * w) / fabs(c2);
+        const double fac = 1.0 + g1 / 2.0 * Ma2;
         m += mc;
         pm += pow((double)W.pv[PP][p], g1 / g) * fac * mc;
         tm += (double)W.pv[PT][p] * fac * mc;
@@ -223,8 +225,8 @@ __global__ void __launch_bounds__(128) k_integrals(Batch B, Phys P, Geo G, Flow<
     const double pti = __shfl_sync(0xffffffffu, pt, 0), pto = __shfl_sync(0xffffffffu, pt, 1);
     const double tti = a[2] / a[0] * P.temp_ref, tto = b[2] / b[0] * P.temp_ref;
     const double PR = pto / pti;
-    // (PR^((g-1)/g) is the quotient of the two bases)
-    const double Ladk = g / g1 * R * tti * ((isnan(PR) ? PR : fb / fa) - 1.0);
+    // (PR^((g-1)/g) is the quotient of the two bases, or PR where that is infinite or not a number)
+    const double Ladk = g / g1 * R * tti * ((isfinite(PR) ? fb / fa : PR) - 1.0);
     const double Lk = g / g1 * R * tti * (tto / tti - 1.0);
     if (lane != 0) return;
     SolveState &st = B.st[s];
