@@ -96,3 +96,27 @@ def test_mixing_plane_over_a_wall(gpu_lib, meshgen, tmp_path):
             got.append((n, s.get("pv", s.slots(0)[0])[1:-1, 1:-1, -1], s.get("pv", s.slots(0)[1])[1:-1, 1:-1, 0]))
     assert got[0][0] < got[1][0]
     assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][2], got[1][2])
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED"])
+@pytest.mark.parametrize("extra", [_none, _wall_on_inlet, _wall_on_periodic])
+def test_variable_of_the_turbulence_model_in_order(extra, precision, gpu_lib, meshgen, tmp_path):
+    """the Spalart-Allmaras variable's ghosts: the configured ratio on the inlet, zero on a wall that lies on it, and on a
+    periodic face its partner's cells, also where a wall lies there"""
+    im, jm, km = 9, 9, 13
+    case = meshgen.annular_duct(IM=im, JM=jm, KM=km, options={"turb": "200", "ev_ratio": "3.0"})
+    wall = extra(meshgen, im, jm, km)
+    meshgen.write_case(dataclasses.replace(case, patches=list(case.patches) + wall), str(tmp_path))
+    with gpu_lib.Solver(str(tmp_path), getattr(gpu_lib, precision)) as s:
+        s.init_uniform()
+        s.iterate(3, history=False)
+        s.resflux(1)
+        ev = s.get("ev").reshape(im + 1, jm + 1, km + 1)
+    inlet = np.full((im + 1, jm + 1), 3.0)
+    if extra is _wall_on_inlet:
+        a, b, c, d = wall[0].rng[:4]
+        inlet[a:b + 1, c:d + 1] = 0.0
+    assert np.array_equal(ev[1:-1, 1:-1, 0], inlet[1:-1, 1:-1])
+    assert np.array_equal(ev[1:-1, 1:-1, -1], ev[1:-1, 1:-1, -2])
+    assert np.array_equal(ev[1:-1, 0, 1:-1], ev[1:-1, -2, 1:-1]) and np.array_equal(ev[1:-1, -1, 1:-1], ev[1:-1, 1, 1:-1])
+    assert np.all(ev[0, 1:-1, 1:-1] == 0.0) and np.all(ev[-1, 1:-1, 1:-1] == 0.0)
