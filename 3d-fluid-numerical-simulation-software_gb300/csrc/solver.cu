@@ -1465,7 +1465,7 @@ public:
 
     // a box [i0,i1]x[j0,j1]x[k0,k1] of several component arrays, components fastest
     struct Comp { const double *d; const T *t; };
-    long box(int l, const Lvl &v, const std::vector<Comp> &cs, int i0, int i1, int j0, int j1, int k0, int k1, double *out, long cap)
+    long box(const Lvl &v, const std::vector<Comp> &cs, int i0, int i1, int j0, int j1, int k0, int k1, double *out, long cap)
     {
         const long n = (long)(i1 - i0 + 1) * (j1 - j0 + 1) * (k1 - k0 + 1) * (long)cs.size();
         if (n > cap) return -1;
@@ -1569,41 +1569,41 @@ public:
         auto D = [](const double *p) { return Comp{p, nullptr}; };
         auto Tt = [](const T *p) { return Comp{nullptr, p}; };
         std::vector<Comp> cs;
-        if (name == "cv") { for (int c = 0; c < 5; c++) cs.push_back(D(W.cv[c])); return box(l, v, cs, 0, IM, 0, JM, 0, KM, out, cap); }
-        if (name == "pv") { for (int c = 0; c < 6; c++) cs.push_back(Tt(W.pv[c])); return box(l, v, cs, 0, IM, 0, JM, 0, KM, out, cap); }
-        if (name == "mut") return box(l, v, {Tt(W.mut)}, 0, IM, 0, JM, 0, KM, out, cap);
+        if (name == "cv") { for (int c = 0; c < 5; c++) cs.push_back(D(W.cv[c])); return box(v, cs, 0, IM, 0, JM, 0, KM, out, cap); }
+        if (name == "pv") { for (int c = 0; c < 6; c++) cs.push_back(Tt(W.pv[c])); return box(v, cs, 0, IM, 0, JM, 0, KM, out, cap); }
+        if (name == "mut") return box(v, {Tt(W.mut)}, 0, IM, 0, JM, 0, KM, out, cap);
         if (name == "ev" || name == "res_ev" || name == "dwall") {
             if (!W.ev) return -1;                  // Spalart-Allmaras cases, fine level
-            if (name == "ev") return box(l, v, {D(W.ev)}, 0, IM, 0, JM, 0, KM, out, cap);
-            if (name == "res_ev") return box(l, v, {Tt(W.res_ev)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
-            return box(l, v, {D(W.dwall)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+            if (name == "ev") return box(v, {D(W.ev)}, 0, IM, 0, JM, 0, KM, out, cap);
+            if (name == "res_ev") return box(v, {Tt(W.res_ev)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+            return box(v, {D(W.dwall)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
         }
-        if (name == "res") { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.res[c])); return box(l, v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap); }
-        if (name == "dq") { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.dq[c])); return box(l, v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap); }
-        if (name == "dt") return box(l, v, {Tt(W.dt)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
-        if (name == "omega") return box(l, v, {Tt(W.omega)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+        if (name == "res") { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.res[c])); return box(v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap); }
+        if (name == "dq") { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.dq[c])); return box(v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap); }
+        if (name == "dt") return box(v, {Tt(W.dt)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+        if (name == "omega") return box(v, {Tt(W.omega)}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
         const char *lam[6] = {"lamcI", "lamcJ", "lamcK", "lamvI", "lamvJ", "lamvK"};
         for (int q = 0; q < 6; q++)
-            if (name == lam[q]) return box(l, v, {Tt(q < 3 ? W.lamc[q] : W.lamv[q - 3])}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+            if (name == lam[q]) return box(v, {Tt(q < 3 ? W.lamc[q] : W.lamv[q - 3])}, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
         const char *fcn[3] = {"FcI", "FcJ", "FcK"}, *fvn[3] = {"FvI", "FvJ", "FvK"}, *gn[3] = {"faceI", "faceJ", "faceK"};
         for (int f = 0; f < 3; f++) {
             int i1 = f == 0 ? IM : IM - 1, j1 = f == 1 ? JM : JM - 1, k1 = f == 2 ? KM : KM - 1;
-            if (name == fcn[f]) { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.Ff[f][c])); return box(l, v, cs, 1, i1, 1, j1, 1, k1, out, cap); }
-            if (name == fvn[f]) { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.Vf[f][c])); return box(l, v, cs, 1, i1, 1, j1, 1, k1, out, cap); }
+            if (name == fcn[f]) { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.Ff[f][c])); return box(v, cs, 1, i1, 1, j1, 1, k1, out, cap); }
+            if (name == fvn[f]) { for (int c = 0; c < 5; c++) cs.push_back(Tt(W.Vf[f][c])); return box(v, cs, 1, i1, 1, j1, 1, k1, out, cap); }
             if (name == gn[f]) {
                 for (int c = 0; c < 3; c++) cs.push_back(D(G.S[f][c]));
                 cs.push_back(D(G.s[f]));
                 for (int c = 0; c < 3; c++) cs.push_back(D(G.c[f][c]));
                 cs.push_back(D(G.r[f])); cs.push_back(D(G.th[f]));
                 for (int c = 0; c < 9; c++) cs.push_back(D(G.m[f][c]));
-                return box(l, v, cs, 1, i1, 1, j1, 1, k1, out, cap);
+                return box(v, cs, 1, i1, 1, j1, 1, k1, out, cap);
             }
         }
         if (name == "cell") {
             cs.push_back(D(G.vol));
             for (int c = 0; c < 3; c++) cs.push_back(D(G.cc[c]));
             for (int c = 0; c < 9; c++) cs.push_back(D(G.cm[c]));
-            return box(l, v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
+            return box(v, cs, 1, IM - 1, 1, JM - 1, 1, KM - 1, out, cap);
         }
         if (name == "totalvol") {
             if (cap < 1) return -1;

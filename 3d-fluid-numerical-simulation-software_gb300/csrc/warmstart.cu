@@ -167,22 +167,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
-// 32 rows x 32 BF16 columns (one row per lane in v) to rows row0.. of dst through the warp's 2 KB
-__device__ __forceinline__ void store_rows32(unsigned char *st, int lane, const bf16 v[32], bf16 *dst, long long row0, long long M, long long ld)
-{
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-        *reinterpret_cast<uint4 *>(st + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = reinterpret_cast<const uint4 *>(v)[c];
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int r = q * 8 + (lane >> 2), c = lane & 3;
-        const uint4 w = *reinterpret_cast<const uint4 *>(st + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
-        if (row0 + r < M) *reinterpret_cast<uint4 *>(dst + (row0 + r) * ld + c * 8) = w;
-    }
-    __syncwarp();
-}
-
 // ---------------------------------------------------------------- the row products, all layers fused
 // The products of rows (cells) with the layers' matrices, D[128 x N] = A[128 x K] . B[N x K]^T per tile of 128
 // rows and layer, a tile's activations kept on chip from layer to layer:
