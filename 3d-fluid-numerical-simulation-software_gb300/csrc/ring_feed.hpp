@@ -1,9 +1,9 @@
 // The groups of a ring of asynchronous copies, asked for in order by one thread: group g goes into stage
-// g % STAGES and completes phase g / STAGES of that stage's barrier. A barrier is armed for a group only once the
-// group before it in the same stage has landed, also where the consumers gave up waiting and run ahead of the
-// copies: armed twice in a phase, its count of arrivals would underflow and two copies would write the same
-// bytes. After a wait that ran out nothing more is asked for, and drain() waits for exactly the groups that were,
-// so that no copy is in flight when the block's shared memory goes.
+// g % STAGES and completes phase g / STAGES of that stage's barrier. The thread asks for a group once the consumers
+// have said that they are done with the group before it in the same stage, and they say so only of a group that
+// they have seen land: a barrier armed twice in a phase would lose count of its arrivals, and two copies would write
+// the same bytes. After a wait that ran out nothing more is said or asked for, and drain() waits for exactly the
+// groups that were asked for, so that no copy is in flight when the block's shared memory goes.
 #pragma once
 
 #ifdef __CUDACC__
@@ -17,14 +17,13 @@ namespace gbt {
 template <int STAGES>
 struct RingFeed {
     int groups, asked = 0;
-    // wait(stage, parity): false once a wait has run out; ask(group, stage) arms the barrier and starts the copies
-    template <typename Wait, typename Ask>
-    GBT_HD void next(bool ok, Wait wait, Ask ask)
+    // ok: no wait of the calling thread has run out; ask(group, stage) arms the barrier and starts the copies
+    template <typename Ask>
+    GBT_HD void next(bool ok, Ask ask)
     {
         if (!ok || asked >= groups) return;
-        const int stage = asked % STAGES;
-        if (asked >= STAGES && !wait(stage, (unsigned)(asked / STAGES - 1) & 1u)) return;
-        ask(asked++, stage);
+        ask(asked, asked % STAGES);
+        asked++;
     }
     template <typename Wait>
     GBT_HD void drain(Wait wait) const

@@ -368,6 +368,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
     if (warp < 4) {
         const int cell = threadIdx.x / kLanes<T, N>, q = threadIdx.x % kLanes<T, N>, a = cell / PB, b = cell % PB;
         const bool column = w.PI * PA + a < w.S.nI && w.PJ * PB + b < w.S.nJ;
+        // (a step is called done only by a thread whose waits have all been met: its inputs have landed then)
         constexpr int F = DIR > 0 ? 1 : 0;          // forward: halo first
         // terms read: FP64, component q (or the fifth) of the three directions; otherwise both groups of I and J
         int r_off[4] = {off_ia<L>(a + 1 - F, b), off_ib<L>(a + 1 - F, b), off_ja<L>(a, b + 1 - F), off_jb<L>(a, b + 1 - F)};
@@ -410,7 +411,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
                 char *wr = terms + slot * L::slot;
                 Step::run(now, rd, wr, cell, q, r_off, w_off, w_off4, column && (unsigned)k < (unsigned)w.S.nK, gm1, dq);
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (threadIdx.x == 0) bar_arrive(done + 8 * slot);
+                if (threadIdx.x == 0 && ok) bar_arrive(done + 8 * slot);
                 now = then;
                 rd = wr;
                 k += DIR;
@@ -433,7 +434,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
                     Step::run(Step::pre(in + (DIR > 0 ? u : cnt - 1 - u) * L::step, cell, q), rd, wr, cell, q, r_off, w_off, w_off4,
                               column && (unsigned)k < (unsigned)w.S.nK, gm1, dq);
                     asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (threadIdx.x == 0) bar_arrive(done + 8 * slot);
+                    if (threadIdx.x == 0 && ok) bar_arrive(done + 8 * slot);
                     rd = wr;
                     k += DIR;
                     dq += DIR * L::dq;
@@ -527,7 +528,6 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
     } else {
         // inputs of a group of steps into its stage, on lane 0
         RingFeed<kStages> feed{(T_ + kGroup - 1) / kGroup};
-        auto landed = [&](int stage, unsigned parity) { bar_wait(full + 8 * stage, parity, ok); return ok; };
         auto fetch = [&](int g, int stage) {
             const int n = g * kGroup, cnt = min(kGroup, T_ - n);
             const long long t = w.step0 + (DIR > 0 ? n : T_ - n - cnt);
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
             }
         };
         if (lane == 0)
-            for (int s = 0; s < kStages; s++) feed.next(ok, landed, fetch);
+            for (int s = 0; s < kStages; s++) feed.next(ok, fetch);
         constexpr int RND = (L::pkt + 31) / 32;
         int from[RND];
         bool mine[RND];
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
             }
             dst += DIR * L::pkt;
             __syncwarp();
-            if ((n + 1) % kGroup == 0 && lane == 0) feed.next(ok, landed, fetch);
+            if ((n + 1) % kGroup == 0 && lane == 0) feed.next(ok, fetch);
             if (++slot == kSlots) { slot = 0; ph ^= 1; }
         }
         // no copy is in flight when the block ends, also where a wait ran out
