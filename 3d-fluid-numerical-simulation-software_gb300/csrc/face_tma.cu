@@ -75,7 +75,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
         : "memory");
     return ok != 0;
 }
-// about a second at most
+// some 17 s at most (a poll of a barrier that does not complete takes 4 us)
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
 {
     for (int t = 0; t < (1 << 22); t++) {

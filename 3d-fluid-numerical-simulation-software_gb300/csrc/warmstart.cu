@@ -92,7 +92,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
         : "memory");
     return ok != 0;
 }
-// about a second at most; a wait that runs out is reported through the error flag
+// some 17 s at most (a poll of a barrier that does not complete takes 4 us); a wait that runs out is reported through
+// the error flag
 constexpr int kMbarWaitLimit = 1 << 22;
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
 {

@@ -2,12 +2,14 @@
 // batch. The forward sweep's cell (i, j, k) needs the terms of (i-1, j, k), (i, j-1, k), (i, j, k-1); the
 // backward sweep is its mirror image.
 //
-// What bounds it: the chain of i + j + k planes, not the arithmetic or the bytes. One kernel launch per
-// plane (programmatic dependent launches, neighbours re-read through L2) cost 1.8 us per plane in FP32 and
-// 3.4 us in FP64. Here a block owns a tile of 4 x 8 grid columns (i, j; 2 x 8 in FP64) and marches it along k skewed: at
-// step t the column (a, b) of the tile is at k = t - a - b, so that the terms it needs from inside the
-// tile are the ones its neighbours formed one step earlier, and a step costs the block one barrier. Tiles
-// run side by side on as many SMs as there are, each a few steps behind the two it reads from.
+// What bounds it is the chain of i + j + k planes, not the arithmetic or the bytes. A block owns a tile of 4 x 8 grid
+// columns (i, j; 2 x 8 in FP64) and marches it along k skewed: at step t the column (a, b) of the tile is at
+// k = t - a - b, so that the terms it needs from inside the tile are the ones its neighbours formed one step
+// earlier, and a step costs the block one barrier. Tiles run side by side on as many SMs as there are,
+// each a few steps behind the two it reads from. The 224 planes of the 129x49x49 passage take 314 us in FP64, where a
+// step of 1.4 us hides the way of a term from tile to tile. In FP32 a step takes 0.3 us, and of the 120 us of a
+// sweep the planes are 67: the rest is some 3 us for each of 17 crossings (term to the outgoing warp, to L2, to
+// the incoming warp that polls for it, to the tile). With a launch per plane a plane took 1.8 us in FP32, 3.4 in FP64.
 //
 // What a step costs is the number of instructions one warp issues (a lone warp of a sub-partition issues
 // one every three to four cycles, and an FP64 instruction holds its sub-partition for some 70): with a
@@ -75,7 +77,8 @@ constexpr int kAhead = 2;                       // steps that the incoming warp 
                                                 // longer than a step; asked earlier, it is more often too early and
                                                 // costs a second round (137, 146, 154, 186 us a forward sweep of the
                                                 // 129x49x49 passage in FP32 with 2, 3, 4, 8)
-constexpr unsigned kWaitLimit = 1u << 21;       // polls of a wait before it gives up (seconds)
+constexpr unsigned kWaitLimit = 1u << 21;       // polls of a wait before it gives up: 8 s on a barrier (a poll of one that
+                                                // does not complete takes 4 us), some 2 s on a packet
 constexpr int kSteps32 = 16;                    // steps of a block of the FP32 gather kernel
 template <typename T, int N> constexpr int kSteps = 256 / kCells<T, N>;                   // of the kernels with a thread per cell
 

@@ -127,7 +127,8 @@ int gb_get_outlet_pressure(gb_solver *h, double *out);
 int gb_sync(gb_solver *h);
 /* block shape of the plane-by-plane sweep launches of earlier versions: out[0] cells per warp (10),
  * out[1] warps per block (1). The sweeps now march tiles of grid columns in one launch per direction and
- * have no shape to choose; the call is kept for programs that report it */
+ * have no shape to choose, and the environment variable GBTURBO_SWEEP_SHAPE, which set it, has no
+ * effect; the call is kept for programs that report it */
 int gb_sweep_tuning(gb_solver *h, int level, int out[2]);
 /* whether a level's face stage runs on tiles of faces staged in shared memory by the tensor memory
  * accelerator (*tma = 1; the mixed form's default scheme on meshes whose k extent KM is 4n + 1 and
@@ -209,7 +210,9 @@ int gb_case_info(const char *case_dir, long long info[9], double *nodes_out, lon
  *   target mean[6], std[6]).
  * gb_ws_forward / gb_ws_forward_backward: the network on given features (n x 64, FP32, rounded to
  *   BF16 on upload): outputs (n x 16); with targets (n x 6, normalised) the mean-squared loss and
- *   the gradient of every parameter (the layout of gb_ws_get_params). */
+ *   the gradient of every parameter (the layout of gb_ws_get_params). The features may lie in host
+ *   (pageable or pinned), managed or device memory, the outputs in any of them, inside the features
+ *   too; they are read after the work that the default stream holds at the call. */
 /* After gb_init_uniform and gb_set_cv of the fine level (level 1) of every slot, before the first
  * iteration: the iterations run full multigrid cycles from that fine field, as a restarted case
  * does, with the coarse levels' time steps and spectral radii evaluated once at the fine field
