@@ -17,4 +17,11 @@ inline void read_every_page(const void *p, size_t bytes)
     for (uintptr_t q = (a / page + 1) * page; q <= last && q > a; q += page) (void)*(const volatile char *)q;
 }
 
+// Whether a kernel may read the caller's FP32 rows at p where they lie: the device reaches the host's memory (reaches), the
+// rows are there (host), and p is aligned, which a copy does not need and a kernel's load does.
+inline bool rows_in_place(const void *p, bool reaches, bool host)
+{
+    return reaches && host && (uintptr_t)p % alignof(float) == 0;
+}
+
 }  // namespace gbt

@@ -1034,12 +1034,13 @@ struct WarmStart::Impl {
     }
 
     // Whether the device is to read the rows at feat where they are: host memory, where it reaches that through the
-    // host's page tables. Rows in device or managed memory are copied, as the host cannot look at them first.
+    // host's page tables. Rows in device or managed memory, which the host cannot look at first, and rows that are not
+    // aligned are copied.
     bool in_place(const float *feat) const
     {
         cudaPointerAttributes a{};
         WCK(cudaPointerGetAttributes(&a, feat));
-        return host_rows && a.type != cudaMemoryTypeDevice && a.type != cudaMemoryTypeManaged;
+        return rows_in_place(feat, host_rows, a.type != cudaMemoryTypeDevice && a.type != cudaMemoryTypeManaged);
     }
     // what the caller has under way on the default stream and the streams that it waits for, which may still
     // write the rows
