@@ -103,6 +103,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
     }
     return false;
 }
+// the same for a whole warp, which goes on together: a wait that runs out on one of its lanes has run out on all
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity)
+{
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity)) != 0;
+}
 // 32 TMEM lanes x 16 columns of 32 bits: thread t of the warp receives lane (base lane + t)
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16])
 {
@@ -365,7 +370,7 @@ __global__ void __launch_bounds__(32 * (kEpiWarps + 2), 1) k_mlp_chain(
                                 zl[c][q] = zr < g.M ? *reinterpret_cast<const uint4 *>(Z + zr * kWsHidden + c * 32) : make_uint4(0u, 0u, 0u, 0u);
                             }
                     }
-                    const bool ok = mbar_wait_bounded(acc_full(h), au[h] & 1u);
+                    const bool ok = mbar_wait_warp(acc_full(h), au[h] & 1u);
                     au[h]++;
                     tc_fence_after();
                     if (!ok) { failed = true; break; }
@@ -539,7 +544,7 @@ __global__ void __launch_bounds__(192, 2) k_mlp_wgrad(const __grid_constant__ Wg
         float *out = g.part[layer] + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 128 * Nb + warp * 32 + lane;
         bool ok = true;
         if (nch > 0) {
-            ok = mbar_wait_bounded(accf, 0u);
+            ok = mbar_wait_warp(accf, 0u);
             tc_fence_after();
         }
         if (!ok) failed = true;
