@@ -6,12 +6,10 @@
 // groups that were asked for, so that no copy is in flight when the block's shared memory goes.
 #pragma once
 
-#ifndef GBT_HD
 #ifdef __CUDACC__
 #define GBT_HD __host__ __device__ __forceinline__
 #else
 #define GBT_HD inline
-#endif
 #endif
 
 namespace gbt {

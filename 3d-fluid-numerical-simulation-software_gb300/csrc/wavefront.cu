@@ -53,7 +53,6 @@
 #include "flux.cuh"
 #include "update.cuh"
 #include "ring_feed.hpp"
-#include "warp_wait.hpp"
 #include <type_traits>
 
 namespace gbt {
@@ -494,18 +493,16 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
                 if (n >= T_) break;
                 // the slot's halo cells are free once the step that read them last is done
                 if (n >= kSlots) bar_wait(done + 8 * slot, ph ^ 1, ok);
-                poll_together(ok, kWaitLimit, [](bool v) { return __any_sync(0xffffffffu, v) != 0; },
-                              [&] {
-                                  bool late = false;
+                for (unsigned polls = 0; ok; polls++) {
+                    bool late = false;
 #pragma unroll
-                                  for (int r = 0; r < RND; r++) late = late || (wants(r, n) && !fresh(hi[u][r]));
-                                  return late;
-                              },
-                              [&] {
+                    for (int r = 0; r < RND; r++) late = late || (wants(r, n) && !fresh(hi[u][r]));
+                    if (!__any_sync(0xffffffffu, late)) break;
+                    if (polls > kWaitLimit) { ok = false; break; }
 #pragma unroll
-                                  for (int r = 0; r < RND; r++)
-                                      if (wants(r, n) && !fresh(hi[u][r])) ask(r, n, lo[u][r], hi[u][r]);
-                              });
+                    for (int r = 0; r < RND; r++)
+                        if (wants(r, n) && !fresh(hi[u][r])) ask(r, n, lo[u][r], hi[u][r]);
+                }
                 // beside the terms of the last step
                 char *s = terms + (slot == 0 ? kSlots - 1 : slot - 1) * L::slot;
 #pragma unroll
