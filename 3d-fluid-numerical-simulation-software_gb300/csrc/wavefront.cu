@@ -153,6 +153,13 @@ __device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, bool &ok
         if (bar_try(bar, parity)) return;
     ok = false;
 }
+// the same for a whole warp whose lanes vote later on: a wait that runs out on one of them has run out on all. (Votes of
+// all lanes in every poll instead, met or not, cost the 129x49x49 passage 1.5% in FP64; this costs nothing.)
+__device__ __forceinline__ void bar_wait_warp(unsigned bar, unsigned parity, bool &ok)
+{
+    bar_wait(bar, parity, ok);
+    ok = __all_sync(0xffffffffu, ok) != 0;
+}
 __device__ __forceinline__ void bulk_copy(unsigned dst, const char *src, unsigned bytes, unsigned bar)
 {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
@@ -492,7 +499,7 @@ __global__ void __launch_bounds__(192, sizeof(T) == 4 ? 4 : 2) k_wave(Batch B, W
                 const int n = n0 + u;
                 if (n >= T_) break;
                 // the slot's halo cells are free once the step that read them last is done
-                if (n >= kSlots) bar_wait(done + 8 * slot, ph ^ 1, ok);
+                if (n >= kSlots) bar_wait_warp(done + 8 * slot, ph ^ 1, ok);
                 for (unsigned polls = 0; ok; polls++) {
                     bool late = false;
 #pragma unroll
